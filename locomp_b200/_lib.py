@@ -7,7 +7,7 @@ from __future__ import annotations
 import ctypes
 import os
 
-from .build import LIB_PATH
+from .build import CALLS_PATH, LIB_PATH
 
 OK = 0
 ERR_BAD_ARG, ERR_UNSUPPORTED, ERR_CUDA, ERR_WORKSPACE, ERR_TIMEOUT = -1, -2, -3, -4, -5
@@ -91,3 +91,22 @@ def check(status: int) -> None:
         if status == ERR_BAD_ARG:
             raise ValueError(f"locomp_b200: {msg}")
         raise LcqError(status, msg)
+
+
+class _TorchCalls:
+    """The functions of the extension module _torch_calls (csrc/torch_calls.cpp), loaded and bound to
+    the library on first use.  Each takes torch CUDA tensors only and returns NotImplemented for
+    anything else."""
+
+    def __getattr__(self, name):
+        if not os.path.exists(CALLS_PATH):
+            raise ImportError(f"{CALLS_PATH} is missing: it has not been built (run `python -m locomp_b200.build`)")
+        lib()
+        from . import _torch_calls
+        from .tensor import workspace
+        _torch_calls.bind(LIB_PATH, check, workspace)
+        self.__dict__.update((n, f) for n, f in vars(_torch_calls).items() if not n.startswith("_"))
+        return self.__dict__[name]
+
+
+calls = _TorchCalls()

@@ -48,6 +48,10 @@ def _finish(out_op: Operand, res):
 # ------------------------------------------------------------------------------------------ norm / activation / residual
 def rms_norm(x, weight, eps: float = 1e-5, *, out=None, stream=None, bf16: bool = False):
     """out[r, :] = x[r, :] * rsqrt(mean(x[r, :]^2) + eps) * weight; x is [n] or [rows, n]."""
+    if stream is None and not bf16 and isinstance(x, torch.Tensor):
+        res = _lib.calls.rms_norm(x, weight, eps, out)
+        if res is not NotImplemented:
+            return res
     xo, wo = resolve(x, "x", bf16), resolve(weight, "weight", bf16)
     n = xo.shape[-1] if xo.shape else 0
     if wo.size != n:
@@ -72,6 +76,10 @@ def residual_rms_norm(hidden, delta, weight, eps: float = 1e-5, *, out=None, str
     """hidden += delta (in place), then out = rms_norm(hidden, weight): the residual add and the
     norm that follows it in the layer (examples/54_smollm2_inference.py:529-534) as one launch.
     `hidden` must be device-resident (it is updated in place).  Returns out."""
+    if stream is None and not bf16 and isinstance(hidden, torch.Tensor):
+        res = _lib.calls.residual_rms_norm(hidden, delta, weight, eps, out)
+        if res is not NotImplemented:
+            return res
     ho, do, wo = resolve(hidden, "hidden", bf16), resolve(delta, "delta", bf16), resolve(weight, "weight", bf16)
     if ho.host is not None:
         raise TypeError("hidden is updated in place and must be a device tensor")
@@ -97,6 +105,10 @@ def residual_rms_norm(hidden, delta, weight, eps: float = 1e-5, *, out=None, str
 
 def silu_mul(gate, up, *, out=None, stream=None, bf16: bool = False):
     """out = gate * sigmoid(gate) * up, elementwise."""
+    if stream is None and not bf16 and isinstance(gate, torch.Tensor):
+        res = _lib.calls.silu_mul(gate, up, out)
+        if res is not NotImplemented:
+            return res
     go, uo = resolve(gate, "gate", bf16), resolve(up, "up", bf16)
     if go.size != uo.size:
         raise ValueError("gate and up must have the same number of elements")
@@ -117,6 +129,10 @@ def silu_mul(gate, up, *, out=None, stream=None, bf16: bool = False):
 
 def add_inplace(a, b, *, stream=None, bf16: bool = False):
     """a += b, elementwise; `a` must be device-resident.  Returns a."""
+    if stream is None and not bf16 and isinstance(a, torch.Tensor):
+        res = _lib.calls.add_inplace(a, b)
+        if res is not NotImplemented:
+            return res
     ao, bo = resolve(a, "a", bf16), resolve(b, "b", bf16)
     if ao.host is not None:
         raise TypeError("a is updated in place and must be a device tensor")
@@ -134,6 +150,9 @@ def add_inplace(a, b, *, stream=None, bf16: bool = False):
 def embed_lookup(token_ids, table, out, seq_len: int, dim: int, *, stream=None, bf16: bool = False) -> None:
     """out[i] = table[token_ids[i]] for i in range(seq_len) (locomp.embed_lookup, locomp/api.py:1025-1038).
     token_ids: int32 [seq_len]; table: [vocab, dim]; out: [seq_len * dim], same dtype as table."""
+    if stream is None and not bf16 and isinstance(table, torch.Tensor):
+        if _lib.calls.embed_lookup(token_ids, table, out, seq_len, dim) is not NotImplemented:
+            return
     io, to, oo = resolve(token_ids, "token_ids"), resolve(table, "table", bf16), resolve(out, "out", bf16)
     if io.kind != "i32":
         raise TypeError(f"token_ids must be int32, got {io.kind}")
@@ -156,6 +175,10 @@ def embed_lookup(token_ids, table, out, seq_len: int, dim: int, *, stream=None, 
 def argmax(x, *, out=None, stream=None, bf16: bool = False):
     """Index of the first maximum of each row of x ([n] or [rows, n]) as int32, computed on the
     device: the host-side np.argmax of examples/54_smollm2_inference.py:606 without the download."""
+    if stream is None and not bf16 and isinstance(x, torch.Tensor):
+        res = _lib.calls.argmax(x, out)
+        if res is not NotImplemented:
+            return res
     xo = resolve(x, "x", bf16)
     if not xo.shape or xo.shape[-1] == 0:
         raise ValueError("argmax needs at least one element per row")
@@ -271,6 +294,10 @@ def quantize(weights, group_size: int = 32, *, bits: int = 4, style: str = "ex38
     style "ex52": quantize_int4_ref of examples/52_dequantize.py:110-126.
     Scales are float32 as in the reference; scale_dtype="f16" additionally rounds them to fp16
     (the W4A16 kernels' scale type)."""
+    if stream is None and scale_dtype is None and style in ("ex38", "ex52") and isinstance(weights, torch.Tensor):
+        res = _lib.calls.quantize(weights, group_size, bits, 0 if style == "ex38" else 1)
+        if res is not NotImplemented:
+            return QuantizedWeight(res[0], res[1], group_size, bits)
     wo = resolve(weights, "weights")
     if len(wo.shape) != 2:
         raise ValueError(f"weights must be 2-D [N, K], got shape {wo.shape}")

@@ -13,6 +13,7 @@ from typing import List, Optional, Sequence, Tuple
 
 import torch
 
+from . import _lib
 from .ops import matmul_workspace_bytes, quantized_matmul
 from .tensor import _TORCH_TO_KIND
 
@@ -29,6 +30,10 @@ class QuantLinear:
         self.in_features = w.shape[1] * (2 if bits == 4 else 1)
 
     def __call__(self, x: torch.Tensor, out: Optional[torch.Tensor] = None, **kw) -> torch.Tensor:
+        if not kw:
+            res = _lib.calls.matmul(x, self.w, self.scales, self.group_size, self.bits, out, None)
+            if res is not NotImplemented:
+                return res
         return quantized_matmul(x, self.w, self.scales, self.group_size, bits=self.bits, out=out, **kw)
 
     @property

@@ -60,6 +60,10 @@ def quantized_matmul(x, w, scales, group_size: int = 32, *, bits: int = 4, out=N
     per-stream buffer this module keeps (needed under CUDA-graph capture, where nothing may be
     allocated; see matmul_workspace_bytes).
     """
+    if isinstance(x, torch.Tensor) and algo is None and out_dtype is None and stream is None and not bf16:
+        res = _lib.calls.matmul(x, w, scales, group_size, bits, out, workspace_buf)
+        if res is not NotImplemented:
+            return res
     xo = resolve(x, "x", bf16)
     wo = resolve(w, "w")
     so = resolve(scales, "scales")
@@ -143,6 +147,10 @@ def dequantize(w, scales, N: Optional[int] = None, K: Optional[int] = None, grou
                out=None, out_dtype: str = "f32", stream=None):
     """out[r, k] = dequant(w)[r, k]; returns a torch CUDA tensor [N, K] (or `out`).
     w and scales may be flat, as the reference's wrappers pass them (examples/52_dequantize.py:86-87)."""
+    if isinstance(w, torch.Tensor) and out is None and stream is None and N is not None and K is not None and out_dtype in KIND_TO_CODE:
+        res = _lib.calls.dequantize(w, scales, N, K, group_size, bits, KIND_TO_CODE[out_dtype])
+        if res is not NotImplemented:
+            return res
     wo = resolve(w, "w")
     so = resolve(scales, "scales")
     if bits not in (4, 8):

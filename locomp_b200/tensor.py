@@ -220,4 +220,5 @@ def workspace(nbytes: int, device: int, stream_ptr: int) -> torch.Tensor:
         buf = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", device))
         torch.cuda.synchronize(device)   # zero-fill ran on torch's stream; the caller's may differ
         _workspaces[key] = buf
+        _lib.calls.set_workspace(device, stream_ptr, buf.data_ptr(), buf.numel())
     return buf

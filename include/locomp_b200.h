@@ -47,7 +47,7 @@ extern "C" {
 #define LCQ_ALGO_AUTO    0   /* pick by shape and dtype                                         */
 #define LCQ_ALGO_SIMT    1   /* warp-per-row CUDA-core kernel; any K % group_size == 0           */
 #define LCQ_ALGO_GEMV_TC 2   /* int4, M <= 16, K % 64 == 0: TMA-staged int4 stream + warp-level MMA, split-K */
-#define LCQ_ALGO_GEMM_TC 3   /* M >= 17: TMA + in-kernel dequant + tcgen05 MMA, TMEM accumulators */
+#define LCQ_ALGO_GEMM_TC 3   /* int4, M >= 17, K % 64 == 0: TMA + in-kernel dequant + tcgen05 MMA on one or two SMs */
 #define LCQ_ALGO_GEMV_W8 4   /* int8, M <= 8: TMA-staged int8 stream, 128-bit shared loads, float32 math */
 
 int         lcq_version(void);
@@ -288,6 +288,15 @@ int lcq_gemv_tc_plan_check(int M, int N, int K, int sm_count, int* fields);
  * cluster mode, partial sums meet in the first CTA's shared memory).  Negative: status code.
  */
 int lcq_gemv_tc_plan_cluster(int M, int N, int K, int sm_count);
+
+/*
+ * The same check for the GEMM_TC kernel: replays the schedule of its CTAs or CTA pairs on the CPU (every
+ * (tile, 256-k weight stage) exactly once, partials of tiles cut along K in slots of their own,
+ * contributor counts) and checks its shared-memory and tensor-memory budgets.  fields (may be NULL)
+ * receives {CTAs, tile rows of x, tiles, tiles cut along K, shared-memory bytes, CTAs per MMA, CTAs per cluster
+ * that share a tile's K}.
+ */
+int lcq_gemm_tc_plan_check(int M, int N, int K, int sm_count, int* fields);
 
 #ifdef __cplusplus
 }

@@ -55,6 +55,7 @@ SIGNATURES = {
     "lcq_set_wait_limit_ns": (_c.c_int, [_c.c_ulonglong]),
     "lcq_gemv_tc_plan_check": (_c.c_int, [_c.c_int] * 4 + [_c.POINTER(_c.c_int)]),
     "lcq_gemv_tc_plan_cluster": (_c.c_int, [_c.c_int] * 4),
+    "lcq_gemm_tc_plan_check": (_c.c_int, [_c.c_int] * 4 + [_c.POINTER(_c.c_int)]),
 }
 
 

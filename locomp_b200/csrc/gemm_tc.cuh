@@ -1,23 +1,36 @@
-// W4A16 prefill GEMM (M > 16) on 5th-generation tensor cores: tcgen05.mma with the
-// accumulator AND the dequantised weight operand in tensor memory.
+// W4A16 GEMM (M > 16: serving batches and prompts) on 5th-generation tensor cores: tcgen05.mma with the
+// accumulators AND the dequantised weight operand in tensor memory.
 //
 //   out[m, n] = sum_k x[m, k] * (nib(n, k) - 8) * scales[n, k / 32]      (float32 accumulate)
 //
 // Orientation ("swap A/B"): the MMA's M dimension is the weight row n, its N dimension the
-// activation row m:   D[128 n x BM m] += Wdq[128 n x 64 k] * X^T[64 k x BM m].
-//   * X tiles [BM x 64] fp16 arrive by TMA (128-byte swizzle) and are the shared-memory B operand.
-//   * Packed int4 tiles [128 n x 256 k] (+ their fp16 scales) arrive by TMA; eight dequant
-//     warps turn them into fp16 (exactly RN((q - 8) * s)) in registers and write them with
-//     tcgen05.st into a ring of TMEM slots that the MMA reads as its A operand.  The packed
-//     weights therefore cross shared memory once (0.5 B/weight) and never as 2-byte values.
-//   * One thread issues the MMAs; tcgen05.commit releases X stages and TMEM slots and, after
-//     the last k tile, hands the accumulator to four epilogue warps (tcgen05.ld -> global).
-// TMEM map (512 columns): [0, 256) accumulator, [256, 512) eight A slots of 32 columns
-// (64 k as packed fp16 pairs).  Weight tiles are fp16 because bf16's 8-bit significand
-// cannot hold (q-8)*s within the 1e-2 output tolerance; bf16 activations are converted to
-// fp16 by a small pre-pass into the caller's workspace.
+// activation row m.  A team -- one CTA (CG = 1) or the two CTAs of a cluster (CG = 2) -- owns
+// D[128 * CG n x bm m], CTA r its rows 128 r .. 128 r + 127:
+//   * Packed int4 tiles [128 n x 256 k] (+ their fp16 scales) arrive by TMA in each CTA; sixteen
+//     dequant warps turn them into fp16 (exactly RN((q - 8) * s)) and write them with tcgen05.st into
+//     a ring of TMEM slots that the MMA reads as its A operand.  The packed weights cross shared
+//     memory once (0.5 B/weight) and never as 2-byte values.
+//   * X tiles [bm x 256 k] fp16 are the shared-memory B operand; in a pair each CTA holds half of their
+//     rows, which both SMs' tensor cores read (cta_group::2).
+//   * One warp of the team issues the MMAs; tcgen05.commit releases X stages and TMEM slots (in both
+//     CTAs) and hands a finished accumulator to four epilogue warps (tcgen05.ld -> global).
+// TMEM (512 columns): up to two accumulators of bm columns, so that the epilogue of one tile runs under
+// the MMAs of the next; the A slots (128 columns each: 256 k as packed fp16 pairs) at the end.
 //
-// Tensor-bound: 2*M*N*K flops per call against the dense 16-bit tensor peak.
+// What bounds it.  At bm >= 192 the tensor cores; below, an MMA costs what reading its A operand from
+// TMEM costs (~56 clocks for 128 x 16, whatever the N), and the hand-over between the dequant warps,
+// the MMA warp and back is a chain of barrier round trips -- hence whole 256-k stages per barrier (with
+// 64-k steps every step took ~750 clocks whatever bm), two sets of dequant warps that take the stages in
+// turn, and MMAs issued by an elected lane of a uniform warp.
+//
+// Split of the work: whole tiles in turn while they fill all teams; the rest is cut along K into equal
+// shares (stream-K).  A tile produced by several teams is combined through scratch: every contributor
+// publishes its float32 partial and bumps a counter, the last one sums all in a fixed order and writes
+// the output.  Nobody waits for another team.  With fewer tiles than SMs a cluster of 2, 4 or 8 CTAs shares
+// the K of each tile and adds up the partials over distributed shared memory.
+//
+// Weight tiles are fp16 because bf16's 8-bit significand cannot hold (q-8)*s within the 1e-2 output
+// tolerance; bf16 activations are converted to fp16 by a small pre-pass into the caller's workspace.
 // Every mbarrier wait is bounded; on expiry the kernel records a status code and unwinds.
 #pragma once
 #include "common.cuh"
@@ -25,51 +38,90 @@
 namespace lcq {
 namespace gemm_tc {
 
-constexpr int BN = 128;                 // weight rows per tile (MMA M)
-constexpr int BK = 64;                  // k per MMA stage (one 128-byte swizzle row of fp16)
-constexpr int WK = 256;                 // k per packed-weight stage
+constexpr int BN = 128;                 // weight rows per CTA
+constexpr int BK = 64;                  // k per step (one 128-byte swizzle row of fp16): four MMAs
+constexpr int WK = 256;                 // k per stage: of packed weights, of X and of TMEM
 constexpr int W_STAGE = BN * (WK / 2);  // 16384
 constexpr int S_STAGE = BN * (WK / 32) * 2;   // 2048
 constexpr int WS_STAGE = W_STAGE + S_STAGE;
-constexpr int NXS = 4;                  // X stages
-constexpr int NWS = 2;                  // packed-weight stages
-constexpr int NAS = 8;                  // TMEM A slots
-constexpr int A_COL0 = 256;             // first TMEM column of the A ring
-constexpr int A_SLOT_COLS = 32;
+constexpr int MAX_XS = 6, MAX_WS = 9, MAX_AS = 3;    // ring depths: X stages, weight stages, TMEM A slots
+constexpr int A_STEP_COLS = BK / 2;     // TMEM columns of 64 k as packed fp16 pairs
+constexpr int A_SLOT_COLS = WK / 2;     // an A slot holds a whole weight stage
 constexpr int TMEM_COLS = 512;
-constexpr int WARP_TMA = 4, WARP_MMA = 5, WARP_DQ0 = 8;
-constexpr int N_DQ_WARPS = 8;                 // 8 or 16 (16: two sets of warps take alternate 64-k tiles)
-constexpr int DQ_PAR = N_DQ_WARPS / 8;
-constexpr int NTHREADS = (WARP_DQ0 + N_DQ_WARPS) * 32;
+constexpr int N_DQ_WARPS = 16;          // two sets of two warpgroups
+constexpr int WARP_EPI0 = N_DQ_WARPS, WARP_W = WARP_EPI0 + 4, WARP_X = WARP_W + 1, WARP_MMA = WARP_X + 1;
+constexpr int NTHREADS = (WARP_MMA + 1) * 32;
+constexpr int BAR_EPI = 1;              // named barrier of the epilogue warps
 
-// ---------------------------------------------------------------- tcgen05 wrappers
+// ---------------------------------------------------------------- tcgen05 / cluster wrappers
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_alloc(uint32_t* smem_slot, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)), "r"(cols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+// CG = 1: the CTA alone; CG = 2: the pair of CTAs of a cluster (the two forms of every instruction below).
+template <int CG> __device__ __forceinline__ void tmem_alloc(uint32_t* smem_slot, uint32_t cols) {
+  if (CG == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
 }
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+template <int CG> __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
+  if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+  else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem descriptor]
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] * B[smem descriptor].  Called by a whole warp, issued by one elected lane: with
+// every operand uniform over the warp the compiler keeps them in uniform registers, where the
+// instruction wants them.  From a branch that one lane takes alone they are moved there one by one,
+// and an MMA takes ~80 clocks to issue whatever its size (M = 64 on 8192 -> 28672: 55.6 us, this way 48.2).
+template <int CG> __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  if (CG == 2) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+  }
+}
+// Arrives on this barrier (CG = 2: and on its counterpart in the other CTA) once the MMAs issued so far
+// have completed.  Whole warp, like the MMAs: the same lane is elected.
+template <int CG> __device__ __forceinline__ void umma_commit(uint64_t* bar) {
+  if (CG == 2)
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+                 "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+                 ::"r"(smem_u32(bar)), "h"(static_cast<uint16_t>(3)) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+                 "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
+// TMA load into this CTA's shared memory whose bytes are counted by a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const void* tmap, uint32_t bar_cluster_addr, int x, int y) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(tmap), "r"(bar_cluster_addr), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
       ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+        "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+        "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -92,297 +144,563 @@ __device__ __forceinline__ uint64_t make_b_desc(uint32_t smem_addr) {
   d |= static_cast<uint64_t>(2) << 61;                        // 128-byte swizzle
   return d;
 }
-// kind::f16 instruction descriptor: D=f32, A=B=f16, both K-major, M=128, N=bm.
-__host__ __device__ inline uint32_t make_idesc(int bm) {
-  return (1u << 4) | (static_cast<uint32_t>(bm >> 3) << 17) | (static_cast<uint32_t>(BN >> 4) << 24);
+// kind::f16 instruction descriptor: D=f32, A=B=f16, both K-major, M=128*CG, N=bm.
+__host__ __device__ inline uint32_t make_idesc(int bm, int cg) {
+  return (1u << 4) | (static_cast<uint32_t>(bm >> 3) << 17) | (static_cast<uint32_t>((BN * cg) >> 4) << 24);
 }
 
+// ---------------------------------------------------------------- work schedule
 struct Params {
   void* out;            // [M, N]
+  const void* scales;   // [N, K/32] fp16 (read directly when K % 256 != 0)
+  float* partials;      // [2 * teams][CTA of the team][bm][BN]
+  int* counters;        // [sk_tiles][CTA of the team], zero on entry, zero on exit
   int M, N, K;
   int bm;               // activation rows per tile (MMA N): multiple of 32, <= 256
-  int n_tiles_n, n_tiles_m;
-  int splits;           // split-K factor (1 = none); with > 1 `out` is float scratch [splits][M][N]
-  int k_tiles_per_split;  // 64-k tiles per split, a multiple of 4
-  int out_dtype;
-  int vec_store;        // N and out allow 16-byte stores
+  int n_tiles_n, n_tiles;
+  int nst;              // 256-k weight stages per tile
+  int teams;            // CTAs (CG = 1) or pairs (CG = 2) launched
+  int sk_tiles;         // tiles 0 .. sk_tiles-1 are cut along K, the others go whole to team (tile - sk_tiles) % teams
+  int split;            // > 1: a cluster of `split` teams per tile, each with its share of K (no whole tiles, no scratch)
+  int nxs, nws;         // ring depths: X stages, weight stages
+  int nas;              // TMEM A slots
+  int nd;               // accumulators (1 or 2)
+};
+
+// First unit (a tile's weight stage, tile-major) of team p's share of the tiles that are cut along K.
+__host__ __device__ inline unsigned share_begin(const Params& p, int team) {
+  const unsigned units = static_cast<unsigned>(p.sk_tiles) * static_cast<unsigned>(p.nst);
+  return static_cast<unsigned>(static_cast<unsigned long long>(units) * static_cast<unsigned>(team) / static_cast<unsigned>(p.teams));
+}
+__host__ __device__ inline int share_owner(const Params& p, unsigned unit) {
+  const unsigned units = static_cast<unsigned>(p.sk_tiles) * static_cast<unsigned>(p.nst);
+  return static_cast<int>((static_cast<unsigned long long>(unit + 1u) * static_cast<unsigned>(p.teams) - 1u) / units);
+}
+
+// The segments of one team: (tile, stages st0 .. st1-1).  Every role walks them in the same order.
+struct Walk {
+  unsigned u, u1;       // what is left of the team's share of the cut tiles
+  int next_tile;        // then the whole tiles
+  int tile, st0, st1;
+  __host__ __device__ Walk(const Params& p, int team) {
+    if (p.split > 1) {
+      const int t = team / p.split, r = team - t * p.split;
+      u = static_cast<unsigned>(t * p.nst + p.nst * r / p.split);
+      u1 = static_cast<unsigned>(t * p.nst + p.nst * (r + 1) / p.split);
+      next_tile = p.n_tiles;
+      return;
+    }
+    u = share_begin(p, team);
+    u1 = share_begin(p, team + 1);
+    next_tile = p.sk_tiles + team;
+  }
+  __host__ __device__ bool next(const Params& p) {
+    if (u < u1) {
+      tile = static_cast<int>(u / static_cast<unsigned>(p.nst));
+      st0 = static_cast<int>(u - static_cast<unsigned>(tile) * static_cast<unsigned>(p.nst));
+      const unsigned left = u1 - u, in_tile = static_cast<unsigned>(p.nst - st0);
+      const unsigned take = left < in_tile ? left : in_tile;
+      st1 = st0 + static_cast<int>(take);
+      u += take;
+      return true;
+    }
+    if (next_tile >= p.n_tiles) return false;
+    tile = next_tile;
+    next_tile += p.teams;
+    st0 = 0;
+    st1 = p.nst;
+    return true;
+  }
 };
 
 struct Smem {           // offsets from the 1024-byte aligned dynamic shared memory base
-  int x;                // NXS stages of bm x 128 B
-  int w;                // NWS stages of WS_STAGE
+  int w;                // nws stages of WS_STAGE
   int bars;
   int tmem_slot;
-  int flags;
-  int stage;            // epilogue staging: 2 x [32 m][128 n] of the output type (sized for float)
+  int flags;            // abort flag, epilogue broadcast
   int total;
 };
-__host__ __device__ inline Smem smem_map(int bm) {
+__host__ __device__ inline int x_step_bytes(int bm, int cg) { return (bm / cg) * 128; }   // this CTA's share of a tile's rows, 64 k
+__host__ __device__ inline int x_stage_bytes(int bm, int cg) { return (WK / BK) * x_step_bytes(bm, cg); }
+__host__ __device__ inline Smem smem_map(int bm, int cg, int nxs, int nws) {
   Smem s;
-  s.x = 0;
-  s.w = NXS * bm * 128;
-  s.bars = s.w + NWS * WS_STAGE;
-  // full_x, empty_x [NXS]; full_w, empty_w [NWS]; full_a, empty_a [NAS]; full_d, empty_d
-  s.tmem_slot = s.bars + (2 * NXS + 2 * NWS + 2 * NAS + 2) * 8;
+  s.w = nxs * x_stage_bytes(bm, cg);    // X stages first: steps are multiples of 2048 bytes
+  s.bars = s.w + nws * WS_STAGE;
+  // full_x, empty_x [MAX_XS]; full_w, empty_w [MAX_WS]; full_a, empty_a [MAX_AS]; full_d, empty_d [2]
+  s.tmem_slot = s.bars + (2 * MAX_XS + 2 * MAX_WS + 2 * MAX_AS + 4) * 8;
   s.flags = s.tmem_slot + 8;
-  s.stage = (s.flags + 8 + 15) & ~15;
-  s.total = s.stage + 2 * 32 * BN * 4;
+  s.total = s.flags + 8;
   return s;
 }
 
-// RN((q - 8) * s) for the 8 nibbles of a word, as 4 half2 in natural k order.
-// PERM = true leaves them in the order the masks deliver -- (e0,e4) (e1,e5) (e2,e6) (e3,e7) --
-// for activations whose k order was permuted the same way by the pre-pass (saves 4 PRMT).
+// ---------------------------------------------------------------- dequantisation
+__device__ __forceinline__ uint32_t lop_and_or(uint32_t a, uint32_t mask, uint32_t magic) {   // (a & mask) | magic
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(mask), "r"(magic));
+  return r;
+}
+__device__ __forceinline__ uint32_t sub_mul(uint32_t v, uint32_t offset, __half2 s2) {        // (v - offset) * s, halves alike
+  const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&offset));
+  const __half2 r = __hmul2(d, s2);
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+// RN((q - 8) * s) for the 8 nibbles of a word, as 4 half2.  A nibble in bits 0-3 of a 16-bit lane under
+// 0x6400 is the fp16 number 1024 + q, one in bits 4-7 under 0x5400 is 64 + q; the subtraction is exact.
+// PERM = true leaves the pairs as the masks deliver them -- (e0,e4) (e1,e5) (e2,e6) (e3,e7) -- for
+// activations whose k order was permuted the same way by the pre-pass (13 instructions a word); else
+// each byte is copied to both halves first, so that its two nibbles come out as a natural pair (16).
 template <bool PERM>
-__device__ __forceinline__ void dequant_word(uint32_t w, __half2 s2, uint32_t (&o)[4]) {
-  const __half2 k1032 = __half2half2(__ushort_as_half(0x6408));   // 1032.0
-  const __half2 k16th = __half2half2(__ushort_as_half(0x2C00));   // 1/16
-  const __half2 km72 = __half2half2(__ushort_as_half(0xD480));    // -72.0
-  const uint32_t w8 = w >> 8;
-  uint32_t l0 = (w & 0x000F000Fu) | 0x64006400u;     // 1024 + (e0, e4)
-  uint32_t h0 = (w & 0x00F000F0u) | 0x64006400u;     // 1024 + 16*(e1, e5)
-  uint32_t l1 = (w8 & 0x000F000Fu) | 0x64006400u;    // 1024 + (e2, e6)
-  uint32_t h1 = (w8 & 0x00F000F0u) | 0x64006400u;    // 1024 + 16*(e3, e7)
-  __half2 p0 = __hsub2(*reinterpret_cast<__half2*>(&l0), k1032);
-  __half2 p1 = __hfma2(*reinterpret_cast<__half2*>(&h0), k16th, km72);
-  __half2 p2 = __hsub2(*reinterpret_cast<__half2*>(&l1), k1032);
-  __half2 p3 = __hfma2(*reinterpret_cast<__half2*>(&h1), k16th, km72);
-  p0 = __hmul2(p0, s2); p1 = __hmul2(p1, s2); p2 = __hmul2(p2, s2); p3 = __hmul2(p3, s2);
-  const uint32_t u0 = *reinterpret_cast<uint32_t*>(&p0), u1 = *reinterpret_cast<uint32_t*>(&p1);
-  const uint32_t u2 = *reinterpret_cast<uint32_t*>(&p2), u3 = *reinterpret_cast<uint32_t*>(&p3);
+__device__ __forceinline__ void dequant_word(uint32_t w, __half2 s2, uint32_t* o) {
   if (PERM) {
-    o[0] = u0; o[1] = u1; o[2] = u2; o[3] = u3;
+    const uint32_t w8 = w >> 8;
+    o[0] = sub_mul(lop_and_or(w, 0x000F000Fu, 0x64006400u), 0x64086408u, s2);
+    o[1] = sub_mul(lop_and_or(w, 0x00F000F0u, 0x54005400u), 0x54805480u, s2);
+    o[2] = sub_mul(lop_and_or(w8, 0x000F000Fu, 0x64006400u), 0x64086408u, s2);
+    o[3] = sub_mul(lop_and_or(w8, 0x00F000F0u, 0x54005400u), 0x54805480u, s2);
   } else {
-    o[0] = __byte_perm(u0, u1, 0x5410);   // (e0, e1)
-    o[1] = __byte_perm(u2, u3, 0x5410);   // (e2, e3)
-    o[2] = __byte_perm(u0, u1, 0x7632);   // (e4, e5)
-    o[3] = __byte_perm(u2, u3, 0x7632);   // (e6, e7)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      o[j] = sub_mul(lop_and_or(__byte_perm(w, 0u, 0x4040 + 0x0101 * j), 0x00F0000Fu, 0x54006400u), 0x54806408u, s2);
   }
 }
 
-// Bounded wait whose verdict is the same in every lane, so warp-aligned instructions that
-// follow it never run with a partial warp.
+__device__ __forceinline__ uint32_t peer_addr(uint32_t local_addr, uint32_t rank) {   // same offset in the CTA of that rank
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// Barriers of the MMA issuer's CTA, as the CTAs of the team address them.  What these arrivals hand over
+// lives in tensor memory and is ordered by the tcgen05 fences around them.
+template <int CG> __device__ __forceinline__ uint32_t leader_addr(uint64_t* bar) {
+  return CG == 2 ? peer_addr(smem_u32(bar), 0) : smem_u32(bar);
+}
+template <int CG> __device__ __forceinline__ void arrive_leader(uint32_t addr) {
+  if (CG == 2) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+  else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// Bounded wait; gives up when the CTA's abort flag is set or the library's wait limit has passed.  The
+// clock is read only after many polls: waits of the ordinary kind end before that.
+__device__ __noinline__ bool wait_slow(volatile int* flag_abort, uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
+  for (int i = 0; i < 1024; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+  }
+  const uint64_t t0 = global_timer_ns();
+  const uint64_t limit = wait_limit_ns();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i) {
+      if (mbar_try_wait(bar, parity)) return true;
+    }
+    if (*flag_abort != 0 || global_timer_ns() - t0 > limit) return false;
+  }
+}
+__device__ __forceinline__ bool wait_bar(volatile int* flag_abort, uint64_t* bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  return wait_slow(flag_abort, bar, parity);
+}
+// The same with one verdict for the whole warp, so that warp-aligned instructions after it never run
+// with a partial warp.
 __device__ __forceinline__ bool warp_wait(volatile int* flag_abort, uint64_t* bar, uint32_t parity) {
-  const bool ok = (*flag_abort == 0) && mbar_wait_bounded(bar, parity);
-  return __all_sync(0xffffffffu, ok);
+  return __all_sync(0xffffffffu, wait_bar(flag_abort, bar, parity));
+}
+__device__ __forceinline__ int load_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ bool all_epilogue_warps(bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all) : "r"(ok ? 1u : 0u), "n"(BAR_EPI) : "memory");
+  return all != 0;
 }
 
-template <typename OT, bool PERM>
+// A position in a ring of n slots and the parity of its current lap.
+struct Ring {
+  uint32_t i, phase;
+  __device__ __forceinline__ void step(uint32_t n) { if (++i == n) { i = 0; phase ^= 1u; } }
+};
+
+// Adds up the partials of a tile that was cut along K and writes its row r of the outputs: `count`
+// contributors in team order, bit for bit the same whoever finishes; contributor `mine` (this CTA) is still
+// in tensor memory.  16 columns at a time: a round trip to L2 under the stream of weights takes 2-3 us.
+// With one other contributor (nearly always) its next columns are fetched while the current ones are added.
+// Out of line: its registers would otherwise cost the dequant warps some of theirs.
+template <typename OT>
+__device__ __noinline__ void finish_tile(uint32_t d_t, OT* out, int rows_out, int rows, int N, const float* first, const float* second,
+                                         long long stride, int count, int mine) {
+  const bool two = count == 2;
+  const float* other = mine == 0 ? second : first;
+  float next[16];
+  if (two) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) next[i] = __ldcg(other + i * BN);
+  }
+#pragma unroll 1
+  for (int c0 = 0; c0 < rows; c0 += 16) {
+    uint32_t v[16];
+    tmem_ld16(d_t + c0, v);
+    tmem_wait_ld();
+    if (two) {
+      other += 16 * BN;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        v[i] = __float_as_uint(__uint_as_float(v[i]) + next[i]);
+        if (c0 + 16 < rows) next[i] = __ldcg(other + i * BN);
+      }
+    } else {
+      float sum[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sum[i] = 0.0f;
+#pragma unroll 1
+      for (int q = 0; q < count; ++q) {
+        const float* src = (q == 0 ? first : second + (q - 1) * stride) + c0 * BN;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) next[i] = q == mine ? __uint_as_float(v[i]) : __ldcg(src + i * BN);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum[i] += next[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(sum[i]);
+    }
+    OT* o = out + static_cast<long long>(c0) * N;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if (c0 + i < rows_out) *o = from_f32<OT>(__uint_as_float(v[i]));
+      o += N;
+    }
+  }
+}
+
+// RAGGED: K % 256 != 0 -- the last weight stage of a tile is partial, and the scale rows are no 16-byte
+// multiples, so no tensor map can describe them: the dequant warps load their scales from global
+// memory, a stage ahead.
+template <int CG, typename OT, bool PERM, bool RAGGED>
 __global__ void __launch_bounds__(NTHREADS, 1)
 w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
-                  const __grid_constant__ CUtensorMap tmap_s, const Params p) {
+                  const __grid_constant__ CUtensorMap tmap_s, const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  if ((smem_u32(smem) & 1023u) != 0u) {
-    if (threadIdx.x == 0) atomicExch(&g_device_status, 13);
-    return;
-  }
-  const Smem L = smem_map(p.bm);
+  const Smem L = smem_map(p.bm, CG, p.nxs, p.nws);
   uint64_t* full_x = reinterpret_cast<uint64_t*>(smem + L.bars);
-  uint64_t* empty_x = full_x + NXS;
-  uint64_t* full_w = empty_x + NXS;
-  uint64_t* empty_w = full_w + NWS;
-  uint64_t* full_a = empty_w + NWS;
-  uint64_t* empty_a = full_a + NAS;
-  uint64_t* full_d = empty_a + NAS;
-  uint64_t* empty_d = full_d + 1;
+  uint64_t* empty_x = full_x + MAX_XS;
+  uint64_t* full_w = empty_x + MAX_XS;
+  uint64_t* empty_w = full_w + MAX_WS;
+  uint64_t* full_a = empty_w + MAX_WS;
+  uint64_t* empty_a = full_a + MAX_AS;
+  uint64_t* full_d = empty_a + MAX_AS;
+  uint64_t* empty_d = full_d + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L.tmem_slot);
   volatile int* flag_abort = reinterpret_cast<volatile int*>(smem + L.flags);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int x_stage_bytes = p.bm * 128;
-  // a work item is (output tile, k split); k_tiles counts the 64-k tiles of one item
-  const int k_tiles = p.k_tiles_per_split;
-  const int total_tiles = p.n_tiles_n * p.n_tiles_m * p.splits;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform over the warp)
+  const uint32_t crank = CG == 2 ? blockIdx.x & 1 : 0;    // rank in the pair: clusters are consecutive blocks
+  const int team = blockIdx.x / CG;
+  const int nk = p.K / BK;                    // 64-k steps of a tile
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NXS; ++i) { mbar_init(&full_x[i], 1); mbar_init(&empty_x[i], 1); }
-    for (int i = 0; i < NWS; ++i) { mbar_init(&full_w[i], 1); mbar_init(&empty_w[i], N_DQ_WARPS); }
-    for (int i = 0; i < NAS; ++i) { mbar_init(&full_a[i], 8); mbar_init(&empty_a[i], 1); }
-    mbar_init(full_d, 1);
-    mbar_init(empty_d, 4);
+    // full_x, full_a and empty_d are used in the pair's first CTA only; commits arrive in both CTAs
+    for (int i = 0; i < MAX_XS; ++i) { mbar_init(&full_x[i], 1); mbar_init(&empty_x[i], 1); }
+    for (int i = 0; i < MAX_WS; ++i) { mbar_init(&full_w[i], 1); mbar_init(&empty_w[i], N_DQ_WARPS / 2); }
+    for (int i = 0; i < MAX_AS; ++i) { mbar_init(&full_a[i], CG * N_DQ_WARPS / 2); mbar_init(&empty_a[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&full_d[i], 1); mbar_init(&empty_d[i], 4 * CG); }
     *flag_abort = 0;
     fence_barrier_init();
+    griddep_launch_dependents();
   }
-  if (warp == WARP_MMA) tmem_alloc(tmem_slot, TMEM_COLS);
+  if (warp == WARP_MMA) tmem_alloc<CG>(tmem_slot, TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (CG == 2) cluster_barrier();             // the other CTA's barriers exist
   const uint32_t tmem_base = *tmem_slot;
+  const uint32_t a_base = tmem_base + TMEM_COLS - p.nas * A_SLOT_COLS;
 
 #define LCQ_GIVE_UP(code) do { *flag_abort = 1; atomicExch(&g_device_status, (code)); } while (0)
 
-  if (warp == WARP_TMA) {
-    // ------------------------------------------------------------ TMA producer
+  if (warp == WARP_W) {
+    // ------------------------------------------------------------ weights and scales (constants: no dependency wait)
     if (lane == 0) {
-      tma_prefetch_desc(&tmap_x); tma_prefetch_desc(&tmap_w); tma_prefetch_desc(&tmap_s);
-      uint32_t xi = 0, wi = 0;   // running stage counters
+      tma_prefetch_desc(&tmap_w);
+      if (!RAGGED) tma_prefetch_desc(&tmap_s);
+      Ring r = {0, 0};
       bool ok = true;
-      for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x) {
-        const int tile = item / p.splits, kt0 = (item % p.splits) * k_tiles;
-        const int m0 = (tile / p.n_tiles_n) * p.bm, n0 = (tile % p.n_tiles_n) * BN;
-        for (int kt = 0; kt < k_tiles && ok; ++kt) {
-          if ((kt & 3) == 0) {
-            const uint32_t s = wi % NWS, ph = (wi / NWS) & 1;
-            if (*flag_abort || !mbar_wait_bounded(&empty_w[s], ph ^ 1)) { LCQ_GIVE_UP(10); ok = false; break; }
-            uint8_t* dst = smem + L.w + s * WS_STAGE;
-            mbar_expect_tx(&full_w[s], WS_STAGE);
-            tma_load_2d(dst, &tmap_w, &full_w[s], ((kt0 + kt) / 4) * (WK / 2), n0);
-            tma_load_2d(dst + W_STAGE, &tmap_s, &full_w[s], ((kt0 + kt) / 4) * (WK / 32), n0);
-            ++wi;
+      for (Walk w(p, team); ok && w.next(p);) {
+        const int n0 = (w.tile % p.n_tiles_n) * (CG * BN) + static_cast<int>(crank) * BN;
+        for (int st = w.st0; st < w.st1; ++st, r.step(p.nws)) {
+          if (!wait_bar(flag_abort, &empty_w[r.i], r.phase ^ 1u)) { LCQ_GIVE_UP(10); ok = false; break; }
+          uint8_t* dst = smem + L.w + r.i * WS_STAGE;
+          mbar_expect_tx(&full_w[r.i], RAGGED ? W_STAGE : WS_STAGE);
+          tma_load_2d(dst, &tmap_w, &full_w[r.i], st * (WK / 2), n0);
+          if (!RAGGED) tma_load_2d(dst + W_STAGE, &tmap_s, &full_w[r.i], st * (WK / 32), n0);
+        }
+      }
+    }
+  } else if (warp == WARP_X) {
+    // ------------------------------------------------------------ activations: this CTA's share of the rows of each tile
+    if (lane == 0) {
+      tma_prefetch_desc(&tmap_x);
+      griddep_wait();                    // x is the preceding kernel's output
+      const int half = p.bm / CG, bytes = x_step_bytes(p.bm, CG);
+      Ring r = {0, 0};
+      bool ok = true;
+      for (Walk w(p, team); ok && w.next(p);) {
+        const int m0 = (w.tile / p.n_tiles_n) * p.bm + static_cast<int>(crank) * half;
+        for (int st = w.st0; st < w.st1; ++st, r.step(p.nxs)) {
+          const int steps = RAGGED && nk - st * 4 < 4 ? nk - st * 4 : 4;
+          if (!wait_bar(flag_abort, &empty_x[r.i], r.phase ^ 1u)) { LCQ_GIVE_UP(11); ok = false; break; }
+          if (crank == 0) mbar_expect_tx(&full_x[r.i], CG * steps * bytes);
+          const uint32_t bar = leader_addr<CG>(full_x + r.i);
+          uint8_t* dst = smem + r.i * (4 * bytes);
+          for (int j = 0; j < steps; ++j) {
+            if (CG == 2) tma_load_2d_pair(dst + j * bytes, &tmap_x, bar, (st * 4 + j) * BK, m0);
+            else tma_load_2d(dst + j * bytes, &tmap_x, full_x + r.i, (st * 4 + j) * BK, m0);
           }
-          const uint32_t s = xi % NXS, ph = (xi / NXS) & 1;
-          if (*flag_abort || !mbar_wait_bounded(&empty_x[s], ph ^ 1)) { LCQ_GIVE_UP(11); ok = false; break; }
-          mbar_expect_tx(&full_x[s], x_stage_bytes);
-          tma_load_2d(smem + L.x + s * x_stage_bytes, &tmap_x, &full_x[s], (kt0 + kt) * BK, m0);
-          ++xi;
         }
       }
     }
   } else if (warp == WARP_MMA) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(p.bm);
-      uint32_t xi = 0, ai = 0, di = 0;
+    // ------------------------------------------------------------ MMA issuer: one warp for the team
+    if (crank == 0) {
+      const uint32_t idesc = make_idesc(p.bm, CG);
+      const uint64_t desc0 = make_b_desc(smem_u32(smem));
+      const uint64_t desc_step = static_cast<uint64_t>(x_step_bytes(p.bm, CG) >> 4);      // descriptors count 16-byte units
+      Ring rx = {0, 0}, ra = {0, 0}, rd = {0, 0};
       bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++di) {
-        if (*flag_abort || !mbar_wait_bounded(empty_d, (di & 1) ^ 1)) { LCQ_GIVE_UP(12); ok = false; break; }
+      for (Walk w(p, team); ok && w.next(p); rd.step(p.nd)) {
+        if (!warp_wait(flag_abort, &empty_d[rd.i], rd.phase ^ 1u)) { if (lane == 0) LCQ_GIVE_UP(12); ok = false; break; }
         tc_fence_after();
-        for (int kt = 0; kt < k_tiles && ok; ++kt, ++xi, ++ai) {
-          const uint32_t sx = xi % NXS, phx = (xi / NXS) & 1;
-          const uint32_t sa = ai % NAS, pha = (ai / NAS) & 1;
-          if (*flag_abort || !mbar_wait_bounded(&full_x[sx], phx) || !mbar_wait_bounded(&full_a[sa], pha)) {
-            LCQ_GIVE_UP(14); ok = false; break;
+        const uint32_t d_t = tmem_base + rd.i * p.bm;
+        uint32_t acc = 0;
+        for (int st = w.st0; st < w.st1; ++st, rx.step(p.nxs), ra.step(p.nas)) {
+          const int steps = RAGGED && nk - st * 4 < 4 ? nk - st * 4 : 4;
+          if (!warp_wait(flag_abort, &full_x[rx.i], rx.phase) || !warp_wait(flag_abort, &full_a[ra.i], ra.phase)) {
+            if (lane == 0) LCQ_GIVE_UP(14);
+            ok = false;
+            break;
           }
           tc_fence_after();
-          const uint64_t bdesc = make_b_desc(smem_u32(smem + L.x + sx * x_stage_bytes));
-          const uint32_t a_t = tmem_base + A_COL0 + sa * A_SLOT_COLS;
+          uint64_t bdesc = desc0 + rx.i * (desc_step * 4);
+          uint32_t a_t = a_base + ra.i * A_SLOT_COLS;
+          for (int k = 0; k < steps; ++k, bdesc += desc_step, a_t += A_STEP_COLS) {
 #pragma unroll
-          for (int j = 0; j < BK / 16; ++j)
-            umma_f16_ts(tmem_base, a_t + j * 8, bdesc + static_cast<uint64_t>(2 * j), idesc, (kt | j) != 0 ? 1u : 0u);
-          umma_commit(&empty_x[sx]);
-          umma_commit(&empty_a[sa]);
-        }
-        if (ok) umma_commit(full_d);
-      }
-    }
-  } else if (warp >= WARP_DQ0) {
-    // ------------------------------------------------------------ dequant warps: smem int4 -> TMEM fp16
-    // Thread = weight row = TMEM lane; warpgroup bit 0 picks the 32-wide half of a 64-k tile.  With
-    // 16 warps the second pair of warpgroups takes the odd tiles (DQ_PAR = 2).  Software-pipelined
-    // by one tile: the registers of a warp's next tile are computed while the tcgen05.st of its
-    // current one is in flight; only then is that store waited for and the slot handed to the MMA.
-    const int q4 = warp & 3;                    // TMEM lane quarter this warp may touch
-    const int wg = (warp - WARP_DQ0) >> 2;      // 0..3
-    const int h = wg & 1;                       // which 32-wide half of the 64-k tile
-    const int par = wg >> 1;                    // which tiles: kt % 2 == par
-    const int r = q4 * 32 + lane;               // weight row inside the tile = TMEM lane
-    const uint32_t lane_taddr = tmem_base + (static_cast<uint32_t>(q4 * 32) << 16) + A_COL0 + h * 16;
-    const int my_tiles = (total_tiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
-    const long long n_steps = static_cast<long long>(my_tiles) * k_tiles;   // 64-k tiles this CTA processes (even)
-    bool ok = true;
-    uint32_t v[16];
-
-    // registers of step `st` (packed tile q = st % 4 of weight stage st / 4)
-    auto produce = [&](long long st) -> bool {
-      const int q = static_cast<int>(st & 3);
-      const uint32_t wi = static_cast<uint32_t>(st >> 2);
-      const uint32_t sw = wi % NWS;
-      if (q < DQ_PAR) {                         // this warp's first tile in the weight stage
-        if (!warp_wait(flag_abort, &full_w[sw], (wi / NWS) & 1)) return false;
-      }
-      const uint8_t* wst = smem + L.w + sw * WS_STAGE;
-      const int c = q * 2 + h;                  // 16-byte chunk (= one 32-wide group) of the 128-byte row
-      const uint4 pk = *reinterpret_cast<const uint4*>(wst + r * 128 + ((c ^ (r & 7)) << 4));
-      const __half2 s2 = __half2half2(*reinterpret_cast<const __half*>(wst + W_STAGE + r * 16 + c * 2));
-      uint32_t o[4];
-      dequant_word<PERM>(pk.x, s2, o); v[0] = o[0]; v[1] = o[1]; v[2] = o[2]; v[3] = o[3];
-      dequant_word<PERM>(pk.y, s2, o); v[4] = o[0]; v[5] = o[1]; v[6] = o[2]; v[7] = o[3];
-      dequant_word<PERM>(pk.z, s2, o); v[8] = o[0]; v[9] = o[1]; v[10] = o[2]; v[11] = o[3];
-      dequant_word<PERM>(pk.w, s2, o); v[12] = o[0]; v[13] = o[1]; v[14] = o[2]; v[15] = o[3];
-      __syncwarp();
-      if (q >= 4 - DQ_PAR && lane == 0) mbar_arrive(&empty_w[sw]);   // this warp's last read of the weight stage
-      return true;
-    };
-
-    if (n_steps > par && !produce(par)) { LCQ_GIVE_UP(15); ok = false; }
-    for (long long st = par; st < n_steps && ok; st += DQ_PAR) {
-      const uint32_t ai = static_cast<uint32_t>(st);
-      const uint32_t sa = ai % NAS;
-      if (!warp_wait(flag_abort, &empty_a[sa], ((ai / NAS) & 1) ^ 1)) { LCQ_GIVE_UP(16); ok = false; break; }
-      tc_fence_after();
-      tmem_st16(lane_taddr + sa * A_SLOT_COLS, v);         // registers are read at issue
-      if (st + DQ_PAR < n_steps) {
-        if (!produce(st + DQ_PAR)) { LCQ_GIVE_UP(15); ok = false; }   // overlaps the store in flight
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&full_a[sa]);
-    }
-  } else if (warp < 4) {
-    // ------------------------------------------------------------ epilogue warps: TMEM -> smem -> global
-    // The accumulator is n-major (lane = n, column = m) while out is [M, N]: 32 columns at a
-    // time are converted and transposed through a double-buffered staging tile [32 m][128 n],
-    // then written with 16-byte stores, 256 contiguous bytes (128 n) per output row.
-    OT* out_base = static_cast<OT*>(p.out);
-    OT* stage = reinterpret_cast<OT*>(smem + L.stage);
-    constexpr int VEC = 16 / sizeof(OT);                 // outputs per 16-byte store
-    constexpr int ROW_VECS = BN / VEC;                   // 16-byte pieces per staged row
-    const int et = warp * 32 + lane;                     // 0..127
-    uint32_t di = 0, chunk = 0;
-    bool ok = true;
-    for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x, ++di) {
-      const int tile = item / p.splits;
-      const int m0 = (tile / p.n_tiles_n) * p.bm, n0 = (tile % p.n_tiles_n) * BN;
-      OT* out = out_base + static_cast<long long>(item % p.splits) * p.M * p.N;   // split-K: this split's partial
-      if (!warp_wait(flag_abort, full_d, di & 1)) { LCQ_GIVE_UP(17); ok = false; break; }
-      tc_fence_after();
-      const int n_cb = p.bm / 32;
-      for (int cb = 0; cb < n_cb; ++cb, ++chunk) {
-        uint32_t v[32];
-        tmem_ld32(tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + cb * 32, v);
-        tmem_wait_ld();
-        if (cb == n_cb - 1) {                            // accumulator fully read: the next tile's MMAs may start
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(empty_d);
-        }
-        OT* sb = stage + (chunk & 1) * (32 * BN);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) sb[i * BN + et] = from_f32<OT>(__uint_as_float(v[i]));
-        named_bar_sync(2, 128);
-        {
-          if (p.vec_store) {
-#pragma unroll
-            for (int j = 0; j < (32 * ROW_VECS) / 128; ++j) {
-              const int idx = j * 128 + et;
-              const int mi = idx / ROW_VECS, cv = idx - mi * ROW_VECS;
-              const int m = m0 + cb * 32 + mi, n = n0 + cv * VEC;
-              if (m < p.M && n < p.N) {
-                const uint4 val = *reinterpret_cast<const uint4*>(sb + mi * BN + cv * VEC);
-                *reinterpret_cast<uint4*>(out + static_cast<long long>(m) * p.N + n) = val;
-              }
+            for (int j = 0; j < BK / 16; ++j) {
+              umma_ts<CG>(d_t, a_t + j * 8, bdesc + static_cast<uint64_t>(2 * j), idesc, acc);
+              acc = 1;
             }
-          } else {
-            const int n = n0 + et;
-            if (n < p.N) {
-              for (int i = 0; i < 32; ++i) {
-                const int m = m0 + cb * 32 + i;
-                if (m < p.M) out[static_cast<long long>(m) * p.N + n] = sb[i * BN + et];
-              }
+          }
+          umma_commit<CG>(&empty_x[rx.i]);
+          umma_commit<CG>(&empty_a[ra.i]);
+        }
+        if (ok) umma_commit<CG>(&full_d[rd.i]);
+      }
+    }
+  } else if (warp < N_DQ_WARPS) {
+    // ------------------------------------------------------------ dequant warps: smem int4 -> TMEM fp16
+    // Two sets of two warpgroups take the stages in turn, so that one set computes while the other loads,
+    // stores or waits.  Thread = weight row = TMEM lane; warpgroup g of a set takes the 64-k steps 2g and
+    // 2g + 1 of its stages (four scale groups).
+    const int set = warp >> 3, g = (warp >> 2) & 1;
+    const int r = (warp & 3) * 32 + lane;
+    const uint32_t lane_taddr = a_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 2 * g * A_STEP_COLS;
+    const uint32_t full_a0 = leader_addr<CG>(full_a);
+    const uint8_t* wrow = smem + L.w + r * 128;
+    const uint8_t* srow = smem + L.w + W_STAGE + r * 16 + g * 8;
+    const int swz = (4 * g) ^ (r & 7);         // 16-byte chunk 4g + j of the row sits at chunk (4g + j) ^ (r & 7): 128-byte swizzle
+    Ring rw = {0, 0}, ra = {0, 0};
+    int turn = 0;                              // whose stage it is
+    bool ok = true;
+    for (Walk w(p, team); ok && w.next(p);) {
+      const uint32_t* gs = nullptr;            // RAGGED: this row's scales in global memory, two groups a word
+      uint2 s_next = make_uint2(0u, 0u);
+      const auto fetch = [&](int st) {
+        const int k = st * 4 + 2 * g;
+        s_next.x = __ldg(gs + (k < nk ? k : nk - 1));
+        s_next.y = __ldg(gs + (k + 1 < nk ? k + 1 : nk - 1));
+      };
+      if (RAGGED) {
+        const int n = (w.tile % p.n_tiles_n) * (CG * BN) + static_cast<int>(crank) * BN + r;
+        gs = reinterpret_cast<const uint32_t*>(p.scales) + static_cast<long long>(n < p.N ? n : p.N - 1) * nk;
+        fetch(w.st0 + (turn == set ? 0 : 1));
+      }
+      for (int st = w.st0; st < w.st1; ++st, turn ^= 1, rw.step(p.nws), ra.step(p.nas)) {
+        if (turn != set) continue;
+        uint2 sc = s_next;
+        if (RAGGED) fetch(st + 2);
+        if (!warp_wait(flag_abort, &full_w[rw.i], rw.phase)) { if (lane == 0) LCQ_GIVE_UP(15); ok = false; break; }
+        const uint8_t* src = wrow + rw.i * WS_STAGE;
+        uint4 pk[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) pk[j] = *reinterpret_cast<const uint4*>(src + ((swz ^ j) << 4));
+        if (!RAGGED) sc = *reinterpret_cast<const uint2*>(srow + rw.i * WS_STAGE);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty_w[rw.i]);
+        const uint32_t dst = lane_taddr + ra.i * A_SLOT_COLS;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {          // RAGGED: steps past K are stored too, and not multiplied
+          const __half2 s01 = *reinterpret_cast<const __half2*>(h == 0 ? &sc.x : &sc.y);
+          const __half2 s0 = __low2half2(s01), s1 = __high2half2(s01);
+          uint32_t v[32];
+          dequant_word<PERM>(pk[2 * h].x, s0, v);
+          dequant_word<PERM>(pk[2 * h].y, s0, v + 4);
+          dequant_word<PERM>(pk[2 * h].z, s0, v + 8);
+          dequant_word<PERM>(pk[2 * h].w, s0, v + 12);
+          dequant_word<PERM>(pk[2 * h + 1].x, s1, v + 16);
+          dequant_word<PERM>(pk[2 * h + 1].y, s1, v + 20);
+          dequant_word<PERM>(pk[2 * h + 1].z, s1, v + 24);
+          dequant_word<PERM>(pk[2 * h + 1].w, s1, v + 28);
+          if (h == 0) {
+            if (!warp_wait(flag_abort, &empty_a[ra.i], ra.phase ^ 1u)) { if (lane == 0) LCQ_GIVE_UP(16); ok = false; break; }
+            tc_fence_after();
+          }
+          tmem_st32(dst + h * A_STEP_COLS, v);
+        }
+        if (!ok) break;
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive_leader<CG>(full_a0 + ra.i * 8);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue warps: TMEM -> global
+    // The accumulator is n-major (lane = n, column = m) while out is [M, N]: a warp writes 32
+    // consecutive n of one m per store (64 or 128 contiguous bytes: whole sectors).
+    griddep_wait();                            // out and the scratch may still be in the preceding kernel's use
+    const int q4 = warp - WARP_EPI0;
+    const int r = q4 * 32 + lane;
+    const uint32_t lane_taddr = tmem_base + (static_cast<uint32_t>(q4 * 32) << 16);
+    const uint32_t empty_d0 = leader_addr<CG>(empty_d);
+    volatile int* shared_int = flag_abort + 1;
+    const long long part_elems = static_cast<long long>(p.bm) * BN;
+    Ring rd = {0, 0};
+    for (Walk w(p, team); w.next(p); rd.step(p.nd)) {
+      const int m0 = (w.tile / p.n_tiles_n) * p.bm;
+      const int n = (w.tile % p.n_tiles_n) * (CG * BN) + static_cast<int>(crank) * BN + r;
+      const uint32_t d_t = lane_taddr + rd.i * p.bm;
+      int rows = p.M - m0;                     // rows of out in this tile
+      if (rows > p.bm) rows = p.bm;
+      OT* out = static_cast<OT*>(p.out) + static_cast<long long>(m0) * p.N + n;
+      // one verdict for the four warps: they meet at named barriers below
+      if (!all_epilogue_warps(wait_bar(flag_abort, &full_d[rd.i], rd.phase))) { if (lane == 0) LCQ_GIVE_UP(17); break; }
+      tc_fence_after();
+      if (CG == 1 && p.split > 1) break;       // the cluster adds up its shares below
+      // who else contributes to this tile: teams p0 .. p1
+      int p0 = team, p1 = team, slot1 = 0;
+      if (w.tile < p.sk_tiles) {
+        const unsigned t0 = static_cast<unsigned>(w.tile) * static_cast<unsigned>(p.nst);
+        p0 = share_owner(p, t0);
+        p1 = share_owner(p, t0 + static_cast<unsigned>(p.nst) - 1u);
+        slot1 = share_begin(p, p0) < t0;       // p0 came from the tile before (slot 0); the others' shares begin here
+      }
+      const auto part = [&](int q) {
+        return p.partials + (static_cast<long long>(2 * q + (q == p0 ? slot1 : 0)) * CG + crank) * part_elems + r;
+      };
+      if (p1 == p0) {
+        for (int c0 = 0; c0 < rows; c0 += 32) {
+          uint32_t v[32];
+          tmem_ld32(d_t + c0, v);
+          tmem_wait_ld();
+          if (n < p.N) {
+            OT* o = out + static_cast<long long>(c0) * p.N;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              if (c0 + i < rows) *o = from_f32<OT>(__uint_as_float(v[i]));
+              o += p.N;
             }
           }
         }
+      } else {
+        int* counter = p.counters + w.tile * CG + crank;
+        // published already by all the others?  Then this CTA finishes the tile without publishing.
+        if (threadIdx.x == WARP_EPI0 * 32) *shared_int = load_acquire(counter);
+        named_bar_sync(BAR_EPI, 128);
+        bool finish = *shared_int == p1 - p0;
+        named_bar_sync(BAR_EPI, 128);
+        if (!finish) {
+          float* mine = part(team);
+          for (int c0 = 0; c0 < rows; c0 += 32) {
+            uint32_t v[32];
+            tmem_ld32(d_t + c0, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) __stcg(mine + (c0 + i) * BN, __uint_as_float(v[i]));
+          }
+          __threadfence();
+          named_bar_sync(BAR_EPI, 128);
+          if (threadIdx.x == WARP_EPI0 * 32) *shared_int = atomicAdd(counter, 1);
+          named_bar_sync(BAR_EPI, 128);
+          finish = *shared_int == p1 - p0;
+          named_bar_sync(BAR_EPI, 128);
+        }
+        __threadfence();
+        if (finish) {
+          finish_tile<OT>(d_t, out, n < p.N ? rows : 0, rows, p.N, part(p0), part(p0) + (2 - slot1) * CG * part_elems,
+                          2 * CG * part_elems, p1 - p0 + 1, team - p0);
+          if (threadIdx.x == WARP_EPI0 * 32) *counter = 0;
+        }
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) arrive_leader<CG>(empty_d0 + rd.i * 8);
     }
   }
 #undef LCQ_GIVE_UP
 
   tc_fence_before();
   __syncthreads();
+  if (CG == 2) {
+    // neither CTA leaves while the other may still arrive on its barriers or the pair's MMAs read its memory
+    cluster_barrier();
+  } else if (p.split > 1) {
+    // One tile per cluster, its K shared out: CTA d settles columns d * cw .. of the tile.  Every CTA sends
+    // each of the others its part of their columns (distributed shared memory, into the rings, which
+    // nobody uses any more), and adds up what it got in rank order.
+    const int me = team % p.split, tile = team / p.split, cw = p.bm / p.split;
+    const int m0 = (tile / p.n_tiles_n) * p.bm;
+    const int rows = p.M - m0 < p.bm ? p.M - m0 : p.bm;
+    const int r = (warp - WARP_EPI0) * 32 + lane;
+    const bool epilogue = warp >= WARP_EPI0 && warp < WARP_W;
+    cluster_barrier();
+    if (epilogue) {
+      tc_fence_after();
+      int d = 0, j = 0;
+      const uint32_t mine = smem_u32(smem) + (me * cw * BN + r) * 4;
+      uint32_t dst = peer_addr(mine, 0);
+      for (int c0 = 0; c0 < rows; c0 += 16) {
+        uint32_t v[16];
+        tmem_ld16(tmem_base + (static_cast<uint32_t>((warp - WARP_EPI0) * 32) << 16) + c0, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst), "r"(v[i]) : "memory");
+          dst += BN * 4;
+          if (++j == cw) { j = 0; ++d; dst = peer_addr(mine, d < p.split ? d : 0); }
+        }
+      }
+      tc_fence_before();
+    }
+    cluster_barrier();
+    const int n = (tile % p.n_tiles_n) * BN + r;
+    if (epilogue && n < p.N) {
+      const float* got = reinterpret_cast<const float*>(smem) + r;
+      OT* out = static_cast<OT*>(p.out) + static_cast<long long>(m0 + me * cw) * p.N + n;
+      for (int j = 0; j < cw && me * cw + j < rows; ++j) {
+        float sum = 0.0f;
+        for (int q = 0; q < p.split; ++q) sum += got[(q * cw + j) * BN];
+        out[static_cast<long long>(j) * p.N] = from_f32<OT>(sum);
+      }
+    }
+  }
   if (warp == WARP_MMA) {
+    __syncwarp();
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc<CG>(tmem_base, TMEM_COLS);
   }
 }
 
@@ -390,6 +708,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 // of every 16-byte piece reordered to (0,4,1,5,2,6,3,7): the order in which the nibble masks
 // deliver the weights, so the dequant warps need no re-pairing.
 __global__ void __launch_bounds__(256) bf16_to_f16_perm_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, long long n16) {
+  griddep_launch_dependents();
+  griddep_wait();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n16; i += stride) {
     const uint4 a = __ldg(in + i);
@@ -404,75 +724,100 @@ __global__ void __launch_bounds__(256) bf16_to_f16_perm_kernel(const uint4* __re
   }
 }
 
-// out[i] = sum over splits of partial[s][i], rounded once to the output type
-template <typename OT>
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ part, OT* __restrict__ out,
-                                                            long long n, int splits) {
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-    float acc = 0.0f;
-    for (int s = 0; s < splits; ++s) acc += __ldcs(part + static_cast<long long>(s) * n + i);
-    out[i] = from_f32<OT>(acc);
-  }
-}
-
 // ---------------------------------------------------------------------------- host side
-struct Tiling { int bm, n_tiles_n, n_tiles_m, splits, k_tiles_per_split; };
+struct Tiling { int cg, bm, n_tiles_n, n_tiles, teams, sk_tiles, split, nd, nas, nxs, nws; };
 
-// Tile shape and split-K factor.  Few output tiles (small M and modest N) would leave most SMs
-// idle, so K is cut into `splits` ranges (multiples of 256 k) whose float partials are summed by
-// a small second kernel.
+// Tile shape, and how the tiles are dealt out.  The estimate is in tensor clocks (see the terms).
 inline Tiling choose_tiling(int M, int N, int K, int sm_count) {
-  Tiling t;
-  t.n_tiles_n = (N + BN - 1) / BN;
-  if (M < 256) {
-    t.bm = ((M + 31) / 32) * 32;
-  } else {
-    double best = -1.0;
-    t.bm = 256;
-    for (int bm : {256, 128}) {
-      const long long tiles = static_cast<long long>(t.n_tiles_n) * ((M + bm - 1) / bm);
-      const long long waves = (tiles + sm_count - 1) / sm_count;
-      const double fill = static_cast<double>(tiles) / static_cast<double>(waves * sm_count);
-      const double score = fill * (bm == 256 ? 1.0 : 0.8);
-      if (score > best) { best = score; t.bm = bm; }
+  const long long nk = K / BK, nst = (K + WK - 1) / WK;
+  Tiling best;
+  memset(&best, 0, sizeof(best));
+  double best_cost = 1e300;
+  const char* env_bm = getenv("LCQ_BM"); const char* env_cg = getenv("LCQ_CG"); const char* env_sp = getenv("LCQ_SPLIT"); const char* env_sk = getenv("LCQ_SK");
+  for (int cg = 1; cg <= 2; ++cg) {
+    if (env_cg && atoi(env_cg) != cg) continue;
+    const int P = sm_count / cg > 0 ? sm_count / cg : 1;
+    if (cg > sm_count) continue;
+    const int tn = (N + cg * BN - 1) / (cg * BN);
+    for (int bm = 32; bm <= (cg == 1 ? 128 : 256); bm += 32) {
+      const int tm = (M + bm - 1) / bm;
+      if (env_bm) { if (bm != atoi(env_bm)) continue; }
+      else if (bm > 32 && tm == (M + bm - 33) / (bm - 32)) continue;      // the same number of tiles fit a lower tile
+      const long long tiles = static_cast<long long>(tn) * tm;
+      Tiling t;
+      t.cg = cg; t.bm = bm; t.n_tiles_n = tn; t.n_tiles = static_cast<int>(tiles);
+      t.nd = bm <= 128 ? 2 : 1;
+      t.nas = bm <= 64 ? 3 : 2;
+      const int per_cta = bm / cg;                    // rows of x a CTA stages
+      t.nxs = per_cta <= 16 ? 6 : per_cta <= 32 ? 5 : per_cta <= 64 ? 3 : 2;
+      t.nws = (227 * 1024 - 1024 - t.nxs * x_stage_bytes(bm, cg)) / WS_STAGE;
+      if (t.nws > MAX_WS) t.nws = MAX_WS;
+      const double least = cg == 1 ? 330.0 : 400.0;
+      const double step = 2.0 * bm > least ? 2.0 * bm : least;
+      const double tile = nk * step + (t.nd == 1 ? 14.0 * bm : 0.0);
+      const auto consider = [&](long long teams, long long sk, int split, double cost) {
+        if (env_sp && atoi(env_sp) != split) return;
+        if (env_sk && (atoi(env_sk) != 0) != (sk != 0)) return;
+        if (cost < best_cost) {
+          best_cost = cost;
+          t.teams = static_cast<int>(teams); t.sk_tiles = static_cast<int>(sk); t.split = split;
+          best = t;
+        }
+      };
+      // whole tiles only
+      consider(tiles < P ? tiles : P, 0, 1, static_cast<double>((tiles + P - 1) / P) * tile);
+      const long long waves = tiles / P, rem = tiles % P;
+      if (waves == 0) {
+        // fewer tiles than SMs: a cluster per tile
+        for (int c = 2; c <= 8 && cg == 1; c *= 2) {
+          if (tiles * c > (c == 8 ? P * 7 / 8 : P) || c > nst) continue;
+          consider(tiles * c, 0, c, ((nst + c - 1) / c) * 4 * step + 1500);
+        }
+      } else if (rem != 0) {
+        const long long sk = rem * 3 >= P ? rem : rem + P;
+        const long long share = (sk * nst + P - 1) / P;
+        consider(P, sk, 1, static_cast<double>((tiles - sk) / P) * tile + share * 4 * step + 1500 + 15.0 * bm + 50.0 * bm);
+      }
     }
   }
-  t.n_tiles_m = (M + t.bm - 1) / t.bm;
-  const long long tiles = static_cast<long long>(t.n_tiles_n) * t.n_tiles_m;
-  const int w_stages = K / WK;                       // 256-k weight stages
-  t.splits = 1;
-  if (tiles * 2 <= sm_count && w_stages >= 2) {
-    int s = static_cast<int>(sm_count / tiles);
-    if (s > w_stages) s = w_stages;
-    if (s > 16) s = 16;
-    while (s > 1 && w_stages % s != 0) --s;            // equal ranges only
-    t.splits = s < 1 ? 1 : s;
-  }
-  t.k_tiles_per_split = (w_stages / t.splits) * (WK / BK);
-  return t;
+  return best;
 }
 
 inline bool supported(int M, int N, int K, int G, int x_dtype, int scale_dtype) {
-  return M >= 1 && N >= 1 && K >= WK && (K % WK) == 0 && G == 32 &&
+  return M >= 1 && N >= 1 && K >= BK && (K % BK) == 0 && G == 32 &&
          (x_dtype == LCQ_F16 || x_dtype == LCQ_BF16) && scale_dtype == LCQ_F16;
 }
 
 inline size_t x_copy_bytes(int M, int K, int x_dtype) {
   return x_dtype == LCQ_BF16 ? ((static_cast<size_t>(M) * K * 2 + 255) & ~static_cast<size_t>(255)) : 0;
 }
-// [shared counter region][fp16 copy of bf16 activations][split-K float partials]
+inline size_t partial_bytes(const Tiling& t) {
+  return t.sk_tiles ? static_cast<size_t>(t.teams) * 2 * t.cg * t.bm * BN * sizeof(float) : 0;
+}
+// [shared counter region][fp16 copy of bf16 activations][float partials of the tiles cut along K]
+inline size_t workspace_bytes(const Tiling& t, int M, int K, int x_dtype) {
+  const size_t scratch = x_copy_bytes(M, K, x_dtype) + partial_bytes(t);
+  return scratch ? kWorkspaceCounterBytes + scratch : 0;
+}
 inline size_t workspace_bytes(int M, int N, int K, int x_dtype, int sm_count = 148) {
-  const Tiling t = choose_tiling(M, N, K, sm_count);
-  const size_t part = t.splits > 1 ? static_cast<size_t>(t.splits) * M * N * sizeof(float) : 0;
-  const size_t xc = x_copy_bytes(M, K, x_dtype);
-  return (xc + part) ? kWorkspaceCounterBytes + xc + part : 0;
+  return workspace_bytes(choose_tiling(M, N, K, sm_count), M, K, x_dtype);
 }
 
-template <typename OT, bool PERM>
-int launch_t(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& ts, const Params& p, int grid,
-             size_t smem_bytes, cudaStream_t stream) {
-  auto kern = w4a16_gemm_kernel<OT, PERM>;
+inline void pdl_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int grid, int block, size_t smem, cudaStream_t stream) {
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+}
+
+template <int CG, typename OT, bool PERM, bool RAGGED>
+int launch_t(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& ts, const Params& p, cudaStream_t stream) {
+  auto kern = w4a16_gemm_kernel<CG, OT, PERM, RAGGED>;
   static thread_local int configured_device = -1;
   int dev = 0;
   LCQ_CUDA_TRY(cudaGetDevice(&dev));
@@ -480,22 +825,41 @@ int launch_t(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& ts
     LCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     configured_device = dev;
   }
-  kern<<<grid, NTHREADS, smem_bytes, stream>>>(tx, tw, ts, p);
-  LCQ_CUDA_TRY(cudaGetLastError());
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  pdl_launch_config(cfg, attr, CG * p.teams, NTHREADS, smem_map(p.bm, CG, p.nxs, p.nws).total, stream);
+  const int cluster = CG == 2 ? 2 : p.split;
+  if (cluster > 1) {
+    cudaLaunchAttribute& a = attr[cfg.numAttrs++];
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim.x = cluster;
+    a.val.clusterDim.y = 1;
+    a.val.clusterDim.z = 1;
+  }
+  LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tx, tw, ts, p));
   return LCQ_OK;
 }
+template <int CG, typename OT>
+int launch_by_kind(bool perm, bool ragged, const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& ts, const Params& p,
+                   cudaStream_t stream) {
+  if (perm) return ragged ? launch_t<CG, OT, true, true>(tx, tw, ts, p, stream) : launch_t<CG, OT, true, false>(tx, tw, ts, p, stream);
+  return ragged ? launch_t<CG, OT, false, true>(tx, tw, ts, p, stream) : launch_t<CG, OT, false, false>(tx, tw, ts, p, stream);
+}
+template <typename OT>
+int launch_by_team(int cg, bool perm, bool ragged, const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& ts, const Params& p,
+                   cudaStream_t stream) {
+  return cg == 2 ? launch_by_kind<2, OT>(perm, ragged, tx, tw, ts, p, stream) : launch_by_kind<1, OT>(perm, ragged, tx, tw, ts, p, stream);
+}
 
-template <bool PERM>
-int launch_by_out(int out_dtype, const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& ts, const Params& p,
-                  int grid, size_t smem_bytes, cudaStream_t stream) {
-  switch (out_dtype) {
-    case LCQ_F32: return launch_t<float, PERM>(tx, tw, ts, p, grid, smem_bytes, stream);
-    case LCQ_F16: return launch_t<__half, PERM>(tx, tw, ts, p, grid, smem_bytes, stream);
-    case LCQ_BF16: return launch_t<__nv_bfloat16, PERM>(tx, tw, ts, p, grid, smem_bytes, stream);
-    default: break;
-  }
-  set_error("w4a16 gemm: bad out_dtype %d", out_dtype);
-  return LCQ_ERR_BAD_ARG;
+inline Params make_params(const Tiling& t, int M, int N, int K) {
+  Params p;
+  memset(&p, 0, sizeof(p));
+  p.M = M; p.N = N; p.K = K;
+  p.bm = t.bm; p.n_tiles_n = t.n_tiles_n; p.n_tiles = t.n_tiles;
+  p.nst = (K + WK - 1) / WK;
+  p.teams = t.teams; p.sk_tiles = t.sk_tiles; p.split = t.split;
+  p.nxs = t.nxs; p.nws = t.nws; p.nas = t.nas; p.nd = t.nd;
+  return p;
 }
 
 inline int launch(const void* x, const void* w, const void* s, void* out, int M, int N, int K, int x_dtype,
@@ -505,65 +869,53 @@ inline int launch(const void* x, const void* w, const void* s, void* out, int M,
     return LCQ_ERR_BAD_ARG;
   }
   const Tiling t = choose_tiling(M, N, K, sm_count);
-  const size_t need = workspace_bytes(M, N, K, x_dtype, sm_count);
+  const size_t need = workspace_bytes(t, M, K, x_dtype);
   if (need && (workspace == nullptr || ws_bytes < need || !aligned(workspace, 256))) {
     set_error("w4a16 gemm: workspace of %zu bytes (256-byte aligned) required, got %zu", need, ws_bytes);
     return LCQ_ERR_WORKSPACE;
   }
   uint8_t* scratch = need ? static_cast<uint8_t*>(workspace) + kWorkspaceCounterBytes : nullptr;
+  const bool perm = x_dtype == LCQ_BF16, ragged = K % WK != 0;
   const void* xh = x;
   // kind::f16 wants both operands in one 16-bit format and the weight tiles must be fp16, so bf16
   // activations are converted once into the workspace.
-  if (x_dtype == LCQ_BF16) {
+  if (perm) {
     const long long n16 = static_cast<long long>(M) * K / 8;
     long long blocks = (n16 + 255) / 256;
     if (blocks > static_cast<long long>(sm_count) * 8) blocks = static_cast<long long>(sm_count) * 8;
-    bf16_to_f16_perm_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(static_cast<const uint4*>(x),
-                                                                          reinterpret_cast<uint4*>(scratch), n16);
-    LCQ_CUDA_TRY(cudaGetLastError());
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    pdl_launch_config(cfg, attr, static_cast<int>(blocks), 256, 0, stream);
+    LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, bf16_to_f16_perm_kernel, static_cast<const uint4*>(x), reinterpret_cast<uint4*>(scratch), n16));
     xh = scratch;
   }
-  float* partials = reinterpret_cast<float*>(scratch + x_copy_bytes(M, K, x_dtype));
-  Params p;
-  memset(&p, 0, sizeof(p));
-  p.M = M; p.N = N; p.K = K;
-  p.bm = t.bm; p.n_tiles_n = t.n_tiles_n; p.n_tiles_m = t.n_tiles_m;
-  p.splits = t.splits; p.k_tiles_per_split = t.k_tiles_per_split;
-  const int kernel_out_dtype = t.splits > 1 ? LCQ_F32 : out_dtype;
-  p.out = t.splits > 1 ? static_cast<void*>(partials) : out;
-  p.out_dtype = kernel_out_dtype;
-  {
-    const int vec = kernel_out_dtype == LCQ_F32 ? 4 : 8;
-    p.vec_store = (N % vec == 0) && aligned(p.out, 16) && ((static_cast<long long>(M) * N) % vec == 0);
-  }
-  const long long items = static_cast<long long>(p.n_tiles_n) * p.n_tiles_m * p.splits;
-  const int grid = static_cast<int>(items < sm_count ? items : sm_count);
+  Params p = make_params(t, M, N, K);
+  p.out = out;
+  p.scales = s;
+  p.counters = static_cast<int*>(workspace);
+  p.partials = reinterpret_cast<float*>(scratch + x_copy_bytes(M, K, x_dtype));
   CUtensorMap tx, tw, ts;
   int rc = encode_tmap_2d(&tx, 1, xh, static_cast<uint64_t>(K), static_cast<uint64_t>(M),
-                          static_cast<uint64_t>(K) * 2, BK, p.bm, 3);
+                          static_cast<uint64_t>(K) * 2, BK, p.bm / t.cg, 3);
   if (rc != LCQ_OK) return rc;
   rc = encode_tmap_2d(&tw, 0, w, static_cast<uint64_t>(K) / 2, static_cast<uint64_t>(N),
                       static_cast<uint64_t>(K) / 2, WK / 2, BN, 3);
   if (rc != LCQ_OK) return rc;
-  rc = encode_tmap_2d(&ts, 1, s, static_cast<uint64_t>(K) / 32, static_cast<uint64_t>(N),
-                      static_cast<uint64_t>(K) / 16, WK / 32, BN, 0);
-  if (rc != LCQ_OK) return rc;
-  const size_t smem_bytes = smem_map(p.bm).total;
-  const bool perm = (x_dtype == LCQ_BF16);   // the pre-pass already permuted k inside every 8-block
-  rc = perm ? launch_by_out<true>(kernel_out_dtype, tx, tw, ts, p, grid, smem_bytes, stream)
-            : launch_by_out<false>(kernel_out_dtype, tx, tw, ts, p, grid, smem_bytes, stream);
-  if (rc != LCQ_OK || t.splits == 1) return rc;
-  const long long n = static_cast<long long>(M) * N;
-  long long blocks = (n + 255) / 256;
-  if (blocks > static_cast<long long>(sm_count) * 8) blocks = static_cast<long long>(sm_count) * 8;
-  switch (out_dtype) {
-    case LCQ_F32: splitk_reduce_kernel<float><<<static_cast<int>(blocks), 256, 0, stream>>>(partials, static_cast<float*>(out), n, t.splits); break;
-    case LCQ_F16: splitk_reduce_kernel<__half><<<static_cast<int>(blocks), 256, 0, stream>>>(partials, static_cast<__half*>(out), n, t.splits); break;
-    case LCQ_BF16: splitk_reduce_kernel<__nv_bfloat16><<<static_cast<int>(blocks), 256, 0, stream>>>(partials, static_cast<__nv_bfloat16*>(out), n, t.splits); break;
-    default: set_error("w4a16 gemm: bad out_dtype %d", out_dtype); return LCQ_ERR_BAD_ARG;
+  if (ragged) {
+    memset(&ts, 0, sizeof(ts));
+  } else {
+    rc = encode_tmap_2d(&ts, 1, s, static_cast<uint64_t>(K) / 32, static_cast<uint64_t>(N),
+                        static_cast<uint64_t>(K) / 16, WK / 32, BN, 0);
+    if (rc != LCQ_OK) return rc;
   }
-  LCQ_CUDA_TRY(cudaGetLastError());
-  return LCQ_OK;
+  switch (out_dtype) {
+    case LCQ_F32: return launch_by_team<float>(t.cg, perm, ragged, tx, tw, ts, p, stream);
+    case LCQ_F16: return launch_by_team<__half>(t.cg, perm, ragged, tx, tw, ts, p, stream);
+    case LCQ_BF16: return launch_by_team<__nv_bfloat16>(t.cg, perm, ragged, tx, tw, ts, p, stream);
+    default: break;
+  }
+  set_error("w4a16 gemm: bad out_dtype %d", out_dtype);
+  return LCQ_ERR_BAD_ARG;
 }
 
 }  // namespace gemm_tc

@@ -271,7 +271,7 @@ static int matmul_entry(int wbits, const void* x, const void* w, const void* s, 
       }
     case LCQ_ALGO_GEMM_TC:
       if (wbits != 4 || !gemm_tc::supported(M, N, K, G, x_dtype, scale_dtype)) {
-        set_error("GEMM_TC needs int4, group_size 32, K %% 256 == 0, f16 scales, f16/bf16 x");
+        set_error("GEMM_TC needs int4, group_size 32, K %% 64 == 0, f16 scales, f16/bf16 x");
         return LCQ_ERR_UNSUPPORTED;
       }
       return gemm_tc::launch(x, w, s, out, M, N, K, x_dtype, out_dtype, workspace, workspace_bytes, di.sm_count, st);
@@ -440,6 +440,56 @@ int lcq_gemv_tc_plan_cluster(int M, int N, int K, int sm_count) {
     return LCQ_ERR_UNSUPPORTED;
   }
   return gemv_tc::make_plan(M, N, K, sm_count).p.cluster;
+}
+
+int lcq_gemm_tc_plan_check(int M, int N, int K, int sm_count, int* fields) {
+  if (!gemm_tc::supported(M, N, K, 32, LCQ_F16, LCQ_F16) || sm_count < 1) {
+    set_error("plan check: problem not covered by GEMM_TC");
+    return LCQ_ERR_UNSUPPORTED;
+  }
+  const gemm_tc::Tiling t = gemm_tc::choose_tiling(M, N, K, sm_count);
+  const gemm_tc::Params p = gemm_tc::make_params(t, M, N, K);
+  const int smem = gemm_tc::smem_map(t.bm, t.cg, t.nxs, t.nws).total;
+  if (fields) {
+    fields[0] = t.teams * t.cg; fields[1] = t.bm; fields[2] = t.n_tiles; fields[3] = t.sk_tiles; fields[4] = smem; fields[5] = t.cg; fields[6] = t.split;
+  }
+  if (t.teams < 1 || t.teams * t.cg > sm_count || (t.split > 1 && (t.cg != 1 || t.teams != t.n_tiles * t.split || t.split > 8)) ||
+      t.bm % 32 != 0 || t.bm < 32 || t.bm > (t.cg == 2 ? 256 : 128) || smem > 227 * 1024 || t.nxs < 2 || t.nws < 2 ||
+      t.nxs > gemm_tc::MAX_XS || t.nws > gemm_tc::MAX_WS || t.nas > gemm_tc::MAX_AS ||
+      t.nd * t.bm + t.nas * gemm_tc::A_SLOT_COLS > gemm_tc::TMEM_COLS ||
+      static_cast<size_t>(t.sk_tiles) * t.cg * sizeof(int) > kWorkspaceCounterBytes) {
+    set_error("plan check: bad tiling (teams %d, bm %d, %d bytes of shared memory)", t.teams, t.bm, smem);
+    return LCQ_ERR_BAD_ARG;
+  }
+  // Replay the device-side schedule: every (tile, weight stage) exactly once, partials in slots of
+  // their own, contributors as the kernel counts them.
+  std::vector<int> seen(static_cast<size_t>(t.n_tiles) * p.nst, 0);
+  std::vector<int> slot_of(static_cast<size_t>(2) * t.teams, -1);
+  std::vector<int> contributors(t.n_tiles, 0);
+  for (int team = 0; team < t.teams; ++team) {
+    for (gemm_tc::Walk w(p, team); w.next(p);) {
+      if (w.tile < 0 || w.tile >= t.n_tiles || w.st0 < 0 || w.st0 >= w.st1 || w.st1 > p.nst) { set_error("plan check: segment out of range"); return LCQ_ERR_BAD_ARG; }
+      for (int st = w.st0; st < w.st1; ++st) seen[static_cast<size_t>(w.tile) * p.nst + st]++;
+      contributors[w.tile]++;
+      if ((w.st0 == 0 && w.st1 == p.nst) || t.split > 1) continue;
+      const unsigned t0 = static_cast<unsigned>(w.tile) * static_cast<unsigned>(p.nst);
+      const int slot1 = team == gemm_tc::share_owner(p, t0) && gemm_tc::share_begin(p, team) < t0;     // as the kernel's part()
+      int& owner = slot_of[2 * team + slot1];
+      if (w.tile >= t.sk_tiles || owner >= 0) { set_error("plan check: tile %d has no slot of its own", w.tile); return LCQ_ERR_BAD_ARG; }
+      owner = w.tile;
+    }
+  }
+  for (size_t i = 0; i < seen.size(); ++i)
+    if (seen[i] != 1) { set_error("plan check: stage %zu covered %d times", i, seen[i]); return LCQ_ERR_BAD_ARG; }
+  for (int tile = 0; tile < t.n_tiles; ++tile) {
+    int expect = t.split;
+    if (tile < t.sk_tiles) {
+      const unsigned t0 = static_cast<unsigned>(tile) * static_cast<unsigned>(p.nst);
+      expect = gemm_tc::share_owner(p, t0 + p.nst - 1) - gemm_tc::share_owner(p, t0) + 1;
+    }
+    if (contributors[tile] != expect) { set_error("plan check: tile %d has %d contributors, the kernel expects %d", tile, contributors[tile], expect); return LCQ_ERR_BAD_ARG; }
+  }
+  return LCQ_OK;
 }
 
 // ---------------------------------------------------------------- allocation-free decode entry

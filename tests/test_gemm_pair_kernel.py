@@ -1,0 +1,53 @@
+"""The tcgen05 kernel on single SMs and SM pairs at the edges of its tiles and of its dispatch: rows of x
+around the tile heights, weight rows around 128 and 256, K that is no whole number of 256-k stages,
+tiles cut along K between CTAs.
+
+Bound: each dequantised weight is rounded once to fp16 (relative error <= 2^-11), products are exact in
+float32 and summed over K <= 4096 with float32 rounding; |err| <= 2^-11 * sum_k |x w| + 2^-12 * the same
+covers both, and the fp16 / bf16 output adds half an ulp of the result (2^-11 / 2^-8 relative).
+"""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import locomp_b200 as L
+from locomp_b200 import _lib
+from oracle import qmm_oracle as O
+
+
+def test_plan_covers_every_stage_once():
+    lib, f = _lib.lib(), (ctypes.c_int * 7)()
+    for m in (1, 17, 32, 33, 64, 100, 192, 193, 256, 512, 1000, 2048, 8192):
+        for n in (1, 100, 256, 257, 1024, 4096, 14336, 28672):
+            for k in (64, 256, 320, 576, 4096, 14336):
+                for sms in (148, 132, 7, 1):
+                    assert lib.lcq_gemm_tc_plan_check(m, n, k, sms, f) == 0, (m, n, k, sms, lib.lcq_last_error())
+    assert lib.lcq_gemm_tc_plan_check(64, 100, 96, 148, f) == _lib.ERR_UNSUPPORTED
+
+
+CASES = [(17, 1, 64), (17, 257, 320), (31, 255, 256), (32, 256, 576), (33, 513, 1984), (64, 300, 4096), (96, 1000, 832),
+         (128, 129, 4096), (160, 640, 1024), (161, 128, 768), (193, 700, 512), (224, 256, 2048), (250, 384, 448), (257, 2000, 1088),
+         (40, 30000, 512), (300, 20000, 320), (1000, 4000, 512), (520, 9600, 1024)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k", CASES)
+def test_against_oracle(m, n, k, kind):
+    rng = np.random.default_rng(m * 31 + n + k)
+    wp, s = O.make_w4(rng, n, k, 32, np.float16)
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).to(kind)
+    wd, sd = torch.from_numpy(wp).cuda(), torch.from_numpy(s).cuda()
+    w = O.dequant_int4(wp, s, 32).astype(np.float64)
+    x64 = x.double().numpy()
+    ref, mag = x64 @ w.T, np.abs(x64) @ np.abs(w).T
+    bound = (2.0 ** -11 + 2.0 ** -12) * mag
+    y = L.quantized_matmul(x.cuda(), wd, sd, 32, algo="gemm_tc", out_dtype="f32")
+    assert np.all(np.abs(y.double().cpu().numpy() - ref) <= bound)
+    z = L.quantized_matmul(x.cuda(), wd, sd, 32, algo="gemm_tc")
+    ulp = 2.0 ** -11 if kind == torch.float16 else 2.0 ** -8
+    assert np.all(np.abs(z.double().cpu().numpy() - ref) <= bound + ulp * np.abs(ref))
+    assert torch.equal(L.quantized_matmul(x.cuda(), wd, sd, 32, algo="gemm_tc"), z)     # fixed order of summation
+    assert _lib.lib().lcq_check_device_status(None) == 0, _lib.lib().lcq_last_error()

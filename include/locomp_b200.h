@@ -294,7 +294,7 @@ int lcq_gemv_tc_plan_cluster(int M, int N, int K, int sm_count);
  * (tile, 256-k weight stage) exactly once, partials of tiles cut along K in slots of their own,
  * contributor counts) and checks its shared-memory and tensor-memory budgets.  fields (may be NULL)
  * receives {CTAs, tile rows of x, tiles, tiles cut along K, shared-memory bytes, CTAs per MMA, CTAs per cluster
- * that share a tile's K}.
+ * that share a tile's K, pieces per tile of the last wave}.
  */
 int lcq_gemm_tc_plan_check(int M, int N, int K, int sm_count, int* fields);
 

@@ -161,6 +161,7 @@ struct Params {
   int nst;              // 256-k weight stages per tile
   int teams;            // CTAs (CG = 1) or pairs (CG = 2) launched
   int sk_tiles;         // tiles 0 .. sk_tiles-1 are cut along K, the others go whole to team (tile - sk_tiles) % teams
+  int full, tail;       // tiles full .. are cut into `tail` pieces of bm / tail rows of x (a last wave that would be mostly empty)
   int split;            // > 1: a cluster of `split` teams per tile, each with its share of K (no whole tiles, no scratch)
   int nxs, nws;         // ring depths: X stages, weight stages
   int nas;              // TMEM A slots
@@ -180,19 +181,20 @@ __host__ __device__ inline int share_owner(const Params& p, unsigned unit) {
 // The segments of one team: (tile, stages st0 .. st1-1).  Every role walks them in the same order.
 struct Walk {
   unsigned u, u1;       // what is left of the team's share of the cut tiles
-  int next_tile;        // then the whole tiles
+  int next_item;        // then the whole tiles and the pieces of the last ones
   int tile, st0, st1;
+  int m0, bm;           // first row of x and their number
   __host__ __device__ Walk(const Params& p, int team) {
     if (p.split > 1) {
       const int t = team / p.split, r = team - t * p.split;
       u = static_cast<unsigned>(t * p.nst + p.nst * r / p.split);
       u1 = static_cast<unsigned>(t * p.nst + p.nst * (r + 1) / p.split);
-      next_tile = p.n_tiles;
+      next_item = p.n_tiles;
       return;
     }
     u = share_begin(p, team);
     u1 = share_begin(p, team + 1);
-    next_tile = p.sk_tiles + team;
+    next_item = p.sk_tiles + team;
   }
   __host__ __device__ bool next(const Params& p) {
     if (u < u1) {
@@ -202,14 +204,27 @@ struct Walk {
       const unsigned take = left < in_tile ? left : in_tile;
       st1 = st0 + static_cast<int>(take);
       u += take;
+      m0 = (tile / p.n_tiles_n) * p.bm;
+      bm = p.bm;
       return true;
     }
-    if (next_tile >= p.n_tiles) return false;
-    tile = next_tile;
-    next_tile += p.teams;
     st0 = 0;
     st1 = p.nst;
-    return true;
+    for (;;) {
+      tile = next_item;
+      bm = p.bm;
+      int piece = 0;
+      if (tile >= p.full) {
+        const int i = tile - p.full;
+        tile = p.full + i / p.tail;
+        piece = i - (tile - p.full) * p.tail;
+        bm = p.bm / p.tail;
+      }
+      if (tile >= p.n_tiles) return false;
+      next_item += p.teams;
+      m0 = (tile / p.n_tiles_n) * p.bm + piece * bm;
+      if (m0 < p.M) return true;              // (a piece below the last row of x is no work)
+    }
   }
 };
 
@@ -383,8 +398,9 @@ __device__ __noinline__ void finish_tile(uint32_t d_t, OT* out, int rows_out, in
 // memory, a stage ahead.
 template <int CG, typename OT, bool PERM, bool RAGGED>
 __global__ void __launch_bounds__(NTHREADS, 1)
-w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
-                  const __grid_constant__ CUtensorMap tmap_s, const __grid_constant__ Params p) {
+w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_piece,
+                  const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
+                  const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const Smem L = smem_map(p.bm, CG, p.nxs, p.nws);
   uint64_t* full_x = reinterpret_cast<uint64_t*>(smem + L.bars);
@@ -446,20 +462,22 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     if (lane == 0) {
       tma_prefetch_desc(&tmap_x);
       griddep_wait();                    // x is the preceding kernel's output
-      const int half = p.bm / CG, bytes = x_step_bytes(p.bm, CG);
+      const int stage_bytes = x_stage_bytes(p.bm, CG);
       Ring r = {0, 0};
       bool ok = true;
       for (Walk w(p, team); ok && w.next(p);) {
-        const int m0 = (w.tile / p.n_tiles_n) * p.bm + static_cast<int>(crank) * half;
+        const int rows = w.bm / CG, bytes = x_step_bytes(w.bm, CG);
+        const int m0 = w.m0 + static_cast<int>(crank) * rows;
+        const CUtensorMap* tmap = w.bm == p.bm ? &tmap_x : &tmap_piece;
         for (int st = w.st0; st < w.st1; ++st, r.step(p.nxs)) {
           const int steps = RAGGED && nk - st * 4 < 4 ? nk - st * 4 : 4;
           if (!wait_bar(flag_abort, &empty_x[r.i], r.phase ^ 1u)) { LCQ_GIVE_UP(11); ok = false; break; }
           if (crank == 0) mbar_expect_tx(&full_x[r.i], CG * steps * bytes);
           const uint32_t bar = leader_addr<CG>(full_x + r.i);
-          uint8_t* dst = smem + r.i * (4 * bytes);
+          uint8_t* dst = smem + r.i * stage_bytes;
           for (int j = 0; j < steps; ++j) {
-            if (CG == 2) tma_load_2d_pair(dst + j * bytes, &tmap_x, bar, (st * 4 + j) * BK, m0);
-            else tma_load_2d(dst + j * bytes, &tmap_x, full_x + r.i, (st * 4 + j) * BK, m0);
+            if (CG == 2) tma_load_2d_pair(dst + j * bytes, tmap, bar, (st * 4 + j) * BK, m0);
+            else tma_load_2d(dst + j * bytes, tmap, full_x + r.i, (st * 4 + j) * BK, m0);
           }
         }
       }
@@ -467,14 +485,15 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   } else if (warp == WARP_MMA) {
     // ------------------------------------------------------------ MMA issuer: one warp for the team
     if (crank == 0) {
-      const uint32_t idesc = make_idesc(p.bm, CG);
-      const uint64_t desc0 = make_b_desc(smem_u32(smem));
-      const uint64_t desc_step = static_cast<uint64_t>(x_step_bytes(p.bm, CG) >> 4);      // descriptors count 16-byte units
+      const uint64_t desc0 = make_b_desc(smem_u32(smem));                                 // descriptors count 16-byte units
+      const uint64_t desc_stage = static_cast<uint64_t>(x_stage_bytes(p.bm, CG) >> 4);
       Ring rx = {0, 0}, ra = {0, 0}, rd = {0, 0};
       bool ok = true;
       for (Walk w(p, team); ok && w.next(p); rd.step(p.nd)) {
         if (!warp_wait(flag_abort, &empty_d[rd.i], rd.phase ^ 1u)) { if (lane == 0) LCQ_GIVE_UP(12); ok = false; break; }
         tc_fence_after();
+        const uint32_t idesc = make_idesc(w.bm, CG);
+        const uint64_t desc_step = static_cast<uint64_t>(x_step_bytes(w.bm, CG) >> 4);
         const uint32_t d_t = tmem_base + rd.i * p.bm;
         uint32_t acc = 0;
         for (int st = w.st0; st < w.st1; ++st, rx.step(p.nxs), ra.step(p.nas)) {
@@ -485,7 +504,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             break;
           }
           tc_fence_after();
-          uint64_t bdesc = desc0 + rx.i * (desc_step * 4);
+          uint64_t bdesc = desc0 + rx.i * desc_stage;
           uint32_t a_t = a_base + ra.i * A_SLOT_COLS;
           for (int k = 0; k < steps; ++k, bdesc += desc_step, a_t += A_STEP_COLS) {
 #pragma unroll
@@ -580,12 +599,11 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const long long part_elems = static_cast<long long>(p.bm) * BN;
     Ring rd = {0, 0};
     for (Walk w(p, team); w.next(p); rd.step(p.nd)) {
-      const int m0 = (w.tile / p.n_tiles_n) * p.bm;
       const int n = (w.tile % p.n_tiles_n) * (CG * BN) + static_cast<int>(crank) * BN + r;
       const uint32_t d_t = lane_taddr + rd.i * p.bm;
-      int rows = p.M - m0;                     // rows of out in this tile
-      if (rows > p.bm) rows = p.bm;
-      OT* out = static_cast<OT*>(p.out) + static_cast<long long>(m0) * p.N + n;
+      int rows = p.M - w.m0;                   // rows of out in this tile
+      if (rows > w.bm) rows = w.bm;
+      OT* out = static_cast<OT*>(p.out) + static_cast<long long>(w.m0) * p.N + n;
       // one verdict for the four warps: they meet at named barriers below
       if (!all_epilogue_warps(wait_bar(flag_abort, &full_d[rd.i], rd.phase))) { if (lane == 0) LCQ_GIVE_UP(17); break; }
       tc_fence_after();
@@ -661,36 +679,37 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     // One tile per cluster, its K shared out: CTA d settles columns d * cw .. of the tile.  Every CTA sends
     // each of the others its part of their columns (distributed shared memory, into the rings, which
     // nobody uses any more), and adds up what it got in rank order.
-    const int me = team % p.split, tile = team / p.split, cw = p.bm / p.split;
+    // The twenty dequant and epilogue warps each take 16 columns at a time.
+    const int me = team % p.split, tile = team / p.split, cw = (p.bm + p.split - 1) / p.split;
     const int m0 = (tile / p.n_tiles_n) * p.bm;
     const int rows = p.M - m0 < p.bm ? p.M - m0 : p.bm;
-    const int r = (warp - WARP_EPI0) * 32 + lane;
-    const bool epilogue = warp >= WARP_EPI0 && warp < WARP_W;
+    const int r = (warp & 3) * 32 + lane;
     cluster_barrier();
-    if (epilogue) {
+    if (warp < WARP_W) {
       tc_fence_after();
-      int d = 0, j = 0;
       const uint32_t mine = smem_u32(smem) + (me * cw * BN + r) * 4;
-      uint32_t dst = peer_addr(mine, 0);
-      for (int c0 = 0; c0 < rows; c0 += 16) {
+      for (int c0 = (warp >> 2) * 16; c0 < rows; c0 += (WARP_W / 4) * 16) {
         uint32_t v[16];
-        tmem_ld16(tmem_base + (static_cast<uint32_t>((warp - WARP_EPI0) * 32) << 16) + c0, v);
+        tmem_ld16(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c0, v);
         tmem_wait_ld();
+        int d = c0 / cw, j = c0 - d * cw;
+        uint32_t dst = peer_addr(mine + j * (BN * 4), d);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst), "r"(v[i]) : "memory");
+          if (c0 + i < rows) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst), "r"(v[i]) : "memory");
           dst += BN * 4;
-          if (++j == cw) { j = 0; ++d; dst = peer_addr(mine, d < p.split ? d : 0); }
+          if (++j == cw && d + 1 < p.split) { j = 0; ++d; dst = peer_addr(mine, d); }
         }
       }
       tc_fence_before();
     }
     cluster_barrier();
     const int n = (tile % p.n_tiles_n) * BN + r;
-    if (epilogue && n < p.N) {
+    if (warp < WARP_W && n < p.N) {
       const float* got = reinterpret_cast<const float*>(smem) + r;
       OT* out = static_cast<OT*>(p.out) + static_cast<long long>(m0 + me * cw) * p.N + n;
-      for (int j = 0; j < cw && me * cw + j < rows; ++j) {
+#pragma unroll 2
+      for (int j = warp >> 2; j < cw && me * cw + j < rows; j += WARP_W / 4) {
         float sum = 0.0f;
         for (int q = 0; q < p.split; ++q) sum += got[(q * cw + j) * BN];
         out[static_cast<long long>(j) * p.N] = from_f32<OT>(sum);
@@ -725,24 +744,29 @@ __global__ void __launch_bounds__(256) bf16_to_f16_perm_kernel(const uint4* __re
 }
 
 // ---------------------------------------------------------------------------- host side
-struct Tiling { int cg, bm, n_tiles_n, n_tiles, teams, sk_tiles, split, nd, nas, nxs, nws; };
+struct Tiling { int cg, bm, n_tiles_n, n_tiles, teams, sk_tiles, full, tail, split, nd, nas, nxs, nws; };
 
-// Tile shape, and how the tiles are dealt out.  The estimate is in tensor clocks (see the terms).
+// Microseconds of a 64-k step of a tile, measured at K = 8192: with few teams at work the hand-over of the
+// weights through TMEM and the MMAs bound it; with all SMs busy (`used` = 1) L2 and power add to that.
+inline double step_us(int cg, int bm, double used) {
+  const double alone = 0.145 + 0.0005 * bm;
+  const double busy = cg == 1 ? 0.145 + 0.00117 * bm : bm <= 128 ? 0.152 + 0.00088 * bm : 0.150 + 0.00100 * bm;
+  const double f = used <= 0.5 ? 0.0 : used >= 1.0 ? 1.0 : 2.0 * used - 1.0;
+  return alone + (busy - alone) * f;
+}
+
+// Tile shape, and how the tiles are dealt out: the cheapest of a few forms by that estimate.
 inline Tiling choose_tiling(int M, int N, int K, int sm_count) {
-  const long long nk = K / BK, nst = (K + WK - 1) / WK;
+  const int nk = K / BK, nst = (K + WK - 1) / WK;
   Tiling best;
   memset(&best, 0, sizeof(best));
   double best_cost = 1e300;
-  const char* env_bm = getenv("LCQ_BM"); const char* env_cg = getenv("LCQ_CG"); const char* env_sp = getenv("LCQ_SPLIT"); const char* env_sk = getenv("LCQ_SK");
-  for (int cg = 1; cg <= 2; ++cg) {
-    if (env_cg && atoi(env_cg) != cg) continue;
-    const int P = sm_count / cg > 0 ? sm_count / cg : 1;
-    if (cg > sm_count) continue;
+  for (int cg = 1; cg <= 2 && cg <= sm_count; ++cg) {
+    const int P = sm_count / cg;
     const int tn = (N + cg * BN - 1) / (cg * BN);
     for (int bm = 32; bm <= (cg == 1 ? 128 : 256); bm += 32) {
       const int tm = (M + bm - 1) / bm;
-      if (env_bm) { if (bm != atoi(env_bm)) continue; }
-      else if (bm > 32 && tm == (M + bm - 33) / (bm - 32)) continue;      // the same number of tiles fit a lower tile
+      if (bm > 32 && tm == (M + bm - 33) / (bm - 32)) continue;      // the same number of tiles fit a lower tile
       const long long tiles = static_cast<long long>(tn) * tm;
       Tiling t;
       t.cg = cg; t.bm = bm; t.n_tiles_n = tn; t.n_tiles = static_cast<int>(tiles);
@@ -752,31 +776,43 @@ inline Tiling choose_tiling(int M, int N, int K, int sm_count) {
       t.nxs = per_cta <= 16 ? 6 : per_cta <= 32 ? 5 : per_cta <= 64 ? 3 : 2;
       t.nws = (227 * 1024 - 1024 - t.nxs * x_stage_bytes(bm, cg)) / WS_STAGE;
       if (t.nws > MAX_WS) t.nws = MAX_WS;
-      const double least = cg == 1 ? 330.0 : 400.0;
-      const double step = 2.0 * bm > least ? 2.0 * bm : least;
-      const double tile = nk * step + (t.nd == 1 ? 14.0 * bm : 0.0);
-      const auto consider = [&](long long teams, long long sk, int split, double cost) {
-        if (env_sp && atoi(env_sp) != split) return;
-        if (env_sk && (atoi(env_sk) != 0) != (sk != 0)) return;
-        if (cost < best_cost) {
-          best_cost = cost;
-          t.teams = static_cast<int>(teams); t.sk_tiles = static_cast<int>(sk); t.split = split;
-          best = t;
-        }
+      const auto consider = [&](long long teams, long long sk, long long full, int tail, int split, double cost) {
+        if (cost >= best_cost) return;
+        best_cost = cost;
+        t.teams = static_cast<int>(teams); t.sk_tiles = static_cast<int>(sk); t.split = split;
+        t.full = static_cast<int>(full); t.tail = tail;
+        best = t;
       };
-      // whole tiles only
-      consider(tiles < P ? tiles : P, 0, 1, static_cast<double>((tiles + P - 1) / P) * tile);
+      const auto step = [&](int rows, double teams) { return step_us(cg, rows, teams / P); };
+      const double start = cg == 1 ? 4.5 : 5.5, epilogue = t.nd == 1 ? 0.0075 * bm : 0.0;   // one accumulator: its epilogue shows
       const long long waves = tiles / P, rem = tiles % P;
+      const double full_waves = static_cast<double>(waves) * (nk * step(bm, P) + epilogue);
+      // whole tiles
+      consider(tiles < P ? tiles : P, 0, tiles, 1, 1, start + full_waves + (rem ? nk * step(bm, static_cast<double>(rem)) + epilogue : 0.0));
+      if (rem == 0) continue;
+      // the tiles of the last wave in pieces of fewer rows of x
+      for (int tail = 2; tail <= 8; tail *= 2) {
+        const int piece = bm / tail;
+        if (piece < 32 || piece % 16 != 0 || piece * tail != bm) continue;
+        const long long pieces = rem * tail, last = (pieces + P - 1) / P;
+        consider(waves == 0 && pieces < P ? pieces : P, 0, tiles - rem, tail, 1,
+                 start + full_waves + last * nk * step(piece, static_cast<double>(pieces) / last) + 0.5);
+      }
+      if (cg == 2) continue;
       if (waves == 0) {
-        // fewer tiles than SMs: a cluster per tile
-        for (int c = 2; c <= 8 && cg == 1; c *= 2) {
-          if (tiles * c > (c == 8 ? P * 7 / 8 : P) || c > nst) continue;
-          consider(tiles * c, 0, c, ((nst + c - 1) / c) * 4 * step + 1500);
+        // fewer tiles than SMs: a cluster per tile.  Clusters pack the ~16 SMs that are sure of each GPC
+        // (18 SMs on average); more of them than fit at once take turns, at twice the time.
+        for (int c = 2; c <= 6 && c <= nst; ++c) {
+          if (tiles > static_cast<long long>(sm_count / 18) * (16 / c)) continue;
+          consider(tiles * c, 0, tiles, 1, c, start + ((nst + c - 1) / c) * 4 * step(bm, static_cast<double>(tiles * c)) + 2.5);
         }
-      } else if (rem != 0) {
+      } else {
+        // equal shares of K for what does not fill all SMs, with a wave of whole tiles added when the shares
+        // would be short (each contributor costs the one who adds up a round trip per 16 rows)
         const long long sk = rem * 3 >= P ? rem : rem + P;
         const long long share = (sk * nst + P - 1) / P;
-        consider(P, sk, 1, static_cast<double>((tiles - sk) / P) * tile + share * 4 * step + 1500 + 15.0 * bm + 50.0 * bm);
+        consider(P, sk, tiles, 1, 1, start + static_cast<double>((tiles - sk) / P) * (nk * step(bm, P) + epilogue) +
+                                         share * 4 * step(bm, P) + (sk == rem ? 2.0 : 6.0));
       }
     }
   }
@@ -816,7 +852,7 @@ inline void pdl_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr
 }
 
 template <int CG, typename OT, bool PERM, bool RAGGED>
-int launch_t(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& ts, const Params& p, cudaStream_t stream) {
+int launch_t(const CUtensorMap* tm, const Params& p, cudaStream_t stream) {
   auto kern = w4a16_gemm_kernel<CG, OT, PERM, RAGGED>;
   static thread_local int configured_device = -1;
   int dev = 0;
@@ -836,19 +872,19 @@ int launch_t(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& ts
     a.val.clusterDim.y = 1;
     a.val.clusterDim.z = 1;
   }
-  LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tx, tw, ts, p));
+  LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], p));
   return LCQ_OK;
 }
 template <int CG, typename OT>
-int launch_by_kind(bool perm, bool ragged, const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& ts, const Params& p,
+int launch_by_kind(bool perm, bool ragged, const CUtensorMap* tm, const Params& p,
                    cudaStream_t stream) {
-  if (perm) return ragged ? launch_t<CG, OT, true, true>(tx, tw, ts, p, stream) : launch_t<CG, OT, true, false>(tx, tw, ts, p, stream);
-  return ragged ? launch_t<CG, OT, false, true>(tx, tw, ts, p, stream) : launch_t<CG, OT, false, false>(tx, tw, ts, p, stream);
+  if (perm) return ragged ? launch_t<CG, OT, true, true>(tm, p, stream) : launch_t<CG, OT, true, false>(tm, p, stream);
+  return ragged ? launch_t<CG, OT, false, true>(tm, p, stream) : launch_t<CG, OT, false, false>(tm, p, stream);
 }
 template <typename OT>
-int launch_by_team(int cg, bool perm, bool ragged, const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& ts, const Params& p,
+int launch_by_team(int cg, bool perm, bool ragged, const CUtensorMap* tm, const Params& p,
                    cudaStream_t stream) {
-  return cg == 2 ? launch_by_kind<2, OT>(perm, ragged, tx, tw, ts, p, stream) : launch_by_kind<1, OT>(perm, ragged, tx, tw, ts, p, stream);
+  return cg == 2 ? launch_by_kind<2, OT>(perm, ragged, tm, p, stream) : launch_by_kind<1, OT>(perm, ragged, tm, p, stream);
 }
 
 inline Params make_params(const Tiling& t, int M, int N, int K) {
@@ -857,7 +893,7 @@ inline Params make_params(const Tiling& t, int M, int N, int K) {
   p.M = M; p.N = N; p.K = K;
   p.bm = t.bm; p.n_tiles_n = t.n_tiles_n; p.n_tiles = t.n_tiles;
   p.nst = (K + WK - 1) / WK;
-  p.teams = t.teams; p.sk_tiles = t.sk_tiles; p.split = t.split;
+  p.teams = t.teams; p.sk_tiles = t.sk_tiles; p.full = t.full; p.tail = t.tail; p.split = t.split;
   p.nxs = t.nxs; p.nws = t.nws; p.nas = t.nas; p.nd = t.nd;
   return p;
 }
@@ -894,24 +930,19 @@ inline int launch(const void* x, const void* w, const void* s, void* out, int M,
   p.scales = s;
   p.counters = static_cast<int*>(workspace);
   p.partials = reinterpret_cast<float*>(scratch + x_copy_bytes(M, K, x_dtype));
-  CUtensorMap tx, tw, ts;
-  int rc = encode_tmap_2d(&tx, 1, xh, static_cast<uint64_t>(K), static_cast<uint64_t>(M),
-                          static_cast<uint64_t>(K) * 2, BK, p.bm / t.cg, 3);
+  CUtensorMap tm[4];    // x in whole tiles, x in pieces of a tile, weights, scales
+  const uint64_t k64 = static_cast<uint64_t>(K), m64 = static_cast<uint64_t>(M), n64 = static_cast<uint64_t>(N);
+  int rc = encode_tmap_2d(&tm[0], 1, xh, k64, m64, k64 * 2, BK, p.bm / t.cg, 3);
   if (rc != LCQ_OK) return rc;
-  rc = encode_tmap_2d(&tw, 0, w, static_cast<uint64_t>(K) / 2, static_cast<uint64_t>(N),
-                      static_cast<uint64_t>(K) / 2, WK / 2, BN, 3);
-  if (rc != LCQ_OK) return rc;
-  if (ragged) {
-    memset(&ts, 0, sizeof(ts));
-  } else {
-    rc = encode_tmap_2d(&ts, 1, s, static_cast<uint64_t>(K) / 32, static_cast<uint64_t>(N),
-                        static_cast<uint64_t>(K) / 16, WK / 32, BN, 0);
-    if (rc != LCQ_OK) return rc;
-  }
+  if (t.tail == 1) tm[1] = tm[0];
+  else if ((rc = encode_tmap_2d(&tm[1], 1, xh, k64, m64, k64 * 2, BK, p.bm / t.tail / t.cg, 3)) != LCQ_OK) return rc;
+  if ((rc = encode_tmap_2d(&tm[2], 0, w, k64 / 2, n64, k64 / 2, WK / 2, BN, 3)) != LCQ_OK) return rc;
+  if (ragged) tm[3] = tm[2];                     // not used
+  else if ((rc = encode_tmap_2d(&tm[3], 1, s, k64 / 32, n64, k64 / 16, WK / 32, BN, 0)) != LCQ_OK) return rc;
   switch (out_dtype) {
-    case LCQ_F32: return launch_by_team<float>(t.cg, perm, ragged, tx, tw, ts, p, stream);
-    case LCQ_F16: return launch_by_team<__half>(t.cg, perm, ragged, tx, tw, ts, p, stream);
-    case LCQ_BF16: return launch_by_team<__nv_bfloat16>(t.cg, perm, ragged, tx, tw, ts, p, stream);
+    case LCQ_F32: return launch_by_team<float>(t.cg, perm, ragged, tm, p, stream);
+    case LCQ_F16: return launch_by_team<__half>(t.cg, perm, ragged, tm, p, stream);
+    case LCQ_BF16: return launch_by_team<__nv_bfloat16>(t.cg, perm, ragged, tm, p, stream);
     default: break;
   }
   set_error("w4a16 gemm: bad out_dtype %d", out_dtype);

@@ -449,9 +449,9 @@ int lcq_gemm_tc_plan_check(int M, int N, int K, int sm_count, int* fields) {
   }
   const gemm_tc::Tiling t = gemm_tc::choose_tiling(M, N, K, sm_count);
   const gemm_tc::Params p = gemm_tc::make_params(t, M, N, K);
-  const int smem = gemm_tc::smem_map(t.bm, t.cg, t.nxs, t.nws).total;
+  const int smem = t.teams < 1 ? 0 : gemm_tc::smem_map(t.bm, t.cg, t.nxs, t.nws).total;
   if (fields) {
-    fields[0] = t.teams * t.cg; fields[1] = t.bm; fields[2] = t.n_tiles; fields[3] = t.sk_tiles; fields[4] = smem; fields[5] = t.cg; fields[6] = t.split;
+    fields[0] = t.teams * t.cg; fields[1] = t.bm; fields[2] = t.n_tiles; fields[3] = t.sk_tiles; fields[4] = smem; fields[5] = t.cg; fields[6] = t.split; fields[7] = t.tail;
   }
   if (t.teams < 1 || t.teams * t.cg > sm_count || (t.split > 1 && (t.cg != 1 || t.teams != t.n_tiles * t.split || t.split > 8)) ||
       t.bm % 32 != 0 || t.bm < 32 || t.bm > (t.cg == 2 ? 256 : 128) || smem > 227 * 1024 || t.nxs < 2 || t.nws < 2 ||
@@ -463,14 +463,16 @@ int lcq_gemm_tc_plan_check(int M, int N, int K, int sm_count, int* fields) {
   }
   // Replay the device-side schedule: every (tile, weight stage) exactly once, partials in slots of
   // their own, contributors as the kernel counts them.
-  std::vector<int> seen(static_cast<size_t>(t.n_tiles) * p.nst, 0);
+  std::vector<int> seen(static_cast<size_t>(t.n_tiles) * t.tail * p.nst, 0);     // per piece of a tile; whole tiles count in their first
   std::vector<int> slot_of(static_cast<size_t>(2) * t.teams, -1);
   std::vector<int> contributors(t.n_tiles, 0);
   for (int team = 0; team < t.teams; ++team) {
     for (gemm_tc::Walk w(p, team); w.next(p);) {
       if (w.tile < 0 || w.tile >= t.n_tiles || w.st0 < 0 || w.st0 >= w.st1 || w.st1 > p.nst) { set_error("plan check: segment out of range"); return LCQ_ERR_BAD_ARG; }
-      for (int st = w.st0; st < w.st1; ++st) seen[static_cast<size_t>(w.tile) * p.nst + st]++;
-      contributors[w.tile]++;
+      const int row = w.m0 - (w.tile / p.n_tiles_n) * p.bm;
+      if (row < 0 || row % w.bm != 0 || w.bm != (w.tile < p.full ? p.bm : p.bm / p.tail)) { set_error("plan check: bad piece"); return LCQ_ERR_BAD_ARG; }
+      for (int st = w.st0; st < w.st1; ++st) seen[(static_cast<size_t>(w.tile) * t.tail + row / w.bm) * p.nst + st]++;
+      if (row == 0) contributors[w.tile]++;
       if ((w.st0 == 0 && w.st1 == p.nst) || t.split > 1) continue;
       const unsigned t0 = static_cast<unsigned>(w.tile) * static_cast<unsigned>(p.nst);
       const int slot1 = team == gemm_tc::share_owner(p, t0) && gemm_tc::share_begin(p, team) < t0;     // as the kernel's part()
@@ -479,8 +481,13 @@ int lcq_gemm_tc_plan_check(int M, int N, int K, int sm_count, int* fields) {
       owner = w.tile;
     }
   }
-  for (size_t i = 0; i < seen.size(); ++i)
-    if (seen[i] != 1) { set_error("plan check: stage %zu covered %d times", i, seen[i]); return LCQ_ERR_BAD_ARG; }
+  for (int tile = 0; tile < t.n_tiles; ++tile)
+    for (int piece = 0; piece < t.tail; ++piece)
+      for (int st = 0; st < p.nst; ++st) {
+        const int row = (tile / p.n_tiles_n) * p.bm + piece * (p.bm / p.tail);
+        const int want = tile < p.full ? piece == 0 : row < M;
+        if (seen[(static_cast<size_t>(tile) * t.tail + piece) * p.nst + st] != want) { set_error("plan check: tile %d stage %d not covered once", tile, st); return LCQ_ERR_BAD_ARG; }
+      }
   for (int tile = 0; tile < t.n_tiles; ++tile) {
     int expect = t.split;
     if (tile < t.sk_tiles) {

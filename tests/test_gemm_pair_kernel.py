@@ -18,7 +18,7 @@ from oracle import qmm_oracle as O
 
 
 def test_plan_covers_every_stage_once():
-    lib, f = _lib.lib(), (ctypes.c_int * 7)()
+    lib, f = _lib.lib(), (ctypes.c_int * 8)()
     for m in (1, 17, 32, 33, 64, 100, 192, 193, 256, 512, 1000, 2048, 8192):
         for n in (1, 100, 256, 257, 1024, 4096, 14336, 28672):
             for k in (64, 256, 320, 576, 4096, 14336):

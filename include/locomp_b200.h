@@ -190,6 +190,44 @@ int lcq_embed_lookup(const void* token_ids, const void* table, void* out, int64_
 int lcq_argmax(const void* x, void* out, int64_t rows, int n, int dtype, void* stream);
 
 /*
+ * One decode step of a Llama-style stack as one kernel (fp16 activations, int4 weights in groups of 32, fp16
+ * scales): embedding of `token`; per layer RMS norm, q|k|v and o projections (o reads x_q), residual add +
+ * RMS norm, gate|up, SiLU * up, down, residual add; final norm, lm_head, greedy argmax into `next_token`.
+ * Every result (logits, outputs, *_out) is written.  The same chain as lcq_embed_lookup, lcq_rms_norm,
+ * lcq_matmul_int4, lcq_residual_rms_norm, lcq_silu_mul, lcq_add_inplace and lcq_argmax in
+ * examples/54_smollm2_inference.py:494-578 order.
+ *
+ * The kernel fills the GPU (one CTA per SM, cooperative launch) and its CTAs wait for one another, with the
+ * limit of lcq_set_wait_limit_ns.  `layers` points to n_layers lcq_decode_layer records in DEVICE memory;
+ * weights, scales and records must be complete before the launch.  `state`: lcq_decode_step_state_bytes()
+ * bytes of device memory, zero-filled once, used by one stack on one stream.  Pointers 16-byte aligned.
+ * lcq_decode_step_state_bytes returns 0 when the shape is not covered (hidden, inter and q_dim multiples of
+ * 64, hidden at most 4096, qkv and vocab multiples of 4, rows short enough for shared memory).
+ */
+typedef struct {
+  const void *qkv_w, *qkv_s;          /* [qkv, hidden] */
+  const void *o_w, *o_s;              /* [hidden, q_dim] */
+  const void *gate_up_w, *gate_up_s;  /* [2 * inter, hidden], gate rows first */
+  const void *down_w, *down_s;        /* [hidden, inter] */
+} lcq_decode_layer;
+
+typedef struct {
+  const void* layers;
+  const void *head_w, *head_s;        /* [vocab, hidden] */
+  void* logits;
+  const void* norms;                  /* [2 * n_layers + 1, hidden]: each layer's input and post-attention norm, the final one */
+  void* outputs;                      /* [n_layers, qkv + hidden + 2 * inter + hidden]: q|k|v, o, gate|up, down */
+  const void *token, *table, *x_q;
+  void *hidden_out, *normed_out, *mlp_out, *next_token, *state;
+  size_t state_bytes;
+  int n_layers, hidden, inter, qkv, q_dim, vocab;
+  float eps;
+} lcq_decode_stack;
+
+size_t lcq_decode_step_state_bytes(const lcq_decode_stack* stack);
+int lcq_decode_step(const lcq_decode_stack* stack, void* stream);
+
+/*
  * Weight quantisers with the reference's arithmetic, bit for bit: w [N, K] of `w_dtype` ->
  * w_packed uint8 [N, K/2] (or w_int8 int8 [N, K]) and scales float32 [N, K/group_size].
  * style 0 = quantize_int4 / quantize_int8 of examples/38_quantized_matmul.py:248-293

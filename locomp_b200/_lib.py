@@ -16,6 +16,16 @@ ALGO_AUTO, ALGO_SIMT, ALGO_GEMV_TC, ALGO_GEMM_TC, ALGO_GEMV_W8 = 0, 1, 2, 3, 4
 
 # name -> (restype, argtypes); mirrors include/locomp_b200.h one to one
 _c = ctypes
+
+
+class DecodeStackDesc(_c.Structure):
+    """lcq_decode_stack."""
+    _fields_ = ([(n, _c.c_void_p) for n in ("layers", "head_w", "head_s", "logits", "norms", "outputs", "token", "table", "x_q",
+                                            "hidden_out", "normed_out", "mlp_out", "next_token", "state")] +
+                [("state_bytes", _c.c_size_t)] + [(n, _c.c_int) for n in ("n_layers", "hidden", "inter", "qkv", "q_dim", "vocab")] +
+                [("eps", _c.c_float)])
+
+
 SIGNATURES = {
     "lcq_version": (_c.c_int, []),
     "lcq_status_string": (_c.c_char_p, [_c.c_int]),
@@ -38,6 +48,8 @@ SIGNATURES = {
     "lcq_add_inplace": (_c.c_int, [_c.c_void_p] * 2 + [_c.c_int64, _c.c_int, _c.c_void_p]),
     "lcq_embed_lookup": (_c.c_int, [_c.c_void_p] * 3 + [_c.c_int64, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p]),
     "lcq_argmax": (_c.c_int, [_c.c_void_p] * 2 + [_c.c_int64, _c.c_int, _c.c_int, _c.c_void_p]),
+    "lcq_decode_step_state_bytes": (_c.c_size_t, [_c.POINTER(DecodeStackDesc)]),
+    "lcq_decode_step": (_c.c_int, [_c.POINTER(DecodeStackDesc), _c.c_void_p]),
     "lcq_quantize_int4": (_c.c_int, [_c.c_void_p] * 3 + [_c.c_int64, _c.c_int64, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p]),
     "lcq_quantize_int8": (_c.c_int, [_c.c_void_p] * 3 + [_c.c_int64, _c.c_int64, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p]),
     "lcq_peer_alloc": (_c.c_int, [_c.c_size_t, _c.POINTER(_c.c_void_p), _c.c_char_p]),

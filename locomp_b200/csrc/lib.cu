@@ -14,6 +14,7 @@
 #include "peer_gather.cuh"
 #include "glue.cuh"
 #include "quantize.cuh"
+#include "decode_step.cuh"
 
 namespace lcq {
 
@@ -685,6 +686,28 @@ int lcq_argmax(const void* x, void* out, int64_t rows, int n, int dtype, void* s
   if (!x || !out) { set_error("null pointer argument"); return LCQ_ERR_BAD_ARG; }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LCQ_BY_DTYPE(dtype, (glue::launch_argmax<T>(x, out, rows, n, st)))
+}
+
+// ---------------------------------------------------------------- one kernel per decode step
+size_t lcq_decode_step_state_bytes(const lcq_decode_stack* stack) {
+  int sm = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) {
+    int v = 0;
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0) sm = v;
+  } else {
+    (void)cudaGetLastError();
+  }
+  step::Plan pl;
+  return stack && step::make_plan(*stack, sm, pl) ? pl.state_bytes : 0;
+}
+
+int lcq_decode_step(const lcq_decode_stack* stack, void* stream) {
+  if (!stack) { set_error("decode_step: null argument"); return LCQ_ERR_BAD_ARG; }
+  DevInfo di;
+  int rc = current_dev_info(di);
+  if (rc != LCQ_OK) return rc;
+  if (di.major != 10) { set_error("built for sm_100a only; device is sm_%d%d", di.major, di.minor); return LCQ_ERR_UNSUPPORTED; }
+  return step::launch(*stack, di.sm_count, static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------- quantisers

@@ -9,13 +9,14 @@ launch and one read of x instead of several (the dense analogue is examples/42_f
 """
 from __future__ import annotations
 
+import ctypes
 from typing import List, Optional, Sequence, Tuple
 
 import torch
 
 from . import _lib
 from .ops import matmul_workspace_bytes, quantized_matmul
-from .tensor import _TORCH_TO_KIND
+from .tensor import _TORCH_TO_KIND, current_stream_ptr
 
 
 class QuantLinear:
@@ -69,7 +70,7 @@ class DecodeStack:
     (examples/54_smollm2_inference.py:494-554, :556-578) except attention itself: embedding lookup,
     input RMS norm, residual add + post-attention norm (one kernel), SiLU * up, residual add, final
     norm, and a greedy argmax of the logits on the device -- a real dependency chain on one hidden
-    state, 8 launches per layer."""
+    state.  In fp16 the whole step is one kernel where that covers the shape, else 8 launches per layer."""
 
     def __init__(self, layers: int = 30, hidden: int = 576, inter: int = 1536, q_heads: int = 9, kv_heads: int = 3,
                  head_dim: int = 64, vocab: int = 49152, fused: bool = False, device="cuda", seed: int = 0,
@@ -85,6 +86,7 @@ class DecodeStack:
             raise ValueError("glue=True runs the fused layer form")
         self.glue = glue
         self.ops = []                                  # with glue: the step as a list of zero-argument launches
+        self._desc = None                              # with glue, where one kernel covers the shape: its description
         self.calls: List[Tuple[QuantLinear, torch.Tensor, torch.Tensor]] = []   # (linear, x, out)
         x_h = torch.randn(1, hidden, device=device, generator=g).to(dtype)
         x_i = torch.randn(1, inter, device=device, generator=g).to(dtype)
@@ -101,8 +103,20 @@ class DecodeStack:
             self.normed = torch.zeros(1, hidden, dtype=dtype, device=device)
             self.mlp = torch.zeros(1, inter, dtype=dtype, device=device)
 
+            # one block for all norm weights and one for all layer outputs: the step kernel finds them by offset
+            widths = (qd + 2 * kvd, hidden, 2 * inter, hidden)
+            self.norms = torch.empty(2 * layers + 1, hidden, dtype=dtype, device=device)
+            self.outputs = torch.zeros(layers, sum(widths), dtype=dtype, device=device)
+            norm_w = iter(self.norms)
+            outs = (o.unsqueeze(0) for row in self.outputs for o in row.split(widths))
+
+            def draw_norm():
+                return next(norm_w).copy_(1 + 0.1 * torch.randn(hidden, device=device, generator=g))
+
             def lin_op(lin, x):
-                out = torch.empty(1, lin.out_features, dtype=dtype, device=device)
+                out = next(outs, None)
+                if out is None:                                # the lm_head
+                    out = torch.empty(1, lin.out_features, dtype=dtype, device=device)
                 self.calls.append((lin, x, out))
                 self.ops.append(lambda: lin(x, out=out, workspace_buf=self.workspace))
                 return out
@@ -110,8 +124,7 @@ class DecodeStack:
             for _ in range(layers):
                 q, k, v, o = make(qd, hidden), make(kvd, hidden), make(kvd, hidden), make(hidden, qd)
                 gate, up, down = make(inter, hidden), make(inter, hidden), make(hidden, inter)
-                w_in = (1 + 0.1 * torch.randn(hidden, device=device, generator=g)).to(dtype)
-                w_post = (1 + 0.1 * torch.randn(hidden, device=device, generator=g)).to(dtype)
+                w_in, w_post = draw_norm(), draw_norm()
                 self.ops.append(lambda w=w_in: D.rms_norm(self.hidden, w, 1e-5, out=self.normed))
                 lin_op(fuse_rows([q, k, v])[0], self.normed)
                 o_out = lin_op(QuantLinear(*o), x_q)            # attention is not part of this path: o reads a prepared buffer
@@ -120,10 +133,11 @@ class DecodeStack:
                 self.ops.append(lambda gu=gu: D.silu_mul(gu[:, :inter], gu[:, inter:], out=self.mlp))
                 d_out = lin_op(QuantLinear(*down), self.mlp)
                 self.ops.append(lambda d=d_out: D.add_inplace(self.hidden, d))
-            w_fin = (1 + 0.1 * torch.randn(hidden, device=device, generator=g)).to(dtype)
+            w_fin = draw_norm()
             self.ops.append(lambda: D.rms_norm(self.hidden, w_fin, 1e-5, out=self.normed))
             self.logits = lin_op(QuantLinear(*make(vocab, hidden)), self.normed)
             self.ops.append(lambda: D.argmax(self.logits, out=self.next_token))
+            self._one_kernel(x_q, layers, hidden, inter, qd, qd + 2 * kvd, vocab)
             layers = 0                                 # the plain construction below adds nothing more
         for _ in range(layers):
             q, k, v, o = make(qd, hidden), make(kvd, hidden), make(kvd, hidden), make(hidden, qd)
@@ -142,7 +156,7 @@ class DecodeStack:
                 add(QuantLinear(*down), x_i)
         if not glue:
             add(QuantLinear(*make(vocab, hidden)), x_h)
-        self.launches_per_step = len(self.ops) if glue else len(self.calls)
+        self.launches_per_step = 1 if self._desc is not None else len(self.ops) if glue else len(self.calls)
         self.weight_bytes = sum(c[0].weight_bytes for c in self.calls)
         # one scratch buffer for the whole stack (calls are stream-ordered), allocated up front so
         # that nothing is allocated while a CUDA graph is being captured
@@ -152,7 +166,32 @@ class DecodeStack:
         self.workspace = torch.zeros(max(need, 256), dtype=torch.uint8, device=device)
         self._graph = None
 
+    def _one_kernel(self, x_q, layers, hidden, inter, qd, qkv, vocab):
+        """Describe the step to the kernel that runs all of it, if it covers the shape (fp16 only)."""
+        if self.norms.dtype != torch.float16:
+            return
+        pointers = [[t.data_ptr() for lin, _, _ in self.calls[4 * i:4 * i + 4] for t in (lin.w, lin.scales)] for i in range(layers)]
+        head = self.calls[-1][0]
+        desc = _lib.DecodeStackDesc(n_layers=layers, hidden=hidden, inter=inter, qkv=qkv, q_dim=qd, vocab=vocab, eps=1e-5)
+        need = _lib.lib().lcq_decode_step_state_bytes(ctypes.byref(desc))
+        if need == 0:
+            return
+        device = self.hidden.device
+        self._state = torch.zeros(need, dtype=torch.uint8, device=device)
+        self._table = torch.tensor(pointers, dtype=torch.int64, device=device)
+        self._x_q = x_q
+        for name, t in (("layers", self._table), ("head_w", head.w), ("head_s", head.scales), ("logits", self.logits), ("norms", self.norms),
+                        ("outputs", self.outputs), ("token", self.token), ("table", self.table), ("x_q", x_q), ("hidden_out", self.hidden),
+                        ("normed_out", self.normed), ("mlp_out", self.mlp), ("next_token", self.next_token), ("state", self._state)):
+            setattr(desc, name, t.data_ptr())
+        desc.state_bytes = need
+        self._desc = desc
+
     def step(self):
+        if self._desc is not None:
+            with torch.cuda.device(self.hidden.device):
+                _lib.check(_lib.lib().lcq_decode_step(ctypes.byref(self._desc), current_stream_ptr()))
+            return
         if self.glue:
             for op in self.ops:
                 op()

@@ -202,7 +202,7 @@ int lcq_argmax(const void* x, void* out, int64_t rows, int n, int dtype, void* s
  * weights, scales and records must be complete before the launch.  `state`: lcq_decode_step_state_bytes()
  * bytes of device memory, zero-filled once, used by one stack on one stream.  Pointers 16-byte aligned.
  * lcq_decode_step_state_bytes returns 0 when the shape is not covered (hidden, inter and q_dim multiples of
- * 64, hidden at most 4096, qkv and vocab multiples of 4, rows short enough for shared memory).
+ * 64, hidden at most 8192, qkv and vocab multiples of 4, rows short enough for shared memory).
  */
 typedef struct {
   const void *qkv_w, *qkv_s;          /* [qkv, hidden] */

@@ -13,7 +13,7 @@
 //   * results that the next phase needs are published as words {fp16 value, 16-bit tag of the phase}: a
 //     consumer polls the data itself until every tag is the one it expects.  No grid barrier, no fence, no
 //     flag: one store and one load through L2 between dependent matvecs;
-//   * every CTA keeps the hidden state (in registers) and does the norms redundantly.
+//   * every CTA keeps the hidden state and does the norms redundantly.
 // Every CTA has at least one unit of 4 rows in every phase.  So whoever has all results of a phase knows
 // that all CTAs have read what they needed for it, and a buffer that is rewritten three phases later (the
 // next layer's) has no reader left.
@@ -32,7 +32,7 @@ namespace step {
 constexpr int NCW = 16;                        // consumer warps
 constexpr int NCT = NCW * 32;
 constexpr int NTHREADS = NCT + 32;             // + the producer warp
-constexpr int MAX_STAGES = 16;
+constexpr int MAX_STAGES = 32;
 constexpr int BAR_C = 1;                       // named barrier of the consumers
 constexpr int STATE_BYTES = 64;                // epoch, argmax counter, argmax key
 
@@ -43,31 +43,37 @@ struct Params {
   Shape sh;
   int n_layers, ctas;
   int stage_bytes, n_stages;
-  uint32_t* o_buf;      // published words: o projection, down projection [hidden], activation [inter]
+  int copies;           // of the published words: a CTA polls copy b % copies
+  int copy_words;       // 2 * hidden + inter
+  uint32_t* o_buf;      // published words, first copy: o projection, down projection [hidden], activation [inter]
   uint32_t* d_buf;
   uint32_t* m_buf;
 };
 
 // Rows of an [n, K] weight that CTA b streams: whole units of 4 (so that rows of scales start on 16 bytes).
-__host__ __device__ inline int share(int n, int b, int ctas) { return 4 * static_cast<int>(static_cast<long long>(n / 4) * b / ctas); }
+__host__ __device__ inline int share(int n, int b, int ctas) { return static_cast<int>(static_cast<unsigned>(n / 4) * static_cast<unsigned>(b) / static_cast<unsigned>(ctas)) * 4; }
 __host__ __device__ inline int row_bytes(int K) { return K / 2 + K / 16; }
 __host__ __device__ inline int tile_rows(int stage_bytes, int K) { return (stage_bytes / row_bytes(K)) & ~3; }
 
-struct Smem { int stages, xn, xq, xm, res, red, bars, flags, total; };
+struct Smem { int stages, xn, xq, xm, hid, gam, res, red, bars, flags, rows, table, total; };
 __host__ __device__ inline int max2(int a, int b) { return a > b ? a : b; }
-__host__ __device__ inline Smem smem_map(const Shape& s, int ctas, int stage_bytes, int n_stages) {
+__host__ __device__ inline Smem smem_map(const Shape& s, int n_layers, int ctas, int stage_bytes, int n_stages) {
   Smem m;
   m.stages = 0;
   m.xn = n_stages * stage_bytes;
   m.xq = m.xn + s.hidden * 2;
   m.xm = m.xq + s.q_dim * 2;
-  m.res = m.xm + s.inter * 2;
+  m.hid = m.xm + s.inter * 2;
+  m.gam = m.hid + s.hidden * 2;
+  m.res = m.gam + s.hidden * 2;
   const int per = 4;                           // a share is at most one unit above the average
   const int rows = max2(max2((s.qkv + s.hidden) / ctas + 4 * per, 2 * s.inter / ctas + 4 * per), s.vocab / ctas + 2 * per);
   m.red = m.res + rows * 16;
   m.bars = m.red + 2 * NCW * 8;
   m.flags = m.bars + 2 * MAX_STAGES * 8;
-  m.total = m.flags + 16;
+  m.rows = m.flags + 16;                       // Rows
+  m.table = m.rows + 32;                       // the layer records
+  m.total = m.table + n_layers * static_cast<int>(sizeof(lcq_decode_layer));
   return m;
 }
 
@@ -102,98 +108,105 @@ __device__ __forceinline__ float dot8(uint32_t w, const uint4& x) {
   const uint32_t b = nibbles(w, 0x00F000F0u, 0x54005400u, 0x54805480u);     // q1, q5
   const uint32_t c = nibbles(w8, 0x000F000Fu, 0x64006400u, 0x64086408u);    // q2, q6
   const uint32_t d = nibbles(w8, 0x00F000F0u, 0x54005400u, 0x54805480u);    // q3, q7
-  float p = 0.0f;
+  float p = 0.0f, q = 0.0f;
   p = fma_lo(a, x.x, false, false, p);
+  q = fma_lo(a, x.z, true, false, q);
   p = fma_lo(b, x.x, false, true, p);
+  q = fma_lo(b, x.z, true, true, q);
   p = fma_lo(c, x.y, false, false, p);
+  q = fma_lo(c, x.w, true, false, q);
   p = fma_lo(d, x.y, false, true, p);
-  p = fma_lo(a, x.z, true, false, p);
-  p = fma_lo(b, x.z, true, true, p);
-  p = fma_lo(c, x.w, true, false, p);
-  p = fma_lo(d, x.w, true, true, p);
-  return p;
+  q = fma_lo(d, x.w, true, true, q);
+  return p + q;
 }
 
 // The tiles of a CTA in the order in which the producer streams and the consumers use them: per layer q|k|v
 // rows, o rows, gate rows, up rows, down rows; then the lm_head.
+struct Rows { int qkv0, qkv, hid0, hid, int0, inter, voc0, voc; };   // this CTA's shares: first row, rows
 struct Segment { const uint8_t* w; const uint8_t* s; int row0, rows, K; };
-__device__ __forceinline__ Segment segment(const Params& p, int layer, int part, int b) {
+__device__ __forceinline__ Segment segment(const Params& p, const lcq_decode_layer* table, const Rows& r, int layer, int part) {
   Segment g;
   const Shape& sh = p.sh;
-  int n, base = 0;
-  if (layer == p.n_layers) {
-    g.w = static_cast<const uint8_t*>(p.d.head_w); g.s = static_cast<const uint8_t*>(p.d.head_s);
-    n = sh.vocab; g.K = sh.hidden;
-  } else {
-    const lcq_decode_layer* l = static_cast<const lcq_decode_layer*>(p.d.layers) + layer;
-    if (part == 0) { g.w = static_cast<const uint8_t*>(l->qkv_w); g.s = static_cast<const uint8_t*>(l->qkv_s); n = sh.qkv; g.K = sh.hidden; }
-    else if (part == 1) { g.w = static_cast<const uint8_t*>(l->o_w); g.s = static_cast<const uint8_t*>(l->o_s); n = sh.hidden; g.K = sh.q_dim; }
-    else if (part == 4) { g.w = static_cast<const uint8_t*>(l->down_w); g.s = static_cast<const uint8_t*>(l->down_s); n = sh.hidden; g.K = sh.inter; }
-    else { g.w = static_cast<const uint8_t*>(l->gate_up_w); g.s = static_cast<const uint8_t*>(l->gate_up_s); n = sh.inter; g.K = sh.hidden; base = part == 3 ? sh.inter : 0; }
-  }
-  const int r0 = share(n, b, p.ctas), r1 = share(n, b + 1, p.ctas);
-  g.row0 = base + r0;
-  g.rows = r1 - r0;
+  if (layer == p.n_layers)
+    return {static_cast<const uint8_t*>(p.d.head_w), static_cast<const uint8_t*>(p.d.head_s), r.voc0, r.voc, sh.hidden};
+  const lcq_decode_layer* l = table + layer;
+  if (part == 0) g = {static_cast<const uint8_t*>(l->qkv_w), static_cast<const uint8_t*>(l->qkv_s), r.qkv0, r.qkv, sh.hidden};
+  else if (part == 1) g = {static_cast<const uint8_t*>(l->o_w), static_cast<const uint8_t*>(l->o_s), r.hid0, r.hid, sh.q_dim};
+  else if (part == 4) g = {static_cast<const uint8_t*>(l->down_w), static_cast<const uint8_t*>(l->down_s), r.hid0, r.hid, sh.inter};
+  else g = {static_cast<const uint8_t*>(l->gate_up_w), static_cast<const uint8_t*>(l->gate_up_s), r.int0 + (part == 3 ? sh.inter : 0), r.inter, sh.hidden};
   return g;
 }
 
-// A lane's sums over the words lane, lane + step, ... of NR rows that are `row_step` rows apart.
+// Shared memory by 32-bit addresses: generic pointers would take two registers each and a slower load.
+__device__ __forceinline__ uint32_t ld32(uint32_t a) { uint32_t v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ uint4 ld128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float ld_half(uint32_t a) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+  return __half2float(__ushort_as_half(v));
+}
+__device__ __forceinline__ void st128(uint32_t a, float x, float y, float z, float w) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+__device__ __forceinline__ void st32(uint32_t a, float x) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory"); }
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+// A lane's sums over the words word0, word0 + step, ... of NR rows that are NCW rows apart.
+// w, sc, x: addresses of the first row's weights and scales and of the input.
 template <int NR>
-__device__ __forceinline__ void rows_dot(const uint8_t* w, const __half* sc, const uint4* x, int K, int row_step, int word0, int step, float (&acc)[4]) {
-  const int words = K / 8, groups = K / 32;
+__device__ __forceinline__ void rows_dot(uint32_t w, uint32_t sc, uint32_t x, int K, int word0, int step, float (&acc)[NR]) {
+  const int words = K / 8;
 #pragma unroll
   for (int r = 0; r < NR; ++r) acc[r] = 0.0f;
-#pragma unroll 2
+#pragma unroll (NR == 1 ? 2 : 1)
   for (int j = word0; j < words; j += step) {
-    const uint4 xv = x[j];
+    const uint4 xv = ld128(x + j * 16);
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      const uint32_t word = *reinterpret_cast<const uint32_t*>(w + (static_cast<size_t>(r * row_step) * words + j) * 4);
-      acc[r] = fmaf(__half2float(sc[r * row_step * groups + (j >> 2)]), dot8(word, xv), acc[r]);
-    }
+    for (int r = 0; r < NR; ++r)
+      acc[r] = fmaf(ld_half(sc + r * NCW * (K / 16) + (j >> 2) * 2), dot8(ld32(w + r * NCW * (K / 2) + j * 4), xv), acc[r]);
   }
 }
 
-// One tile (rows x K in shared memory) times x; row i's sum goes to res[4 i .. 4 i + 3] as up to four parts.
-__device__ __forceinline__ void tile_matvec(const uint8_t* stage, int rows, int K, const uint4* x, float4* res, int warp, int lane) {
-  const __half* sc = reinterpret_cast<const __half*>(stage + rows * (K / 2));
+// One tile (rows x K in shared memory) times x; row i's sum goes to res + 16 i as up to four parts.
+__device__ __forceinline__ void tile_matvec(uint32_t stage, int rows, int K, uint32_t x, uint32_t res, int warp, int lane) {
+  const uint32_t sc = stage + rows * (K / 2);
   if (rows <= 8) {                             // several warps a row
-    const int parts = rows <= 4 ? 4 : 2, row = warp / parts, part = warp - row * parts;
+    const int shift = rows <= 4 ? 2 : 1, row = warp >> shift, part = warp & ((1 << shift) - 1);
     if (row >= rows) return;
-    float acc[4];
-    rows_dot<1>(stage + row * (K / 2), sc + row * (K / 32), x, K, 0, part * 32 + lane, parts * 32, acc);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
-    float* out = reinterpret_cast<float*>(res + row);
-    if (lane == 0) { out[part] = acc[0]; if (parts == 2) out[part + 2] = 0.0f; }
+    float acc[1];
+    rows_dot<1>(stage + row * (K / 2), sc + row * (K / 16), x, K, part * 32 + lane, 32 << shift, acc);
+    acc[0] = warp_sum(acc[0]);
+    if (lane == 0) { st32(res + row * 16 + part * 4, acc[0]); if (shift == 1) st32(res + row * 16 + part * 4 + 8, 0.0f); }
     return;
   }
-  for (int row = warp; row < rows; row += 4 * NCW) {
-    float acc[4];
-    const uint8_t* w = stage + row * (K / 2);
-    const __half* s = sc + row * (K / 32);
-    const int n = (rows - row + NCW - 1) / NCW;          // rows of this pass: 1 .. 4
-    if (n >= 4) rows_dot<4>(w, s, x, K, NCW, lane, 32, acc);
-    else if (n == 3) rows_dot<3>(w, s, x, K, NCW, lane, 32, acc);
-    else if (n == 2) rows_dot<2>(w, s, x, K, NCW, lane, 32, acc);
-    else rows_dot<1>(w, s, x, K, NCW, lane, 32, acc);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      if (r < n) {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], off);
-        if (lane == 0) res[row + r * NCW] = make_float4(acc[r], 0.0f, 0.0f, 0.0f);
-      }
-    }
+  int row = warp;
+  for (; row + NCW < rows; row += 2 * NCW) {
+    float acc[2];
+    rows_dot<2>(stage + row * (K / 2), sc + row * (K / 16), x, K, lane, 32, acc);
+    acc[0] = warp_sum(acc[0]);
+    acc[1] = warp_sum(acc[1]);
+    if (lane == 0) { st128(res + row * 16, acc[0], 0.0f, 0.0f, 0.0f); st128(res + (row + NCW) * 16, acc[1], 0.0f, 0.0f, 0.0f); }
+  }
+  if (row < rows) {
+    float acc[1];
+    rows_dot<1>(stage + row * (K / 2), sc + row * (K / 16), x, K, lane, 32, acc);
+    acc[0] = warp_sum(acc[0]);
+    if (lane == 0) st128(res + row * 16, acc[0], 0.0f, 0.0f, 0.0f);
   }
 }
 
-// CH: chunks of 4 * NCT hidden values (a thread keeps 4 of each in registers).
-template <int CH>
 __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(128) uint8_t smem[];
   const Shape& sh = p.sh;
-  const Smem L = smem_map(sh, p.ctas, p.stage_bytes, p.n_stages);
+  const Smem L = smem_map(sh, p.n_layers, p.ctas, p.stage_bytes, p.n_stages);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.bars);
   uint64_t* empty = full + MAX_STAGES;
   volatile int* flag_abort = reinterpret_cast<volatile int*>(smem + L.flags);
@@ -207,9 +220,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
     for (int i = 0; i < p.n_stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], NCW); }
     *flag_abort = 0;
     *smem_epoch = *reinterpret_cast<volatile uint32_t*>(epoch);
+    Rows r;
+    r.qkv0 = share(sh.qkv, b, p.ctas); r.qkv = share(sh.qkv, b + 1, p.ctas) - r.qkv0;
+    r.hid0 = share(sh.hidden, b, p.ctas); r.hid = share(sh.hidden, b + 1, p.ctas) - r.hid0;
+    r.int0 = share(sh.inter, b, p.ctas); r.inter = share(sh.inter, b + 1, p.ctas) - r.int0;
+    r.voc0 = share(sh.vocab, b, p.ctas); r.voc = share(sh.vocab, b + 1, p.ctas) - r.voc0;
+    *reinterpret_cast<Rows*>(smem + L.rows) = r;
     fence_barrier_init();
   }
+  for (int i = tid; i < p.n_layers * static_cast<int>(sizeof(lcq_decode_layer) / 8); i += NTHREADS)
+    reinterpret_cast<uint64_t*>(smem + L.table)[i] = static_cast<const uint64_t*>(p.d.layers)[i];
   __syncthreads();
+  const Rows& mine = *reinterpret_cast<const Rows*>(smem + L.rows);
+  const int step_h = tile_rows(p.stage_bytes, sh.hidden), step_q = tile_rows(p.stage_bytes, sh.q_dim), step_i = tile_rows(p.stage_bytes, sh.inter);
 
   if (warp == NCW) {
     // ------------------------------------------------------------ producer: one thread, all layers in order
@@ -219,8 +242,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
       bool ok = true;
       for (int layer = 0; layer <= p.n_layers && ok; ++layer) {
         for (int part = 0; part < (layer < p.n_layers ? 5 : 1) && ok; ++part) {
-          const Segment g = segment(p, layer, part, b);
-          const int step = tile_rows(p.stage_bytes, g.K);
+          const Segment g = segment(p, reinterpret_cast<const lcq_decode_layer*>(smem + L.table), mine, layer, part);
+          const int step = part == 1 && layer < p.n_layers ? step_q : part == 4 ? step_i : step_h;
           for (int r = 0; r < g.rows; r += step) {
             const int rows = g.rows - r < step ? g.rows - r : step;
             if (*flag_abort || !mbar_wait_bounded(&empty[s], phase ^ 1u)) { *flag_abort = 1; atomicExch(&g_device_status, 50); ok = false; break; }
@@ -236,29 +259,27 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
     }
   } else {
     // ------------------------------------------------------------ consumers
-    __half* xn = reinterpret_cast<__half*>(smem + L.xn);
-    __half* xq = reinterpret_cast<__half*>(smem + L.xq);
-    __half* xm = reinterpret_cast<__half*>(smem + L.xm);
-    float4* res = reinterpret_cast<float4*>(smem + L.res);
+    const uint32_t base = smem_u32(smem);
+    const uint32_t xn = base + L.xn, xq = base + L.xq, xm = base + L.xm;
+    __half* xn_p = reinterpret_cast<__half*>(smem + L.xn);
     float* red = reinterpret_cast<float*>(smem + L.red);
     const uint32_t tag0 = *smem_epoch * static_cast<uint32_t>(3 * p.n_layers) + 1u;
+    const int copy = (b % p.copies) * p.copy_words;
     int s = 0;
     uint32_t phase = 0;
     bool dead = false;
 
-    const auto use_tiles = [&](int layer, int part, const __half* x, int res0) {
-      const Segment g = segment(p, layer, part, b);
-      const int step = tile_rows(p.stage_bytes, g.K);
-      for (int r = 0; r < g.rows; r += step) {
-        const int rows = g.rows - r < step ? g.rows - r : step;
+    // the next `n` rows of the stream (K columns, `step` rows a tile) times x
+    const auto use_tiles = [&](int n, int K, int step, uint32_t x, int res0) {
+      for (int r = 0; r < n; r += step) {
+        const int rows = n - r < step ? n - r : step;
         if (!dead && (*flag_abort || !mbar_wait_bounded(&full[s], phase))) { dead = true; *flag_abort = 1; atomicExch(&g_device_status, 51); }
         dead = __any_sync(0xffffffffu, dead);
-        if (!dead) tile_matvec(smem + s * p.stage_bytes, rows, g.K, reinterpret_cast<const uint4*>(x), res + res0 + r, warp, lane);
+        if (!dead) tile_matvec(base + s * p.stage_bytes, rows, K, x, base + L.res + (res0 + r) * 16, warp, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
         if (++s == p.n_stages) { s = 0; phase ^= 1u; }
       }
-      return g.rows;
     };
     // four published values, once they carry `tag`
     const auto take = [&](const uint32_t* src, uint32_t tag, __half (&v)[4]) {
@@ -275,40 +296,40 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
       v[0] = __ushort_as_half(static_cast<unsigned short>(w.x >> 16)); v[1] = __ushort_as_half(static_cast<unsigned short>(w.y >> 16));
       v[2] = __ushort_as_half(static_cast<unsigned short>(w.z >> 16)); v[3] = __ushort_as_half(static_cast<unsigned short>(w.w >> 16));
     };
-    __half h[CH][4];                           // the hidden state, values 4 * (c * NCT + tid) ..
-    // hidden (+= what was published in src); xn = rms_norm(hidden) * weight
-    // (the weights of the next norm are fetched a phase ahead: they may come from HBM)
-    uint2 next_g[CH];
-    int norm_index = 0;
-    const auto fetch_norm = [&]() {
-#pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        const int i = 4 * (c * NCT + tid);
-        next_g[c] = make_uint2(0u, 0u);
-        if (i < sh.hidden && norm_index <= 2 * p.n_layers)
-          next_g[c] = __ldg(reinterpret_cast<const uint2*>(static_cast<const __half*>(p.d.norms) + static_cast<long long>(norm_index) * sh.hidden + i));
+    // A thread's share of the hidden state and of the next norm's weights, 4 values of every 4 * NCT, lies in
+    // shared memory: in registers they cost the matvec loops theirs, and a spill goes to L2 here.
+    __half* hid = reinterpret_cast<__half*>(smem + L.hid);
+    const uint32_t gam = smem_u32(smem + L.gam);
+    const __half* next_norm = static_cast<const __half*>(p.d.norms);
+    int norms_left = 2 * p.n_layers + 1;
+    const auto fetch_norm = [&]() {            // a phase ahead: they may come from HBM
+      if (norms_left > 0) {
+        for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(gam + 2 * i), "l"(next_norm + i) : "memory");
       }
-      ++norm_index;
+      next_norm += sh.hidden;
+      --norms_left;
     };
+    // hidden (+= what was published in src); xn = rms_norm(hidden) * weight
     const auto norm = [&](const uint32_t* src, uint32_t tag) {
       float ss = 0.0f;
+      for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT) {
+        __half h[4];
+        *reinterpret_cast<uint2*>(h) = *reinterpret_cast<const uint2*>(hid + i);
+        if (src != nullptr) {
+          __half v[4];
+          take(src + i, tag, v);
 #pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        const int i = 4 * (c * NCT + tid);
-        if (i < sh.hidden) {
-          if (src != nullptr) {
-            __half v[4];
-            take(src + i, tag, v);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) h[c][e] = __float2half_rn(__half2float(h[c][e]) + __half2float(v[e]));
-          }
-#pragma unroll
-          for (int e = 0; e < 4; ++e) ss = fmaf(__half2float(h[c][e]), __half2float(h[c][e]), ss);
+          for (int e = 0; e < 4; ++e) h[e] = __float2half_rn(__half2float(h[e]) + __half2float(v[e]));
+          *reinterpret_cast<uint2*>(hid + i) = *reinterpret_cast<const uint2*>(h);
         }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ss = fmaf(__half2float(h[e]), __half2float(h[e]), ss);
       }
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
       if (lane == 0) red[warp] = ss;
+      asm volatile("cp.async.wait_all;" ::: "memory");
       named_bar_sync(BAR_C, NCT);
       float total = 0.0f;
 #pragma unroll
@@ -317,21 +338,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
         total += (q.x + q.y) + (q.z + q.w);
       }
       const float rms = rsqrtf(total / static_cast<float>(sh.hidden) + p.d.eps);
+      for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT) {
+        __half o[4], g[4], h[4];
+        *reinterpret_cast<uint2*>(g) = *reinterpret_cast<const uint2*>(smem + L.gam + 2 * i);
+        *reinterpret_cast<uint2*>(h) = *reinterpret_cast<const uint2*>(hid + i);
 #pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        const int i = 4 * (c * NCT + tid);
-        if (i < sh.hidden) {
-          __half o[4], g[4];
-          *reinterpret_cast<uint2*>(g) = next_g[c];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) o[e] = __float2half_rn(__half2float(h[c][e]) * rms * __half2float(g[e]));
-          *reinterpret_cast<uint2*>(xn + i) = *reinterpret_cast<const uint2*>(o);
-        }
+        for (int e = 0; e < 4; ++e) o[e] = __float2half_rn(__half2float(h[e]) * rms * __half2float(g[e]));
+        *reinterpret_cast<uint2*>(xn_p + i) = *reinterpret_cast<const uint2*>(o);
       }
       named_bar_sync(BAR_C, NCT);
       fetch_norm();
     };
-    const auto sum4 = [&](int i) { const float4 v = res[i]; return (v.x + v.y) + (v.z + v.w); };
+    const auto sum4 = [&](int i) {
+      const uint4 v = ld128(base + L.res + i * 16);
+      return (__uint_as_float(v.x) + __uint_as_float(v.y)) + (__uint_as_float(v.z) + __uint_as_float(v.w));
+    };
 
     // embedding; the prepared input of the o projections
     fetch_norm();
@@ -340,89 +361,71 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
       const bool known = id >= 0 && id < sh.vocab;
       if (!known && b == 0 && tid == 0) atomicExch(&g_device_status, 40);
       const __half* row = static_cast<const __half*>(p.d.table) + static_cast<long long>(known ? id : 0) * sh.hidden;
-#pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        const int i = 4 * (c * NCT + tid);
-        uint2 raw = make_uint2(0u, 0u);
-        if (known && i < sh.hidden) raw = *reinterpret_cast<const uint2*>(row + i);
-        *reinterpret_cast<uint2*>(h[c]) = raw;
-      }
+      for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT)
+        *reinterpret_cast<uint2*>(hid + i) = known ? *reinterpret_cast<const uint2*>(row + i) : make_uint2(0u, 0u);
       for (int i = 8 * tid; i < sh.q_dim; i += 8 * NCT)
-        *reinterpret_cast<uint4*>(xq + i) = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.d.x_q) + i);
+        *reinterpret_cast<uint4*>(smem + L.xq + 2 * i) = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.d.x_q) + i);
     }
 
-    for (int layer = 0; layer < p.n_layers; ++layer) {
-      // this layer's outputs: q|k|v, o, gate|up, down
-      __half* qkv_out = static_cast<__half*>(p.d.outputs) + static_cast<long long>(layer) * (sh.qkv + 2 * sh.hidden + 2 * sh.inter);
-      __half *o_out = qkv_out + sh.qkv, *gate_up_out = o_out + sh.hidden, *down_out = gate_up_out + 2 * sh.inter;
-      const uint32_t tag = (tag0 + 3u * layer) & 0xFFFFu, tag1 = (tag + 1u) & 0xFFFFu, tag2 = (tag + 2u) & 0xFFFFu;
-      // ---- q|k|v and o
-      norm(layer == 0 ? nullptr : p.d_buf, (tag - 1u) & 0xFFFFu);
-      {
-        const int q0 = share(sh.qkv, b, p.ctas), o0 = share(sh.hidden, b, p.ctas);
-        const int n_q = use_tiles(layer, 0, xn, 0);
-        const int n_o = use_tiles(layer, 1, xq, n_q);
-        named_bar_sync(BAR_C, NCT);
-        for (int i = tid; i < n_o + n_q; i += NCT) {
-          if (i < n_o) {
-            const __half v = __float2half_rn(sum4(n_q + i));
-            publish(p.o_buf + o0 + i, v, tag);
-            o_out[o0 + i] = v;
-          } else {
-            qkv_out[q0 + i - n_o] = __float2half_rn(sum4(i - n_o));
-          }
-        }
-      }
-      // ---- gate|up and the activation
-      norm(p.o_buf, tag);
-      {
-        const int i0 = share(sh.inter, b, p.ctas);
-        const int n = use_tiles(layer, 2, xn, 0);
-        use_tiles(layer, 3, xn, n);
-        named_bar_sync(BAR_C, NCT);
-        for (int i = tid; i < n; i += NCT) {
-          const __half g = __float2half_rn(sum4(i)), u = __float2half_rn(sum4(n + i));
-          const float x = __half2float(g);
-          const __half v = __float2half_rn((x * (1.0f / (1.0f + expf(-x)))) * __half2float(u));
-          publish(p.m_buf + i0 + i, v, tag1);
-          gate_up_out[i0 + i] = g;
-          gate_up_out[sh.inter + i0 + i] = u;
-          if (layer == p.n_layers - 1) static_cast<__half*>(p.d.mlp_out)[i0 + i] = v;
-        }
-      }
-      // ---- down
-      {
+    // Phases 3 l, 3 l + 1, 3 l + 2 of layer l: {norm, q|k|v and o}, {norm, gate|up, activation}, {down}; then the
+    // lm_head.  One loop body for all of them: three times the code would be fetched anew every phase.
+    const int last = 3 * p.n_layers;
+    __half* out = static_cast<__half*>(p.d.outputs);     // this layer's q|k|v, o, gate|up, down
+    for (int ph = 0, kind = 0; ph <= last; ++ph) {
+      const uint32_t tag = (tag0 + ph) & 0xFFFFu, before = (tag - 1u) & 0xFFFFu;
+      const bool head = ph == last;
+      if (kind == 2) {
         for (int i = 4 * tid; i < sh.inter; i += 4 * NCT) {
           __half v[4];
-          take(p.m_buf + i, tag1, v);
-          *reinterpret_cast<uint2*>(xm + i) = *reinterpret_cast<const uint2*>(v);
+          take(p.m_buf + copy + i, before, v);
+          *reinterpret_cast<uint2*>(smem + L.xm + 2 * i) = *reinterpret_cast<const uint2*>(v);
         }
-        const int d0 = share(sh.hidden, b, p.ctas);
         named_bar_sync(BAR_C, NCT);
-        const int n = use_tiles(layer, 4, xm, 0);
-        named_bar_sync(BAR_C, NCT);
-        for (int i = tid; i < n; i += NCT) {
-          const __half v = __float2half_rn(sum4(i));
-          publish(p.d_buf + d0 + i, v, tag2);
-          down_out[d0 + i] = v;
-        }
+      } else {
+        norm(ph == 0 ? nullptr : (kind == 0 ? p.d_buf : p.o_buf) + copy, before);
       }
+      // the rows that are published (pub, from sum `first` on) and those beside them
+      const int pub = head ? 0 : kind == 1 ? mine.inter : mine.hid;
+      const int first = kind == 0 ? (head ? mine.voc : mine.qkv) : 0;
+      for (int part = 0; part < (kind == 2 || head ? 1 : 2); ++part) {
+        const int n = part == 1 ? pub : kind == 0 ? first : pub;
+        const bool o_rows = kind == 0 && part == 1;
+        use_tiles(n, kind == 2 ? sh.inter : o_rows ? sh.q_dim : sh.hidden, kind == 2 ? step_i : o_rows ? step_q : step_h,
+                  kind == 2 ? xm : o_rows ? xq : xn, part == 0 ? 0 : kind == 0 ? first : pub);
+      }
+      named_bar_sync(BAR_C, NCT);
+      if (head) break;
+      {
+        uint32_t* dst = kind == 0 ? p.o_buf + mine.hid0 : kind == 1 ? p.m_buf + mine.int0 : p.d_buf + mine.hid0;
+        __half* plain = kind == 0 ? out + sh.qkv + mine.hid0 : kind == 1 ? out + sh.qkv + sh.hidden + mine.int0
+                                                                        : out + sh.qkv + sh.hidden + 2 * sh.inter + mine.hid0;
+        // warp w writes copies w, w + NCW, ...; the first also what the caller sees
+        for (int c = warp; c < p.copies; c += NCW) {
+          for (int i = lane; i < pub; i += 32) {
+            __half v = __float2half_rn(sum4(first + i));
+            if (c == 0) plain[i] = v;
+            if (kind == 1) {
+              const __half u = __float2half_rn(sum4(pub + i));
+              const float x = __half2float(v);
+              if (c == 0) plain[sh.inter + i] = u;
+              v = __float2half_rn((x * (1.0f / (1.0f + expf(-x)))) * __half2float(u));
+              if (c == 0 && ph == last - 2) static_cast<__half*>(p.d.mlp_out)[mine.int0 + i] = v;
+            }
+            publish(dst + c * p.copy_words + i, v, tag);
+          }
+        }
+        if (kind == 0)
+          for (int i = tid; i < first; i += NCT) out[mine.qkv0 + i] = __float2half_rn(sum4(i));
+      }
+      if (++kind == 3) { kind = 0; out += sh.qkv + 2 * sh.hidden + 2 * sh.inter; }
     }
-    // ---- final norm, lm_head, argmax
-    norm(p.d_buf, (tag0 + 3u * p.n_layers - 1u) & 0xFFFFu);
     if (b == 0) {
-#pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        const int i = 4 * (c * NCT + tid);
-        if (i < sh.hidden) {
-          *reinterpret_cast<uint2*>(static_cast<__half*>(p.d.hidden_out) + i) = *reinterpret_cast<const uint2*>(h[c]);
-          *reinterpret_cast<uint2*>(static_cast<__half*>(p.d.normed_out) + i) = *reinterpret_cast<const uint2*>(xn + i);
-        }
+      for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT) {
+        *reinterpret_cast<uint2*>(static_cast<__half*>(p.d.hidden_out) + i) = *reinterpret_cast<const uint2*>(hid + i);
+        *reinterpret_cast<uint2*>(static_cast<__half*>(p.d.normed_out) + i) = *reinterpret_cast<const uint2*>(xn_p + i);
       }
     }
-    const int v0 = share(sh.vocab, b, p.ctas);
-    const int n = use_tiles(p.n_layers, 0, xn, 0);
-    named_bar_sync(BAR_C, NCT);
+    const int v0 = mine.voc0, n = mine.voc;
     // the key of a logit orders as np.argmax does: by value, NaN above all, the lowest index among equals
     unsigned long long key = 0;
     for (int i = tid; i < n; i += NCT) {
@@ -459,52 +462,28 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
 }
 
 // ---------------------------------------------------------------------------- host side
-struct Plan { int ctas, stage_bytes, n_stages, chunks; size_t smem, state_bytes; };
+struct Plan { int ctas, stage_bytes, n_stages, copies; size_t smem, state_bytes; };
 
 inline bool make_plan(const lcq_decode_stack& d, int sm_count, Plan& pl) {
   const int H = d.hidden, I = d.inter;
-  if (d.n_layers < 1 || H < 64 || I < 64 || d.qkv < 4 || d.q_dim < 64 || d.vocab < 4) return false;
-  if (H % 64 || I % 64 || d.q_dim % 64 || d.qkv % 4 || d.vocab % 4 || H > 8 * NCT || I > (1 << 20) || d.vocab > (1 << 28)) return false;
+  if (d.n_layers < 1 || H < 64 || I < 64 || d.qkv < 4 || d.q_dim < 64 || d.vocab < 4 || d.n_layers > 256) return false;
+  if (H % 64 || I % 64 || d.q_dim % 64 || d.qkv % 4 || d.vocab % 4 || H > 8192 || I > (1 << 20) || d.vocab > (1 << 24)) return false;
   int units = H / 4;                           // every CTA needs a unit of 4 rows in every phase
   if (I / 4 < units) units = I / 4;
   if (d.vocab / 4 < units) units = d.vocab / 4;
   pl.ctas = sm_count < units ? sm_count : units;
-  pl.chunks = H <= 4 * NCT ? 1 : 2;
-  // a stage holds at least 4 rows of the longest kind, and 16 KB of the others
+  // a stage holds at least 4 rows of the longest kind, and 8 KB of the others
   const int longest = max2(max2(row_bytes(H), row_bytes(I)), row_bytes(d.q_dim)) * 4;
-  pl.stage_bytes = (max2(longest, 16 * 1024) + 127) & ~127;
+  pl.stage_bytes = (max2(longest, getenv("LCQ_STG") ? atoi(getenv("LCQ_STG")) : 8 * 1024) + 127) & ~127;
   const Shape sh = {H, I, d.qkv, d.q_dim, d.vocab};
-  const int rest = smem_map(sh, pl.ctas, 0, 0).total;
+  const int rest = smem_map(sh, d.n_layers, pl.ctas, 0, 0).total;
   pl.n_stages = (227 * 1024 - rest) / pl.stage_bytes;
   if (pl.n_stages > MAX_STAGES) pl.n_stages = MAX_STAGES;
   if (pl.n_stages < 2) return false;
-  pl.smem = static_cast<size_t>(smem_map(sh, pl.ctas, pl.stage_bytes, pl.n_stages).total);
-  pl.state_bytes = STATE_BYTES + (static_cast<size_t>(2) * H + I) * 4;
+  pl.smem = static_cast<size_t>(smem_map(sh, d.n_layers, pl.ctas, pl.stage_bytes, pl.n_stages).total);
+  pl.copies = getenv("LCQ_COPIES") ? atoi(getenv("LCQ_COPIES")) : 8;
+  pl.state_bytes = STATE_BYTES + (static_cast<size_t>(2) * H + I) * 4 * pl.copies;
   return true;
-}
-
-template <int CH>
-int launch_t(const Params& p, size_t smem, cudaStream_t stream) {
-  static thread_local int configured_device = -1;
-  int dev = 0;
-  LCQ_CUDA_TRY(cudaGetDevice(&dev));
-  if (configured_device != dev) {
-    LCQ_CUDA_TRY(cudaFuncSetAttribute(decode_step_kernel<CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    configured_device = dev;
-  }
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(p.ctas);
-  cfg.blockDim = dim3(NTHREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;           // all CTAs resident at once, or the launch fails
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, decode_step_kernel<CH>, p));
-  return LCQ_OK;
 }
 
 inline int launch(const lcq_decode_stack& d, int sm_count, cudaStream_t stream) {
@@ -520,11 +499,32 @@ inline int launch(const lcq_decode_stack& d, int sm_count, cudaStream_t stream) 
   p.sh = {d.hidden, d.inter, d.qkv, d.q_dim, d.vocab};
   p.n_layers = d.n_layers;
   p.ctas = pl.ctas;
+  p.copies = pl.copies;
+  p.copy_words = 2 * d.hidden + d.inter;
   p.stage_bytes = pl.stage_bytes; p.n_stages = pl.n_stages;
   p.o_buf = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(d.state) + STATE_BYTES);
   p.d_buf = p.o_buf + d.hidden;
   p.m_buf = p.d_buf + d.hidden;
-  return pl.chunks == 1 ? launch_t<1>(p, pl.smem, stream) : launch_t<2>(p, pl.smem, stream);
+  static thread_local int configured_device = -1;
+  int dev = 0;
+  LCQ_CUDA_TRY(cudaGetDevice(&dev));
+  if (configured_device != dev) {
+    LCQ_CUDA_TRY(cudaFuncSetAttribute(decode_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    configured_device = dev;
+  }
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(p.ctas);
+  cfg.blockDim = dim3(NTHREADS);
+  cfg.dynamicSmemBytes = pl.smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;           // all CTAs resident at once, or the launch fails
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, decode_step_kernel, p));
+  return LCQ_OK;
 }
 
 }  // namespace step

@@ -2,11 +2,13 @@
 // kernel: embedding, per layer {RMS norm, q|k|v and o projections, residual add + RMS norm, gate|up, SiLU *
 // up, down, residual add}, final norm, lm_head and greedy argmax -- the chain that locomp_b200.DecodeStack
 // runs as 8 launches a layer otherwise (examples/54_smollm2_inference.py:494-578 without the attention
-// itself; o reads a prepared buffer, so it depends on nothing in its layer and runs beside q|k|v).
+// itself; o reads a prepared buffer, so it depends on nothing in its layer and runs beside the down projection
+// before it: two phases a layer).
 //
 // What bounds it.  SmolLM2-135M has 30 layers of 2 MB: 12 us of HBM time for the whole token, but ~90
 // dependent matvecs.  As separate kernels each costs ~2 us (launch, dependency wait, first loads, drain):
-// 506 us a token.  Here
+// 506 us a token, now 297; 5 layers of width 2048 167 us, now 135.  What is left is instruction latency: a phase
+// is ~1000 dependent instructions of a warp (norm 1.2 us, tiles 1.3, publishing 0.9, waiting 1.3).  Here
 //   * one CTA per SM stays for the whole step; a producer thread streams the CTA's rows of ALL layers
 //     through one shared-memory ring (bulk copies), running ahead across layers, so that weights are there
 //     when their input is;
@@ -15,7 +17,7 @@
 //     flag: one store and one load through L2 between dependent matvecs;
 //   * every CTA keeps the hidden state and does the norms redundantly.
 // Every CTA has at least one unit of 4 rows in every phase.  So whoever has all results of a phase knows
-// that all CTAs have read what they needed for it, and a buffer that is rewritten three phases later (the
+// that all CTAs have read what they needed for it, and a buffer that is rewritten two phases later (the
 // next layer's) has no reader left.
 //
 // The CTAs wait for one another: the launch is cooperative, and every wait is bounded (on expiry the CTA
@@ -61,13 +63,13 @@ __host__ __device__ inline Smem smem_map(const Shape& s, int n_layers, int ctas,
   Smem m;
   m.stages = 0;
   m.xn = n_stages * stage_bytes;
-  m.xq = m.xn + s.hidden * 2;
+  m.xq = m.xn + 2 * s.hidden * 2;              // both norms of a layer
   m.xm = m.xq + s.q_dim * 2;
   m.hid = m.xm + s.inter * 2;
-  m.gam = m.hid + s.hidden * 2;
-  m.res = m.gam + s.hidden * 2;
+  m.gam = m.hid + 2 * s.hidden * 2;            // before and after o
+  m.res = m.gam + 2 * s.hidden * 2;
   const int per = 4;                           // a share is at most one unit above the average
-  const int rows = max2(max2((s.qkv + s.hidden) / ctas + 4 * per, 2 * s.inter / ctas + 4 * per), s.vocab / ctas + 2 * per);
+  const int rows = max2(max2((s.qkv + 2 * s.inter) / ctas + 6 * per, 2 * s.hidden / ctas + 4 * per), s.vocab / ctas + 2 * per);
   m.red = m.res + rows * 16;
   m.bars = m.red + 2 * NCW * 8;
   m.flags = m.bars + 2 * MAX_STAGES * 8;
@@ -120,21 +122,32 @@ __device__ __forceinline__ float dot8(uint32_t w, const uint4& x) {
   return p + q;
 }
 
-// The tiles of a CTA in the order in which the producer streams and the consumers use them: per layer q|k|v
-// rows, o rows, gate rows, up rows, down rows; then the lm_head.
+// The phases of a step.  0: the first layer's o.  1 + 2 l: q|k|v, gate|up and the activation of layer l -- o
+// depends on x_q alone, so it is there already and both norms of a layer follow from the down projection
+// before it.  2 + 2 l: down of layer l, and o of the next layer.  1 + 2 n_layers: the lm_head.
+enum { PART_QKV, PART_GATE, PART_UP, PART_DOWN, PART_O, PART_HEAD };
+__device__ __forceinline__ int first_part(int ph, int n_layers) {
+  return ph == 0 ? PART_O : ph > 2 * n_layers + 1 ? -1 : ph == 2 * n_layers + 1 ? PART_HEAD : (ph & 1) ? PART_QKV : PART_DOWN;
+}
+__device__ __forceinline__ int next_part(int part, int ph, int n_layers) {
+  if (part == PART_QKV || part == PART_GATE) return part + 1;
+  return part == PART_DOWN && ph < 2 * n_layers ? PART_O : -1;
+}
+
+// What a CTA streams for a part of a phase: rows of a weight and of its scales.
 struct Rows { int qkv0, qkv, hid0, hid, int0, inter, voc0, voc; };   // this CTA's shares: first row, rows
 struct Segment { const uint8_t* w; const uint8_t* s; int row0, rows, K; };
-__device__ __forceinline__ Segment segment(const Params& p, const lcq_decode_layer* table, const Rows& r, int layer, int part) {
-  Segment g;
+__device__ __forceinline__ Segment segment(const Params& p, const lcq_decode_layer* table, const Rows& r, int ph, int part) {
   const Shape& sh = p.sh;
-  if (layer == p.n_layers)
-    return {static_cast<const uint8_t*>(p.d.head_w), static_cast<const uint8_t*>(p.d.head_s), r.voc0, r.voc, sh.hidden};
-  const lcq_decode_layer* l = table + layer;
-  if (part == 0) g = {static_cast<const uint8_t*>(l->qkv_w), static_cast<const uint8_t*>(l->qkv_s), r.qkv0, r.qkv, sh.hidden};
-  else if (part == 1) g = {static_cast<const uint8_t*>(l->o_w), static_cast<const uint8_t*>(l->o_s), r.hid0, r.hid, sh.q_dim};
-  else if (part == 4) g = {static_cast<const uint8_t*>(l->down_w), static_cast<const uint8_t*>(l->down_s), r.hid0, r.hid, sh.inter};
-  else g = {static_cast<const uint8_t*>(l->gate_up_w), static_cast<const uint8_t*>(l->gate_up_s), r.int0 + (part == 3 ? sh.inter : 0), r.inter, sh.hidden};
-  return g;
+  const lcq_decode_layer* l = table + (part == PART_O ? ph / 2 : (ph - 1) / 2);
+  switch (part) {
+    case PART_QKV: return {static_cast<const uint8_t*>(l->qkv_w), static_cast<const uint8_t*>(l->qkv_s), r.qkv0, r.qkv, sh.hidden};
+    case PART_GATE: return {static_cast<const uint8_t*>(l->gate_up_w), static_cast<const uint8_t*>(l->gate_up_s), r.int0, r.inter, sh.hidden};
+    case PART_UP: return {static_cast<const uint8_t*>(l->gate_up_w), static_cast<const uint8_t*>(l->gate_up_s), sh.inter + r.int0, r.inter, sh.hidden};
+    case PART_DOWN: return {static_cast<const uint8_t*>(l->down_w), static_cast<const uint8_t*>(l->down_s), r.hid0, r.hid, sh.inter};
+    case PART_O: return {static_cast<const uint8_t*>(l->o_w), static_cast<const uint8_t*>(l->o_s), r.hid0, r.hid, sh.q_dim};
+    default: return {static_cast<const uint8_t*>(p.d.head_w), static_cast<const uint8_t*>(p.d.head_s), r.voc0, r.voc, sh.hidden};
+  }
 }
 
 // Shared memory by 32-bit addresses: generic pointers would take two registers each and a slower load.
@@ -149,15 +162,15 @@ __device__ __forceinline__ float ld_half(uint32_t a) {
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
   return __half2float(__ushort_as_half(v));
 }
-__device__ __forceinline__ void st128(uint32_t a, float x, float y, float z, float w) {
-  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
-}
-__device__ __forceinline__ void st32(uint32_t a, float x) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory"); }
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   return v;
 }
+__device__ __forceinline__ void st128(uint32_t a, float x, float y, float z, float w) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+__device__ __forceinline__ void st32(uint32_t a, float x) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory"); }
 
 // A lane's sums over the words word0, word0 + step, ... of NR rows that are NCW rows apart.
 // w, sc, x: addresses of the first row's weights and scales and of the input.
@@ -234,16 +247,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
   const Rows& mine = *reinterpret_cast<const Rows*>(smem + L.rows);
   const int step_h = tile_rows(p.stage_bytes, sh.hidden), step_q = tile_rows(p.stage_bytes, sh.q_dim), step_i = tile_rows(p.stage_bytes, sh.inter);
 
-  if (warp == NCW) {
-    // ------------------------------------------------------------ producer: one thread, all layers in order
+  if (warp >= NCW) {
+    // ------------------------------------------------------------ producer: one thread, all phases in order
     if (lane == 0) {
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int layer = 0; layer <= p.n_layers && ok; ++layer) {
-        for (int part = 0; part < (layer < p.n_layers ? 5 : 1) && ok; ++part) {
-          const Segment g = segment(p, reinterpret_cast<const lcq_decode_layer*>(smem + L.table), mine, layer, part);
-          const int step = part == 1 && layer < p.n_layers ? step_q : part == 4 ? step_i : step_h;
+      for (int ph = 0, part; ok && (part = first_part(ph, p.n_layers)) >= 0; ++ph) {
+        for (; part >= 0 && ok; part = next_part(part, ph, p.n_layers)) {
+          const Segment g = segment(p, reinterpret_cast<const lcq_decode_layer*>(smem + L.table), mine, ph, part);
+          const int step = part == PART_O ? step_q : part == PART_DOWN ? step_i : step_h;
           for (int r = 0; r < g.rows; r += step) {
             const int rows = g.rows - r < step ? g.rows - r : step;
             if (*flag_abort || !mbar_wait_bounded(&empty[s], phase ^ 1u)) { *flag_abort = 1; atomicExch(&g_device_status, 50); ok = false; break; }
@@ -263,7 +276,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
     const uint32_t xn = base + L.xn, xq = base + L.xq, xm = base + L.xm;
     __half* xn_p = reinterpret_cast<__half*>(smem + L.xn);
     float* red = reinterpret_cast<float*>(smem + L.red);
-    const uint32_t tag0 = *smem_epoch * static_cast<uint32_t>(3 * p.n_layers) + 1u;
+    const uint32_t tag0 = *smem_epoch * static_cast<uint32_t>(2 * p.n_layers + 1) + 1u;
     const int copy = (b % p.copies) * p.copy_words;
     int s = 0;
     uint32_t phase = 0;
@@ -296,66 +309,80 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
       v[0] = __ushort_as_half(static_cast<unsigned short>(w.x >> 16)); v[1] = __ushort_as_half(static_cast<unsigned short>(w.y >> 16));
       v[2] = __ushort_as_half(static_cast<unsigned short>(w.z >> 16)); v[3] = __ushort_as_half(static_cast<unsigned short>(w.w >> 16));
     };
-    // A thread's share of the hidden state and of the next norm's weights, 4 values of every 4 * NCT, lies in
+    // A thread's share of the hidden state and of the next norms' weights, 4 values of every 4 * NCT, lies in
     // shared memory: in registers they cost the matvec loops theirs, and a spill goes to L2 here.
     __half* hid = reinterpret_cast<__half*>(smem + L.hid);
-    const uint32_t gam = smem_u32(smem + L.gam);
     const __half* next_norm = static_cast<const __half*>(p.d.norms);
     int norms_left = 2 * p.n_layers + 1;
-    const auto fetch_norm = [&]() {            // a phase ahead: they may come from HBM
-      if (norms_left > 0) {
-        for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(gam + 2 * i), "l"(next_norm + i) : "memory");
-      }
-      next_norm += sh.hidden;
-      --norms_left;
+    const auto fetch_norms = [&]() {           // a phase ahead: they may come from HBM
+      const int two = norms_left > 1 ? 2 * sh.hidden : norms_left * sh.hidden;
+      for (int i = 4 * tid; i < two; i += 4 * NCT)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(base + L.gam + 2 * i), "l"(next_norm + i) : "memory");
+      next_norm += two;
+      norms_left -= 2;
     };
-    // hidden (+= what was published in src); xn = rms_norm(hidden) * weight
-    const auto norm = [&](const uint32_t* src, uint32_t tag) {
-      float ss = 0.0f;
+    // hidden += the down projection; x = rms_norm(hidden); hidden += the o projection; x2 = rms_norm(hidden)
+    // (the first phase has no down projection before it, the last one no o)
+    const auto norms = [&](const uint32_t* down, const uint32_t* o, uint32_t tag) {
+      float ss = 0.0f, ss2 = 0.0f;
       for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT) {
-        __half h[4];
+        __half h[4], v[4];
         *reinterpret_cast<uint2*>(h) = *reinterpret_cast<const uint2*>(hid + i);
-        if (src != nullptr) {
-          __half v[4];
-          take(src + i, tag, v);
+        if (down != nullptr) {
+          take(down + i, tag, v);
 #pragma unroll
           for (int e = 0; e < 4; ++e) h[e] = __float2half_rn(__half2float(h[e]) + __half2float(v[e]));
-          *reinterpret_cast<uint2*>(hid + i) = *reinterpret_cast<const uint2*>(h);
         }
+        *reinterpret_cast<uint2*>(hid + i) = *reinterpret_cast<const uint2*>(h);
 #pragma unroll
         for (int e = 0; e < 4; ++e) ss = fmaf(__half2float(h[e]), __half2float(h[e]), ss);
-      }
+        if (o != nullptr) {
+          take(o + i, tag, v);
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-      if (lane == 0) red[warp] = ss;
+          for (int e = 0; e < 4; ++e) h[e] = __float2half_rn(__half2float(h[e]) + __half2float(v[e]));
+          *reinterpret_cast<uint2*>(hid + sh.hidden + i) = *reinterpret_cast<const uint2*>(h);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) ss2 = fmaf(__half2float(h[e]), __half2float(h[e]), ss2);
+        }
+      }
+      ss = warp_sum(ss);
+      ss2 = warp_sum(ss2);
+      if (lane == 0) { red[warp] = ss; red[NCW + warp] = ss2; }
       asm volatile("cp.async.wait_all;" ::: "memory");
       named_bar_sync(BAR_C, NCT);
-      float total = 0.0f;
+      float total[2];
 #pragma unroll
-      for (int i = 0; i < NCW / 4; ++i) {
-        const float4 q = reinterpret_cast<const float4*>(red)[i];
-        total += (q.x + q.y) + (q.z + q.w);
+      for (int j = 0; j < 2; ++j) {
+        total[j] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NCW / 4; ++i) {
+          const float4 q = reinterpret_cast<const float4*>(red)[j * (NCW / 4) + i];
+          total[j] += (q.x + q.y) + (q.z + q.w);
+        }
+        total[j] = rsqrtf(total[j] / static_cast<float>(sh.hidden) + p.d.eps);
       }
-      const float rms = rsqrtf(total / static_cast<float>(sh.hidden) + p.d.eps);
       for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT) {
-        __half o[4], g[4], h[4];
-        *reinterpret_cast<uint2*>(g) = *reinterpret_cast<const uint2*>(smem + L.gam + 2 * i);
-        *reinterpret_cast<uint2*>(h) = *reinterpret_cast<const uint2*>(hid + i);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[e] = __float2half_rn(__half2float(h[e]) * rms * __half2float(g[e]));
-        *reinterpret_cast<uint2*>(xn_p + i) = *reinterpret_cast<const uint2*>(o);
+        for (int j = 0; j < 2; ++j) {
+          __half g[4], h[4], o4[4];
+          *reinterpret_cast<uint2*>(g) = *reinterpret_cast<const uint2*>(smem + L.gam + 2 * (j * sh.hidden + i));
+          *reinterpret_cast<uint2*>(h) = *reinterpret_cast<const uint2*>(hid + j * sh.hidden + i);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o4[e] = __float2half_rn(__half2float(h[e]) * total[j] * __half2float(g[e]));
+          *reinterpret_cast<uint2*>(xn_p + j * sh.hidden + i) = *reinterpret_cast<const uint2*>(o4);
+          if (j == 1 && o != nullptr) *reinterpret_cast<uint2*>(hid + i) = *reinterpret_cast<const uint2*>(h);
+        }
       }
       named_bar_sync(BAR_C, NCT);
-      fetch_norm();
+      fetch_norms();
     };
-    const auto sum4 = [&](int i) {
+    const auto row_sum = [&](int i) {
       const uint4 v = ld128(base + L.res + i * 16);
       return (__uint_as_float(v.x) + __uint_as_float(v.y)) + (__uint_as_float(v.z) + __uint_as_float(v.w));
     };
 
     // embedding; the prepared input of the o projections
-    fetch_norm();
+    fetch_norms();
     {
       const int id = *static_cast<const int*>(p.d.token);
       const bool known = id >= 0 && id < sh.vocab;
@@ -367,14 +394,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
         *reinterpret_cast<uint4*>(smem + L.xq + 2 * i) = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.d.x_q) + i);
     }
 
-    // Phases 3 l, 3 l + 1, 3 l + 2 of layer l: {norm, q|k|v and o}, {norm, gate|up, activation}, {down}; then the
-    // lm_head.  One loop body for all of them: three times the code would be fetched anew every phase.
-    const int last = 3 * p.n_layers;
+    // One loop body for all phases: code that runs once a phase is fetched anew each time.
     __half* out = static_cast<__half*>(p.d.outputs);     // this layer's q|k|v, o, gate|up, down
-    for (int ph = 0, kind = 0; ph <= last; ++ph) {
+    const int layer_out = sh.qkv + 2 * sh.hidden + 2 * sh.inter, last = 2 * p.n_layers + 1;
+    for (int ph = 0; ph <= last; ++ph) {
       const uint32_t tag = (tag0 + ph) & 0xFFFFu, before = (tag - 1u) & 0xFFFFu;
-      const bool head = ph == last;
-      if (kind == 2) {
+      const bool wide = (ph & 1) && ph != last;          // q|k|v, gate|up
+      if (ph & 1) {
+        norms(ph == 1 ? nullptr : p.d_buf + copy, ph == last ? nullptr : p.o_buf + copy, before);
+      } else if (ph != 0) {
         for (int i = 4 * tid; i < sh.inter; i += 4 * NCT) {
           __half v[4];
           take(p.m_buf + copy + i, before, v);
@@ -382,42 +410,48 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
         }
         named_bar_sync(BAR_C, NCT);
       } else {
-        norm(ph == 0 ? nullptr : (kind == 0 ? p.d_buf : p.o_buf) + copy, before);
+        named_bar_sync(BAR_C, NCT);
       }
-      // the rows that are published (pub, from sum `first` on) and those beside them
-      const int pub = head ? 0 : kind == 1 ? mine.inter : mine.hid;
-      const int first = kind == 0 ? (head ? mine.voc : mine.qkv) : 0;
-      for (int part = 0; part < (kind == 2 || head ? 1 : 2); ++part) {
-        const int n = part == 1 ? pub : kind == 0 ? first : pub;
-        const bool o_rows = kind == 0 && part == 1;
-        use_tiles(n, kind == 2 ? sh.inter : o_rows ? sh.q_dim : sh.hidden, kind == 2 ? step_i : o_rows ? step_q : step_h,
-                  kind == 2 ? xm : o_rows ? xq : xn, part == 0 ? 0 : kind == 0 ? first : pub);
+      int sums = 0;
+      for (int part = first_part(ph, p.n_layers); part >= 0; part = next_part(part, ph, p.n_layers)) {
+        const int n = part == PART_QKV ? mine.qkv : part == PART_HEAD ? mine.voc : part <= PART_UP ? mine.inter : mine.hid;
+        use_tiles(n, part == PART_DOWN ? sh.inter : part == PART_O ? sh.q_dim : sh.hidden,
+                  part == PART_DOWN ? step_i : part == PART_O ? step_q : step_h,
+                  part == PART_DOWN ? xm : part == PART_O ? xq : part == PART_GATE || part == PART_UP ? xn + 2 * sh.hidden : xn, sums);
+        sums += n;
       }
       named_bar_sync(BAR_C, NCT);
-      if (head) break;
-      {
-        uint32_t* dst = kind == 0 ? p.o_buf + mine.hid0 : kind == 1 ? p.m_buf + mine.int0 : p.d_buf + mine.hid0;
-        __half* plain = kind == 0 ? out + sh.qkv + mine.hid0 : kind == 1 ? out + sh.qkv + sh.hidden + mine.int0
-                                                                        : out + sh.qkv + sh.hidden + 2 * sh.inter + mine.hid0;
-        // warp w writes copies w, w + NCW, ...; the first also what the caller sees
-        for (int c = warp; c < p.copies; c += NCW) {
-          for (int i = lane; i < pub; i += 32) {
-            __half v = __float2half_rn(sum4(first + i));
-            if (c == 0) plain[i] = v;
-            if (kind == 1) {
-              const __half u = __float2half_rn(sum4(pub + i));
-              const float x = __half2float(v);
-              if (c == 0) plain[sh.inter + i] = u;
-              v = __float2half_rn((x * (1.0f / (1.0f + expf(-x)))) * __half2float(u));
-              if (c == 0 && ph == last - 2) static_cast<__half*>(p.d.mlp_out)[mine.int0 + i] = v;
+      if (ph == last) break;
+      // warp w writes copies w, w + NCW, ... of what is published; the first also what the caller sees
+      for (int c = warp; c < p.copies; c += NCW) {
+        if (wide) {
+          for (int i = lane; i < mine.inter; i += 32) {
+            const __half gate = __float2half_rn(row_sum(mine.qkv + i)), up = __float2half_rn(row_sum(mine.qkv + mine.inter + i));
+            const float x = __half2float(gate);
+            const __half v = __float2half_rn((x * (1.0f / (1.0f + expf(-x)))) * __half2float(up));
+            publish(p.m_buf + c * p.copy_words + mine.int0 + i, v, tag);
+            if (c == 0) {
+              __half* o = out + sh.qkv + sh.hidden + mine.int0 + i;
+              o[0] = gate;
+              o[sh.inter] = up;
+              if (ph == last - 2) static_cast<__half*>(p.d.mlp_out)[mine.int0 + i] = v;
             }
-            publish(dst + c * p.copy_words + i, v, tag);
+          }
+        } else {
+          // down rows of this layer, then o rows of the next (phase 0: o rows only; the last layer: down only)
+          const int n_down = ph == 0 ? 0 : mine.hid;
+          for (int i = lane; i < sums; i += 32) {
+            const __half v = __float2half_rn(row_sum(i));
+            const bool down = i < n_down;
+            const int row = mine.hid0 + (down ? i : i - n_down);
+            publish((down ? p.d_buf : p.o_buf) + c * p.copy_words + row, v, tag);
+            if (c == 0) (down ? out + layer_out - sh.hidden : (ph == 0 ? out : out + layer_out) + sh.qkv)[row] = v;
           }
         }
-        if (kind == 0)
-          for (int i = tid; i < first; i += NCT) out[mine.qkv0 + i] = __float2half_rn(sum4(i));
       }
-      if (++kind == 3) { kind = 0; out += sh.qkv + 2 * sh.hidden + 2 * sh.inter; }
+      if (wide)
+        for (int i = tid; i < mine.qkv; i += NCT) out[mine.qkv0 + i] = __float2half_rn(row_sum(i));
+      if (!(ph & 1) && ph != 0) out += layer_out;
     }
     if (b == 0) {
       for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT) {
@@ -429,7 +463,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
     // the key of a logit orders as np.argmax does: by value, NaN above all, the lowest index among equals
     unsigned long long key = 0;
     for (int i = tid; i < n; i += NCT) {
-      const __half v = __float2half_rn(sum4(i));
+      const __half v = __float2half_rn(row_sum(i));
       static_cast<__half*>(p.d.logits)[v0 + i] = v;
       const float f = __half2float(v) + 0.0f;            // -0 counts as 0
       uint32_t u = __float_as_uint(f);
@@ -472,16 +506,16 @@ inline bool make_plan(const lcq_decode_stack& d, int sm_count, Plan& pl) {
   if (I / 4 < units) units = I / 4;
   if (d.vocab / 4 < units) units = d.vocab / 4;
   pl.ctas = sm_count < units ? sm_count : units;
-  // a stage holds at least 4 rows of the longest kind, and 8 KB of the others
+  // a stage holds at least 4 rows of the longest kind, and 24 KB of the others
   const int longest = max2(max2(row_bytes(H), row_bytes(I)), row_bytes(d.q_dim)) * 4;
-  pl.stage_bytes = (max2(longest, getenv("LCQ_STG") ? atoi(getenv("LCQ_STG")) : 8 * 1024) + 127) & ~127;
+  pl.stage_bytes = (max2(longest, 24 * 1024) + 127) & ~127;
   const Shape sh = {H, I, d.qkv, d.q_dim, d.vocab};
   const int rest = smem_map(sh, d.n_layers, pl.ctas, 0, 0).total;
   pl.n_stages = (227 * 1024 - rest) / pl.stage_bytes;
   if (pl.n_stages > MAX_STAGES) pl.n_stages = MAX_STAGES;
   if (pl.n_stages < 2) return false;
   pl.smem = static_cast<size_t>(smem_map(sh, d.n_layers, pl.ctas, pl.stage_bytes, pl.n_stages).total);
-  pl.copies = getenv("LCQ_COPIES") ? atoi(getenv("LCQ_COPIES")) : 8;
+  pl.copies = 8;                               // 30 layers of width 576: 1 copy 420 us, 2 363, 4 337, 8 332, 16 325 (an earlier build)
   pl.state_bytes = STATE_BYTES + (static_cast<size_t>(2) * H + I) * 4 * pl.copies;
   return true;
 }

@@ -1,4 +1,4 @@
-// Warp-per-row quantized matmul on CUDA cores: the general kernel (any K % G == 0, any
+// Quantized matmul on CUDA cores, a warp per row (per four rows when M > 1): the general kernels (any K % G == 0, any
 // dtype combination, float32 math end to end).  It is the path for the reference's own
 // dtypes -- float32 x / scales / out, M = 1 (examples/38_quantized_matmul.py:30-134) --
 // and the fallback for shapes the tensor-core kernels do not take.
@@ -164,6 +164,109 @@ __global__ void __launch_bounds__(256) gemv_simt_kernel(const XT* __restrict__ x
   }
 }
 
+// Several rows of x (M > 1), float32 math end to end: a warp owns R = 4 weight rows and MT rows of x, lanes
+// stride over K in chunks of 8.  With one weight row per warp every warp re-read all of x -- M * 4 bytes of
+// it from L1 per half byte of weight -- and that bound the kernel; here a chunk of x serves four rows and a
+// dequantised weight MT rows of x.  `splits` warps of a block share a row group's K when N alone gives too few
+// warps, and add up in shared memory.
+// M = 4, K = 2176, N = 8056, int8, f16: 21.1 us before, now XX us; M = 8, K = 8192, N = 7000, int4, f32: XX.
+template <int WBITS, typename XT, typename ST, typename OT, int MT>
+__global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w,
+                                                        const ST* __restrict__ scales, OT* __restrict__ out,
+                                                        int M, int N, int K, int G, int gshift, int split_shift) {
+  constexpr int R = 4;
+  __shared__ float red[8][R * MT];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int splits = 1 << split_shift, part = warp & (splits - 1);
+  const int n0 = (blockIdx.x * (8 >> split_shift) + (warp >> split_shift)) * R;
+  const int m0 = blockIdx.y * MT;
+  const int nchunks = K >> 3, ns = K / G, row_bytes = WBITS == 4 ? (K >> 1) : K;
+  const uint8_t* wrow[R];
+  const ST* srow[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {                // (rows past N read the last one and are not written)
+    const int n = n0 + r < N ? n0 + r : N - 1;
+    wrow[r] = w + static_cast<long long>(n) * row_bytes;
+    srow[r] = scales + static_cast<long long>(n) * ns;
+  }
+  const XT* xrow[MT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) xrow[m] = x + static_cast<long long>(m0 + m < M ? m0 + m : M - 1) * K;
+  float acc[MT][R];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[m][r] = 0.0f;
+  }
+  uint32_t lo[R], hi[R];
+  float sc[R];
+  const auto fetch = [&](int c) {
+    if (c >= nchunks) return;
+    const int g = gshift >= 0 ? (c << 3) >> gshift : (c << 3) / G;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (WBITS == 4) {
+        lo[r] = __ldg(reinterpret_cast<const uint32_t*>(wrow[r]) + c);
+      } else {
+        const uint2 two = __ldg(reinterpret_cast<const uint2*>(wrow[r]) + c);
+        lo[r] = two.x; hi[r] = two.y;
+      }
+      sc[r] = to_f32<ST>(__ldg(srow[r] + g));
+    }
+  };
+  int c = part * 32 + lane;
+  fetch(c);                                    // weights are constants: ahead of the wait for the preceding kernel
+  griddep_launch_dependents();
+  griddep_wait();
+  for (; c < nchunks; c += 32 << split_shift) {
+    float wq[R][8], s[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      s[r] = sc[r];
+      if (WBITS == 4) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) wq[r][i] = small_uint_to_f32((lo[r] >> (4 * i)) & 15u) - 8.0f;
+      } else {
+        float f[4];
+        int8x4_to_f32(lo[r], f); wq[r][0] = f[0]; wq[r][1] = f[1]; wq[r][2] = f[2]; wq[r][3] = f[3];
+        int8x4_to_f32(hi[r], f); wq[r][4] = f[0]; wq[r][5] = f[1]; wq[r][6] = f[2]; wq[r][7] = f[3];
+      }
+    }
+    fetch(c + (32 << split_shift));
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      float xv[8];
+      load8<XT>(xrow[m] + (c << 3), xv);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float p = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) p = fmaf(xv[i], wq[r][i], p);
+        acc[m][r] = fmaf(s[r], p, acc[m][r]);
+      }
+    }
+  }
+  // lane m * R + r collects output (m, r)
+  float mine = 0.0f;
+#pragma unroll
+  for (int i = 0; i < R * MT; ++i) {
+    float v = acc[i / R][i % R];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    if (lane == i) mine = v;
+  }
+  if (splits > 1) {
+    if (lane < R * MT) red[warp][lane] = mine;
+    __syncthreads();
+    if (part != 0) return;
+    if (lane < R * MT) {
+      for (int q = 1; q < splits; ++q) mine += red[warp + q][lane];
+    }
+  }
+  const int m = m0 + lane / R, n = n0 + lane % R;
+  if (lane < R * MT && m < M && n < N) out[static_cast<long long>(m) * N + n] = from_f32<OT>(mine);
+}
+
 template <int WBITS, typename XT, typename ST, typename OT>
 int launch_gemv_simt(const void* x, const void* w, const void* s, void* out, int M, int N, int K, int G,
                      cudaStream_t stream) {
@@ -190,10 +293,28 @@ int launch_gemv_simt(const void* x, const void* w, const void* s, void* out, int
     LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_simt_kernel<WBITS, XT, ST, OT, MT_, VEC_>, xp, wp, sp, \
                                     op, M, N, K, G));                                                \
   } while (0)
-  if (vec) {
-    if (M == 1) LCQ_SIMT_LAUNCH(1, true);
-    else if (M == 2) LCQ_SIMT_LAUNCH(2, true);
-    else LCQ_SIMT_LAUNCH(4, true);
+  if (vec && M > 1) {
+    // 8 warps a block; K is shared while the warps fill less than two thirds of the SMs twice over (8 warps each
+    // way) and every one of them still has a chunk per lane
+    int split = 0;
+    const long long groups = (N + 3) / 4;
+    const int m_blocks = (M + 7) / 8;
+    while (split < 3 && ((groups * m_blocks) << split) < 148 * 12 && (K >> 3) >= (64 << split)) ++split;
+    int gshift = -1;
+    if ((G & (G - 1)) == 0) { gshift = 0; while ((1 << gshift) < G) ++gshift; }
+    const unsigned blocks = static_cast<unsigned>((groups + (8 >> split) - 1) / (8 >> split));
+    if (M == 2) {
+      cfg.gridDim = dim3(blocks, 1);
+      LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 2>, xp, wp, sp, op, M, N, K, G, gshift, split));
+    } else if (M <= 4) {
+      cfg.gridDim = dim3(blocks, 1);
+      LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 4>, xp, wp, sp, op, M, N, K, G, gshift, split));
+    } else {
+      cfg.gridDim = dim3(blocks, m_blocks);
+      LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 8>, xp, wp, sp, op, M, N, K, G, gshift, split));
+    }
+  } else if (vec) {
+    LCQ_SIMT_LAUNCH(1, true);
   } else {
     if (M == 1) LCQ_SIMT_LAUNCH(1, false);
     else LCQ_SIMT_LAUNCH(4, false);

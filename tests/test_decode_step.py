@@ -1,0 +1,60 @@
+"""The one-kernel decode step against the chain of separate kernels it stands for (same arithmetic, other order
+of the float32 sums): per result a relative 2-norm error of 1e-2 -- fp16 rounding (2^-11) of each stored
+value, compounded over at most four layers."""
+import pytest
+import torch
+
+import locomp_b200 as L
+from locomp_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+# fewer rows than SMs in some phase, hidden beyond one pass of the threads, rows that fill no tile, many tiles
+SHAPES = [dict(layers=1, hidden=64, inter=64, q_heads=1, kv_heads=1, vocab=4), dict(layers=2, hidden=128, inter=192, q_heads=2, kv_heads=1, vocab=1000),
+          dict(layers=4, hidden=576, inter=1536, q_heads=9, kv_heads=3, vocab=49152), dict(layers=3, hidden=640, inter=2624, q_heads=7, kv_heads=2, vocab=5004),
+          dict(layers=2, hidden=2112, inter=5632, q_heads=33, kv_heads=3, vocab=3000), dict(layers=2, hidden=2048, inter=8192, q_heads=32, kv_heads=32, vocab=16384)]
+
+
+def _results(st):
+    return [t.clone() for t in (st.logits, st.hidden, st.normed, st.mlp, st.outputs)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_matches_the_chain_of_kernels(shape):
+    st = L.DecodeStack(fused=True, glue=True, seed=7, **shape)
+    assert st._desc is not None and st.launches_per_step == 1
+    st.token.fill_(shape["vocab"] // 2)
+    for op in st.ops:
+        op()
+    ref = _results(st)
+    for t in (st.logits, st.hidden, st.normed, st.mlp, st.outputs):
+        t.fill_(float("nan"))
+    st.step()
+    got = _results(st)
+    for g, r in zip(got, ref):
+        assert torch.isfinite(r).all()
+        assert float((g.double() - r.double()).norm()) <= 1e-2 * float(r.double().norm())
+    assert int(st.next_token) == int(st.logits.float().argmax())
+    st.capture()
+    for _ in range(3):                        # again and again on the same state: the same bits
+        st.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(_results(st), got))
+    assert _lib.lib().lcq_check_device_status(None) == 0, _lib.lib().lcq_last_error()
+
+
+def test_unknown_token_is_reported():
+    st = L.DecodeStack(layers=1, hidden=128, inter=192, q_heads=2, kv_heads=1, vocab=1000, fused=True, glue=True)
+    st.token.fill_(1000)
+    st.step()
+    assert _lib.lib().lcq_check_device_status(None) == _lib.ERR_TIMEOUT and b"code 40" in _lib.lib().lcq_last_error()
+    assert float(st.hidden.abs().max()) >= 0.0 and _lib.lib().lcq_check_device_status(None) == 0
+
+
+def test_other_shapes_and_types_keep_the_chain():
+    st = L.DecodeStack(layers=1, hidden=96, inter=192, q_heads=2, kv_heads=1, vocab=1000, fused=True, glue=True)
+    assert st._desc is None and st.launches_per_step == len(st.ops)
+    st = L.DecodeStack(layers=1, hidden=128, inter=192, q_heads=2, kv_heads=1, vocab=1000, fused=True, glue=True, dtype=torch.bfloat16)
+    assert st._desc is None
+    st.step()
+    assert torch.isfinite(st.logits).all()

@@ -164,12 +164,13 @@ __global__ void __launch_bounds__(256) gemv_simt_kernel(const XT* __restrict__ x
   }
 }
 
-// Several rows of x (M > 1), float32 math end to end: a warp owns R = 4 weight rows and MT rows of x, lanes
+// Several rows of x, or one and a weight beyond 2 Mi elements; float32 math end to end: a warp owns R = 4 weight rows and MT rows of x, lanes
 // stride over K in chunks of 8.  With one weight row per warp every warp re-read all of x -- M * 4 bytes of
 // it from L1 per half byte of weight -- and that bound the kernel; here a chunk of x serves four rows and a
 // dequantised weight MT rows of x.  `splits` warps of a block share a row group's K when N alone gives too few
 // warps, and add up in shared memory.
-// M = 4, K = 2176, N = 8056, int8, f16: 21.1 us before, now XX us; M = 8, K = 8192, N = 7000, int4, f32: XX.
+// M = 4, K = 2176, N = 8056, int8, f16: 23.8 us before, now 10.5; M = 8, K = 8192, N = 7000, int4, f32: 129, now 61;
+// M = 1, K = 8192, N = 16000, int8, f32: 56.7, now 36.7.
 template <int WBITS, typename XT, typename ST, typename OT, int MT>
 __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w,
                                                         const ST* __restrict__ scales, OT* __restrict__ out,
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[m][r] = 0.0f;
   }
-  uint32_t lo[R], hi[R];
+  uint32_t lo[R], hi[R];                       // the next chunk, on its way (four chunks ahead cost occupancy: 37 -> 90 us for one case)
   float sc[R];
   const auto fetch = [&](int c) {
     if (c >= nchunks) return;
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
       s[r] = sc[r];
       if (WBITS == 4) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) wq[r][i] = small_uint_to_f32((lo[r] >> (4 * i)) & 15u) - 8.0f;
+        for (int i = 0; i < 8; ++i) wq[r][i] = __uint_as_float(0x4B000000u | ((lo[r] >> (4 * i)) & 15u)) - 8388616.0f;   // 2^23 + q, exact
       } else {
         float f[4];
         int8x4_to_f32(lo[r], f); wq[r][0] = f[0]; wq[r][1] = f[1]; wq[r][2] = f[2]; wq[r][3] = f[3];
@@ -293,26 +294,19 @@ int launch_gemv_simt(const void* x, const void* w, const void* s, void* out, int
     LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_simt_kernel<WBITS, XT, ST, OT, MT_, VEC_>, xp, wp, sp, \
                                     op, M, N, K, G));                                                \
   } while (0)
-  if (vec && M > 1) {
+  if (vec && (M > 1 || static_cast<long long>(N) * K > (1LL << 21))) {
     // 8 warps a block; K is shared while the warps fill less than two thirds of the SMs twice over (8 warps each
     // way) and every one of them still has a chunk per lane
     int split = 0;
     const long long groups = (N + 3) / 4;
-    const int m_blocks = (M + 7) / 8;
+    const int mt = M == 1 ? 1 : M == 2 ? 2 : 4, m_blocks = (M + mt - 1) / mt;
     while (split < 3 && ((groups * m_blocks) << split) < 148 * 12 && (K >> 3) >= (64 << split)) ++split;
     int gshift = -1;
     if ((G & (G - 1)) == 0) { gshift = 0; while ((1 << gshift) < G) ++gshift; }
-    const unsigned blocks = static_cast<unsigned>((groups + (8 >> split) - 1) / (8 >> split));
-    if (M == 2) {
-      cfg.gridDim = dim3(blocks, 1);
-      LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 2>, xp, wp, sp, op, M, N, K, G, gshift, split));
-    } else if (M <= 4) {
-      cfg.gridDim = dim3(blocks, 1);
-      LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 4>, xp, wp, sp, op, M, N, K, G, gshift, split));
-    } else {
-      cfg.gridDim = dim3(blocks, m_blocks);
-      LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 8>, xp, wp, sp, op, M, N, K, G, gshift, split));
-    }
+    cfg.gridDim = dim3(static_cast<unsigned>((groups + (8 >> split) - 1) / (8 >> split)), m_blocks);
+    if (mt == 1) LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 1>, xp, wp, sp, op, M, N, K, G, gshift, split));
+    else if (mt == 2) LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 2>, xp, wp, sp, op, M, N, K, G, gshift, split));
+    else LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 4>, xp, wp, sp, op, M, N, K, G, gshift, split));
   } else if (vec) {
     LCQ_SIMT_LAUNCH(1, true);
   } else {

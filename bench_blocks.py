@@ -136,7 +136,7 @@ class Problem:
     def kernel_name(self) -> str:
         _lib = self.ctx._lib
         return {_lib.ALGO_SIMT: "gemv_simt_kernel", _lib.ALGO_GEMV_TC: "w4a16_gemv_kernel", _lib.ALGO_GEMM_TC: "w4a16_gemm_kernel",
-                _lib.ALGO_GEMV_W8: "w8_gemv_kernel"}.get(self.selected, "?")
+                _lib.ALGO_GEMV_W8: "gemv_rows_kernel"}.get(self.selected, "?")
 
 
 # ------------------------------------------------------------------------------------------ roofline of the dominant kernel

@@ -370,6 +370,55 @@ PyObject* bind(PyObject*, PyObject* args) {
   Py_RETURN_NONE;
 }
 
+// The base class of QuantLinear: its weights as members and the call itself in native code, so that a call
+// enters no Python frame (4.0 -> 3.7 us for the smallest).  What is not `linear(x)` or `linear(x, out)` goes to the
+// method _general of the subclass.
+struct Linear {
+  PyObject_HEAD
+  PyObject *w, *scales, *group_size, *bits;
+};
+PyObject* general_name = nullptr;
+
+PyObject* linear_call(PyObject* self, PyObject* args, PyObject* kwargs) {
+  Linear* l = reinterpret_cast<Linear*>(self);
+  const Py_ssize_t n = PyTuple_GET_SIZE(args);
+  if ((kwargs == nullptr || PyDict_GET_SIZE(kwargs) == 0) && (n == 1 || n == 2) && l->w && l->scales && l->group_size && l->bits) {
+    PyObject* const a[7] = {PyTuple_GET_ITEM(args, 0), l->w, l->scales, l->group_size, l->bits, n == 2 ? PyTuple_GET_ITEM(args, 1) : Py_None, Py_None};
+    PyObject* r;
+    {
+      HANDLE_TH_ERRORS
+      r = matmul(nullptr, a, 7);
+      END_HANDLE_TH_ERRORS
+    }
+    if (r != Py_NotImplemented) return r;
+    Py_DECREF(r);
+  }
+  PyObject* method = PyObject_GetAttr(self, general_name);
+  if (!method) return nullptr;
+  PyObject* r = PyObject_Call(method, args, kwargs);
+  Py_DECREF(method);
+  return r;
+}
+int linear_traverse(PyObject* self, visitproc visit, void* arg) {
+  Linear* l = reinterpret_cast<Linear*>(self);
+  Py_VISIT(l->w); Py_VISIT(l->scales); Py_VISIT(l->group_size); Py_VISIT(l->bits);
+  return 0;
+}
+int linear_clear(PyObject* self) {
+  Linear* l = reinterpret_cast<Linear*>(self);
+  Py_CLEAR(l->w); Py_CLEAR(l->scales); Py_CLEAR(l->group_size); Py_CLEAR(l->bits);
+  return 0;
+}
+void linear_dealloc(PyObject* self) {
+  PyObject_GC_UnTrack(self);
+  linear_clear(self);
+  Py_TYPE(self)->tp_free(self);
+}
+PyMemberDef linear_members[] = {{"w", Py_T_OBJECT_EX, offsetof(Linear, w), 0, nullptr}, {"scales", Py_T_OBJECT_EX, offsetof(Linear, scales), 0, nullptr},
+                                {"group_size", Py_T_OBJECT_EX, offsetof(Linear, group_size), 0, nullptr},
+                                {"bits", Py_T_OBJECT_EX, offsetof(Linear, bits), 0, nullptr}, {nullptr, 0, 0, 0, nullptr}};
+PyTypeObject linear_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
 // A C++ exception (out of memory, a CUDA error seen by torch) becomes the Python exception torch gives it.
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
@@ -387,4 +436,20 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_torch_calls", nullptr, -1, method
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__torch_calls(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__torch_calls(void) {
+  general_name = PyUnicode_InternFromString("_general");
+  linear_type.tp_name = "locomp_b200._torch_calls.LinearBase";
+  linear_type.tp_basicsize = sizeof(Linear);
+  linear_type.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE | Py_TPFLAGS_HAVE_GC;
+  linear_type.tp_call = linear_call;
+  linear_type.tp_traverse = linear_traverse;
+  linear_type.tp_clear = linear_clear;
+  linear_type.tp_dealloc = linear_dealloc;
+  linear_type.tp_members = linear_members;
+  linear_type.tp_new = PyType_GenericNew;
+  PyObject* m = PyModule_Create(&module);
+  if (!general_name || !m || PyType_Ready(&linear_type) < 0) return nullptr;
+  Py_INCREF(&linear_type);
+  if (PyModule_AddObject(m, "LinearBase", reinterpret_cast<PyObject*>(&linear_type)) < 0) return nullptr;
+  return m;
+}

@@ -19,8 +19,17 @@ from .ops import matmul_workspace_bytes, quantized_matmul
 from .tensor import _TORCH_TO_KIND, current_stream_ptr
 
 
-class QuantLinear:
-    """y = x @ dequant(W)^T with W int4 (uint8 [N, K/2]) or int8 ([N, K]) and per-group scales."""
+try:
+    from ._torch_calls import LinearBase
+except ImportError:            # not built yet: the package can be imported (to build it), a layer cannot be called
+    LinearBase = object
+
+
+class QuantLinear(LinearBase):
+    """y = x @ dequant(W)^T with W int4 (uint8 [N, K/2]) or int8 ([N, K]) and per-group scales.
+
+    linear(x, out=None, **kw): as quantized_matmul(x, w, scales, group_size, bits=bits, out=out, **kw).  The plain
+    call on torch CUDA tensors runs in native code (the base class); everything else arrives in _general."""
 
     def __init__(self, w: torch.Tensor, scales: torch.Tensor, group_size: int = 32, bits: int = 4):
         if not (w.is_cuda and scales.is_cuda):
@@ -29,12 +38,9 @@ class QuantLinear:
         self.group_size, self.bits = group_size, bits
         self.out_features = w.shape[0]
         self.in_features = w.shape[1] * (2 if bits == 4 else 1)
+        _lib.calls.matmul                                      # loads and binds the library
 
-    def __call__(self, x: torch.Tensor, out: Optional[torch.Tensor] = None, **kw) -> torch.Tensor:
-        if not kw:
-            res = _lib.calls.matmul(x, self.w, self.scales, self.group_size, self.bits, out, None)
-            if res is not NotImplemented:
-                return res
+    def _general(self, x: torch.Tensor, out: Optional[torch.Tensor] = None, **kw) -> torch.Tensor:
         return quantized_matmul(x, self.w, self.scales, self.group_size, bits=self.bits, out=out, **kw)
 
     @property

@@ -247,25 +247,39 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
       }
     }
   }
-  // lane m * R + r collects output (m, r)
-  float mine = 0.0f;
+  // Sums over the lanes: at each step a lane gives half of its values to its partner and keeps the other half, so V
+  // values take V - 1 shuffles and log2(32 / V) more instead of 5 V. The high bits of the lane number say which value
+  // (index = m * R + r) it ends with; its low log2(32 / V) bits tell copies apart. M = 5, 4-bit, 1536 -> 3690:
+  // 8.15 -> 7.73 us; M = 3, 1024 -> 16000: 11.70 -> 11.24 us; M = 1, 8-bit, 8192 -> 16000: 36.8 -> 35.4 us.
+  constexpr int V = R * MT;
+  float v[V];
 #pragma unroll
-  for (int i = 0; i < R * MT; ++i) {
-    float v = acc[i / R][i % R];
+  for (int i = 0; i < V; ++i) v[i] = acc[i / R][i % R];
+  int index = 0;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if (lane == i) mine = v;
-  }
-  if (splits > 1) {
-    if (lane < R * MT) red[warp][lane] = mine;
-    __syncthreads();
-    if (part != 0) return;
-    if (lane < R * MT) {
-      for (int q = 1; q < splits; ++q) mine += red[warp + q][lane];
+  for (int h = V / 2, off = 16; h > 0; h >>= 1, off >>= 1) {
+    const bool upper = lane & off;
+    if (upper) index += h;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const float keep = upper ? v[i + h] : v[i], give = upper ? v[i] : v[i + h];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
     }
   }
-  const int m = m0 + lane / R, n = n0 + lane % R;
-  if (lane < R * MT && m < M && n < N) out[static_cast<long long>(m) * N + n] = from_f32<OT>(mine);
+  float mine = v[0];
+#pragma unroll
+  for (int off = 16 / V; off > 0; off >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, off);
+  const bool writer = (lane & (32 / V - 1)) == 0;
+  if (splits > 1) {
+    if (writer) red[warp][index] = mine;
+    __syncthreads();
+    if (part != 0) return;
+    if (writer) {
+      for (int q = 1; q < splits; ++q) mine += red[warp + q][index];
+    }
+  }
+  const int m = m0 + index / R, n = n0 + index % R;
+  if (writer && m < M && n < N) out[static_cast<long long>(m) * N + n] = from_f32<OT>(mine);
 }
 
 template <int WBITS, typename XT, typename ST, typename OT>

@@ -185,16 +185,28 @@ class DecodeStack:
         device = self.hidden.device
         self._state = torch.zeros(need, dtype=torch.uint8, device=device)
         self._table = torch.tensor(pointers, dtype=torch.int64, device=device)
-        self._x_q = x_q
+        buffers = (self.norms, self.outputs, x_q)
         for name, t in (("layers", self._table), ("head_w", head.w), ("head_s", head.scales), ("logits", self.logits), ("norms", self.norms),
                         ("outputs", self.outputs), ("token", self.token), ("table", self.table), ("x_q", x_q), ("hidden_out", self.hidden),
                         ("normed_out", self.normed), ("mlp_out", self.mlp), ("next_token", self.next_token), ("state", self._state)):
             setattr(desc, name, t.data_ptr())
         desc.state_bytes = need
         self._desc = desc
+        # The description holds raw addresses: keep their tensors, and what it takes to see that one was replaced.
+        owners = [(self, n) for n in ("token", "table", "hidden", "normed", "mlp", "logits", "next_token")]
+        owners += [(lin, n) for lin, _, _ in self.calls for n in ("w", "scales")]
+        self._described = ([(o, n, getattr(o, n), getattr(o, n).data_ptr()) for o, n in owners],
+                           [(t, t.data_ptr()) for t in buffers], list(self.ops))
+
+    def _as_described(self) -> bool:
+        """Whether everything the description points to is still what the chain of launches would use.  (~50 us of host time for
+        30 layers; a replayed graph does not come here.)"""
+        attributes, buffers, ops = self._described
+        return (self.ops == ops and all(getattr(o, n) is t and t.data_ptr() == p for o, n, t, p in attributes) and
+                all(t.data_ptr() == p for t, p in buffers) and all(lin.group_size == 32 and lin.bits == 4 for lin, _, _ in self.calls))
 
     def step(self):
-        if self._desc is not None:
+        if self._desc is not None and self._as_described():
             with torch.cuda.device(self.hidden.device):
                 _lib.check(_lib.lib().lcq_decode_step(ctypes.byref(self._desc), current_stream_ptr()))
             return

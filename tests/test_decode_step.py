@@ -48,7 +48,40 @@ def test_unknown_token_is_reported():
     st.token.fill_(1000)
     st.step()
     assert _lib.lib().lcq_check_device_status(None) == _lib.ERR_TIMEOUT and b"code 40" in _lib.lib().lcq_last_error()
+    assert _lib.lib().lcq_check_device_status(None) == 0
     assert float(st.hidden.abs().max()) >= 0.0 and _lib.lib().lcq_check_device_status(None) == 0
+
+
+def _plain_step(st):
+    for op in st.ops:
+        op()
+    return [t.clone() for t in (st.logits, st.hidden)]
+
+
+@pytest.mark.parametrize("replaced", ["token", "table", "w", "scales", "data", "ops"])
+def test_what_was_replaced_since_the_construction_is_used(replaced):
+    """Rebinding a buffer or a weight takes effect, as in the chain of launches (then the chain runs: the same bits)."""
+    st = L.DecodeStack(layers=2, hidden=128, inter=192, q_heads=2, kv_heads=1, vocab=1000, fused=True, glue=True, seed=3)
+    st.step()
+    before = st.logits.clone()
+    lin = st.calls[1][0]
+    if replaced == "token":
+        st.token = torch.full((1,), 77, dtype=torch.int32, device="cuda")
+    elif replaced == "table":
+        st.table = st.table.flip(0).contiguous()
+    elif replaced == "w":
+        lin.w = 255 - lin.w
+    elif replaced == "scales":
+        lin.scales = lin.scales * 4
+    elif replaced == "data":
+        st.token.data = torch.full((1,), 77, dtype=torch.int32, device="cuda")
+    else:
+        st.ops = st.ops[:-2] + [lambda: st.logits.zero_()]
+    want = _plain_step(st)
+    st.logits.fill_(float("nan"))
+    st.step()
+    assert all(torch.equal(a, b) for a, b in zip((st.logits, st.hidden), want)) and not torch.equal(st.logits, before)
+    assert _lib.lib().lcq_check_device_status(None) == 0
 
 
 def test_other_shapes_and_types_keep_the_chain():

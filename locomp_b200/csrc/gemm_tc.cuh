@@ -7,8 +7,8 @@
 // activation row m.  A team -- one CTA (CG = 1) or the two CTAs of a cluster (CG = 2) -- owns
 // D[128 * CG n x bm m], CTA r its rows 128 r .. 128 r + 127:
 //   * Packed int4 tiles [128 n x 256 k] (+ their fp16 scales) arrive by TMA in each CTA; sixteen
-//     dequant warps turn them into fp16 (exactly RN((q - 8) * s)) and write them with tcgen05.st into
-//     a ring of TMEM slots that the MMA reads as its A operand.  The packed weights cross shared
+//     dequant warps turn them into fp16 (exactly RN((q - 8) * s); K % 256 != 0: and the rest, a second term)
+//     and write them with tcgen05.st into a ring of TMEM slots that the MMA reads as its A operand.  The packed weights cross shared
 //     memory once (0.5 B/weight) and never as 2-byte values.
 //   * X tiles [bm x 256 k] fp16 are the shared-memory B operand; in a pair each CTA holds half of their
 //     rows, which both SMs' tensor cores read (cta_group::2).
@@ -51,6 +51,8 @@ constexpr int TMEM_COLS = 512;
 constexpr int N_DQ_WARPS = 16;          // two sets of two warpgroups
 constexpr int WARP_EPI0 = N_DQ_WARPS, WARP_W = WARP_EPI0 + 4, WARP_X = WARP_W + 1, WARP_MMA = WARP_X + 1;
 constexpr int NTHREADS = (WARP_MMA + 1) * 32;
+// fp16 numbers that make up a weight: one where K is whole weight stages, else two (see RAGGED below)
+__host__ __device__ constexpr int terms(bool ragged) { return ragged ? 2 : 1; }
 constexpr int BAR_EPI = 1;              // named barrier of the epilogue warps
 
 // ---------------------------------------------------------------- tcgen05 / cluster wrappers
@@ -259,24 +261,42 @@ __device__ __forceinline__ uint32_t sub_mul(uint32_t v, uint32_t offset, __half2
   const __half2 r = __hmul2(d, s2);
   return *reinterpret_cast<const uint32_t*>(&r);
 }
-// RN((q - 8) * s) for the 8 nibbles of a word, as 4 half2.  A nibble in bits 0-3 of a 16-bit lane under
+__device__ __forceinline__ uint32_t sub_mul_rest(uint32_t v, uint32_t offset, __half2 s2) {   // what sub_mul rounds off, exactly
+  const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&offset));
+  const __half2 r = __hfma2(d, s2, __hneg2(__hmul2(d, s2)));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+// RN((q - 8) * s) for the 8 nibbles of a word, as 4 half2; REST: (q - 8) * s less that.  A nibble in bits 0-3 of a 16-bit lane under
 // 0x6400 is the fp16 number 1024 + q, one in bits 4-7 under 0x5400 is 64 + q; the subtraction is exact.
 // PERM = true leaves the pairs as the masks deliver them -- (e0,e4) (e1,e5) (e2,e6) (e3,e7) -- for
 // activations whose k order was permuted the same way by the pre-pass (13 instructions a word); else
 // each byte is copied to both halves first, so that its two nibbles come out as a natural pair (16).
-template <bool PERM>
+template <bool PERM, bool REST>
 __device__ __forceinline__ void dequant_word(uint32_t w, __half2 s2, uint32_t* o) {
+  const auto scaled = [&](uint32_t v, uint32_t offset) { return REST ? sub_mul_rest(v, offset, s2) : sub_mul(v, offset, s2); };
   if (PERM) {
     const uint32_t w8 = w >> 8;
-    o[0] = sub_mul(lop_and_or(w, 0x000F000Fu, 0x64006400u), 0x64086408u, s2);
-    o[1] = sub_mul(lop_and_or(w, 0x00F000F0u, 0x54005400u), 0x54805480u, s2);
-    o[2] = sub_mul(lop_and_or(w8, 0x000F000Fu, 0x64006400u), 0x64086408u, s2);
-    o[3] = sub_mul(lop_and_or(w8, 0x00F000F0u, 0x54005400u), 0x54805480u, s2);
+    o[0] = scaled(lop_and_or(w, 0x000F000Fu, 0x64006400u), 0x64086408u);
+    o[1] = scaled(lop_and_or(w, 0x00F000F0u, 0x54005400u), 0x54805480u);
+    o[2] = scaled(lop_and_or(w8, 0x000F000Fu, 0x64006400u), 0x64086408u);
+    o[3] = scaled(lop_and_or(w8, 0x00F000F0u, 0x54005400u), 0x54805480u);
   } else {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      o[j] = sub_mul(lop_and_or(__byte_perm(w, 0u, 0x4040 + 0x0101 * j), 0x00F0000Fu, 0x54006400u), 0x54806408u, s2);
+      o[j] = scaled(lop_and_or(__byte_perm(w, 0u, 0x4040 + 0x0101 * j), 0x00F0000Fu, 0x54006400u), 0x54806408u);
   }
+}
+// The 64 weights of a row in two groups of 32, with a scale each.
+template <bool PERM, bool REST>
+__device__ __forceinline__ void dequant_step(const uint4* pk, __half2 s0, __half2 s1, uint32_t (&v)[32]) {
+  dequant_word<PERM, REST>(pk[0].x, s0, v);
+  dequant_word<PERM, REST>(pk[0].y, s0, v + 4);
+  dequant_word<PERM, REST>(pk[0].z, s0, v + 8);
+  dequant_word<PERM, REST>(pk[0].w, s0, v + 12);
+  dequant_word<PERM, REST>(pk[1].x, s1, v + 16);
+  dequant_word<PERM, REST>(pk[1].y, s1, v + 20);
+  dequant_word<PERM, REST>(pk[1].z, s1, v + 24);
+  dequant_word<PERM, REST>(pk[1].w, s1, v + 28);
 }
 
 __device__ __forceinline__ uint32_t peer_addr(uint32_t local_addr, uint32_t rank) {   // same offset in the CTA of that rank
@@ -395,7 +415,10 @@ __device__ __noinline__ void finish_tile(uint32_t d_t, OT* out, int rows_out, in
 
 // RAGGED: K % 256 != 0 -- the last weight stage of a tile is partial, and the scale rows are no 16-byte
 // multiples, so no tensor map can describe them: the dequant warps load their scales from global
-// memory, a stage ahead.
+// memory, a stage ahead.  Such calls have exact products (TERMS = 2), as the decode kernel has that they ran on
+// before this one took them: a weight is the sum of two fp16 numbers, RN((q - 8) * s) and what that rounds off
+// ((q - 8) * s and its rounding are multiples of 2^-24, so the rest is an fp16 number), in two A slots that meet the
+// same X stage.  The first set of dequant warps writes the one, the second set the other.
 template <int CG, typename OT, bool PERM, bool RAGGED>
 __global__ void __launch_bounds__(NTHREADS, 1)
 w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_piece,
@@ -418,11 +441,12 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   const uint32_t crank = CG == 2 ? blockIdx.x & 1 : 0;    // rank in the pair: clusters are consecutive blocks
   const int team = blockIdx.x / CG;
   const int nk = p.K / BK;                    // 64-k steps of a tile
+  constexpr int TERMS = terms(RAGGED);        // A slots per weight stage
 
   if (threadIdx.x == 0) {
     // full_x, full_a and empty_d are used in the pair's first CTA only; commits arrive in both CTAs
     for (int i = 0; i < MAX_XS; ++i) { mbar_init(&full_x[i], 1); mbar_init(&empty_x[i], 1); }
-    for (int i = 0; i < MAX_WS; ++i) { mbar_init(&full_w[i], 1); mbar_init(&empty_w[i], N_DQ_WARPS / 2); }
+    for (int i = 0; i < MAX_WS; ++i) { mbar_init(&full_w[i], 1); mbar_init(&empty_w[i], TERMS * N_DQ_WARPS / 2); }
     for (int i = 0; i < MAX_AS; ++i) { mbar_init(&full_a[i], CG * N_DQ_WARPS / 2); mbar_init(&empty_a[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&full_d[i], 1); mbar_init(&empty_d[i], 4 * CG); }
     *flag_abort = 0;
@@ -496,7 +520,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         const uint64_t desc_step = static_cast<uint64_t>(x_step_bytes(w.bm, CG) >> 4);
         const uint32_t d_t = tmem_base + rd.i * p.bm;
         uint32_t acc = 0;
-        for (int st = w.st0; st < w.st1; ++st, rx.step(p.nxs), ra.step(p.nas)) {
+        for (int i = TERMS * w.st0; i < TERMS * w.st1; ++i, ra.step(p.nas)) {
+          const int st = i / TERMS;
           const int steps = RAGGED && nk - st * 4 < 4 ? nk - st * 4 : 4;
           if (!warp_wait(flag_abort, &full_x[rx.i], rx.phase) || !warp_wait(flag_abort, &full_a[ra.i], ra.phase)) {
             if (lane == 0) LCQ_GIVE_UP(14);
@@ -513,7 +538,10 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
               acc = 1;
             }
           }
-          umma_commit<CG>(&empty_x[rx.i]);
+          if (TERMS == 1 || (i & 1)) {
+            umma_commit<CG>(&empty_x[rx.i]);
+            rx.step(p.nxs);
+          }
           umma_commit<CG>(&empty_a[ra.i]);
         }
         if (ok) umma_commit<CG>(&full_d[rd.i]);
@@ -521,8 +549,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
   } else if (warp < N_DQ_WARPS) {
     // ------------------------------------------------------------ dequant warps: smem int4 -> TMEM fp16
-    // Two sets of two warpgroups take the stages in turn, so that one set computes while the other loads,
-    // stores or waits.  Thread = weight row = TMEM lane; warpgroup g of a set takes the 64-k steps 2g and
+    // Two sets of two warpgroups take the stages (TERMS = 2: the two terms of each stage) in turn, so that one set
+    // computes while the other loads, stores or waits.  Thread = weight row = TMEM lane; warpgroup g of a set takes the 64-k steps 2g and
     // 2g + 1 of its stages (four scale groups).
     const int set = warp >> 3, g = (warp >> 2) & 1;
     const int r = (warp & 3) * 32 + lane;
@@ -532,7 +560,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const uint8_t* srow = smem + L.w + W_STAGE + r * 16 + g * 8;
     const int swz = (4 * g) ^ (r & 7);         // 16-byte chunk 4g + j of the row sits at chunk (4g + j) ^ (r & 7): 128-byte swizzle
     Ring rw = {0, 0}, ra = {0, 0};
-    int turn = 0;                              // whose stage it is
+    int turn = 0;                              // whose A slot it is
     bool ok = true;
     for (Walk w(p, team); ok && w.next(p);) {
       const uint32_t* gs = nullptr;            // RAGGED: this row's scales in global memory, two groups a word
@@ -545,12 +573,16 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       if (RAGGED) {
         const int n = (w.tile % p.n_tiles_n) * (CG * BN) + static_cast<int>(crank) * BN + r;
         gs = reinterpret_cast<const uint32_t*>(p.scales) + static_cast<long long>(n < p.N ? n : p.N - 1) * nk;
-        fetch(w.st0 + (turn == set ? 0 : 1));
+        fetch(w.st0);
       }
-      for (int st = w.st0; st < w.st1; ++st, turn ^= 1, rw.step(p.nws), ra.step(p.nas)) {
-        if (turn != set) continue;
+      for (int i = TERMS * w.st0; i < TERMS * w.st1; ++i, turn ^= 1, ra.step(p.nas)) {
+        const int st = i / TERMS;
+        if (turn != set) {
+          if (TERMS == 1) rw.step(p.nws);
+          continue;
+        }
         uint2 sc = s_next;
-        if (RAGGED) fetch(st + 2);
+        if (RAGGED) fetch(st + 1);
         if (!warp_wait(flag_abort, &full_w[rw.i], rw.phase)) { if (lane == 0) LCQ_GIVE_UP(15); ok = false; break; }
         const uint8_t* src = wrow + rw.i * WS_STAGE;
         uint4 pk[4];
@@ -565,14 +597,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           const __half2 s01 = *reinterpret_cast<const __half2*>(h == 0 ? &sc.x : &sc.y);
           const __half2 s0 = __low2half2(s01), s1 = __high2half2(s01);
           uint32_t v[32];
-          dequant_word<PERM>(pk[2 * h].x, s0, v);
-          dequant_word<PERM>(pk[2 * h].y, s0, v + 4);
-          dequant_word<PERM>(pk[2 * h].z, s0, v + 8);
-          dequant_word<PERM>(pk[2 * h].w, s0, v + 12);
-          dequant_word<PERM>(pk[2 * h + 1].x, s1, v + 16);
-          dequant_word<PERM>(pk[2 * h + 1].y, s1, v + 20);
-          dequant_word<PERM>(pk[2 * h + 1].z, s1, v + 24);
-          dequant_word<PERM>(pk[2 * h + 1].w, s1, v + 28);
+          if (TERMS == 2 && set == 1) dequant_step<PERM, true>(pk + 2 * h, s0, s1, v);
+          else dequant_step<PERM, false>(pk + 2 * h, s0, s1, v);
           if (h == 0) {
             if (!warp_wait(flag_abort, &empty_a[ra.i], ra.phase ^ 1u)) { if (lane == 0) LCQ_GIVE_UP(16); ok = false; break; }
             tc_fence_after();
@@ -584,6 +610,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         tc_fence_before();
         __syncwarp();
         if (lane == 0) arrive_leader<CG>(full_a0 + ra.i * 8);
+        rw.step(p.nws);
       }
     }
   } else {
@@ -783,7 +810,7 @@ inline Tiling choose_tiling(int M, int N, int K, int sm_count) {
         t.full = static_cast<int>(full); t.tail = tail;
         best = t;
       };
-      const auto step = [&](int rows, double teams) { return step_us(cg, rows, teams / P); };
+      const auto step = [&](int rows, double teams) { return terms(K % WK != 0) * step_us(cg, rows, teams / P); };
       const double start = cg == 1 ? 4.5 : 5.5, epilogue = t.nd == 1 ? 0.0075 * bm : 0.0;   // one accumulator: its epilogue shows
       const long long waves = tiles / P, rem = tiles % P;
       const double full_waves = static_cast<double>(waves) * (nk * step(bm, P) + epilogue);

@@ -198,12 +198,16 @@ static bool w8_supported(int M, int N, int K, int G) {
 }
 
 static int select_algo(int wbits, int M, int N, int K, int G, int x_dtype, int scale_dtype, int out_dtype) {
-  (void)out_dtype;
   // The prefill kernel rounds each dequantised weight to fp16 (relative error 2^-12); summed over
   // K > 16384 that error alone reaches the 1e-2 absolute output tolerance in a few outputs per
   // million, so long-K problems with few rows stay on the decode kernel, whose products are exact.
   const bool long_k_few_rows = K > 16384 && M <= 64;
-  if (wbits == 4 && M > 16 && !long_k_few_rows && gemm_tc::supported(M, N, K, G, x_dtype, scale_dtype))
+  // At K % 256 != 0 its products are exact too, but its accumulator truncates at every step: 2.2e-9 K of the result
+  // (2-norm), where the decode kernel stays at 1e-7.  In a bf16 result (rounding 1.66e-3) that is nothing, in an fp16 result
+  // (2.07e-4) it adds less than 0.3 % up to K = 6144; beyond, and for float32 results, such calls run on the
+  // decode kernel, 16 rows at a time, and cost what that costs (M = 1069, 12608 -> 2386: 1218 us, 113 on this kernel).
+  const bool plain_sum = K % 256 == 0 || out_dtype == LCQ_BF16 || (out_dtype == LCQ_F16 && K <= 6144);
+  if (wbits == 4 && M > 16 && !long_k_few_rows && plain_sum && gemm_tc::supported(M, N, K, G, x_dtype, scale_dtype))
     return LCQ_ALGO_GEMM_TC;
   // A single activation row against a weight of at most 2 Mi weights (1 MiB packed) is pure latency:
   // the warp-per-row kernel has no ring to fill and no activations to stage, and measures

@@ -51,3 +51,40 @@ def test_against_oracle(m, n, k, kind):
     assert np.all(np.abs(z.double().cpu().numpy() - ref) <= bound + ulp * np.abs(ref))
     assert torch.equal(L.quantized_matmul(x.cuda(), wd, sd, 32, algo="gemm_tc"), z)     # fixed order of summation
     assert _lib.lib().lcq_check_device_status(None) == 0, _lib.lib().lcq_last_error()
+
+
+def test_ragged_k_stays_on_exact_sums_where_the_result_would_show_it():
+    select, f32, f16, bf16 = _lib.lib().lcq_matmul_select_algo, _lib.F32, _lib.F16, _lib.BF16
+    for m, k in ((17, 64), (64, 576), (500, 6080), (1000, 2112)):
+        assert select(4, m, 1000, k, 32, f16, f16, f32) == select(4, m, 1000, k, 32, bf16, f16, f32) == _lib.ALGO_GEMV_TC
+        assert select(4, m, 1000, k, 32, f16, f16, f16) == select(4, m, 1000, k, 32, bf16, f16, bf16) == _lib.ALGO_GEMM_TC
+    assert select(4, 64, 1000, 6208, 32, f16, f16, f16) == _lib.ALGO_GEMV_TC
+    assert select(4, 64, 1000, 6208, 32, bf16, f16, bf16) == _lib.ALGO_GEMM_TC
+    for out in (f32, f16, bf16):                  # whole weight stages: as ever
+        assert select(4, 64, 1000, 8192, 32, f16, f16, out) == _lib.ALGO_GEMM_TC
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k", [(17, 100, 64), (40, 300, 320), (64, 1000, 2624), (130, 1000, 832), (200, 9000, 1088), (293, 14066, 4032)])
+def test_ragged_k_has_exact_products(m, n, k, kind):
+    """K % 256 != 0: weights as two fp16 terms, so that only the sums round.  Each of the 2 K / 16 MMAs of an output cuts its
+    float32 sum short by less than 2^-23 of it: K / 8 * 2^-23 in the 2-norm (one fp16 term alone gives 1.8e-4, from
+    K = 12,000 on no more than that).  Scales down to fp16's subnormals.  A 16-bit result adds its own rounding, and is as close as the decode
+    kernel's to the third digit; a float32 result is the decode kernel's."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    w = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=g)
+    x = torch.randn(m, k, device="cuda", generator=g).to(kind)
+    for size in (0.02, 1e-6):
+        s = (torch.randn(n, k // 32, device="cuda", generator=g).abs() * size).half()
+        ref = x.double() @ L.dequantize(w, s.float(), n, k, 32).double().t()
+
+        def error(out):
+            return float((out.double() - ref).norm() / ref.norm())
+        out = L.quantized_matmul(x, w, s, 32, algo="gemm_tc", out_dtype="f32")
+        assert error(out) <= k / 8 * 2.0 ** -23
+        assert torch.equal(L.quantized_matmul(x, w, s, 32, algo="gemm_tc", out_dtype="f32"), out)
+        wide = torch.empty_like(out)
+        assert torch.equal(L.quantized_matmul(x, w, s, 32, out=wide), L.quantized_matmul(x, w, s, 32, algo="gemv_tc", out_dtype="f32"))
+        assert error(L.quantized_matmul(x, w, s, 32)) <= 1.003 * error(L.quantized_matmul(x, w, s, 32, algo="gemv_tc"))
+    assert _lib.lib().lcq_check_device_status(None) == 0, _lib.lib().lcq_last_error()

@@ -370,28 +370,38 @@ PyObject* bind(PyObject*, PyObject* args) {
   Py_RETURN_NONE;
 }
 
-// The base class of QuantLinear: its weights as members and the call itself in native code, so that a call
-// enters no Python frame (4.0 -> 3.7 us for the smallest).  What is not `linear(x)` or `linear(x, out)` goes to the
-// method _general of the subclass.
-struct Linear {
-  PyObject_HEAD
-  PyObject *w, *scales, *group_size, *bits;
-};
+// The base class of QuantLinear: the call itself in native code, so that it enters no Python frame.  The layer's weights
+// are ordinary attributes of the instance (it is copied, pickled and changed as any Python object) and are owned here
+// for the duration of the call: another thread may rebind them while the GIL is released.  What is not `linear(x)`
+// or `linear(x, out)` goes to the method _general of the subclass.
 PyObject* general_name = nullptr;
+PyObject* operand_names[4];            // w, scales, group_size, bits
+
+struct Owned {
+  PyObject* p = nullptr;
+  ~Owned() { Py_XDECREF(p); }
+};
 
 PyObject* linear_call(PyObject* self, PyObject* args, PyObject* kwargs) {
-  Linear* l = reinterpret_cast<Linear*>(self);
   const Py_ssize_t n = PyTuple_GET_SIZE(args);
-  if ((kwargs == nullptr || PyDict_GET_SIZE(kwargs) == 0) && (n == 1 || n == 2) && l->w && l->scales && l->group_size && l->bits) {
-    PyObject* const a[7] = {PyTuple_GET_ITEM(args, 0), l->w, l->scales, l->group_size, l->bits, n == 2 ? PyTuple_GET_ITEM(args, 1) : Py_None, Py_None};
-    PyObject* r;
-    {
-      HANDLE_TH_ERRORS
-      r = matmul(nullptr, a, 7);
-      END_HANDLE_TH_ERRORS
+  if (raise_status && (kwargs == nullptr || PyDict_GET_SIZE(kwargs) == 0) && (n == 1 || n == 2)) {
+    Owned of_layer[4];
+    bool all = true;
+    for (int i = 0; i < 4 && all; ++i) all = (of_layer[i].p = PyObject_GetAttr(self, operand_names[i])) != nullptr;
+    if (all) {
+      PyObject* const a[7] = {PyTuple_GET_ITEM(args, 0), of_layer[0].p, of_layer[1].p, of_layer[2].p, of_layer[3].p,
+                              n == 2 ? PyTuple_GET_ITEM(args, 1) : Py_None, Py_None};
+      PyObject* r;
+      {
+        HANDLE_TH_ERRORS
+        r = matmul(nullptr, a, 7);
+        END_HANDLE_TH_ERRORS
+      }
+      if (r != Py_NotImplemented) return r;
+      Py_DECREF(r);
+    } else {
+      PyErr_Clear();                   // (_general raises it)
     }
-    if (r != Py_NotImplemented) return r;
-    Py_DECREF(r);
   }
   PyObject* method = PyObject_GetAttr(self, general_name);
   if (!method) return nullptr;
@@ -399,25 +409,8 @@ PyObject* linear_call(PyObject* self, PyObject* args, PyObject* kwargs) {
   Py_DECREF(method);
   return r;
 }
-int linear_traverse(PyObject* self, visitproc visit, void* arg) {
-  Linear* l = reinterpret_cast<Linear*>(self);
-  Py_VISIT(l->w); Py_VISIT(l->scales); Py_VISIT(l->group_size); Py_VISIT(l->bits);
-  return 0;
-}
-int linear_clear(PyObject* self) {
-  Linear* l = reinterpret_cast<Linear*>(self);
-  Py_CLEAR(l->w); Py_CLEAR(l->scales); Py_CLEAR(l->group_size); Py_CLEAR(l->bits);
-  return 0;
-}
-void linear_dealloc(PyObject* self) {
-  PyObject_GC_UnTrack(self);
-  linear_clear(self);
-  Py_TYPE(self)->tp_free(self);
-}
-PyMemberDef linear_members[] = {{"w", Py_T_OBJECT_EX, offsetof(Linear, w), 0, nullptr}, {"scales", Py_T_OBJECT_EX, offsetof(Linear, scales), 0, nullptr},
-                                {"group_size", Py_T_OBJECT_EX, offsetof(Linear, group_size), 0, nullptr},
-                                {"bits", Py_T_OBJECT_EX, offsetof(Linear, bits), 0, nullptr}, {nullptr, 0, 0, 0, nullptr}};
-PyTypeObject linear_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+PyType_Slot linear_slots[] = {{Py_tp_call, reinterpret_cast<void*>(linear_call)}, {0, nullptr}};
+PyType_Spec linear_spec = {"locomp_b200._torch_calls.LinearBase", 0, 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE, linear_slots};
 
 // A C++ exception (out of memory, a CUDA error seen by torch) becomes the Python exception torch gives it.
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
@@ -438,18 +431,11 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_torch_calls", nullptr, -1, method
 
 PyMODINIT_FUNC PyInit__torch_calls(void) {
   general_name = PyUnicode_InternFromString("_general");
-  linear_type.tp_name = "locomp_b200._torch_calls.LinearBase";
-  linear_type.tp_basicsize = sizeof(Linear);
-  linear_type.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE | Py_TPFLAGS_HAVE_GC;
-  linear_type.tp_call = linear_call;
-  linear_type.tp_traverse = linear_traverse;
-  linear_type.tp_clear = linear_clear;
-  linear_type.tp_dealloc = linear_dealloc;
-  linear_type.tp_members = linear_members;
-  linear_type.tp_new = PyType_GenericNew;
+  const char* const names[4] = {"w", "scales", "group_size", "bits"};
+  bool all = general_name != nullptr;
+  for (int i = 0; i < 4; ++i) all = (operand_names[i] = PyUnicode_InternFromString(names[i])) != nullptr && all;
   PyObject* m = PyModule_Create(&module);
-  if (!general_name || !m || PyType_Ready(&linear_type) < 0) return nullptr;
-  Py_INCREF(&linear_type);
-  if (PyModule_AddObject(m, "LinearBase", reinterpret_cast<PyObject*>(&linear_type)) < 0) return nullptr;
+  PyObject* type = PyType_FromSpec(&linear_spec);      // a heap type without fields of its own, like a class of Python
+  if (!all || !m || !type || PyModule_AddObject(m, "LinearBase", type) < 0) return nullptr;
   return m;
 }

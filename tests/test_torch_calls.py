@@ -1,5 +1,9 @@
 """The native host path for torch CUDA tensors gives what the general path gives, and leaves to the
 general path whatever it does not take."""
+import copy
+import pickle
+import sys
+
 import pytest
 import torch
 
@@ -82,3 +86,47 @@ def test_what_is_not_a_cuda_tensor_is_left_to_the_general_path():
     assert c.argmax(t, None) is NotImplemented
     with pytest.raises(TypeError, match="CUDA"):
         L.quantized_matmul(t, t, t)
+
+
+def test_a_layer_is_copied_and_pickled_as_any_object():
+    layer = L.QuantLinear.__new__(L.QuantLinear)          # (the constructor wants weights on a GPU)
+    layer.w, layer.scales, layer.group_size, layer.bits = torch.randint(0, 256, (6, 32), dtype=torch.uint8), torch.rand(6, 2).half(), 32, 4
+    layer.out_features, layer.in_features, layer.label = 6, 64, "mine"
+    assert set(vars(layer)) == {"w", "scales", "group_size", "bits", "out_features", "in_features", "label"}
+    assert copy.copy(layer).w is layer.w
+    others = [copy.deepcopy(layer)] + [pickle.loads(pickle.dumps(layer, protocol)) for protocol in range(pickle.HIGHEST_PROTOCOL + 1)]
+    for other in others:
+        assert type(other) is L.QuantLinear and other.w is not layer.w and vars(other).keys() == vars(layer).keys()
+        assert torch.equal(other.w, layer.w) and torch.equal(other.scales, layer.scales) and other.bits == 4 and other.label == "mine"
+        with pytest.raises(TypeError, match="CUDA"):
+            other(torch.zeros(1, 64).half())
+    with pytest.raises(AttributeError, match="scales"):
+        del layer.scales
+        layer(torch.zeros(1, 64).half())
+
+
+@pytest.mark.gpu
+def test_weights_rebound_during_a_call_outlive_it(monkeypatch):
+    """The call on a new stream enters Python for its workspace; what happens there (as in another thread while the GIL is
+    released) may drop the layer's last reference to its weights."""
+    module = sys.modules["locomp_b200.tensor"]
+    x, w, s = _linear(16, 2048, 130, 4, 32, torch.float16)
+    want = L.quantized_matmul(x, w, s)
+    layer = L.QuantLinear(w, s)
+    del w, s
+
+    entered = []
+
+    class Table(dict):
+        def get(self, key, default=None):
+            entered.append(key)
+            layer.w, layer.scales = torch.zeros_like(layer.w), torch.zeros_like(layer.scales)
+            return super().get(key, default)
+    monkeypatch.setattr(module, "_workspaces", Table(module._workspaces))
+    side = torch.cuda.Stream(priority=-1)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        got = layer(x)
+        assert torch.equal(layer(x), torch.zeros_like(got))
+    side.synchronize()
+    assert entered and torch.equal(got, want)

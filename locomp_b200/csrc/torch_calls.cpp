@@ -7,13 +7,16 @@
 // Every function returns NotImplemented for whatever is not the ordinary case (NumPy arrays,
 // DeviceTensor, foreign objects, non-contiguous or CPU tensors, wrong types or sizes): the caller then
 // takes the general path in Python, which handles it or raises the error that names what is wrong.
-// The GIL is released around the C ABI call only (a full launch queue makes it wait); the table of
-// workspaces is touched with the GIL held and needs no lock of its own.
+// The GIL is released around the C ABI call only (a full launch queue makes it wait).  The scratch of a stream
+// is locked from its lookup until the call has returned: threads that share a stream (each thread's current stream
+// is the default one unless it changed it) would otherwise mix the launches of calls that use the same scratch, or
+// replace it under a call that has not launched yet.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <dlfcn.h>
 
 #include <map>
+#include <mutex>
 #include <utility>
 
 #include <ATen/core/Tensor.h>
@@ -41,7 +44,23 @@ struct Api {
 } api;
 PyObject* raise_status = nullptr;      // callable(status): raises the exception of a negative status
 PyObject* make_workspace = nullptr;    // callable(nbytes, device, stream): allocates (or grows) and reports it through set_workspace
-std::map<std::pair<int, uintptr_t>, std::pair<void*, size_t>> workspaces;   // (device, stream) -> scratch, owned by the Python side
+
+// The scratch of a (device, stream).  The lock is taken without the GIL (and may be held while the GIL is taken, never
+// the other way round), the table is touched with the GIL only.  Recursive: the allocation below it may run
+// other Python code of the same thread.
+struct Scratch {
+  std::recursive_mutex lock;
+  PyObject* tensor = nullptr;          // owns the memory
+  void* ptr = nullptr;
+  size_t bytes = 0;
+};
+std::map<std::pair<int, uintptr_t>, Scratch> scratches;
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  void end() { if (state) PyEval_RestoreThread(state); state = nullptr; }
+  void again() { state = PyEval_SaveThread(); }
+  ~NoGil() { end(); }
+};
 
 constexpr int NOT_FLOAT = -1;
 int float_code(at::ScalarType t) {
@@ -83,10 +102,8 @@ PyObject* finish(int status, PyObject* given) {
 }
 template <typename F>
 int unlocked(const F& call) {
-  PyThreadState* state = PyEval_SaveThread();
-  const int rc = call();
-  PyEval_RestoreThread(state);
-  return rc;
+  NoGil released;
+  return call();
 }
 void* current_stream(int device) { return c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream(); }
 at::Tensor empty(at::IntArrayRef shape, at::ScalarType type, const at::Tensor& like) {
@@ -121,35 +138,39 @@ PyObject* matmul(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
   }
   const int dev = x->device().index();
   void* stream = current_stream(dev);
-  const auto call = [&](void* ws, size_t ws_bytes) {
-    return unlocked([&] {
-      return api.matmul[bits == 8](x->data_ptr(), w->data_ptr(), s->data_ptr(), out->data_ptr(), static_cast<int>(M), static_cast<int>(N),
-                                   static_cast<int>(K), static_cast<int>(group), xk, sk, ok, LCQ_ALGO_AUTO, ws, ws_bytes, stream);
-    });
+  const void *xp = x->data_ptr(), *wp = w->data_ptr(), *sp = s->data_ptr();
+  void* op = out->data_ptr();
+  const auto call = [&](void* ws, size_t ws_bytes) {       // without the GIL
+    return api.matmul[bits == 8](xp, wp, sp, op, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<int>(group),
+                                 xk, sk, ok, LCQ_ALGO_AUTO, ws, ws_bytes, stream);
   };
-  int rc;
+  int rc = LCQ_ERR_WORKSPACE;
   if (args[6] != Py_None) {
     const at::Tensor* ws = cuda_tensor(args[6]);
     if (!ws || ws->device() != x->device()) return not_implemented();
-    rc = call(ws->data_ptr(), ws->nbytes());
+    void* ws_ptr = ws->data_ptr();
+    const size_t ws_bytes = ws->nbytes();
+    rc = unlocked([&] { return call(ws_ptr, ws_bytes); });
     if (rc == LCQ_ERR_WORKSPACE) return not_implemented();
-  } else {
+  } else if (bits == 8 || xk == LCQ_F32 || sk != LCQ_F16) {
+    rc = unlocked([&] { return call(nullptr, 0); });         // no kernel of these types has scratch
+  }
+  if (args[6] == Py_None && rc == LCQ_ERR_WORKSPACE) {
+    Scratch& scratch = scratches[{dev, reinterpret_cast<uintptr_t>(stream)}];
+    NoGil released;
+    const std::lock_guard<std::recursive_mutex> held(scratch.lock);
     // The call itself says whether the scratch this stream has is enough: no size query on the ordinary path.
-    const auto scratch = [&] {
-      const auto it = workspaces.find({dev, reinterpret_cast<uintptr_t>(stream)});
-      return it == workspaces.end() ? std::pair<void*, size_t>{nullptr, 0} : it->second;
-    };
-    auto ws = scratch();
-    rc = call(ws.first, ws.second);
+    rc = call(scratch.ptr, scratch.bytes);
     if (rc == LCQ_ERR_WORKSPACE) {
+      released.end();
       const size_t need = api.workspace_bytes(static_cast<int>(bits), static_cast<int>(M), static_cast<int>(N), static_cast<int>(K),
                                               static_cast<int>(group), xk, sk, ok, LCQ_ALGO_AUTO);
       PyObject* r = PyObject_CallFunction(make_workspace, "niK", static_cast<Py_ssize_t>(need), dev,
                                           static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream)));
       if (!r) return nullptr;
       Py_DECREF(r);
-      ws = scratch();
-      rc = call(ws.first, ws.second);
+      released.again();
+      rc = call(scratch.ptr, scratch.bytes);
     }
   }
   return args[5] == Py_None ? finish(rc, std::move(made)) : finish(rc, args[5]);
@@ -326,13 +347,41 @@ PyObject* argmax(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
   return args[1] == Py_None ? finish(rc, std::move(made)) : finish(rc, args[1]);
 }
 
-// set_workspace(device, stream, address, nbytes): the scratch that calls on this stream use from now on
+bool stream_key(PyObject* const* args, std::pair<int, uintptr_t>& key) {      // (device, stream)
+  const long dev = PyLong_AsLong(args[0]);
+  const unsigned long long stream = PyErr_Occurred() ? 0 : PyLong_AsUnsignedLongLong(args[1]);
+  key = {static_cast<int>(dev), static_cast<uintptr_t>(stream)};
+  return !PyErr_Occurred();
+}
+// set_workspace(device, stream, tensor): the scratch that calls on this stream use from now on; its lock is held
 PyObject* set_workspace(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
-  long long dev, bytes;
-  if (n_args != 4 || !as_int(args[0], dev) || !as_int(args[3], bytes)) return PyErr_Format(PyExc_TypeError, "set_workspace(device, stream, address, nbytes)");
-  const unsigned long long stream = PyLong_AsUnsignedLongLong(args[1]), ptr = PyLong_AsUnsignedLongLong(args[2]);
-  if (PyErr_Occurred()) return nullptr;
-  workspaces[{static_cast<int>(dev), static_cast<uintptr_t>(stream)}] = {reinterpret_cast<void*>(ptr), static_cast<size_t>(bytes)};
+  std::pair<int, uintptr_t> key;
+  if (n_args != 3 || !THPVariable_Check(args[2])) return PyErr_Format(PyExc_TypeError, "set_workspace(device, stream, tensor)");
+  if (!stream_key(args, key)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(args[2]);
+  Scratch& scratch = scratches[key];
+  scratch.ptr = t.data_ptr();
+  scratch.bytes = t.nbytes();
+  PyObject* old = scratch.tensor;
+  Py_INCREF(args[2]);
+  scratch.tensor = args[2];
+  Py_XDECREF(old);
+  Py_RETURN_NONE;
+}
+// lock_workspace(device, stream), unlock_workspace(device, stream): for the general path
+PyObject* lock_workspace(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
+  std::pair<int, uintptr_t> key;
+  if (n_args != 2) return PyErr_Format(PyExc_TypeError, "lock_workspace(device, stream)");
+  if (!stream_key(args, key)) return nullptr;
+  Scratch& scratch = scratches[key];
+  unlocked([&] { scratch.lock.lock(); return 0; });
+  Py_RETURN_NONE;
+}
+PyObject* unlock_workspace(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
+  std::pair<int, uintptr_t> key;
+  if (n_args != 2) return PyErr_Format(PyExc_TypeError, "unlock_workspace(device, stream)");
+  if (!stream_key(args, key)) return nullptr;
+  scratches[key].lock.unlock();
   Py_RETURN_NONE;
 }
 
@@ -423,6 +472,7 @@ PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef methods[] = {
     LCQ_METHOD(matmul), LCQ_METHOD(dequantize), LCQ_METHOD(quantize), LCQ_METHOD(rms_norm), LCQ_METHOD(residual_rms_norm),
     LCQ_METHOD(silu_mul), LCQ_METHOD(add_inplace), LCQ_METHOD(embed_lookup), LCQ_METHOD(argmax), LCQ_METHOD(set_workspace),
+    LCQ_METHOD(lock_workspace), LCQ_METHOD(unlock_workspace),
     {"bind", bind, METH_VARARGS, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_torch_calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

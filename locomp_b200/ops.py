@@ -25,7 +25,7 @@ import torch
 
 from . import _lib
 from .tensor import (KIND_TO_CODE, KIND_TO_TORCH, DeviceTensor, Operand, _require_cuda, current_stream_ptr,
-                     resolve, workspace)
+                     locked_workspace, resolve, workspace)
 
 _ALGOS = {None: _lib.ALGO_AUTO, "auto": _lib.ALGO_AUTO, "simt": _lib.ALGO_SIMT,
           "gemv_tc": _lib.ALGO_GEMV_TC, "gemm_tc": _lib.ALGO_GEMM_TC, "gemv_w8": _lib.ALGO_GEMV_W8}
@@ -115,15 +115,20 @@ def quantized_matmul(x, w, scales, group_size: int = 32, *, bits: int = 4, out=N
         ws_bytes = L.lcq_matmul_workspace_bytes(bits, M, N, K, group_size, xk, sk, KIND_TO_CODE[okind], a)
         if ws_bytes == (1 << 64) - 1:
             raise _lib.LcqError(_lib.ERR_UNSUPPORTED, f"algo {algo!r} does not cover this problem")
+        fn = L.lcq_matmul_int4 if bits == 4 else L.lcq_matmul_int8
+
+        def launch(ws):
+            _lib.check(fn(xo.ptr, wo.ptr, so.ptr, oo.ptr, M, N, K, group_size, xk, sk, KIND_TO_CODE[okind], a,
+                          ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0, sp))
         if ws_bytes and workspace_buf is not None:
             if workspace_buf.numel() * workspace_buf.element_size() < ws_bytes or workspace_buf.device.index != dev:
                 raise ValueError(f"workspace_buf must hold {ws_bytes} bytes on cuda:{dev}")
-            ws = workspace_buf
+            launch(workspace_buf)
+        elif ws_bytes:
+            with locked_workspace(dev, sp):
+                launch(workspace(ws_bytes, dev, sp))
         else:
-            ws = workspace(ws_bytes, dev, sp) if ws_bytes else None
-        fn = L.lcq_matmul_int4 if bits == 4 else L.lcq_matmul_int8
-        _lib.check(fn(xo.ptr, wo.ptr, so.ptr, oo.ptr, M, N, K, group_size, xk, sk, KIND_TO_CODE[okind], a,
-                      ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0, sp))
+            launch(None)
     if host_out is not None:          # a NumPy output: copy the result back in place
         torch.cuda.current_stream().synchronize()
         host_out[...] = oo.keepalive.cpu().numpy().reshape(host_out.shape)

@@ -14,6 +14,7 @@ dtype is checked here.
 """
 from __future__ import annotations
 
+from contextlib import contextmanager
 from typing import Any, Optional, Tuple
 
 import numpy as np
@@ -208,17 +209,29 @@ def current_stream_ptr(stream=None) -> int:
 _workspaces = {}
 
 
+@contextmanager
+def locked_workspace(device: int, stream_ptr: int):
+    """Holds the lock of a stream's scratch buffer: from the lookup of the buffer until the call that uses it has launched
+    all of its kernels, no other thread replaces the buffer or launches kernels that use it."""
+    _lib.calls.lock_workspace(device, stream_ptr)
+    try:
+        yield
+    finally:
+        _lib.calls.unlock_workspace(device, stream_ptr)
+
+
 def workspace(nbytes: int, device: int, stream_ptr: int) -> torch.Tensor:
-    """Zero-initialised scratch buffer, one per (device, stream); the kernels leave it zeroed."""
+    """Zero-initialised scratch buffer, one per (device, stream); the kernels leave it zeroed.  Used under locked_workspace."""
     key = (device, stream_ptr)
-    buf = _workspaces.get(key)
-    need = max(int(nbytes), 256)
-    if buf is None or buf.numel() < need:
-        if buf is not None:
-            # work queued on the old buffer must finish before the allocator may reuse it
-            torch.cuda.synchronize(device)
-        buf = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", device))
-        torch.cuda.synchronize(device)   # zero-fill ran on torch's stream; the caller's may differ
-        _workspaces[key] = buf
-        _lib.calls.set_workspace(device, stream_ptr, buf.data_ptr(), buf.numel())
-    return buf
+    with locked_workspace(device, stream_ptr):
+        buf = _workspaces.get(key)
+        need = max(int(nbytes), 256)
+        if buf is None or buf.numel() < need:
+            if buf is not None:
+                # work queued on the old buffer must finish before the allocator may reuse it
+                torch.cuda.synchronize(device)
+            buf = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", device))
+            torch.cuda.synchronize(device)   # zero-fill ran on torch's stream; the caller's may differ
+            _workspaces[key] = buf
+            _lib.calls.set_workspace(device, stream_ptr, buf)
+        return buf

@@ -3,6 +3,7 @@ general path whatever it does not take."""
 import copy
 import pickle
 import sys
+import threading
 
 import pytest
 import torch
@@ -130,3 +131,49 @@ def test_weights_rebound_during_a_call_outlive_it(monkeypatch):
         assert torch.equal(layer(x), torch.zeros_like(got))
     side.synchronize()
     assert entered and torch.equal(got, want)
+
+
+def test_the_scratch_of_a_stream_is_one_threads_at_a_time():
+    locked, order = sys.modules["locomp_b200.tensor"].locked_workspace, []
+
+    def other():
+        with locked(0, 12345):
+            order.append("other")
+    thread = threading.Thread(target=other)
+    with locked(0, 12345):
+        with locked(0, 12345):                             # the same thread may come again
+            thread.start()
+        with locked(0, 54321):                             # another stream is another lock
+            thread.join(0.2)
+        order.append("this")
+    thread.join(10)
+    assert order == ["this", "other"]
+
+
+@pytest.mark.gpu
+def test_threads_that_share_a_stream_do_not_share_scratch():
+    """Two threads on the default stream, calls of two launches that pass data through the scratch (bf16, M > 16), sizes that
+    make the scratch grow between them; the native and the general path in turn."""
+    problems = [_linear(m, k, n, 4, 32, torch.bfloat16) for m, k, n in ((300, 1024, 700), (1100, 4096, 300))]
+    want = [L.QuantLinear(w, s)(x, torch.empty(x.shape[0], w.shape[0], dtype=torch.bfloat16, device="cuda")) for x, w, s in problems]
+    torch.cuda.synchronize()
+    failures = []
+
+    def work(i):
+        x, w, s = problems[i]
+        layer, operand = L.QuantLinear(w, s), L.DeviceTensor(x)
+        got = [layer(x) if r % 3 else L.quantized_matmul(operand, w, s) for r in range(120)]
+        torch.cuda.synchronize()
+        failures.extend((i, r) for r, g in enumerate(got) if not torch.equal(g, want[i]))
+    side = torch.cuda.Stream(priority=-1)                  # no large scratch so far: it grows while the other thread launches
+
+    def on_side(i):
+        with torch.cuda.stream(side):
+            work(i)
+    for form in (work, on_side):
+        threads = [threading.Thread(target=form, args=(i,)) for i in (0, 1)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert not failures and _lib.lib().lcq_check_device_status(None) == 0

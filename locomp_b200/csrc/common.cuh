@@ -102,6 +102,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     if (global_timer_ns() - t0 > limit) return false;
   }
 }
+// Waits for a kernel's own copies out of this GPU's memory, which nothing but time stands in the way of: two seconds at
+// most whatever the wait limit is, for kernels that are about to leave after one of their bounded waits ran out.
+__device__ __noinline__ void mbar_wait_landed(uint64_t* bar, uint32_t parity) {
+  const uint64_t t0 = global_timer_ns();
+  while (!mbar_try_wait(bar, parity) && global_timer_ns() - t0 < 2000000000ull) {}
+}
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }

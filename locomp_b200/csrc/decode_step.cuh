@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
   if (warp >= NCW) {
     // ------------------------------------------------------------ producer: one thread, all phases in order
     if (lane == 0) {
-      int s = 0;
+      int s = 0, in_flight = 0;                // the next stage; stages before it whose copies may be on their way
       uint32_t phase = 0;
       bool ok = true;
       for (int ph = 0, part; ok && (part = first_part(ph, p.n_layers)) >= 0; ++ph) {
@@ -259,15 +259,23 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
           const int step = part == PART_O ? step_q : part == PART_DOWN ? step_i : step_h;
           for (int r = 0; r < g.rows; r += step) {
             const int rows = g.rows - r < step ? g.rows - r : step;
-            if (*flag_abort || !mbar_wait_bounded(&empty[s], phase ^ 1u)) { *flag_abort = 1; atomicExch(&g_device_status, 50); ok = false; break; }
+            // (the flag after the wait: consumers that gave up release stages whose copies have not landed)
+            if (!mbar_wait_bounded(&empty[s], phase ^ 1u) || *flag_abort) { *flag_abort = 1; atomicExch(&g_device_status, 50); ok = false; break; }
             const uint32_t wb = static_cast<uint32_t>(rows) * (g.K / 2), sb = static_cast<uint32_t>(rows) * (g.K / 16);
             const uint32_t dst = smem_u32(smem) + s * p.stage_bytes;
             mbar_expect_tx(&full[s], wb + sb);
             bulk_load(dst, g.w + static_cast<long long>(g.row0 + r) * (g.K / 2), wb, &full[s]);
             bulk_load(dst + wb, g.s + static_cast<long long>(g.row0 + r) * (g.K / 16), sb, &full[s]);
             if (++s == p.n_stages) { s = 0; phase ^= 1u; }
+            if (in_flight < p.n_stages) ++in_flight;
           }
         }
+      }
+      // Consumers that gave up wait for no more stages, so the copies into the last ones are waited for here: none may
+      // land after the CTA has left.  They read this GPU's memory and end by themselves, whatever the wait limit.
+      for (; in_flight > 0; --in_flight) {
+        if (--s < 0) { s = p.n_stages - 1; phase ^= 1u; }
+        mbar_wait_landed(&full[s], phase);
       }
     }
   } else {

@@ -230,11 +230,12 @@ struct Walk {
   }
 };
 
+enum { FLAG_ABORT, FLAG_SHARED, ISSUED_W, ISSUED_X0, ISSUED_X1, N_FLAGS = 6 };
 struct Smem {           // offsets from the 1024-byte aligned dynamic shared memory base
   int w;                // nws stages of WS_STAGE
   int bars;
   int tmem_slot;
-  int flags;            // abort flag, epilogue broadcast
+  int flags;            // abort flag, epilogue broadcast, stages issued: weights, X (in the pair's first CTA: of both CTAs)
   int total;
 };
 __host__ __device__ inline int x_step_bytes(int bm, int cg) { return (bm / cg) * 128; }   // this CTA's share of a tile's rows, 64 k
@@ -243,10 +244,10 @@ __host__ __device__ inline Smem smem_map(int bm, int cg, int nxs, int nws) {
   Smem s;
   s.w = nxs * x_stage_bytes(bm, cg);    // X stages first: steps are multiples of 2048 bytes
   s.bars = s.w + nws * WS_STAGE;
-  // full_x, empty_x [MAX_XS]; full_w, empty_w [MAX_WS]; full_a, empty_a [MAX_AS]; full_d, empty_d [2]
-  s.tmem_slot = s.bars + (2 * MAX_XS + 2 * MAX_WS + 2 * MAX_AS + 4) * 8;
+  // full_x, empty_x [MAX_XS]; full_w, empty_w [MAX_WS]; full_a, empty_a [MAX_AS]; full_d, empty_d [2]; drained
+  s.tmem_slot = s.bars + (2 * MAX_XS + 2 * MAX_WS + 2 * MAX_AS + 5) * 8;
   s.flags = s.tmem_slot + 8;
-  s.total = s.flags + 8;
+  s.total = s.flags + 4 * N_FLAGS;
   return s;
 }
 
@@ -303,6 +304,9 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t local_addr, uint32_t rank
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
   return a;
+}
+__device__ __forceinline__ void store_remote(uint32_t cluster_addr, int v) {
+  asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
@@ -413,6 +417,44 @@ __device__ __noinline__ void finish_tile(uint32_t d_t, OT* out, int rows_out, in
   }
 }
 
+// After a wait ran out in the CTA or its partner: waits for what they still have under way -- the MMAs, and the copies
+// into the last stages, which nobody waits for any more -- so that nothing lands in shared memory or reads it after
+// they have left.  A CTA of a pair may have loaded its half of an X stage whose other half was never issued: the
+// barrier is then given the missing half, or armed for the one that comes.  Called by all threads; in a pair between
+// two cluster barriers.
+template <int CG, bool RAGGED>
+__device__ __noinline__ void drain(const Params& p, uint8_t* smem, int team, uint32_t crank) {
+  const Smem L = smem_map(p.bm, CG, p.nxs, p.nws);
+  uint64_t* full_x = reinterpret_cast<uint64_t*>(smem + L.bars);
+  uint64_t* full_w = full_x + 2 * MAX_XS;
+  uint64_t* drained = full_w + 2 * MAX_WS + 2 * MAX_AS + 4;
+  const volatile int* flags = reinterpret_cast<const volatile int*>(smem + L.flags);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  if (warp == WARP_MMA) {
+    if (crank == 0) umma_commit<CG>(drained);            // (arrives in both CTAs, after all that was committed before)
+    __syncwarp();
+    mbar_wait_landed(drained, 0);
+  } else if (warp == WARP_W && lane == 0) {
+    const int n = flags[ISSUED_W];
+    for (int i = n > p.nws ? n - p.nws : 0; i < n; ++i) mbar_wait_landed(full_w + i % p.nws, (i / p.nws) & 1);
+  } else if (warp == WARP_X && lane == 0 && crank == 0) {
+    const int mine = flags[ISSUED_X0], other = CG == 2 ? flags[ISSUED_X1] : mine, n = mine > other ? mine : other;
+    const int nk = p.K / BK;
+    int i = 0;
+    for (Walk w(p, team); i < n && w.next(p);) {
+      for (int st = w.st0; st < w.st1 && i < n; ++st, ++i) {
+        if (i < n - p.nxs) continue;
+        const int steps = RAGGED && nk - st * 4 < 4 ? nk - st * 4 : 4, bytes = steps * x_step_bytes(w.bm, CG);
+        uint64_t* bar = full_x + i % p.nxs;
+        if (i >= mine) mbar_expect_tx(bar, bytes);
+        else if (i >= other) asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+        mbar_wait_landed(bar, (i / p.nxs) & 1);
+      }
+    }
+  }
+  __syncthreads();
+}
+
 // RAGGED: K % 256 != 0 -- the last weight stage of a tile is partial, and the scale rows are no 16-byte
 // multiples, so no tensor map can describe them: the dequant warps load their scales from global
 // memory, a stage ahead.  Such calls have exact products (TERMS = 2), as the decode kernel has that they ran on
@@ -434,6 +476,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   uint64_t* empty_a = full_a + MAX_AS;
   uint64_t* full_d = empty_a + MAX_AS;
   uint64_t* empty_d = full_d + 2;
+  uint64_t* drained = empty_d + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L.tmem_slot);
   volatile int* flag_abort = reinterpret_cast<volatile int*>(smem + L.flags);
 
@@ -449,6 +492,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     for (int i = 0; i < MAX_WS; ++i) { mbar_init(&full_w[i], 1); mbar_init(&empty_w[i], TERMS * N_DQ_WARPS / 2); }
     for (int i = 0; i < MAX_AS; ++i) { mbar_init(&full_a[i], CG * N_DQ_WARPS / 2); mbar_init(&empty_a[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&full_d[i], 1); mbar_init(&empty_d[i], 4 * CG); }
+    mbar_init(drained, 1);
     *flag_abort = 0;
     fence_barrier_init();
     griddep_launch_dependents();
@@ -461,7 +505,13 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t a_base = tmem_base + TMEM_COLS - p.nas * A_SLOT_COLS;
 
-#define LCQ_GIVE_UP(code) do { *flag_abort = 1; atomicExch(&g_device_status, (code)); } while (0)
+  // (a pair gives up together: see drain)
+#define LCQ_GIVE_UP(code)                                                                                                  \
+  do {                                                                                                                     \
+    *flag_abort = 1;                                                                                                       \
+    if (CG == 2) store_remote(peer_addr(smem_u32(smem + L.flags + 4 * FLAG_ABORT), crank ^ 1u), 1);                        \
+    atomicExch(&g_device_status, (code));                                                                                  \
+  } while (0)
 
   if (warp == WARP_W) {
     // ------------------------------------------------------------ weights and scales (constants: no dependency wait)
@@ -470,6 +520,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       if (!RAGGED) tma_prefetch_desc(&tmap_s);
       Ring r = {0, 0};
       bool ok = true;
+      int issued = 0;
       for (Walk w(p, team); ok && w.next(p);) {
         const int n0 = (w.tile % p.n_tiles_n) * (CG * BN) + static_cast<int>(crank) * BN;
         for (int st = w.st0; st < w.st1; ++st, r.step(p.nws)) {
@@ -478,8 +529,10 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           mbar_expect_tx(&full_w[r.i], RAGGED ? W_STAGE : WS_STAGE);
           tma_load_2d(dst, &tmap_w, &full_w[r.i], st * (WK / 2), n0);
           if (!RAGGED) tma_load_2d(dst + W_STAGE, &tmap_s, &full_w[r.i], st * (WK / 32), n0);
+          ++issued;
         }
       }
+      flag_abort[ISSUED_W] = issued;
     }
   } else if (warp == WARP_X) {
     // ------------------------------------------------------------ activations: this CTA's share of the rows of each tile
@@ -489,6 +542,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       const int stage_bytes = x_stage_bytes(p.bm, CG);
       Ring r = {0, 0};
       bool ok = true;
+      int issued = 0;
       for (Walk w(p, team); ok && w.next(p);) {
         const int rows = w.bm / CG, bytes = x_step_bytes(w.bm, CG);
         const int m0 = w.m0 + static_cast<int>(crank) * rows;
@@ -503,8 +557,11 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             if (CG == 2) tma_load_2d_pair(dst + j * bytes, tmap, bar, (st * 4 + j) * BK, m0);
             else tma_load_2d(dst + j * bytes, tmap, full_x + r.i, (st * 4 + j) * BK, m0);
           }
+          ++issued;
         }
       }
+      if (CG == 2) store_remote(peer_addr(smem_u32(smem + L.flags + 4 * (ISSUED_X0 + crank)), 0), issued);
+      else flag_abort[ISSUED_X0] = issued;
     }
   } else if (warp == WARP_MMA) {
     // ------------------------------------------------------------ MMA issuer: one warp for the team
@@ -622,7 +679,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const int r = q4 * 32 + lane;
     const uint32_t lane_taddr = tmem_base + (static_cast<uint32_t>(q4 * 32) << 16);
     const uint32_t empty_d0 = leader_addr<CG>(empty_d);
-    volatile int* shared_int = flag_abort + 1;
+    volatile int* shared_int = flag_abort + FLAG_SHARED;
     const long long part_elems = static_cast<long long>(p.bm) * BN;
     Ring rd = {0, 0};
     for (Walk w(p, team); w.next(p); rd.step(p.nd)) {
@@ -699,10 +756,12 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 
   tc_fence_before();
   __syncthreads();
-  if (CG == 2) {
-    // neither CTA leaves while the other may still arrive on its barriers or the pair's MMAs read its memory
-    cluster_barrier();
-  } else if (p.split > 1) {
+  if (CG == 2) cluster_barrier();    // neither CTA leaves while the other may still arrive on its barriers or the pair's MMAs read its memory
+  if (*flag_abort) {
+    drain<CG, RAGGED>(p, smem, team, crank);
+    if (CG == 2) cluster_barrier();
+  }
+  if (CG == 1 && p.split > 1) {
     // One tile per cluster, its K shared out: CTA d settles columns d * cw .. of the tile.  Every CTA sends
     // each of the others its part of their columns (distributed shared memory, into the rings, which
     // nobody uses any more), and adds up what it got in rank order.
@@ -723,7 +782,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         uint32_t dst = peer_addr(mine + j * (BN * 4), d);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          if (c0 + i < rows) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst), "r"(v[i]) : "memory");
+          if (c0 + i < rows) store_remote(dst, static_cast<int>(v[i]));
           dst += BN * 4;
           if (++j == cw && d + 1 < p.split) { j = 0; ++d; dst = peer_addr(mine, d); }
         }

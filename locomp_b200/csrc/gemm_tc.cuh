@@ -146,6 +146,9 @@ __device__ __forceinline__ uint64_t make_b_desc(uint32_t smem_addr) {
   d |= static_cast<uint64_t>(2) << 61;                        // 128-byte swizzle
   return d;
 }
+// The N of a kind::f16 MMA is a multiple of this.  For the pair form (M = 256) it is 32 that is specified; 48, 80 and 112 gave the
+// right results, and are not used.
+__host__ __device__ constexpr int mma_n_step(int cg) { return 16 * cg; }
 // kind::f16 instruction descriptor: D=f32, A=B=f16, both K-major, M=128*CG, N=bm.
 __host__ __device__ inline uint32_t make_idesc(int bm, int cg) {
   return (1u << 4) | (static_cast<uint32_t>(bm >> 3) << 17) | (static_cast<uint32_t>((BN * cg) >> 4) << 24);
@@ -879,7 +882,7 @@ inline Tiling choose_tiling(int M, int N, int K, int sm_count) {
       // the tiles of the last wave in pieces of fewer rows of x
       for (int tail = 2; tail <= 8; tail *= 2) {
         const int piece = bm / tail;
-        if (piece < 32 || piece % 16 != 0 || piece * tail != bm) continue;
+        if (piece < 32 || piece % mma_n_step(cg) != 0 || piece * tail != bm) continue;
         const long long pieces = rem * tail, last = (pieces + P - 1) / P;
         consider(waves == 0 && pieces < P ? pieces : P, 0, tiles - rem, tail, 1,
                  start + full_waves + last * nk * step(piece, static_cast<double>(pieces) / last) + 0.5);

@@ -474,7 +474,7 @@ int lcq_gemm_tc_plan_check(int M, int N, int K, int sm_count, int* fields) {
     for (gemm_tc::Walk w(p, team); w.next(p);) {
       if (w.tile < 0 || w.tile >= t.n_tiles || w.st0 < 0 || w.st0 >= w.st1 || w.st1 > p.nst) { set_error("plan check: segment out of range"); return LCQ_ERR_BAD_ARG; }
       const int row = w.m0 - (w.tile / p.n_tiles_n) * p.bm;
-      if (row < 0 || row % w.bm != 0 || w.bm != (w.tile < p.full ? p.bm : p.bm / p.tail)) { set_error("plan check: bad piece"); return LCQ_ERR_BAD_ARG; }
+      if (row < 0 || row % w.bm != 0 || w.bm != (w.tile < p.full ? p.bm : p.bm / p.tail) || w.bm % gemm_tc::mma_n_step(t.cg) != 0) { set_error("plan check: bad piece"); return LCQ_ERR_BAD_ARG; }
       for (int st = w.st0; st < w.st1; ++st) seen[(static_cast<size_t>(w.tile) * t.tail + row / w.bm) * p.nst + st]++;
       if (row == 0) contributors[w.tile]++;
       if ((w.st0 == 0 && w.st1 == p.nst) || t.split > 1) continue;

@@ -27,6 +27,15 @@ def test_plan_covers_every_stage_once():
     assert lib.lcq_gemm_tc_plan_check(64, 100, 96, 148, f) == _lib.ERR_UNSUPPORTED
 
 
+@pytest.mark.parametrize("m,n,k", [(293, 14066, 5568), (379, 19152, 9024), (1042, 16637, 6976), (90, 9000, 2048), (700, 6000, 4096)])
+def test_pairs_multiply_rows_in_multiples_of_32(m, n, k):
+    """A pair's MMA takes N in steps of 32, a single SM's in steps of 16: whole tiles and the pieces of the last ones."""
+    f = (ctypes.c_int * 8)()
+    assert _lib.lib().lcq_gemm_tc_plan_check(m, n, k, 148, f) == 0
+    bm, cg, tail = f[1], f[5], f[7]
+    assert bm % (16 * cg) == 0 and bm % tail == 0 and (bm // tail) % (16 * cg) == 0
+
+
 CASES = [(17, 1, 64), (17, 257, 320), (31, 255, 256), (32, 256, 576), (33, 513, 1984), (64, 300, 4096), (96, 1000, 832),
          (128, 129, 4096), (160, 640, 1024), (161, 128, 768), (193, 700, 512), (224, 256, 2048), (250, 384, 448), (257, 2000, 1088),
          (40, 30000, 512), (300, 20000, 320), (1000, 4000, 512), (520, 9600, 1024)]

@@ -97,3 +97,49 @@ def test_ragged_k_has_exact_products(m, n, k, kind):
         assert torch.equal(L.quantized_matmul(x, w, s, 32, out=wide), L.quantized_matmul(x, w, s, 32, algo="gemv_tc", out_dtype="f32"))
         assert error(L.quantized_matmul(x, w, s, 32)) <= 1.003 * error(L.quantized_matmul(x, w, s, 32, algo="gemv_tc"))
     assert _lib.lib().lcq_check_device_status(None) == 0, _lib.lib().lcq_last_error()
+
+
+# Every form of the schedule, each with whole and with partial weight stages: (m, n, k), then what the plan for 148 SMs must say --
+# CTAs per MMA, whether tiles are cut along K, CTAs per cluster that share a tile, rows of a piece of a last tile (0: whole).
+FORMS = [((18, 74, 1792), (1, False, 4, 0)), ((18, 77, 832), (1, False, 4, 0)), ((19, 85, 1280), (1, False, 5, 0)), ((19, 73, 1344), (1, False, 6, 0)),
+         ((23, 5619, 2048), (1, False, 2, 0)), ((18, 2092, 1472), (1, False, 3, 0)),
+         ((20, 26048, 2304), (1, True, 1, 0)), ((20, 25453, 1216), (1, True, 1, 0)), ((64, 28672, 8192), (1, True, 1, 0)),
+         ((33, 21092, 2560), (1, False, 1, 32)), ((36, 20259, 1088), (1, False, 1, 32)), ((68, 21774, 1792), (1, False, 1, 48)),
+         ((69, 19544, 1088), (1, False, 1, 48)), ((114, 23439, 1024), (1, False, 1, 64)),
+         ((142, 12161, 768), (2, False, 1, 0)), ((130, 10336, 448), (2, False, 1, 0)),
+         ((103, 20209, 2304), (2, False, 1, 32)), ((371, 19953, 384), (2, False, 1, 32)), ((111, 20595, 1152), (2, False, 1, 32)),
+         ((113, 24755, 2304), (2, False, 1, 64)), ((229, 21765, 576), (2, False, 1, 64)),
+         ((1264, 3821, 1024), (2, False, 1, 96)), ((190, 19169, 640), (2, False, 1, 96)),
+         ((4805, 1170, 1280), (2, False, 1, 128)), ((711, 7733, 640), (2, False, 1, 128))]
+
+
+def _form(m, n, k, sms):
+    f = (ctypes.c_int * 8)()
+    assert _lib.lib().lcq_gemm_tc_plan_check(m, n, k, sms, f) == 0, _lib.lib().lcq_last_error()
+    return f[5], f[3] > 0, f[6], f[1] // f[7] if f[7] > 1 else 0
+
+
+@pytest.mark.parametrize("problem,form", FORMS)
+def test_the_forms_are_those_the_gpu_test_is_for(problem, form):
+    assert _form(*problem, 148) == form
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("problem,form", FORMS)
+def test_every_form_of_the_schedule(problem, form, kind):
+    """All outputs against the dequantised weights in 64 bits, with the bound at the head of this file: an absolute one on
+    each output, from sum |x w|."""
+    m, n, k = problem
+    assert _form(m, n, k, torch.cuda.get_device_properties(0).multi_processor_count) == form
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    w = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=g)
+    s = (torch.randn(n, k // 32, device="cuda", generator=g).abs() * 0.02).half()
+    x = torch.randn(m, k, device="cuda", generator=g).to(kind)
+    w64 = L.dequantize(w, s.float(), n, k, 32).double()
+    ref, mag = x.double() @ w64.t(), x.double().abs() @ w64.abs().t()
+    out = L.quantized_matmul(x, w, s, 32, algo="gemm_tc", out_dtype="f32")
+    assert bool(((out.double() - ref).abs() <= (2.0 ** -11 + 2.0 ** -12) * mag).all())
+    narrow = L.quantized_matmul(x, w, s, 32, algo="gemm_tc")
+    assert torch.equal(narrow, out.to(kind))                                  # the same sums, rounded once
+    assert _lib.lib().lcq_check_device_status(None) == 0, _lib.lib().lcq_last_error()

@@ -66,6 +66,14 @@ def fuse_rows(parts: Sequence[Tuple[torch.Tensor, torch.Tensor]], group_size: in
     return QuantLinear(w, s, group_size, bits), splits
 
 
+def _one_kernel_pays(layers: int, layer_weights: int, head_weights: int) -> bool:
+    """Whether a step is faster as one kernel than as a chain of launches.  The kernel saves about 10 us a layer of launches and
+    hand-overs; its float32 matvecs stream weights more slowly than the decode kernel: about 1 us per 30 Mi weights of a
+    layer and per 15 Mi of the lm_head.  Kernel and chain in us: 30 layers of 576 / 1536 299 and 484; 24 of 2048 / 8192 539 and 726; 6 of 4096 / 14336 304 and
+    323; 5 of 4608 / 12288 299 and 297; 4 of 6144 / 16384 342 and 296; 6 of 3584 / 18944 with 152,064 rows of lm_head 392 and 370."""
+    return layers * (10.0 - layer_weights / 30e6) > head_weights / 15e6
+
+
 class DecodeStack:
     """The quantized linears of one decode step of a Llama-style stack (SmolLM2 shapes by default),
     chained on fixed activation buffers: q|k|v, o, gate|up, down per layer, then the lm_head.
@@ -76,7 +84,7 @@ class DecodeStack:
     (examples/54_smollm2_inference.py:494-554, :556-578) except attention itself: embedding lookup,
     input RMS norm, residual add + post-attention norm (one kernel), SiLU * up, residual add, final
     norm, and a greedy argmax of the logits on the device -- a real dependency chain on one hidden
-    state.  In fp16 the whole step is one kernel where that covers the shape, else 8 launches per layer."""
+    state.  In fp16 the whole step is one kernel where that covers the shape and is faster, else 8 launches per layer."""
 
     def __init__(self, layers: int = 30, hidden: int = 576, inter: int = 1536, q_heads: int = 9, kv_heads: int = 3,
                  head_dim: int = 64, vocab: int = 49152, fused: bool = False, device="cuda", seed: int = 0,
@@ -173,8 +181,8 @@ class DecodeStack:
         self._graph = None
 
     def _one_kernel(self, x_q, layers, hidden, inter, qd, qkv, vocab):
-        """Describe the step to the kernel that runs all of it, if it covers the shape (fp16 only)."""
-        if self.norms.dtype != torch.float16:
+        """Describe the step to the kernel that runs all of it, if it covers the shape (fp16 only) and is faster."""
+        if self.norms.dtype != torch.float16 or not _one_kernel_pays(layers, hidden * (qkv + qd + 3 * inter), hidden * vocab):
             return
         pointers = [[t.data_ptr() for lin, _, _ in self.calls[4 * i:4 * i + 4] for t in (lin.w, lin.scales)] for i in range(layers)]
         head = self.calls[-1][0]

@@ -6,8 +6,7 @@ import torch
 
 import locomp_b200 as L
 from locomp_b200 import _lib
-
-pytestmark = pytest.mark.gpu
+from locomp_b200.linear import _one_kernel_pays
 
 # fewer rows than SMs in some phase, hidden beyond one pass of the threads, rows that fill no tile, many tiles
 SHAPES = [dict(layers=1, hidden=64, inter=64, q_heads=1, kv_heads=1, vocab=4), dict(layers=2, hidden=128, inter=192, q_heads=2, kv_heads=1, vocab=1000),
@@ -15,10 +14,28 @@ SHAPES = [dict(layers=1, hidden=64, inter=64, q_heads=1, kv_heads=1, vocab=4), d
           dict(layers=2, hidden=2112, inter=5632, q_heads=33, kv_heads=3, vocab=3000), dict(layers=2, hidden=2048, inter=8192, q_heads=32, kv_heads=32, vocab=16384)]
 
 
+# layers, hidden, inter, query and key heads, vocabulary: us of the one kernel, us of the chain
+MEASURED = [((1, 64, 64, 1, 1, 64), 16.6, 16.7), ((12, 256, 768, 4, 4, 32000), 96.8, 140.3), ((30, 576, 1536, 9, 3, 49152), 298.9, 483.7),
+            ((1, 576, 1536, 9, 3, 49152), 26.7, 33.0), ((8, 1024, 3072, 16, 8, 151936), 119.4, 192.6), ((24, 2048, 8192, 32, 32, 49152), 539.2, 726.3),
+            ((1, 2048, 8192, 32, 32, 16384), 37.3, 41.1), ((8, 2560, 9728, 32, 8, 151936), 293.5, 354.6), ((8, 3072, 8192, 24, 8, 128256), 301.3, 344.3),
+            ((4, 3072, 24576, 24, 24, 32000), 238.0, 240.2), ((6, 3584, 18944, 28, 4, 152064), 391.9, 370.0), ((6, 4096, 4096, 32, 8, 32000), 177.0, 210.6),
+            ((8, 4096, 14336, 32, 8, 128256), 466.1, 469.1), ((6, 4096, 14336, 32, 32, 32000), 319.7, 336.4), ((5, 4608, 12288, 36, 36, 32000), 299.0, 296.8),
+            ((5, 5120, 5120, 40, 8, 32000), 201.0, 242.2), ((4, 5120, 13824, 40, 8, 32000), 272.5, 256.9), ((4, 5120, 13824, 40, 40, 32000), 289.5, 281.7),
+            ((4, 6144, 16384, 48, 8, 32000), 342.3, 295.8), ((4, 8192, 8192, 64, 8, 32000), 332.3, 294.4)]
+
+
+def test_the_faster_form_is_taken():
+    """Against times of both forms from 64 to 8192 wide: the rule's choice costs at most 3 % more than the better one."""
+    for (layers, hidden, inter, q, kv, vocab), kernel, chain in MEASURED:
+        pays = _one_kernel_pays(layers, hidden * (64 * (2 * q + 2 * kv) + 3 * inter), hidden * vocab)
+        assert (kernel if pays else chain) <= 1.03 * min(kernel, chain), (layers, hidden, inter, vocab)
+
+
 def _results(st):
     return [t.clone() for t in (st.logits, st.hidden, st.normed, st.mlp, st.outputs)]
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("shape", SHAPES)
 def test_matches_the_chain_of_kernels(shape):
     st = L.DecodeStack(fused=True, glue=True, seed=7, **shape)
@@ -43,6 +60,7 @@ def test_matches_the_chain_of_kernels(shape):
     assert _lib.lib().lcq_check_device_status(None) == 0, _lib.lib().lcq_last_error()
 
 
+@pytest.mark.gpu
 def test_unknown_token_is_reported():
     st = L.DecodeStack(layers=1, hidden=128, inter=192, q_heads=2, kv_heads=1, vocab=1000, fused=True, glue=True)
     st.token.fill_(1000)
@@ -61,6 +79,7 @@ def _plain_step(st):
     return [t.clone() for t in (st.logits, st.hidden)]
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("replaced", ["token", "table", "w", "scales", "data", "ops"])
 def test_what_was_replaced_since_the_construction_is_used(replaced):
     """Rebinding a buffer or a weight takes effect, as in the chain of launches (then the chain runs: the same bits)."""
@@ -87,6 +106,7 @@ def test_what_was_replaced_since_the_construction_is_used(replaced):
     assert _lib.lib().lcq_check_device_status(None) == 0
 
 
+@pytest.mark.gpu
 def test_error_against_64_bits_is_that_of_the_chain():
     """Thirty layers, both forms against the step in 64 bits with nothing rounded in between.  The two round the same values to
     fp16 after float32 sums in different orders, so either may come out ahead; over four inputs the root mean square of the kernel's
@@ -114,9 +134,12 @@ def test_error_against_64_bits_is_that_of_the_chain():
     assert rms[1] <= 1.25 * rms[0], (chain, kernel)
 
 
+@pytest.mark.gpu
 def test_other_shapes_and_types_keep_the_chain():
     st = L.DecodeStack(layers=1, hidden=96, inter=192, q_heads=2, kv_heads=1, vocab=1000, fused=True, glue=True)
     assert st._desc is None and st.launches_per_step == len(st.ops)
+    wide = L.DecodeStack(layers=1, hidden=8192, inter=8192, q_heads=64, kv_heads=8, vocab=4096, fused=True, glue=True)
+    assert wide._desc is None                 # covered, and slower than the chain
     st = L.DecodeStack(layers=1, hidden=128, inter=192, q_heads=2, kv_heads=1, vocab=1000, fused=True, glue=True, dtype=torch.bfloat16)
     assert st._desc is None
     st.step()

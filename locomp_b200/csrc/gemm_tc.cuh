@@ -23,11 +23,12 @@
 // 64-k steps every step took ~750 clocks whatever bm), two sets of dequant warps that take the stages in
 // turn, and MMAs issued by an elected lane of a uniform warp.
 //
-// Split of the work: whole tiles in turn while they fill all teams; the rest is cut along K into equal
-// shares (stream-K).  A tile produced by several teams is combined through scratch: every contributor
-// publishes its float32 partial and bumps a counter, the last one sums all in a fixed order and writes
-// the output.  Nobody waits for another team.  With fewer tiles than SMs a cluster of 2, 4 or 8 CTAs shares
-// the K of each tile and adds up the partials over distributed shared memory.
+// Split of the work: whole tiles in turn while they fill all teams.  The rest goes in pieces of fewer rows, or, on
+// single SMs, is cut along K into equal shares (stream-K): a tile produced by several CTAs is combined through
+// scratch, every contributor publishes its float32 partial and bumps a counter, the last one sums all in a
+// fixed order and writes the output.  Nobody waits for another CTA.  With fewer tiles than SMs a cluster of 2 to 6
+// single CTAs shares the K of each tile and adds up the partials over distributed shared memory.  Pairs are not cut
+// along K: nothing of that kind has been measured on them.
 //
 // Weight tiles are fp16 because bf16's 8-bit significand cannot hold (q-8)*s within the 1e-2 output
 // tolerance; bf16 activations are converted to fp16 by a small pre-pass into the caller's workspace.
@@ -158,14 +159,14 @@ __host__ __device__ inline uint32_t make_idesc(int bm, int cg) {
 struct Params {
   void* out;            // [M, N]
   const void* scales;   // [N, K/32] fp16 (read directly when K % 256 != 0)
-  float* partials;      // [2 * teams][CTA of the team][bm][BN]
-  int* counters;        // [sk_tiles][CTA of the team], zero on entry, zero on exit
+  float* partials;      // CG = 1: [2 * teams][bm][BN]
+  int* counters;        // [sk_tiles], zero on entry, zero on exit
   int M, N, K;
   int bm;               // activation rows per tile (MMA N): multiple of 32, <= 256
   int n_tiles_n, n_tiles;
   int nst;              // 256-k weight stages per tile
   int teams;            // CTAs (CG = 1) or pairs (CG = 2) launched
-  int sk_tiles;         // tiles 0 .. sk_tiles-1 are cut along K, the others go whole to team (tile - sk_tiles) % teams
+  int sk_tiles;         // tiles 0 .. sk_tiles-1 (CG = 2: none) are cut along K, the others go whole to team (tile - sk_tiles) % teams
   int full, tail;       // tiles full .. are cut into `tail` pieces of bm / tail rows of x (a last wave that would be mostly empty)
   int split;            // > 1: a cluster of `split` teams per tile, each with its share of K (no whole tiles, no scratch)
   int nxs, nws;         // ring depths: X stages, weight stages
@@ -245,7 +246,7 @@ __host__ __device__ inline int x_step_bytes(int bm, int cg) { return (bm / cg) *
 __host__ __device__ inline int x_stage_bytes(int bm, int cg) { return (WK / BK) * x_step_bytes(bm, cg); }
 __host__ __device__ inline Smem smem_map(int bm, int cg, int nxs, int nws) {
   Smem s;
-  s.w = nxs * x_stage_bytes(bm, cg);    // X stages first: steps are multiples of 2048 bytes
+  s.w = nxs * x_stage_bytes(bm, cg);    // X stages first: steps are multiples of 1024 bytes, the swizzle's period
   s.bars = s.w + nws * WS_STAGE;
   // full_x, empty_x [MAX_XS]; full_w, empty_w [MAX_WS]; full_a, empty_a [MAX_AS]; full_d, empty_d [2]; drained
   s.tmem_slot = s.bars + (2 * MAX_XS + 2 * MAX_WS + 2 * MAX_AS + 5) * 8;
@@ -697,16 +698,16 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       if (CG == 1 && p.split > 1) break;       // the cluster adds up its shares below
       // who else contributes to this tile: teams p0 .. p1
       int p0 = team, p1 = team, slot1 = 0;
-      if (w.tile < p.sk_tiles) {
+      if (CG == 1 && w.tile < p.sk_tiles) {
         const unsigned t0 = static_cast<unsigned>(w.tile) * static_cast<unsigned>(p.nst);
         p0 = share_owner(p, t0);
         p1 = share_owner(p, t0 + static_cast<unsigned>(p.nst) - 1u);
         slot1 = share_begin(p, p0) < t0;       // p0 came from the tile before (slot 0); the others' shares begin here
       }
       const auto part = [&](int q) {
-        return p.partials + (static_cast<long long>(2 * q + (q == p0 ? slot1 : 0)) * CG + crank) * part_elems + r;
+        return p.partials + static_cast<long long>(2 * q + (q == p0 ? slot1 : 0)) * part_elems + r;
       };
-      if (p1 == p0) {
+      if (CG == 2 || p1 == p0) {
         for (int c0 = 0; c0 < rows; c0 += 32) {
           uint32_t v[32];
           tmem_ld32(d_t + c0, v);
@@ -721,7 +722,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           }
         }
       } else {
-        int* counter = p.counters + w.tile * CG + crank;
+        int* counter = p.counters + w.tile;
         // published already by all the others?  Then this CTA finishes the tile without publishing.
         if (threadIdx.x == WARP_EPI0 * 32) *shared_int = load_acquire(counter);
         named_bar_sync(BAR_EPI, 128);
@@ -745,8 +746,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         }
         __threadfence();
         if (finish) {
-          finish_tile<OT>(d_t, out, n < p.N ? rows : 0, rows, p.N, part(p0), part(p0) + (2 - slot1) * CG * part_elems,
-                          2 * CG * part_elems, p1 - p0 + 1, team - p0);
+          finish_tile<OT>(d_t, out, n < p.N ? rows : 0, rows, p.N, part(p0), part(p0) + (2 - slot1) * part_elems,
+                          2 * part_elems, p1 - p0 + 1, team - p0);
           if (threadIdx.x == WARP_EPI0 * 32) *counter = 0;
         }
       }
@@ -917,7 +918,7 @@ inline size_t x_copy_bytes(int M, int K, int x_dtype) {
   return x_dtype == LCQ_BF16 ? ((static_cast<size_t>(M) * K * 2 + 255) & ~static_cast<size_t>(255)) : 0;
 }
 inline size_t partial_bytes(const Tiling& t) {
-  return t.sk_tiles ? static_cast<size_t>(t.teams) * 2 * t.cg * t.bm * BN * sizeof(float) : 0;
+  return t.sk_tiles ? static_cast<size_t>(t.teams) * 2 * t.bm * BN * sizeof(float) : 0;
 }
 // [shared counter region][fp16 copy of bf16 activations][float partials of the tiles cut along K]
 inline size_t workspace_bytes(const Tiling& t, int M, int K, int x_dtype) {

@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
 
 template <int WBITS, typename XT, typename ST, typename OT>
 int launch_gemv_simt(const void* x, const void* w, const void* s, void* out, int M, int N, int K, int G,
-                     cudaStream_t stream) {
+                     int sm_count, cudaStream_t stream) {
   if (M == 0 || N == 0) return LCQ_OK;
   const bool vec = (K % 8 == 0) && (G % 8 == 0) && aligned(x, 16) && aligned(w, WBITS == 4 ? 4 : 8);
   const XT* xp = static_cast<const XT*>(x);
@@ -309,12 +309,12 @@ int launch_gemv_simt(const void* x, const void* w, const void* s, void* out, int
                                     op, M, N, K, G));                                                \
   } while (0)
   if (vec && (M > 1 || static_cast<long long>(N) * K > (1LL << 21))) {
-    // 8 warps a block; K is shared while the warps fill less than two thirds of the SMs twice over (8 warps each
-    // way) and every one of them still has a chunk per lane
+    // 8 warps a block; the warps of a block share K while there are fewer than 12 warps an SM and each of them still has a
+    // chunk per lane
     int split = 0;
     const long long groups = (N + 3) / 4;
     const int mt = M == 1 ? 1 : M == 2 ? 2 : 4, m_blocks = (M + mt - 1) / mt;
-    while (split < 3 && ((groups * m_blocks) << split) < 148 * 12 && (K >> 3) >= (64 << split)) ++split;
+    while (split < 3 && ((groups * m_blocks) << split) < sm_count * 12LL && (K >> 3) >= (64 << split)) ++split;
     int gshift = -1;
     if ((G & (G - 1)) == 0) { gshift = 0; while ((1 << gshift) < G) ++gshift; }
     cfg.gridDim = dim3(static_cast<unsigned>((groups + (8 >> split) - 1) / (8 >> split)), m_blocks);

@@ -150,32 +150,32 @@ static int dequant_entry(int wbits, const void* w, const void* s, void* out, int
 
 template <int WBITS, typename XT, typename ST>
 static int simt_by_out(const void* x, const void* w, const void* s, void* out, int M, int N, int K, int G,
-                       int out_dtype, cudaStream_t st) {
+                       int out_dtype, int sm, cudaStream_t st) {
   switch (out_dtype) {
-    case LCQ_F32: return launch_gemv_simt<WBITS, XT, ST, float>(x, w, s, out, M, N, K, G, st);
-    case LCQ_F16: return launch_gemv_simt<WBITS, XT, ST, __half>(x, w, s, out, M, N, K, G, st);
-    case LCQ_BF16: return launch_gemv_simt<WBITS, XT, ST, __nv_bfloat16>(x, w, s, out, M, N, K, G, st);
+    case LCQ_F32: return launch_gemv_simt<WBITS, XT, ST, float>(x, w, s, out, M, N, K, G, sm, st);
+    case LCQ_F16: return launch_gemv_simt<WBITS, XT, ST, __half>(x, w, s, out, M, N, K, G, sm, st);
+    case LCQ_BF16: return launch_gemv_simt<WBITS, XT, ST, __nv_bfloat16>(x, w, s, out, M, N, K, G, sm, st);
   }
   return LCQ_ERR_BAD_ARG;
 }
 template <int WBITS, typename XT>
 static int simt_by_scale(const void* x, const void* w, const void* s, void* out, int M, int N, int K, int G,
-                         int scale_dtype, int out_dtype, cudaStream_t st) {
+                         int scale_dtype, int out_dtype, int sm, cudaStream_t st) {
   switch (scale_dtype) {
-    case LCQ_F32: return simt_by_out<WBITS, XT, float>(x, w, s, out, M, N, K, G, out_dtype, st);
-    case LCQ_F16: return simt_by_out<WBITS, XT, __half>(x, w, s, out, M, N, K, G, out_dtype, st);
-    case LCQ_BF16: return simt_by_out<WBITS, XT, __nv_bfloat16>(x, w, s, out, M, N, K, G, out_dtype, st);
+    case LCQ_F32: return simt_by_out<WBITS, XT, float>(x, w, s, out, M, N, K, G, out_dtype, sm, st);
+    case LCQ_F16: return simt_by_out<WBITS, XT, __half>(x, w, s, out, M, N, K, G, out_dtype, sm, st);
+    case LCQ_BF16: return simt_by_out<WBITS, XT, __nv_bfloat16>(x, w, s, out, M, N, K, G, out_dtype, sm, st);
   }
   return LCQ_ERR_BAD_ARG;
 }
 template <int WBITS>
 static int simt_entry(const void* x, const void* w, const void* s, void* out, int M, int N, int K, int G,
-                      int x_dtype, int scale_dtype, int out_dtype, cudaStream_t st) {
+                      int x_dtype, int scale_dtype, int out_dtype, int sm, cudaStream_t st) {
   if (M > 4 * 65535) { set_error("SIMT path supports M <= 262140"); return LCQ_ERR_UNSUPPORTED; }
   switch (x_dtype) {
-    case LCQ_F32: return simt_by_scale<WBITS, float>(x, w, s, out, M, N, K, G, scale_dtype, out_dtype, st);
-    case LCQ_F16: return simt_by_scale<WBITS, __half>(x, w, s, out, M, N, K, G, scale_dtype, out_dtype, st);
-    case LCQ_BF16: return simt_by_scale<WBITS, __nv_bfloat16>(x, w, s, out, M, N, K, G, scale_dtype, out_dtype, st);
+    case LCQ_F32: return simt_by_scale<WBITS, float>(x, w, s, out, M, N, K, G, scale_dtype, out_dtype, sm, st);
+    case LCQ_F16: return simt_by_scale<WBITS, __half>(x, w, s, out, M, N, K, G, scale_dtype, out_dtype, sm, st);
+    case LCQ_BF16: return simt_by_scale<WBITS, __nv_bfloat16>(x, w, s, out, M, N, K, G, scale_dtype, out_dtype, sm, st);
   }
   return LCQ_ERR_BAD_ARG;
 }
@@ -192,7 +192,8 @@ static size_t gemv_tc_workspace_bytes(int M, int N, int K, int sm_count) {
 }
 
 // LCQ_ALGO_GEMV_W8 named a TMA-staged int8 kernel; the float kernels now run such calls in a half to a quarter of
-// its time (M = 1, 2048 -> 49152 float32: 46 us, now 25; M = 7: 380 us, now 95).  The code stays for callers.
+// its time (M = 1, 2048 -> 49152 float32: 46 us, now 25; M = 7: 380 us, now 95).  Callers may still ask for it by that
+// name, and lcq_matmul_select_algo still reports it for the calls that it ran: it is LCQ_ALGO_SIMT under another code.
 static bool w8_supported(int M, int N, int K, int G) {
   return M >= 1 && M <= 8 && N >= 1 && K >= 16 && (K % 16) == 0 && G >= 16 && (G % 16) == 0;
 }
@@ -240,8 +241,8 @@ static int matmul_entry(int wbits, const void* x, const void* w, const void* s, 
   }
   switch (algo) {
     case LCQ_ALGO_SIMT:
-      return wbits == 4 ? simt_entry<4>(x, w, s, out, M, N, K, G, x_dtype, scale_dtype, out_dtype, st)
-                        : simt_entry<8>(x, w, s, out, M, N, K, G, x_dtype, scale_dtype, out_dtype, st);
+      return wbits == 4 ? simt_entry<4>(x, w, s, out, M, N, K, G, x_dtype, scale_dtype, out_dtype, di.sm_count, st)
+                        : simt_entry<8>(x, w, s, out, M, N, K, G, x_dtype, scale_dtype, out_dtype, di.sm_count, st);
     case LCQ_ALGO_GEMV_TC: {
       if (wbits != 4 || !gemv_tc::supported(M < 16 ? M : 16, N, K, G, x_dtype, scale_dtype)) {
         set_error("GEMV_TC needs int4, group_size 32, K %% 64 == 0, f16 scales, f16/bf16 x");
@@ -272,7 +273,7 @@ static int matmul_entry(int wbits, const void* x, const void* w, const void* s, 
         set_error("GEMV_W8 needs int8 weights, M <= 8, K %% 16 == 0, group_size %% 16 == 0");
         return LCQ_ERR_UNSUPPORTED;
       }
-      return simt_entry<8>(x, w, s, out, M, N, K, G, x_dtype, scale_dtype, out_dtype, st);
+      return simt_entry<8>(x, w, s, out, M, N, K, G, x_dtype, scale_dtype, out_dtype, di.sm_count, st);
     case LCQ_ALGO_GEMM_TC:
       if (wbits != 4 || !gemm_tc::supported(M, N, K, G, x_dtype, scale_dtype)) {
         set_error("GEMM_TC needs int4, group_size 32, K %% 64 == 0, f16 scales, f16/bf16 x");
@@ -461,7 +462,7 @@ int lcq_gemm_tc_plan_check(int M, int N, int K, int sm_count, int* fields) {
       t.bm % 32 != 0 || t.bm < 32 || t.bm > (t.cg == 2 ? 256 : 128) || smem > 227 * 1024 || t.nxs < 2 || t.nws < 2 ||
       t.nxs > gemm_tc::MAX_XS || t.nws > gemm_tc::MAX_WS || t.nas > gemm_tc::MAX_AS ||
       t.nd * t.bm + t.nas * gemm_tc::A_SLOT_COLS > gemm_tc::TMEM_COLS ||
-      static_cast<size_t>(t.sk_tiles) * t.cg * sizeof(int) > kWorkspaceCounterBytes) {
+      static_cast<size_t>(t.sk_tiles) * sizeof(int) > kWorkspaceCounterBytes || (t.cg == 2 && t.sk_tiles != 0)) {
     set_error("plan check: bad tiling (teams %d, bm %d, %d bytes of shared memory)", t.teams, t.bm, smem);
     return LCQ_ERR_BAD_ARG;
   }

@@ -195,7 +195,8 @@ int lcq_argmax(const void* x, void* out, int64_t rows, int n, int dtype, void* s
  * RMS norm, gate|up, SiLU * up, down, residual add; final norm, lm_head, greedy argmax into `next_token`.
  * Every result (logits, outputs, *_out) is written.  The same chain as lcq_embed_lookup, lcq_rms_norm,
  * lcq_matmul_int4, lcq_residual_rms_norm, lcq_silu_mul, lcq_add_inplace and lcq_argmax in
- * examples/54_smollm2_inference.py:494-578 order.
+ * examples/54_smollm2_inference.py:494-578 order.  There is no attention in it, and no place for it: o reads x_q, so
+ * the kernel computes it ahead of its turn, and a layer has two dependent phases instead of four.
  *
  * The kernel fills the GPU (one CTA per SM, cooperative launch) and its CTAs wait for one another, with the
  * limit of lcq_set_wait_limit_ns.  `layers` points to n_layers lcq_decode_layer records in DEVICE memory;

@@ -3,7 +3,8 @@
 // up, down, residual add}, final norm, lm_head and greedy argmax -- the chain that locomp_b200.DecodeStack
 // runs as 8 launches a layer otherwise (examples/54_smollm2_inference.py:494-578 without the attention
 // itself; o reads a prepared buffer, so it depends on nothing in its layer and runs beside the down projection
-// before it: two phases a layer).
+// before it).  That makes two dependent phases a layer.  It is an order that only a step without attention has: a
+// layer whose o reads the attention output has four (q|k|v, o, gate|up, down) and cannot take this schedule.
 //
 // What bounds it.  SmolLM2-135M has 30 layers of 2 MB: 12 us of HBM time for the whole token, but ~90
 // dependent matvecs.  As separate kernels each costs ~2 us (launch, dependency wait, first loads, drain):

@@ -24,8 +24,9 @@
 // to the same integer unless t lies that close to a half-integer.  Adding 1.5 * 2^23 rounds t to an integer
 // (to even) and leaves it in the low bits of the sum; t minus that integer is exact, and when it comes
 // within the bound of 1/2 (or t is no number) the thread divides.  Dividing every weight and converting
-// with rint / min / max / float-to-int instructions bound the kernel: 4096 x 14336, int4, float32 weights 82 us,
-// now 41 us (6.6 TB/s); float16 48 us, bfloat16 60 us (its ties: one octet in a few has one).
+// with rint / min / max / float-to-int instructions bound the kernel: 4096 x 14336, int4, float32 weights 84 us a
+// call, now 48 (the kernel alone, from a cold cache, 44 us for 235 MB read and 37 MB written, most of which are still in
+// L2 when it ends); back to back float16 takes 48 us, bfloat16 60 (its ties: one octet in a few has one).
 #pragma once
 #include "common.cuh"
 #include "gemv_simt.cuh"

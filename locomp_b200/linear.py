@@ -84,7 +84,9 @@ class DecodeStack:
     (examples/54_smollm2_inference.py:494-554, :556-578) except attention itself: embedding lookup,
     input RMS norm, residual add + post-attention norm (one kernel), SiLU * up, residual add, final
     norm, and a greedy argmax of the logits on the device -- a real dependency chain on one hidden
-    state.  In fp16 the whole step is one kernel where that covers the shape and is faster, else 8 launches per layer."""
+    state.  In fp16 the whole step is one kernel where that covers the shape and is faster, else 8 launches per layer.
+    Since o reads a prepared buffer and not attention output, that kernel computes it beside the down projection of the layer
+    before: two dependent phases a layer, where a model with attention has four."""
 
     def __init__(self, layers: int = 30, hidden: int = 576, inter: int = 1536, q_heads: int = 9, kv_heads: int = 3,
                  head_dim: int = 64, vocab: int = 49152, fused: bool = False, device="cuda", seed: int = 0,

@@ -2,29 +2,39 @@
 // kernel: embedding, per layer {RMS norm, q|k|v and o projections, residual add + RMS norm, gate|up, SiLU *
 // up, down, residual add}, final norm, lm_head and greedy argmax -- the chain that locomp_b200.DecodeStack
 // runs as 8 launches a layer otherwise (examples/54_smollm2_inference.py:494-578 without the attention
-// itself; o reads a prepared buffer, so it depends on nothing in its layer and runs beside the down projection
-// before it).  That makes two dependent phases a layer.  It is an order that only a step without attention has: a
-// layer whose o reads the attention output has four (q|k|v, o, gate|up, down) and cannot take this schedule.
+// itself; o reads a prepared buffer, so it depends on nothing in its layer).  That makes two dependent
+// exchanges a layer.  It is an order that only a step without attention has: a layer whose o reads the
+// attention output has four (q|k|v, o, gate|up, down) and cannot take this schedule.
 //
-// What bounds it.  SmolLM2-135M has 30 layers of 2 MB: 12 us of HBM time for the whole token, but ~90
-// dependent matvecs.  As separate kernels each costs ~2 us (launch, dependency wait, first loads, drain):
-// 506 us a token, now 297; 5 layers of width 2048 167 us, now 135.  What is left is instruction latency: a phase
-// is ~1000 dependent instructions of a warp (norm 1.2 us, tiles 1.3, publishing 0.9, waiting 1.3).  Here
+// What bounds it.  SmolLM2-135M has 30 layers of 2 MB: 12 us of HBM time for the whole token, but a chain
+// of 60 dependent matvecs whose results every SM needs.  Latency is all there is to it: the round trip
+// through L2 (0.9 us from storing a result to every CTA's having it) and the dependent instructions of a matvec, a norm and
+// an activation.  As separate kernels 484 us a token, as one kernel with float32 FMAs 292, now 191 to 217 (over boxes).  Hence
 //   * one CTA per SM stays for the whole step; a producer thread streams the CTA's rows of ALL layers
 //     through one shared-memory ring (bulk copies), running ahead across layers, so that weights are there
 //     when their input is;
 //   * results that the next phase needs are published as words {fp16 value, 16-bit tag of the phase}: a
 //     consumer polls the data itself until every tag is the one it expects.  No grid barrier, no fence, no
 //     flag: one store and one load through L2 between dependent matvecs;
-//   * every CTA keeps the hidden state and does the norms redundantly.
-// Every CTA has at least one unit of 4 rows in every phase.  So whoever has all results of a phase knows
-// that all CTAs have read what they needed for it, and a buffer that is rewritten two phases later (the
-// next layer's) has no reader left.
+//   * every CTA keeps the hidden state and does the norms redundantly;
+//   * the warps are two sets with roles of their own, so that what is not on the chain runs beside it: the first
+//     set publishes the activation and the down projection and waits for the activations of the others, and computes o two layers ahead;
+//     the second does the norms and q|k|v.  Both multiply gate|up and down;
+//   * all of it is one loop body without calls: registers that a call saves go to the stack, and with all of L1 given to
+//     shared memory that is a trip to L2 (one call a phase cost 60 us a step); and code beyond 32 KB is fetched at half the speed.
+// A matvec runs on mma.sync: 16 rows x 32 k (one group) are two m16n8k16 MMAs whose A operand are the nibbles as q - 8
+// in fp16 (exact) and whose B operand is x; the group's scale multiplies the float32 result.
+// No shuffles: the tensor core adds up a group, a lane the groups of its rows, shared memory the warps.
+//
+// Every CTA has at least one unit of 4 rows in every phase on the chain.  So whoever has all results of a phase knows
+// that all CTAs have read what they needed for it, and a buffer that is rewritten a layer later has no reader left.  The
+// results of o take two buffers in turn: those of layer l + 2 are written after all activations of layer l have come in, which were
+// published after the norms that read o of layer l.
 //
 // The CTAs wait for one another: the launch is cooperative, and every wait is bounded (on expiry the CTA
 // records a status code and runs to its end without waiting).
 //
-// Arithmetic as in the separate kernels: products and sums in float32, each result rounded to fp16 where
+// Arithmetic as in the separate kernels: exact products and float32 sums, each result rounded to fp16 where
 // those kernels store it.
 #pragma once
 #include "common.cuh"
@@ -32,51 +42,74 @@
 namespace lcq {
 namespace step {
 
-constexpr int NCW = 16;                        // consumer warps
-constexpr int NCT = NCW * 32;
-constexpr int NTHREADS = NCT + 32;             // + the producer warp
+// Two sets of SET consumer warps, and the producer; U groups of 32 columns of a warp's share of a stage at a time.
+template <int SET> struct Threads {
+  static constexpr int NCW = 2 * SET, NCT = NCW * 32, SET_T = SET * 32, ALL = NCT + 32, U = SET == 4 ? 5 : 3;
+};
 constexpr int MAX_STAGES = 32;
-constexpr int BAR_C = 1;                       // named barrier of the consumers
+enum { BAR_ALL = 1, BAR_SUMS, BAR_SET0, BAR_SET1 };   // named barriers: all consumers; a phase's sums are there; those of a set
 constexpr int STATE_BYTES = 64;                // epoch, argmax counter, argmax key
+constexpr int HEAD_SLABS = 32;                 // slabs of the lm_head whose sums are kept at a time
+constexpr int COPIES = 8;                      // of the published words: a CTA polls copy b % 8.  (30 layers of width 576: 1 copy 420 us, 2 363, 4 337, 8 332, 16 325 in an early build)
+constexpr int ROW_SUMS = 48;                   // bytes of a row's partial sums of a stage, one per warp of a set (eight at most; rows sit in different banks)
+constexpr int STAGE_SUMS = 16 * ROW_SUMS;
+constexpr int PART_INFO_BYTES = 16 + 32 * 16 + 32 * 8;
 
 struct Shape { int hidden, inter, qkv, q_dim, vocab; };
+enum { PART_O, PART_GATE, PART_QKV, PART_DOWN, PART_HEAD, N_PARTS };
+// How a weight [n, K] is streamed: as [n * v, K / v], a matrix of the same bytes with shorter rows.  A stage is a slab of up to 16 of
+// those, the rows of an MMA's A operand, as they lie in memory: one copy, and one of their scales.  gate|up: up to 8 rows of gate, then the same
+// ones of up, so that both sums of a row end up in the same lane.
+struct Part {
+  int K, v;
+  int groups;           // of 32 columns of a (short) row; 16 bytes each, so that a row is `groups` times 16 bytes
+  int h1, slots;        // short rows of the first half of a slab (at most 8), of both
+  int per;              // rows that a slab advances by (gate|up: of each)
+};
+
+// Offsets in shared memory.
+struct Smem { int stages, xn, xq, xm, hid, gam, sums, side, red, info, bars, flags, rows, table, total; };
 
 struct Params {
   lcq_decode_stack d;
   Shape sh;
+  Part part[N_PARTS];
+  Smem map;
   int n_layers, ctas;
   int stage_bytes, n_stages;
-  int copies;           // of the published words: a CTA polls copy b % copies
-  int copy_words;       // 2 * hidden + inter
-  uint32_t* o_buf;      // published words, first copy: o projection, down projection [hidden], activation [inter]
+  float inv_hidden;
+  uint32_t* o_buf;      // published words, first copy: o projection (two buffers), down projection [hidden], activation [inter]
   uint32_t* d_buf;
   uint32_t* m_buf;
 };
 
 // Rows of an [n, K] weight that CTA b streams: whole units of 4 (so that rows of scales start on 16 bytes).
 __host__ __device__ inline int share(int n, int b, int ctas) { return static_cast<int>(static_cast<unsigned>(n / 4) * static_cast<unsigned>(b) / static_cast<unsigned>(ctas)) * 4; }
-__host__ __device__ inline int row_bytes(int K) { return K / 2 + K / 16; }
-__host__ __device__ inline int tile_rows(int stage_bytes, int K) { return (stage_bytes / row_bytes(K)) & ~3; }
-
-struct Smem { int stages, xn, xq, xm, hid, gam, res, red, bars, flags, rows, table, total; };
+__host__ __device__ inline int max_share(int n, int ctas) { return (n / 4 + ctas - 1) / ctas * 4; }
+__host__ __device__ inline int min2(int a, int b) { return a < b ? a : b; }
 __host__ __device__ inline int max2(int a, int b) { return a > b ? a : b; }
-__host__ __device__ inline Smem smem_map(const Shape& s, int n_layers, int ctas, int stage_bytes, int n_stages) {
+__host__ __device__ inline int stages_of(const Part& q, int rows) { return (rows + q.per - 1) / q.per; }
+
+inline Smem smem_map(const Params& p) {
+  const Shape& s = p.sh;
   Smem m;
   m.stages = 0;
-  m.xn = n_stages * stage_bytes;
+  m.xn = p.n_stages * p.stage_bytes;
   m.xq = m.xn + 2 * s.hidden * 2;              // both norms of a layer
   m.xm = m.xq + s.q_dim * 2;
   m.hid = m.xm + s.inter * 2;
   m.gam = m.hid + 2 * s.hidden * 2;            // before and after o
-  m.res = m.gam + 2 * s.hidden * 2;
-  const int per = 4;                           // a share is at most one unit above the average
-  const int rows = max2(max2((s.qkv + 2 * s.inter) / ctas + 6 * per, 2 * s.hidden / ctas + 4 * per), s.vocab / ctas + 2 * per);
-  m.red = m.res + rows * 16;
-  m.bars = m.red + 2 * NCW * 8;
+  m.sums = m.gam + 2 * s.hidden * 2;           // partial sums of the phases on the chain; of q|k|v, then of o
+  const int head = min2(max_share(s.vocab, p.ctas), HEAD_SLABS * p.part[PART_HEAD].per);
+  m.side = m.sums + max2(max2(stages_of(p.part[PART_GATE], max_share(s.inter, p.ctas)), stages_of(p.part[PART_DOWN], max_share(s.hidden, p.ctas))),
+                         stages_of(p.part[PART_HEAD], head)) * STAGE_SUMS;
+  m.red = m.side + (stages_of(p.part[PART_QKV], max_share(s.qkv, p.ctas)) + stages_of(p.part[PART_O], max_share(s.hidden, p.ctas))) * STAGE_SUMS;
+  m.info = m.red + 32 * 8;
+  m.bars = m.info + N_PARTS * PART_INFO_BYTES;
   m.flags = m.bars + 2 * MAX_STAGES * 8;
   m.rows = m.flags + 16;                       // Rows
-  m.table = m.rows + 32;                       // the layer records
-  m.total = m.table + n_layers * static_cast<int>(sizeof(lcq_decode_layer));
+  m.table = m.rows + 48;                       // the layer records
+  m.total = m.table + p.n_layers * static_cast<int>(sizeof(lcq_decode_layer));
   return m;
 }
 
@@ -93,63 +126,38 @@ __device__ __forceinline__ void publish(uint32_t* p, __half v, uint32_t tag) {
   const uint32_t word = (static_cast<uint32_t>(__half_as_ushort(v)) << 16) | tag;
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(word) : "memory");
 }
-// acc + a * b with float32 accumulation of the exact product; operands are halves of 32-bit registers
-__device__ __forceinline__ float fma_lo(uint32_t a, uint32_t b, bool a_hi, bool b_hi, float acc) {
-  const unsigned short x = static_cast<unsigned short>(a_hi ? a >> 16 : a), y = static_cast<unsigned short>(b_hi ? b >> 16 : b);
-  asm("fma.rn.f32.f16 %0, %1, %2, %0;" : "+f"(acc) : "h"(x), "h"(y));
-  return acc;
-}
 __device__ __forceinline__ uint32_t nibbles(uint32_t w, uint32_t mask, uint32_t magic, uint32_t offset) {   // two q - 8 as fp16, exact
   uint32_t r;
   asm("{\n\t.reg .b32 t;\n\tlop3.b32 t, %1, %2, %3, 0xEA;\n\tsub.f16x2 %0, t, %4;\n\t}" : "=r"(r) : "r"(w), "r"(mask), "r"(magic), "r"(offset));
   return r;
 }
-// sum of x[i] * (q[i] - 8) over the 8 nibbles of a word
-__device__ __forceinline__ float dot8(uint32_t w, const uint4& x) {
+// The 8 nibbles of a word as four operand registers: (0,4) (1,5) (2,6) (3,7).  x is staged in that order.
+__device__ __forceinline__ void unpack(uint32_t w, uint32_t (&v)[4]) {
   const uint32_t w8 = w >> 8;
-  const uint32_t a = nibbles(w, 0x000F000Fu, 0x64006400u, 0x64086408u);     // q0, q4
-  const uint32_t b = nibbles(w, 0x00F000F0u, 0x54005400u, 0x54805480u);     // q1, q5
-  const uint32_t c = nibbles(w8, 0x000F000Fu, 0x64006400u, 0x64086408u);    // q2, q6
-  const uint32_t d = nibbles(w8, 0x00F000F0u, 0x54005400u, 0x54805480u);    // q3, q7
-  float p = 0.0f, q = 0.0f;
-  p = fma_lo(a, x.x, false, false, p);
-  q = fma_lo(a, x.z, true, false, q);
-  p = fma_lo(b, x.x, false, true, p);
-  q = fma_lo(b, x.z, true, true, q);
-  p = fma_lo(c, x.y, false, false, p);
-  q = fma_lo(c, x.w, true, false, q);
-  p = fma_lo(d, x.y, false, true, p);
-  q = fma_lo(d, x.w, true, true, q);
-  return p + q;
+  v[0] = nibbles(w, 0x000F000Fu, 0x64006400u, 0x64086408u);
+  v[1] = nibbles(w, 0x00F000F0u, 0x54005400u, 0x54805480u);
+  v[2] = nibbles(w8, 0x000F000Fu, 0x64006400u, 0x64086408u);
+  v[3] = nibbles(w8, 0x00F000F0u, 0x54005400u, 0x54805480u);
 }
 
-// The phases of a step.  0: the first layer's o.  1 + 2 l: q|k|v, gate|up and the activation of layer l -- o
-// depends on x_q alone, so it is there already and both norms of a layer follow from the down projection
-// before it.  2 + 2 l: down of layer l, and o of the next layer.  1 + 2 n_layers: the lm_head.
-enum { PART_QKV, PART_GATE, PART_UP, PART_DOWN, PART_O, PART_HEAD };
-__device__ __forceinline__ int first_part(int ph, int n_layers) {
-  return ph == 0 ? PART_O : ph > 2 * n_layers + 1 ? -1 : ph == 2 * n_layers + 1 ? PART_HEAD : (ph & 1) ? PART_QKV : PART_DOWN;
-}
-__device__ __forceinline__ int next_part(int part, int ph, int n_layers) {
-  if (part == PART_QKV || part == PART_GATE) return part + 1;
-  return part == PART_DOWN && ph < 2 * n_layers ? PART_O : -1;
-}
-
-// What a CTA streams for a part of a phase: rows of a weight and of its scales.
-struct Rows { int qkv0, qkv, hid0, hid, int0, inter, voc0, voc; };   // this CTA's shares: first row, rows
-struct Segment { const uint8_t* w; const uint8_t* s; int row0, rows, K; };
-__device__ __forceinline__ Segment segment(const Params& p, const lcq_decode_layer* table, const Rows& r, int ph, int part) {
-  const Shape& sh = p.sh;
-  const lcq_decode_layer* l = table + (part == PART_O ? ph / 2 : (ph - 1) / 2);
-  switch (part) {
-    case PART_QKV: return {static_cast<const uint8_t*>(l->qkv_w), static_cast<const uint8_t*>(l->qkv_s), r.qkv0, r.qkv, sh.hidden};
-    case PART_GATE: return {static_cast<const uint8_t*>(l->gate_up_w), static_cast<const uint8_t*>(l->gate_up_s), r.int0, r.inter, sh.hidden};
-    case PART_UP: return {static_cast<const uint8_t*>(l->gate_up_w), static_cast<const uint8_t*>(l->gate_up_s), sh.inter + r.int0, r.inter, sh.hidden};
-    case PART_DOWN: return {static_cast<const uint8_t*>(l->down_w), static_cast<const uint8_t*>(l->down_s), r.hid0, r.hid, sh.inter};
-    case PART_O: return {static_cast<const uint8_t*>(l->o_w), static_cast<const uint8_t*>(l->o_s), r.hid0, r.hid, sh.q_dim};
-    default: return {static_cast<const uint8_t*>(p.d.head_w), static_cast<const uint8_t*>(p.d.head_s), r.voc0, r.voc, sh.hidden};
+// The order of the stream: o of the first two layers; per layer gate|up, q|k|v, down, o of the layer after next; the lm_head.
+struct Order {
+  int layer, part;      // layer of the weight
+  bool begun;
+  __host__ __device__ inline void next(int n_layers) {
+    if (part == PART_O) {
+      if (begun) { --layer; part = PART_GATE; }
+      else if (layer == 0 && n_layers > 1) layer = 1;
+      else { layer = 0; part = PART_GATE; begun = true; }
+    } else if (part == PART_GATE) part = PART_QKV;
+    else if (part == PART_QKV) part = PART_DOWN;
+    else if (part == PART_DOWN) {
+      if (layer + 2 < n_layers) { layer += 2; part = PART_O; }
+      else { ++layer; part = layer < n_layers ? PART_GATE : PART_HEAD; }
+    } else part = N_PARTS;
   }
-}
+};
+struct Rows { int qkv0, qkv, hid0, hid, int0, inter, voc0, voc, stages[4]; };   // this CTA's shares: first row, rows; stages of PART_O .. PART_DOWN
 
 // Shared memory by 32-bit addresses: generic pointers would take two registers each and a slower load.
 __device__ __forceinline__ uint32_t ld32(uint32_t a) { uint32_t v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
@@ -158,337 +166,557 @@ __device__ __forceinline__ uint4 ld128(uint32_t a) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
   return v;
 }
-__device__ __forceinline__ float ld_half(uint32_t a) {
-  unsigned short v;
+__device__ __forceinline__ uint2 ld64(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint16_t ld16(uint32_t a) {
+  uint16_t v;
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
-  return __half2float(__ushort_as_half(v));
+  return v;
+}
+__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
+}
+// The sum of 4 or 8 floats.
+template <int N> __device__ __forceinline__ float sum_words(uint32_t a) {
+  const uint4 u = ld128(a);
+  float t = (__uint_as_float(u.x) + __uint_as_float(u.y)) + (__uint_as_float(u.z) + __uint_as_float(u.w));
+  if (N == 8) {
+    const uint4 v = ld128(a + 16);
+    t += (__uint_as_float(v.x) + __uint_as_float(v.y)) + (__uint_as_float(v.z) + __uint_as_float(v.w));
+  }
+  return t;
 }
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   return v;
 }
-__device__ __forceinline__ void st128(uint32_t a, float x, float y, float z, float w) {
-  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
-}
+__device__ __forceinline__ void st128(uint32_t a, const uint4& v) { asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory"); }
 __device__ __forceinline__ void st32(uint32_t a, float x) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory"); }
-
-// A lane's sums over the words word0, word0 + step, ... of NR rows that are NCW rows apart.
-// w, sc, x: addresses of the first row's weights and scales and of the input.
-template <int NR>
-__device__ __forceinline__ void rows_dot(uint32_t w, uint32_t sc, uint32_t x, int K, int word0, int step, float (&acc)[NR]) {
-  const int words = K / 8;
+// Eight consecutive values of x, from index i (a multiple of 8), in the order that the operand registers want: (0,4) (1,5) (2,6) (3,7).
+__device__ __forceinline__ void stage_x(uint32_t x, int i, const __half2 (&v)[4]) {
+  uint32_t u[4];
 #pragma unroll
-  for (int r = 0; r < NR; ++r) acc[r] = 0.0f;
-#pragma unroll (NR == 1 ? 2 : 1)
-  for (int j = word0; j < words; j += step) {
-    const uint4 xv = ld128(x + j * 16);
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-      acc[r] = fmaf(ld_half(sc + r * NCW * (K / 16) + (j >> 2) * 2), dot8(ld32(w + r * NCW * (K / 2) + j * 4), xv), acc[r]);
-  }
+  for (int e = 0; e < 4; ++e) u[e] = *reinterpret_cast<const uint32_t*>(&v[e]);
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(x + i * 2), "r"(__byte_perm(u[0], u[2], 0x5410)), "r"(__byte_perm(u[0], u[2], 0x7632)),
+               "r"(__byte_perm(u[1], u[3], 0x5410)), "r"(__byte_perm(u[1], u[3], 0x7632)) : "memory");
 }
 
-// One tile (rows x K in shared memory) times x; row i's sum goes to res + 16 i as up to four parts.
-__device__ __forceinline__ void tile_matvec(uint32_t stage, int rows, int K, uint32_t x, uint32_t res, int warp, int lane) {
-  const uint32_t sc = stage + rows * (K / 2);
-  if (rows <= 8) {                             // several warps a row
-    const int shift = rows <= 4 ? 2 : 1, row = warp >> shift, part = warp & ((1 << shift) - 1);
-    if (row >= rows) return;
-    float acc[1];
-    rows_dot<1>(stage + row * (K / 2), sc + row * (K / 16), x, K, part * 32 + lane, 32 << shift, acc);
-    acc[0] = warp_sum(acc[0]);
-    if (lane == 0) { st32(res + row * 16 + part * 4, acc[0]); if (shift == 1) st32(res + row * 16 + part * 4 + 8, 0.0f); }
-    return;
-  }
-  int row = warp;
-  for (; row + NCW < rows; row += 2 * NCW) {
-    float acc[2];
-    rows_dot<2>(stage + row * (K / 2), sc + row * (K / 16), x, K, lane, 32, acc);
-    acc[0] = warp_sum(acc[0]);
-    acc[1] = warp_sum(acc[1]);
-    if (lane == 0) { st128(res + row * 16, acc[0], 0.0f, 0.0f, 0.0f); st128(res + (row + NCW) * 16, acc[1], 0.0f, 0.0f, 0.0f); }
-  }
-  if (row < rows) {
-    float acc[1];
-    rows_dot<1>(stage + row * (K / 2), sc + row * (K / 16), x, K, lane, 32, acc);
-    acc[0] = warp_sum(acc[0]);
-    if (lane == 0) st128(res + row * 16, acc[0], 0.0f, 0.0f, 0.0f);
-  }
+__device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+// Whether a wait that began with the first call has to end: another warp of the CTA has given up, or the limit has passed.
+// (Inline, as all of this kernel: around a call registers go to the stack, and with all of L1 given to shared memory that is a trip to L2.)
+__device__ __forceinline__ bool over(unsigned long long& t0, uint32_t flag_abort) {
+  const unsigned long long now = global_timer_ns();
+  if (t0 == 0) t0 = now;
+  return ld32(flag_abort) != 0u || now - t0 > wait_limit_ns();
+}
+// Bounded wait for a stage; gives up when another warp of the CTA has, too.
+__device__ __forceinline__ bool wait_stage(uint32_t bar, uint32_t parity, uint32_t flag_abort) {
+  unsigned long long t0 = 0;
+#pragma unroll 1
+  while (!try_wait(bar, parity))
+    if (over(t0, flag_abort)) return false;
+  return true;
 }
 
-__global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_constant__ Params p) {
+__device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// What a consumer needs to know of a part, in shared memory: one copy for the CTA, addresses inside a stage and of x per lane.
+struct PartInfo { int groups, second, pad[2]; uint4 lane[32]; uint2 x[32]; };
+static_assert(sizeof(PartInfo) == PART_INFO_BYTES, "PartInfo layout");
+__device__ __forceinline__ void describe(const Part& q, PartInfo& info, int lane, bool turn) {
+  const int g = lane >> 2, t4 = lane & 3, ra = min2(g, q.h1 - 1), rb = q.h1 + min2(g, max2(q.slots - q.h1, 1) - 1), sc = q.slots * q.groups * 16;
+  info.lane[lane] = make_uint4(ra * q.groups * 16 + t4 * 4, rb * q.groups * 16 + t4 * 4, sc + ra * q.groups * 2, sc + rb * q.groups * 2);
+  info.x[lane] = make_uint2((g % q.v) * (q.K / q.v) * 2 + t4 * 16, turn && q.groups % 8 == 0 ? g : 0);
+  if (lane == 0) { info.groups = q.groups; info.second = q.slots > q.h1; }
+}
+
+// The matvec of a part: the next n stages of the stream times x; a set of warps takes every step-th stage from `first`.  Its warps
+// take the groups of a stage in turn.  Rows lie one behind the other; with eight warps, where they are a multiple of 8 groups (128 bytes) long, each row g takes
+// another group of the eight, g further on, so that the eight rows that a quarter of the A operand takes sit in different banks.  Column g of the B
+// operand is x at the group that row g takes (and row g + 8), so the sums of both are in column g of the result.
+// What does not need x -- waiting for the stage, fetching up to U groups of weights -- is done before x is there (fetch).
+template <int SET>
+struct Matvec {
+  static constexpr int U = Threads<SET>::U;
+  int j, n, step;                              // the set's next stage, number of stages, distance
+  int i;                                       // its place in the ring
+  uint32_t phase;
+  int unit, units;                             // of the stage: this warp's next group, and how many it has
+  bool second;
+  uint4 at;                                    // addresses in a stage of the first group of both rows: weights, scales
+  uint32_t xt;                                 // offset of its x
+  // what has been fetched
+  uint32_t a[U], b[U];                         // words of both rows, their scales
+  uint32_t c[U];
+
+  __device__ __forceinline__ void begin(const Params& p, uint32_t info, int n_, int first, int step_, int s, uint32_t phase_) {
+    const int w = (threadIdx.x >> 5) & (SET - 1), lane = threadIdx.x & 31;
+    const uint2 q = ld64(info), x = ld64(info + 16 + 512 + lane * 8);
+    at = ld128(info + 16 + lane * 16);
+    units = (static_cast<int>(q.x) - w + SET - 1) / SET;
+    second = q.y != 0;
+    const uint32_t r = SET == 8 ? (w + x.y) & 7 : w;       // (w where the rows do not turn)
+    at.x += r * 16; at.y += r * 16; at.z += r * 2; at.w += r * 2;
+    xt = x.x + r * 64;
+    j = first; n = n_; step = step_; i = s + first; phase = phase_; unit = 0;
+#pragma unroll 1
+    while (i >= p.n_stages) { i -= p.n_stages; phase ^= 1u; }
+  }
+  // the next groups of stage j
+  __device__ __forceinline__ void fetch(const Params& p, uint32_t base, bool& dead, uint32_t flag_abort) {
+    if (unit == 0 && !dead) {
+      const bool ok = wait_stage(base + p.map.bars + i * 8, phase, flag_abort);
+      if (__any_sync(0xffffffffu, !ok)) { dead = true; st32(flag_abort, 1.0f); atomicExch(&g_device_status, 51); }
+    }
+    const uint32_t st = base + i * p.stage_bytes;
+    const uint32_t a0 = st + at.x + unit * (SET * 16), b0 = st + at.y + unit * (SET * 16), s0 = st + at.z + unit * (SET * 2), t0 = st + at.w + unit * (SET * 2);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      c[u] = 0u; b[u] = 0x88888888u; a[u] = 0x88888888u;           // nothing: zeros
+      if (unit + u < units) {
+        a[u] = ld32(a0 + u * (SET * 16));
+        c[u] = ld16(s0 + u * (SET * 2));
+        if (second) {
+          b[u] = ld32(b0 + u * (SET * 16));
+          c[u] |= static_cast<uint32_t>(ld16(t0 + u * (SET * 2))) << 16;
+        }
+      }
+    }
+  }
+  // all of it, the first groups fetched before; the sums of a stage go to sums + stage * STAGE_SUMS: [row][warp]
+  __device__ __forceinline__ void run(const Params& p, uint32_t base, uint32_t x, uint32_t sums, bool& dead, uint32_t flag_abort) {
+    const int w = (threadIdx.x >> 5) & (SET - 1), lane = threadIdx.x & 31, g = lane >> 2;
+    const bool odd = g & 1;
+    float sum0 = 0.0f, sum1 = 0.0f;
+#pragma unroll 1
+    while (j < n) {
+      const uint32_t x0 = x + xt + unit * (SET * 64);
+      float d[U][4];
+      uint4 xv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) xv[u] = ld128(x0 + (unit + u < units ? u * (SET * 64) : 0));
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        uint32_t va[4], vb[4];
+        unpack(a[u], va);
+        unpack(b[u], vb);
+        const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        mma_m16n8k16_f16(d[u], va[0], vb[0], va[1], vb[1], xv[u].x, xv[u].y, zero);
+        mma_m16n8k16_f16(d[u], va[2], vb[2], va[3], vb[3], xv[u].z, xv[u].w, d[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (unit + u < units) {                // (a group that does not exist is zeros times some x, which may be infinite)
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&c[u]));
+          sum0 = fmaf(f.x, odd ? d[u][1] : d[u][0], sum0);
+          sum1 = fmaf(f.y, odd ? d[u][3] : d[u][2], sum1);
+        }
+      }
+      unit += U;
+      if (unit >= units) {                     // the stage is done
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(base + p.map.bars + (MAX_STAGES + i) * 8) : "memory");
+        if ((lane & 3) == (g >> 1)) {
+          const uint32_t to = sums + j * STAGE_SUMS + g * ROW_SUMS + w * 4;
+          st32(to, sum0);
+          st32(to + 8 * ROW_SUMS, sum1);
+        }
+        sum0 = 0.0f; sum1 = 0.0f;
+        unit = 0; j += step; i += step;
+#pragma unroll 1
+        while (i >= p.n_stages) { i -= p.n_stages; phase ^= 1u; }
+      }
+      if (j < n) fetch(p, base, dead, flag_abort);
+    }
+  }
+};
+
+// Polls eight published words until all carry `tag`.
+struct Poll {
+  const uint32_t* src;
+  uint4 w[2];
+  __device__ __forceinline__ void start(const uint32_t* p) { src = p; w[0] = load_words(p); w[1] = load_words(p + 4); }
+  static __device__ __forceinline__ uint32_t differs(const uint4& w, uint32_t tag) { return (((w.x ^ tag) | (w.y ^ tag)) | ((w.z ^ tag) | (w.w ^ tag))) & 0xFFFFu; }
+  __device__ __forceinline__ void finish(uint32_t tag, bool& dead, uint32_t flag_abort, __half2 (&v)[4]) {
+    unsigned long long t0 = 0;
+#pragma unroll 1
+    for (uint32_t tries = 0; (differs(w[0], tag) | differs(w[1], tag)) != 0 && !dead; ++tries) {
+      if ((tries & 255u) == 255u && over(t0, flag_abort)) { dead = true; st32(flag_abort, 1.0f); atomicExch(&g_device_status, 52); }
+      w[0] = load_words(src);
+      w[1] = load_words(src + 4);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t lo = __byte_perm(w[h].x, w[h].y, 0x7632), hi = __byte_perm(w[h].z, w[h].w, 0x7632);
+      v[2 * h] = *reinterpret_cast<const __half2*>(&lo);
+      v[2 * h + 1] = *reinterpret_cast<const __half2*>(&hi);
+    }
+  }
+};
+
+template <int SET>
+__global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const __grid_constant__ Params p) {
+  constexpr int NCW = Threads<SET>::NCW, NCT = Threads<SET>::NCT, SET_T = Threads<SET>::SET_T;
   extern __shared__ __align__(128) uint8_t smem[];
   const Shape& sh = p.sh;
-  const Smem L = smem_map(sh, p.n_layers, p.ctas, p.stage_bytes, p.n_stages);
+  const Smem& L = p.map;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.bars);
   uint64_t* empty = full + MAX_STAGES;
-  volatile int* flag_abort = reinterpret_cast<volatile int*>(smem + L.flags);
+  const uint32_t flag_abort = smem_u32(smem) + L.flags;     // set when a wait ran out
   uint32_t* smem_epoch = reinterpret_cast<uint32_t*>(smem + L.flags + 4);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x, b = blockIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x, b = blockIdx.x;
   uint32_t* epoch = static_cast<uint32_t*>(p.d.state);
   unsigned int* finished = static_cast<unsigned int*>(p.d.state) + 1;
   unsigned long long* best_key = static_cast<unsigned long long*>(p.d.state) + 1;
 
   if (tid == 0) {
-    for (int i = 0; i < p.n_stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], NCW); }
-    *flag_abort = 0;
+#pragma unroll 1
+    for (int i = 0; i < p.n_stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], SET); }
+    st32(flag_abort, 0.0f);
     *smem_epoch = *reinterpret_cast<volatile uint32_t*>(epoch);
     Rows r;
     r.qkv0 = share(sh.qkv, b, p.ctas); r.qkv = share(sh.qkv, b + 1, p.ctas) - r.qkv0;
     r.hid0 = share(sh.hidden, b, p.ctas); r.hid = share(sh.hidden, b + 1, p.ctas) - r.hid0;
     r.int0 = share(sh.inter, b, p.ctas); r.inter = share(sh.inter, b + 1, p.ctas) - r.int0;
     r.voc0 = share(sh.vocab, b, p.ctas); r.voc = share(sh.vocab, b + 1, p.ctas) - r.voc0;
+    r.stages[PART_O] = stages_of(p.part[PART_O], r.hid); r.stages[PART_GATE] = stages_of(p.part[PART_GATE], r.inter);
+    r.stages[PART_QKV] = stages_of(p.part[PART_QKV], r.qkv); r.stages[PART_DOWN] = stages_of(p.part[PART_DOWN], r.hid);
     *reinterpret_cast<Rows*>(smem + L.rows) = r;
     fence_barrier_init();
   }
-  for (int i = tid; i < p.n_layers * static_cast<int>(sizeof(lcq_decode_layer) / 8); i += NTHREADS)
+#pragma unroll 1
+  for (int i = tid; i < p.n_layers * static_cast<int>(sizeof(lcq_decode_layer) / 8); i += Threads<SET>::ALL)
     reinterpret_cast<uint64_t*>(smem + L.table)[i] = static_cast<const uint64_t*>(p.d.layers)[i];
+  if (warp < N_PARTS) describe(p.part[warp], reinterpret_cast<PartInfo*>(smem + L.info)[warp], lane, SET == 8);
   __syncthreads();
-  const Rows& mine = *reinterpret_cast<const Rows*>(smem + L.rows);
-  const int step_h = tile_rows(p.stage_bytes, sh.hidden), step_q = tile_rows(p.stage_bytes, sh.q_dim), step_i = tile_rows(p.stage_bytes, sh.inter);
+  const volatile Rows& mine = *reinterpret_cast<const volatile Rows*>(smem + L.rows);      // (volatile: read when needed, registers are scarce)
 
   if (warp >= NCW) {
-    // ------------------------------------------------------------ producer: one thread, all phases in order
+    // ------------------------------------------------------------ producer: one thread, the whole stream in order.  (A copy takes it 60 clocks
+    // to issue, also where several lanes issue one each: with a copy per row that alone was 2000 a stage.)
     if (lane == 0) {
-      int s = 0, in_flight = 0;                // the next stage; stages before it whose copies may be on their way
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int ph = 0, part; ok && (part = first_part(ph, p.n_layers)) >= 0; ++ph) {
-        for (; part >= 0 && ok; part = next_part(part, ph, p.n_layers)) {
-          const Segment g = segment(p, reinterpret_cast<const lcq_decode_layer*>(smem + L.table), mine, ph, part);
-          const int step = part == PART_O ? step_q : part == PART_DOWN ? step_i : step_h;
-          for (int r = 0; r < g.rows; r += step) {
-            const int rows = g.rows - r < step ? g.rows - r : step;
-            // (the flag after the wait: consumers that gave up release stages whose copies have not landed)
-            if (!mbar_wait_bounded(&empty[s], phase ^ 1u) || *flag_abort) { *flag_abort = 1; atomicExch(&g_device_status, 50); ok = false; break; }
-            const uint32_t wb = static_cast<uint32_t>(rows) * (g.K / 2), sb = static_cast<uint32_t>(rows) * (g.K / 16);
-            const uint32_t dst = smem_u32(smem) + s * p.stage_bytes;
-            mbar_expect_tx(&full[s], wb + sb);
-            bulk_load(dst, g.w + static_cast<long long>(g.row0 + r) * (g.K / 2), wb, &full[s]);
-            bulk_load(dst + wb, g.s + static_cast<long long>(g.row0 + r) * (g.K / 16), sb, &full[s]);
-            if (++s == p.n_stages) { s = 0; phase ^= 1u; }
-            if (in_flight < p.n_stages) ++in_flight;
-          }
+    int s = 0, in_flight = 0;                  // the next stage; stages before it whose copies may be on their way
+    uint32_t phase = 0;
+    bool ok = true;
+#pragma unroll 1
+    for (Order o = {0, PART_O, false}; ok && o.part != N_PARTS; o.next(p.n_layers)) {
+      const lcq_decode_layer* l = reinterpret_cast<const lcq_decode_layer*>(smem + L.table) + (o.part == PART_HEAD ? 0 : o.layer);
+      const Part& q = p.part[o.part];
+      const bool paired = o.part == PART_GATE;
+      const uint8_t* w = static_cast<const uint8_t*>(o.part == PART_O ? l->o_w : paired ? l->gate_up_w : o.part == PART_QKV ? l->qkv_w : o.part == PART_DOWN ? l->down_w : p.d.head_w);
+      const uint8_t* sc = static_cast<const uint8_t*>(o.part == PART_O ? l->o_s : paired ? l->gate_up_s : o.part == PART_QKV ? l->qkv_s : o.part == PART_DOWN ? l->down_s : p.d.head_s);
+      const int n = paired ? mine.inter : o.part == PART_QKV ? mine.qkv : o.part == PART_HEAD ? mine.voc : mine.hid;
+      const int row0 = paired ? mine.int0 : o.part == PART_QKV ? mine.qkv0 : o.part == PART_HEAD ? mine.voc0 : mine.hid0;
+      const int row_w = q.K / 2, row_s = q.K / 16;
+#pragma unroll 1
+      for (int r = 0; r < n; r += q.per) {
+        const int rows = min2(n - r, q.per);
+        if (!wait_stage(smem_u32(&empty[s]), phase ^ 1u, flag_abort) || ld32(flag_abort) != 0u) {
+          st32(flag_abort, 1.0f);                     // (the flag after the wait: consumers that gave up release stages whose copies have not landed)
+          atomicExch(&g_device_status, 50);
+          ok = false;
+          break;
         }
+        mbar_expect_tx(&full[s], static_cast<uint32_t>(rows * (row_w + row_s)) << (paired ? 1 : 0));
+        const uint32_t dst = smem_u32(smem) + s * p.stage_bytes, dst_s = dst + q.slots * q.groups * 16;
+        bulk_load(dst, w + static_cast<long long>(row0 + r) * row_w, rows * row_w, &full[s]);
+        bulk_load(dst_s, sc + static_cast<long long>(row0 + r) * row_s, rows * row_s, &full[s]);
+        if (paired) {
+          bulk_load(dst + q.h1 * q.groups * 16, w + static_cast<long long>(sh.inter + row0 + r) * row_w, rows * row_w, &full[s]);
+          bulk_load(dst_s + q.h1 * q.groups * 2, sc + static_cast<long long>(sh.inter + row0 + r) * row_s, rows * row_s, &full[s]);
+        }
+        if (++s == p.n_stages) { s = 0; phase ^= 1u; }
+        if (in_flight < p.n_stages) ++in_flight;
       }
-      // Consumers that gave up wait for no more stages, so the copies into the last ones are waited for here: none may
-      // land after the CTA has left.  They read this GPU's memory and end by themselves, whatever the wait limit.
-      for (; in_flight > 0; --in_flight) {
-        if (--s < 0) { s = p.n_stages - 1; phase ^= 1u; }
-        mbar_wait_landed(&full[s], phase);
-      }
+    }
+    // Consumers that gave up wait for no more stages, so the copies into the last ones are waited for here: none may
+    // land after the CTA has left.  They read this GPU's memory and end by themselves, whatever the wait limit.
+#pragma unroll 1
+    for (; in_flight > 0; --in_flight) {
+      if (--s < 0) { s = p.n_stages - 1; phase ^= 1u; }
+      mbar_wait_landed(&full[s], phase);
+    }
     }
   } else {
     // ------------------------------------------------------------ consumers
+    // Both sets of warps multiply.  The first also puts together the activation (publishes it, waits for that of the others) and
+    // publishes the down projection; the second does the norms, and q|k|v and o while the activation travels.
     const uint32_t base = smem_u32(smem);
+    const int set = warp / SET, w = warp & (SET - 1), st = tid & (SET_T - 1);      // warp and thread of the set
     const uint32_t xn = base + L.xn, xq = base + L.xq, xm = base + L.xm;
-    __half* xn_p = reinterpret_cast<__half*>(smem + L.xn);
-    float* red = reinterpret_cast<float*>(smem + L.red);
+    const uint32_t sums_c = base + L.sums, sums_s = base + L.side;
     const uint32_t tag0 = *smem_epoch * static_cast<uint32_t>(2 * p.n_layers + 1) + 1u;
-    const int copy = (b % p.copies) * p.copy_words;
-    int s = 0;
+    const int words = 3 * sh.hidden + sh.inter, copy = (b % COPIES) * words;       // the copy that is read here; warp w writes copy w
+    int s = 0;                                 // the next stage of the stream
     uint32_t phase = 0;
     bool dead = false;
-
-    // the next `n` rows of the stream (K columns, `step` rows a tile) times x
-    const auto use_tiles = [&](int n, int K, int step, uint32_t x, int res0) {
-      for (int r = 0; r < n; r += step) {
-        const int rows = n - r < step ? n - r : step;
-        if (!dead && (*flag_abort || !mbar_wait_bounded(&full[s], phase))) { dead = true; *flag_abort = 1; atomicExch(&g_device_status, 51); }
-        dead = __any_sync(0xffffffffu, dead);
-        if (!dead) tile_matvec(base + s * p.stage_bytes, rows, K, x, base + L.res + (res0 + r) * 16, warp, lane);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[s]);
-        if (++s == p.n_stages) { s = 0; phase ^= 1u; }
-      }
+    const auto pass = [&](int n) {
+      s += n;
+#pragma unroll 1
+      while (s >= p.n_stages) { s -= p.n_stages; phase ^= 1u; }
     };
-    // four published values, once they carry `tag`
-    const auto take = [&](const uint32_t* src, uint32_t tag, __half (&v)[4]) {
-      uint4 w = load_words(src);
-      uint64_t t0 = 0;
-      for (int i = 0; !dead && !(((w.x ^ tag) & 0xFFFFu) == 0 && ((w.y ^ tag) & 0xFFFFu) == 0 && ((w.z ^ tag) & 0xFFFFu) == 0 && ((w.w ^ tag) & 0xFFFFu) == 0); ++i) {
-        if ((i & 1023) == 1023) {
-          const uint64_t now = global_timer_ns();
-          if (t0 == 0) t0 = now;
-          if (*flag_abort || now - t0 > wait_limit_ns()) { dead = true; *flag_abort = 1; atomicExch(&g_device_status, 52); break; }
-        }
-        w = load_words(src);
+    // the sum of row i of a slab (half: of its first or second half) whose sums begin at `sums`: v short rows of a partial sum per warp
+    const auto row_sum = [&](uint32_t sums, int i, int v) {
+      float t = 0.0f;
+#pragma unroll 1
+      for (uint32_t a = sums + i * v * ROW_SUMS; v > 0; --v, a += ROW_SUMS) {
+        t += sum_words<SET>(a);
       }
-      v[0] = __ushort_as_half(static_cast<unsigned short>(w.x >> 16)); v[1] = __ushort_as_half(static_cast<unsigned short>(w.y >> 16));
-      v[2] = __ushort_as_half(static_cast<unsigned short>(w.z >> 16)); v[3] = __ushort_as_half(static_cast<unsigned short>(w.w >> 16));
+      return t;
     };
-    // A thread's share of the hidden state and of the next norms' weights, 4 values of every 4 * NCT, lies in
-    // shared memory: in registers they cost the matvec loops theirs, and a spill goes to L2 here.
-    __half* hid = reinterpret_cast<__half*>(smem + L.hid);
-    const __half* next_norm = static_cast<const __half*>(p.d.norms);
-    int norms_left = 2 * p.n_layers + 1;
-    const auto fetch_norms = [&]() {           // a phase ahead: they may come from HBM
-      const int two = norms_left > 1 ? 2 * sh.hidden : norms_left * sh.hidden;
-      for (int i = 4 * tid; i < two; i += 4 * NCT)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(base + L.gam + 2 * i), "l"(next_norm + i) : "memory");
-      next_norm += two;
-      norms_left -= 2;
+    // row i of a part that is not gate|up: 16 / v rows a slab
+    const auto sum_of = [&](uint32_t sums, int i, int v) { return row_sum(sums + (i * v >> 4) * STAGE_SUMS, i & (16 / v - 1), v); };
+    // A thread's share of the hidden state and of the next norms' weights, 8 values of every 8 * SET_T, lies in shared memory.
+    const uint32_t hid = base + L.hid;
+    const auto fetch_norms = [&](int of) {           // a layer ahead: they may come from HBM.  A thread fetches what it will use.
+#pragma unroll 1
+      for (int j = 0; j < 2 && 2 * of + j <= 2 * p.n_layers; ++j)
+#pragma unroll 1
+        for (int i = 8 * st; i < sh.hidden; i += 8 * SET_T)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(base + L.gam + 2 * (j * sh.hidden + i)), "l"(static_cast<const __half*>(p.d.norms) + static_cast<long long>(2 * of + j) * sh.hidden + i) : "memory");
+    };
+    const auto squares = [&](const __half2 (&h)[4], float ss) {
+      float t[2] = {0.0f, 0.0f};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __half22float2(h[e]);
+        t[e & 1] = fmaf(f.x, f.x, t[e & 1]);
+        t[e & 1] = fmaf(f.y, f.y, t[e & 1]);
+      }
+      return ss + (t[0] + t[1]);
     };
     // hidden += the down projection; x = rms_norm(hidden); hidden += the o projection; x2 = rms_norm(hidden)
-    // (the first phase has no down projection before it, the last one no o)
+    // (the first layer has no down projection before it, the lm_head no o)
     const auto norms = [&](const uint32_t* down, const uint32_t* o, uint32_t tag) {
       float ss = 0.0f, ss2 = 0.0f;
-      for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT) {
-        __half h[4], v[4];
-        *reinterpret_cast<uint2*>(h) = *reinterpret_cast<const uint2*>(hid + i);
+#pragma unroll 1
+      for (int i = 8 * st; i < sh.hidden; i += 8 * SET_T) {
+        Poll pd, po;
+        if (o != nullptr) po.start(o + i);
+        if (down != nullptr) pd.start(down + i);
+        __half2 h[4], v[4];
+        *reinterpret_cast<uint4*>(h) = ld128(hid + 2 * i);
         if (down != nullptr) {
-          take(down + i, tag, v);
+          pd.finish(tag, dead, flag_abort, v);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) h[e] = __float2half_rn(__half2float(h[e]) + __half2float(v[e]));
+          for (int e = 0; e < 4; ++e) h[e] = __hadd2_rn(h[e], v[e]);       // (rounds as the float32 sum rounded to fp16 does)
         }
-        *reinterpret_cast<uint2*>(hid + i) = *reinterpret_cast<const uint2*>(h);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) ss = fmaf(__half2float(h[e]), __half2float(h[e]), ss);
+        st128(hid + 2 * i, *reinterpret_cast<const uint4*>(h));
+        ss = squares(h, ss);
         if (o != nullptr) {
-          take(o + i, tag, v);
+          po.finish(tag, dead, flag_abort, v);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) h[e] = __float2half_rn(__half2float(h[e]) + __half2float(v[e]));
-          *reinterpret_cast<uint2*>(hid + sh.hidden + i) = *reinterpret_cast<const uint2*>(h);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) ss2 = fmaf(__half2float(h[e]), __half2float(h[e]), ss2);
+          for (int e = 0; e < 4; ++e) h[e] = __hadd2_rn(h[e], v[e]);
+          st128(hid + 2 * (sh.hidden + i), *reinterpret_cast<const uint4*>(h));
+          ss2 = squares(h, ss2);
         }
       }
+      dead = __any_sync(0xffffffffu, dead);
       ss = warp_sum(ss);
       ss2 = warp_sum(ss2);
-      if (lane == 0) { red[warp] = ss; red[NCW + warp] = ss2; }
+      const uint32_t red = base + L.red;
+      if (lane == 0) { st32(red + w * 4, ss); st32(red + SET * 4 + w * 4, ss2); }
       asm volatile("cp.async.wait_all;" ::: "memory");
-      named_bar_sync(BAR_C, NCT);
-      float total[2];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        total[j] = 0.0f;
-#pragma unroll
-        for (int i = 0; i < NCW / 4; ++i) {
-          const float4 q = reinterpret_cast<const float4*>(red)[j * (NCW / 4) + i];
-          total[j] += (q.x + q.y) + (q.z + q.w);
-        }
-        total[j] = rsqrtf(total[j] / static_cast<float>(sh.hidden) + p.d.eps);
-      }
-      for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT) {
+      named_bar_sync(BAR_SET1, SET_T);
+      if (8 * (st & ~31) < sh.hidden) {
+        float total[2];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          __half g[4], h[4], o4[4];
-          *reinterpret_cast<uint2*>(g) = *reinterpret_cast<const uint2*>(smem + L.gam + 2 * (j * sh.hidden + i));
-          *reinterpret_cast<uint2*>(h) = *reinterpret_cast<const uint2*>(hid + j * sh.hidden + i);
+          total[j] = rsqrtf(fmaf(sum_words<SET>(red + j * SET * 4), p.inv_hidden, p.d.eps));
+        }
+#pragma unroll 1
+        for (int i = 8 * st; i < sh.hidden; i += 8 * SET_T) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) o4[e] = __float2half_rn(__half2float(h[e]) * total[j] * __half2float(g[e]));
-          *reinterpret_cast<uint2*>(xn_p + j * sh.hidden + i) = *reinterpret_cast<const uint2*>(o4);
-          if (j == 1 && o != nullptr) *reinterpret_cast<uint2*>(hid + i) = *reinterpret_cast<const uint2*>(h);
+          for (int j = 1; j >= 0; --j) {       // (gate|up wait for the second one)
+            __half2 h[4], n[4], y[4];
+            *reinterpret_cast<uint4*>(n) = ld128(base + L.gam + 2 * (j * sh.hidden + i));
+            *reinterpret_cast<uint4*>(h) = ld128(hid + 2 * (j * sh.hidden + i));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 hf = __half22float2(h[e]), nf = __half22float2(n[e]);
+              y[e] = __floats2half2_rn(hf.x * total[j] * nf.x, hf.y * total[j] * nf.y);
+            }
+            stage_x(xn + j * sh.hidden * 2, i, y);
+          }
+          if (o != nullptr) st128(hid + 2 * i, ld128(hid + 2 * (sh.hidden + i)));
         }
       }
-      named_bar_sync(BAR_C, NCT);
-      fetch_norms();
-    };
-    const auto row_sum = [&](int i) {
-      const uint4 v = ld128(base + L.res + i * 16);
-      return (__uint_as_float(v.x) + __uint_as_float(v.y)) + (__uint_as_float(v.z) + __uint_as_float(v.w));
     };
 
     // embedding; the prepared input of the o projections
-    fetch_norms();
-    {
+    if (set == 1) {
+      fetch_norms(0);
       const int id = *static_cast<const int*>(p.d.token);
       const bool known = id >= 0 && id < sh.vocab;
-      if (!known && b == 0 && tid == 0) atomicExch(&g_device_status, 40);
+      if (!known && b == 0 && st == 0) atomicExch(&g_device_status, 40);
       const __half* row = static_cast<const __half*>(p.d.table) + static_cast<long long>(known ? id : 0) * sh.hidden;
-      for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT)
-        *reinterpret_cast<uint2*>(hid + i) = known ? *reinterpret_cast<const uint2*>(row + i) : make_uint2(0u, 0u);
-      for (int i = 8 * tid; i < sh.q_dim; i += 8 * NCT)
-        *reinterpret_cast<uint4*>(smem + L.xq + 2 * i) = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.d.x_q) + i);
+#pragma unroll 1
+      for (int i = 8 * st; i < sh.hidden; i += 8 * SET_T)
+        st128(hid + 2 * i, known ? *reinterpret_cast<const uint4*>(row + i) : make_uint4(0u, 0u, 0u, 0u));
+    } else {
+#pragma unroll 1
+      for (int i = 8 * st; i < sh.q_dim; i += 8 * SET_T) {
+        __half2 v[4];
+        *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.d.x_q) + i);
+        stage_x(xq, i, v);
+      }
     }
+    named_bar_sync(BAR_ALL, NCT);
 
-    // One loop body for all phases: code that runs once a phase is fetched anew each time.
-    __half* out = static_cast<__half*>(p.d.outputs);     // this layer's q|k|v, o, gate|up, down
-    const int layer_out = sh.qkv + 2 * sh.hidden + 2 * sh.inter, last = 2 * p.n_layers + 1;
-    for (int ph = 0; ph <= last; ++ph) {
-      const uint32_t tag = (tag0 + ph) & 0xFFFFu, before = (tag - 1u) & 0xFFFFu;
-      const bool wide = (ph & 1) && ph != last;          // q|k|v, gate|up
-      if (ph & 1) {
-        norms(ph == 1 ? nullptr : p.d_buf + copy, ph == last ? nullptr : p.o_buf + copy, before);
-      } else if (ph != 0) {
-        for (int i = 4 * tid; i < sh.inter; i += 4 * NCT) {
-          __half v[4];
-          take(p.m_buf + copy + i, before, v);
-          *reinterpret_cast<uint2*>(smem + L.xm + 2 * i) = *reinterpret_cast<const uint2*>(v);
-        }
-        named_bar_sync(BAR_C, NCT);
-      } else {
-        named_bar_sync(BAR_C, NCT);
-      }
-      int sums = 0;
-      for (int part = first_part(ph, p.n_layers); part >= 0; part = next_part(part, ph, p.n_layers)) {
-        const int n = part == PART_QKV ? mine.qkv : part == PART_HEAD ? mine.voc : part <= PART_UP ? mine.inter : mine.hid;
-        use_tiles(n, part == PART_DOWN ? sh.inter : part == PART_O ? sh.q_dim : sh.hidden,
-                  part == PART_DOWN ? step_i : part == PART_O ? step_q : step_h,
-                  part == PART_DOWN ? xm : part == PART_O ? xq : part == PART_GATE || part == PART_UP ? xn + 2 * sh.hidden : xn, sums);
-        sums += n;
-      }
-      named_bar_sync(BAR_C, NCT);
-      if (ph == last) break;
-      // warp w writes copies w, w + NCW, ... of what is published; the first also what the caller sees
-      for (int c = warp; c < p.copies; c += NCW) {
-        if (wide) {
-          for (int i = lane; i < mine.inter; i += 32) {
-            const __half gate = __float2half_rn(row_sum(mine.qkv + i)), up = __float2half_rn(row_sum(mine.qkv + mine.inter + i));
-            const float x = __half2float(gate);
-            const __half v = __float2half_rn((x * (1.0f / (1.0f + expf(-x)))) * __half2float(up));
-            publish(p.m_buf + c * p.copy_words + mine.int0 + i, v, tag);
-            if (c == 0) {
-              __half* o = out + sh.qkv + sh.hidden + mine.int0 + i;
-              o[0] = gate;
-              o[sh.inter] = up;
-              if (ph == last - 2) static_cast<__half*>(p.d.mlp_out)[mine.int0 + i] = v;
+    // Three matvecs a layer for each set: gate|up together, then the first one takes its half of down, and o of the layer after next; the
+    // second one q|k|v and its half of down.  (Before the first layer: o of the first two layers.  At the end: the lm_head, in pieces.)
+    // One loop body for all of them: it is small enough to stay in the instruction cache next to the schedulers.
+    // tags: o of layer l 2 l, its activation 2 l + 1, its down projection 2 l + 2 (o has buffers of its own, the layers' in turn)
+    const int layer_out = sh.qkv + 2 * sh.hidden + 2 * sh.inter;
+    int layer = 0, ahead = 0;                  // o is that of layer + ahead
+    int part = set == 0 ? PART_O : PART_GATE, done = 0;  // rows of the lm_head that are done
+    unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem + L.red);     // the best logit of each warp
+    if (set == 1) pass(min2(p.n_layers, 2) * mine.stages[PART_O]);
+#pragma unroll 1
+    for (;;) {
+      const uint32_t tag = tag0 + 2u * layer;
+      __half* out = static_cast<__half*>(p.d.outputs) + static_cast<long long>(layer) * layer_out;     // the layer's q|k|v, o, gate|up, down
+      const bool joint = part == PART_GATE || part == PART_DOWN || part == PART_HEAD;
+      const int head_rows = min2(mine.voc - done, HEAD_SLABS * p.part[PART_HEAD].per);
+      const int n = part == PART_HEAD ? stages_of(p.part[PART_HEAD], head_rows) : mine.stages[part];
+      const uint32_t sums = part == PART_QKV ? sums_s : part == PART_O ? sums_s + mine.stages[PART_QKV] * STAGE_SUMS : sums_c;
+      const int v = p.part[part].v;
+      Matvec<SET> m;
+      m.begin(p, base + L.info + part * PART_INFO_BYTES, n, !joint ? 0 : part == PART_DOWN ? 1 - set : set, joint ? 2 : 1, s, phase);
+      if (m.j < n) m.fetch(p, base, dead, flag_abort);
+      pass(n);
+      if (set == 0) {
+        if (part == PART_DOWN) {               // the activation
+#pragma unroll 1
+          for (int i = 8 * st; i < sh.inter; i += 2 * 8 * SET_T) {
+            const int i2 = i + 8 * SET_T;      // two at a time
+            Poll q, q2;
+            __half2 y[4];
+            q.start(p.m_buf + copy + i);
+            if (i2 < sh.inter) q2.start(p.m_buf + copy + i2);
+            q.finish((tag + 1u) & 0xFFFFu, dead, flag_abort, y);
+            stage_x(xm, i, y);
+            if (i2 < sh.inter) {
+              q2.finish((tag + 1u) & 0xFFFFu, dead, flag_abort, y);
+              stage_x(xm, i2, y);
             }
           }
-        } else {
-          // down rows of this layer, then o rows of the next (phase 0: o rows only; the last layer: down only)
-          const int n_down = ph == 0 ? 0 : mine.hid;
-          for (int i = lane; i < sums; i += 32) {
-            const __half v = __float2half_rn(row_sum(i));
-            const bool down = i < n_down;
-            const int row = mine.hid0 + (down ? i : i - n_down);
-            publish((down ? p.d_buf : p.o_buf) + c * p.copy_words + row, v, tag);
-            if (c == 0) (down ? out + layer_out - sh.hidden : (ph == 0 ? out : out + layer_out) + sh.qkv)[row] = v;
+          dead = __any_sync(0xffffffffu, dead);
+        }
+      } else if (part == PART_GATE || (part == PART_HEAD && done == 0)) {
+        norms(layer == 0 ? nullptr : p.d_buf + copy, part == PART_HEAD ? nullptr : p.o_buf + (layer & 1) * sh.hidden + copy, tag & 0xFFFFu);
+      }
+      if (joint) named_bar_sync(BAR_ALL, NCT);
+      else if (set == 0) named_bar_sync(BAR_SET0, SET_T);          // (the sums of o before have been read)
+      m.run(p, base, part == PART_DOWN ? xm : part == PART_O ? xq : part == PART_GATE ? xn + 2 * sh.hidden : xn, sums, dead, flag_abort);
+
+      if (part == PART_GATE || part == PART_DOWN) {
+        if (set == 1) {
+          bar_arrive(BAR_SUMS, NCT);
+          if (part == PART_GATE) {
+            part = PART_QKV;
+          } else {
+            if (layer + 2 < p.n_layers) pass(mine.stages[PART_O]);
+            part = ++layer < p.n_layers ? PART_GATE : PART_HEAD;
+          }
+          continue;
+        }
+        named_bar_sync(BAR_SUMS, NCT);
+      }
+      if (part == PART_GATE) {
+        const int per = p.part[PART_GATE].per;
+#pragma unroll 1
+        for (int i = lane; i < mine.inter; i += 32) {
+          const int j = i * v >> 3;            // a slab is 8 / v rows of each (the last may be less)
+          const uint32_t slab = sums + j * STAGE_SUMS;
+          const int r = i - j * per;
+          const __half gate = __float2half_rn(row_sum(slab, r, v)), up = __float2half_rn(row_sum(slab + 8 * ROW_SUMS, r, v));
+          const float x = __half2float(gate);
+          const __half y = __float2half_rn((x * (1.0f / (1.0f + expf(-x)))) * __half2float(up));
+#pragma unroll
+          for (int c = 0; c < COPIES / SET; ++c) publish(p.m_buf + (w + c * SET) * words + mine.int0 + i, y, (tag + 1u) & 0xFFFFu);
+          if (w == 0) {                        // what the caller sees
+            __half* o = out + sh.qkv + sh.hidden + mine.int0 + i;
+            o[0] = gate;
+            o[sh.inter] = up;
+            if (layer + 1 == p.n_layers) static_cast<__half*>(p.d.mlp_out)[mine.int0 + i] = y;
           }
         }
+        pass(mine.stages[PART_QKV]);
+        part = PART_DOWN;
+      } else if (part == PART_DOWN || part == PART_O) {
+        const bool down = part == PART_DOWN;
+        if (!down) named_bar_sync(BAR_SET0, SET_T);
+        uint32_t* to = (down ? p.d_buf : p.o_buf + ((layer + ahead) & 1) * sh.hidden) + w * words + mine.hid0;
+        __half* o = out + (down ? layer_out - sh.hidden : ahead * layer_out + sh.qkv) + mine.hid0;
+        const uint32_t t = (tag + (down ? 2u : 2u * ahead)) & 0xFFFFu;
+#pragma unroll 1
+        for (int i = lane; i < mine.hid; i += 32) {
+          const __half y = __float2half_rn(sum_of(sums, i, v));
+#pragma unroll
+          for (int c = 0; c < COPIES / SET; ++c) publish(to + c * SET * words + i, y, t);
+          if (w == 0) o[i] = y;
+        }
+        if (down && layer + 2 < p.n_layers) {
+          part = PART_O;
+        } else if (!down && ahead == 0 && p.n_layers > 1) {
+          ahead = 1;                           // (once: o of the second layer)
+        } else {
+          if (down || ahead == 2) ++layer;
+          ahead = 2;
+          part = layer < p.n_layers ? PART_GATE : PART_HEAD;
+        }
+      } else if (part == PART_QKV) {
+        fetch_norms(layer + 1);
+        named_bar_sync(BAR_SET1, SET_T);
+#pragma unroll 1
+        for (int i = st; i < mine.qkv; i += SET_T) out[mine.qkv0 + i] = __float2half_rn(sum_of(sums, i, v));
+        part = PART_DOWN;
+      } else {
+        // the key of a logit orders as np.argmax does: by value, NaN above all, the lowest index among equals
+        named_bar_sync(BAR_ALL, NCT);
+        const int v0 = mine.voc0 + done;
+        unsigned long long key = 0;
+#pragma unroll 1
+        for (int i = tid; i < head_rows; i += NCT) {
+          const __half y = __float2half_rn(sum_of(sums, i, v));
+          static_cast<__half*>(p.d.logits)[v0 + i] = y;
+          const float f = __half2float(y) + 0.0f;        // -0 counts as 0
+          uint32_t u = __float_as_uint(f);
+          u = f != f ? 0xFFFFFFFFu : (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+          const unsigned long long k = (static_cast<unsigned long long>(u) << 32) | (0xFFFFFFFFu - static_cast<uint32_t>(v0 + i));
+          if (k > key) key = k;
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+          const unsigned long long k = __shfl_xor_sync(0xffffffffu, key, off);
+          if (k > key) key = k;
+        }
+        if (lane == 0 && (done == 0 || key > keys[warp])) keys[warp] = key;
+        done += head_rows;
+        if (done >= mine.voc) break;
+        named_bar_sync(BAR_ALL, NCT);          // the sums have been read
       }
-      if (wide)
-        for (int i = tid; i < mine.qkv; i += NCT) out[mine.qkv0 + i] = __float2half_rn(row_sum(i));
-      if (!(ph & 1) && ph != 0) out += layer_out;
     }
     if (b == 0) {
-      for (int i = 4 * tid; i < sh.hidden; i += 4 * NCT) {
-        *reinterpret_cast<uint2*>(static_cast<__half*>(p.d.hidden_out) + i) = *reinterpret_cast<const uint2*>(hid + i);
-        *reinterpret_cast<uint2*>(static_cast<__half*>(p.d.normed_out) + i) = *reinterpret_cast<const uint2*>(xn_p + i);
+#pragma unroll 1
+      for (int i = tid; i < sh.hidden; i += NCT) {
+        static_cast<__half*>(p.d.hidden_out)[i] = *reinterpret_cast<const __half*>(smem + L.hid + 2 * i);
+        static_cast<__half*>(p.d.normed_out)[i] = *reinterpret_cast<const __half*>(smem + L.xn + (i >> 3) * 16 + 4 * (i & 3) + ((i >> 2) & 1) * 2);
       }
     }
-    const int v0 = mine.voc0, n = mine.voc;
-    // the key of a logit orders as np.argmax does: by value, NaN above all, the lowest index among equals
-    unsigned long long key = 0;
-    for (int i = tid; i < n; i += NCT) {
-      const __half v = __float2half_rn(row_sum(i));
-      static_cast<__half*>(p.d.logits)[v0 + i] = v;
-      const float f = __half2float(v) + 0.0f;            // -0 counts as 0
-      uint32_t u = __float_as_uint(f);
-      u = f != f ? 0xFFFFFFFFu : (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-      const unsigned long long k = (static_cast<unsigned long long>(u) << 32) | (0xFFFFFFFFu - static_cast<uint32_t>(v0 + i));
-      if (k > key) key = k;
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const unsigned long long k = __shfl_xor_sync(0xffffffffu, key, off);
-      if (k > key) key = k;
-    }
-    unsigned long long* keys = reinterpret_cast<unsigned long long*>(red);
-    if (lane == 0) keys[warp] = key;
-    named_bar_sync(BAR_C, NCT);
+    named_bar_sync(BAR_ALL, NCT);
     if (tid == 0) {
+      unsigned long long key = keys[0];
+#pragma unroll 1
       for (int i = 1; i < NCW; ++i) if (keys[i] > key) key = keys[i];
       atomicMax(best_key, key);
       __threadfence();
@@ -505,27 +733,55 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_step_kernel(const __grid_c
 }
 
 // ---------------------------------------------------------------------------- host side
-struct Plan { int ctas, stage_bytes, n_stages, copies; size_t smem, state_bytes; };
+struct Plan { Params p; size_t smem, state_bytes; };
+
+// A weight of rows of K columns, of which a CTA has at most `rows`: cut into short rows where they would be long, or so few that they
+// left rows of the MMA empty.  (Copies of scales start on 16 bytes: a slab is whole units of 4 rows.)
+inline Part make_part(int K, int rows, bool paired) {
+  Part q;
+  q.K = K;
+  q.v = 1;
+  const int slab = paired ? 8 : 16;
+  while (q.v < (paired ? 2 : 4) && K % (64 * q.v) == 0 && (K / q.v > 2560 || rows * q.v * 2 <= slab)) q.v *= 2;
+  q.groups = K / q.v / 32;
+  q.h1 = min2(8, rows * q.v);
+  q.slots = paired ? 2 * q.h1 : min2(16, rows * q.v);
+  q.per = (paired ? q.h1 : q.slots) / q.v;
+  return q;
+}
+
+// Four warps a set, which leave each more registers and fewer of them in each other's way, or eight, which hide each other's latencies when a
+// stage is long.  us a step with four / eight: 30 layers of 576 / 1536 191 / 221, 12 of 256 / 768 88 / 98; 12 of 768 / 2048 106 / 98,
+// 8 of 1024 / 3072 90 / 86, 5 of 2048 / 8192 201 / 135.
+inline bool narrow(const Params& p) { return p.sh.hidden <= 640; }
 
 inline bool make_plan(const lcq_decode_stack& d, int sm_count, Plan& pl) {
   const int H = d.hidden, I = d.inter;
   if (d.n_layers < 1 || H < 64 || I < 64 || d.qkv < 4 || d.q_dim < 64 || d.vocab < 4 || d.n_layers > 256) return false;
   if (H % 64 || I % 64 || d.q_dim % 64 || d.qkv % 4 || d.vocab % 4 || H > 8192 || I > (1 << 20) || d.vocab > (1 << 24)) return false;
+  Params& p = pl.p;
+  memset(&p, 0, sizeof(p));
+  p.d = d;
+  p.sh = {H, I, d.qkv, d.q_dim, d.vocab};
+  p.n_layers = d.n_layers;
+  p.inv_hidden = 1.0f / static_cast<float>(H);
   int units = H / 4;                           // every CTA needs a unit of 4 rows in every phase
   if (I / 4 < units) units = I / 4;
   if (d.vocab / 4 < units) units = d.vocab / 4;
-  pl.ctas = sm_count < units ? sm_count : units;
-  // a stage holds at least 4 rows of the longest kind, and 24 KB of the others
-  const int longest = max2(max2(row_bytes(H), row_bytes(I)), row_bytes(d.q_dim)) * 4;
-  pl.stage_bytes = (max2(longest, 24 * 1024) + 127) & ~127;
-  const Shape sh = {H, I, d.qkv, d.q_dim, d.vocab};
-  const int rest = smem_map(sh, d.n_layers, pl.ctas, 0, 0).total;
-  pl.n_stages = (227 * 1024 - rest) / pl.stage_bytes;
-  if (pl.n_stages > MAX_STAGES) pl.n_stages = MAX_STAGES;
-  if (pl.n_stages < 2) return false;
-  pl.smem = static_cast<size_t>(smem_map(sh, d.n_layers, pl.ctas, pl.stage_bytes, pl.n_stages).total);
-  pl.copies = 8;                               // 30 layers of width 576: 1 copy 420 us, 2 363, 4 337, 8 332, 16 325 (an earlier build)
-  pl.state_bytes = STATE_BYTES + (static_cast<size_t>(2) * H + I) * 4 * pl.copies;
+  p.ctas = sm_count < units ? sm_count : units;
+  const int hid = max_share(H, p.ctas), qkv = max_share(d.qkv, p.ctas);
+  p.part[PART_O] = make_part(d.q_dim, hid, false);
+  p.part[PART_GATE] = make_part(H, max_share(I, p.ctas), true);
+  p.part[PART_QKV] = make_part(H, qkv, false);
+  p.part[PART_DOWN] = make_part(I, hid, false);
+  p.part[PART_HEAD] = make_part(H, max_share(d.vocab, p.ctas), false);
+  for (const Part& q : p.part) p.stage_bytes = max2(p.stage_bytes, (q.slots * q.groups * 18 + 127) & ~127);
+  p.n_stages = (227 * 1024 - smem_map(p).total) / p.stage_bytes;
+  if (p.n_stages > MAX_STAGES) p.n_stages = MAX_STAGES;
+  if (p.n_stages < 2) return false;
+  p.map = smem_map(p);
+  pl.smem = static_cast<size_t>(p.map.total);
+  pl.state_bytes = STATE_BYTES + (static_cast<size_t>(3) * H + I) * 4 * COPIES;
   return true;
 }
 
@@ -536,29 +792,23 @@ inline int launch(const lcq_decode_stack& d, int sm_count, cudaStream_t stream) 
   const void* pointers[] = {d.layers, d.head_w, d.head_s, d.logits, d.norms, d.outputs, d.token, d.table, d.x_q, d.hidden_out, d.normed_out, d.mlp_out, d.next_token, d.state};
   for (const void* q : pointers)
     if (!q || !aligned(q, q == d.token || q == d.next_token ? 4 : 16)) { set_error("decode_step: null or misaligned pointer"); return LCQ_ERR_BAD_ARG; }
-  Params p;
-  memset(&p, 0, sizeof(p));
-  p.d = d;
-  p.sh = {d.hidden, d.inter, d.qkv, d.q_dim, d.vocab};
-  p.n_layers = d.n_layers;
-  p.ctas = pl.ctas;
-  p.copies = pl.copies;
-  p.copy_words = 2 * d.hidden + d.inter;
-  p.stage_bytes = pl.stage_bytes; p.n_stages = pl.n_stages;
+  Params& p = pl.p;
   p.o_buf = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(d.state) + STATE_BYTES);
-  p.d_buf = p.o_buf + d.hidden;
+  p.d_buf = p.o_buf + 2 * d.hidden;
   p.m_buf = p.d_buf + d.hidden;
   static thread_local int configured_device = -1;
   int dev = 0;
   LCQ_CUDA_TRY(cudaGetDevice(&dev));
   if (configured_device != dev) {
-    LCQ_CUDA_TRY(cudaFuncSetAttribute(decode_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    LCQ_CUDA_TRY(cudaFuncSetAttribute(decode_step_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    LCQ_CUDA_TRY(cudaFuncSetAttribute(decode_step_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     configured_device = dev;
   }
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(p.ctas);
-  cfg.blockDim = dim3(NTHREADS);
+  const bool four = narrow(p);
+  cfg.blockDim = dim3(four ? Threads<4>::ALL : Threads<8>::ALL);
   cfg.dynamicSmemBytes = pl.smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -566,7 +816,7 @@ inline int launch(const lcq_decode_stack& d, int sm_count, cudaStream_t stream) 
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, decode_step_kernel, p));
+  LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, four ? decode_step_kernel<4> : decode_step_kernel<8>, p));
   return LCQ_OK;
 }
 

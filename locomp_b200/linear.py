@@ -69,7 +69,7 @@ def fuse_rows(parts: Sequence[Tuple[torch.Tensor, torch.Tensor]], group_size: in
 def _one_kernel_pays(layers: int, layer_weights: int, head_weights: int) -> bool:
     """Whether a step is faster as one kernel than as a chain of launches.  The kernel saves about 10 us a layer of launches and
     hand-overs; its matvecs stream weights more slowly than the decode kernel: about 1 us per 30 Mi weights of a
-    layer and per 15 Mi of the lm_head.  Kernel and chain in us: 30 layers of 576 / 1536 217 and 484; 8 of 2048 / 8192 186 and 248; 8 of 3072 / 8192
+    layer and per 15 Mi of the lm_head.  Kernel and chain in us: 30 layers of 576 / 1536 217 and 484; 8 of 3072 / 8192
     with 128,256 rows of lm_head 289 and 344; 8 of 2560 / 9728 with 151,936 315 and 355; wider ones with an earlier kernel: 5 of 4608 / 12288 299
     and 297; 4 of 6144 / 16384 342 and 296; 6 of 3584 / 18944 with 152,064 rows of lm_head 392 and 370."""
     return layers * (10.0 - layer_weights / 30e6) > head_weights / 15e6

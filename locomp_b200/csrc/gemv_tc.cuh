@@ -26,7 +26,8 @@
 // both 16-row slabs of its row group (shared-memory bandwidth, not issue rate, bounds the
 // M = 16 case), and the slices of a row group are added through shared memory when a row
 // block ends.  K is cut into n_kr ranges so that one range of x fits in shared memory; the
-// CTAs of a range split its tile sequence (row-block major) stream-K style.  A row block
+// CTAs of a range split its tile sequence (row-block major) stream-K style, at row blocks where that
+// leaves their shares nearly even, else anywhere.  A row block
 // whose tiles were produced by more than one CTA is combined through scratch: every
 // contributor writes its float32 partial, bumps a counter (one per row block and row
 // group), and the last one sums all partials in a fixed order, writes the output and resets
@@ -105,6 +106,7 @@ struct Params {
   int max_split;        // scratch slots per (row block, k-range)
   int x_tiles;          // k tiles of x a CTA keeps in shared memory (S, or ceil(S / cluster) in cluster mode)
   int cluster;          // CTAs per row block that reduce through distributed shared memory (1 = none)
+  int whole;            // a CTA's share is whole row blocks
 };
 
 // The share of one k-range's tile sequence owned by one CTA.  Tile counts are 32-bit: the plan
@@ -112,7 +114,8 @@ struct Params {
 struct Sched {
   int S_kr;             // tiles per row block in this k-range
   unsigned T;           // n_rb * S_kr
-  int G;                // CTAs on this k-range (<= T)
+  int G;                // CTAs on this k-range (<= T / unit)
+  unsigned unit;        // tiles that are not split: 1, or a row block's
 };
 
 __host__ __device__ inline Sched make_sched(const Params& p, int kr) {
@@ -120,12 +123,16 @@ __host__ __device__ inline Sched make_sched(const Params& p, int kr) {
   const int left = p.nst - kr * p.S;
   s.S_kr = left < p.S ? left : p.S;
   s.T = static_cast<unsigned>(p.n_rb) * static_cast<unsigned>(s.S_kr);
-  s.G = static_cast<unsigned>(p.ctas_per_kr) < s.T ? p.ctas_per_kr : static_cast<int>(s.T);
+  s.unit = p.whole ? static_cast<unsigned>(s.S_kr) : 1u;
+  const unsigned units = p.whole ? static_cast<unsigned>(p.n_rb) : s.T;
+  s.G = static_cast<unsigned>(p.ctas_per_kr) < units ? p.ctas_per_kr : static_cast<int>(units);
   return s;
 }
-__host__ __device__ inline unsigned tile_begin(const Sched& s, int j) { return (static_cast<unsigned>(j) * s.T) / static_cast<unsigned>(s.G); }
+__host__ __device__ inline unsigned tile_begin(const Sched& s, int j) {
+  return (static_cast<unsigned>(j) * (s.T / s.unit)) / static_cast<unsigned>(s.G) * s.unit;
+}
 __host__ __device__ inline int owner_of(const Sched& s, unsigned t) {
-  return static_cast<int>(((t + 1u) * static_cast<unsigned>(s.G) - 1u) / s.T);
+  return static_cast<int>(((t / s.unit + 1u) * static_cast<unsigned>(s.G) - 1u) / (s.T / s.unit));
 }
 // CTAs j0..j1 (inclusive) of this k-range contribute to row block rb.
 __host__ __device__ inline void cover(const Sched& s, int rb, int& j0, int& j1) {
@@ -374,7 +381,7 @@ template <int MT, int NC>
 __device__ __forceinline__ void flush_row_group(const Params& p, const float (&y)[2][MT][4], int rb, int rg, int g, int t4,
                                              int lane, int seen_lane0, const CtaInfo* info) {
   Sched sch;
-  sch.S_kr = info->S_kr; sch.T = info->T; sch.G = info->G;
+  sch.S_kr = info->S_kr; sch.T = info->T; sch.G = info->G; sch.unit = 1;       // (whole row blocks do not come here)
   const int kr = info->kr, j = info->j;
   // contributors: identical for every full-length k-range, the last range may differ
   int j0, j1, c_full, c_last;
@@ -1068,6 +1075,17 @@ inline Plan make_plan(int M, int N, int K, int sm_count) {
     int c = (p.S + lim - 1) / lim;
     long long want = static_cast<long long>(p.n_rb) * c;
     if (want < p.ctas_per_kr) p.ctas_per_kr = static_cast<int>(want);
+  }
+  // Whole row blocks where they leave no CTA with much more than its equal share: no scratch, no counters, and the tail of a
+  // row block that two CTAs share (a round trip to L2 under full load) costs as much as three to four tiles.  us a call, cut / whole,
+  // tiles of the busiest CTA: M = 1 512 -> 49152 8.1 / 5.9 (2.6, 4), 2048 -> 32000 13.4 / 9.3 (6.8, 8), 4096 -> 28672 17.7 / 16.0 (12.1, 16),
+  // 1536 -> 49152 13.1 / 12.4 (7.8, 12), 2048 -> 49152 14.9 / 15.7 (10.4, 16), 4096 -> 40000 21.4 / 26.0 (16.9, 32); M = 16 512 -> 49152
+  // 12.5 / 9.8 (5.2, 6), 2048 -> 49152 23.5 / 23.1 (20.8, 24), 2048 -> 20000 14.2 / 16.2 (8.5, 16).
+  if (!pl.cluster && p.n_kr == 1) {
+    const int ctas = p.ctas_per_kr < p.n_rb ? p.ctas_per_kr : p.n_rb;
+    const long long most = static_cast<long long>((p.n_rb + ctas - 1) / ctas) * p.S;
+    p.whole = 16 * most * p.ctas_per_kr <= 17 * T + 64LL * p.ctas_per_kr;
+    if (p.whole) p.ctas_per_kr = ctas;
   }
   // a row block of S tiles can straddle at most S / min_tiles_per_cta + 2 CTAs of a k-range;
   // the last (shorter) range has its own, smaller T -- bound with the worst of the two

@@ -337,6 +337,15 @@ int lcq_gemv_tc_plan_cluster(int M, int N, int K, int sm_count);
  */
 int lcq_gemm_tc_plan_check(int M, int N, int K, int sm_count, int* fields);
 
+/*
+ * The same check for the decode-step kernel (only the sizes of `stack` are read): every row in the stages of one CTA, every
+ * stage used once by the set of warps that waits for it, no wait that ends before its stage has landed, no stage or partial sum
+ * overwritten in use, no CTA that waits for itself, under several orders of events; copies and shared memory within bounds.  fields (may be NULL) receives
+ * {CTAs, stages in the ring, bytes of a stage, shared-memory bytes, warps that multiply, waits at which the stage's barrier alone would have let a warp on too
+ * early}.  LCQ_ERR_UNSUPPORTED: a shape that the kernel does not cover.
+ */
+int lcq_decode_step_plan_check(const lcq_decode_stack* stack, int sm_count, int* fields);
+
 #ifdef __cplusplus
 }
 #endif

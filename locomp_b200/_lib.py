@@ -68,6 +68,7 @@ SIGNATURES = {
     "lcq_gemv_tc_plan_check": (_c.c_int, [_c.c_int] * 4 + [_c.POINTER(_c.c_int)]),
     "lcq_gemv_tc_plan_cluster": (_c.c_int, [_c.c_int] * 4),
     "lcq_gemm_tc_plan_check": (_c.c_int, [_c.c_int] * 4 + [_c.POINTER(_c.c_int)]),
+    "lcq_decode_step_plan_check": (_c.c_int, [_c.POINTER(DecodeStackDesc), _c.c_int, _c.POINTER(_c.c_int)]),
 }
 
 

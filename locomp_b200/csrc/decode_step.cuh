@@ -26,6 +26,9 @@
 // in fp16 (exact) and whose B operand is x; the group's scale multiplies the float32 result.
 // No shuffles: the tensor core adds up a group, a lane the groups of its rows, shared memory the warps.
 //
+// A set waits for the stages that it uses itself and skips the other's, up to more than a round of the ring.  A barrier's parity tells only
+// neighbouring rounds apart, so before it a set waits for the producer's count of issued stages, which says which round a place of the ring is in.
+//
 // Every CTA has at least one unit of 4 rows in every phase on the chain.  So whoever has all results of a phase knows
 // that all CTAs have read what they needed for it, and a buffer that is rewritten a layer later has no reader left.  The
 // results of o take two buffers in turn: those of layer l + 2 are written after all activations of layer l have come in, which were
@@ -107,8 +110,8 @@ inline Smem smem_map(const Params& p) {
   m.info = m.red + 32 * 8;
   m.bars = m.info + N_PARTS * PART_INFO_BYTES;
   m.flags = m.bars + 2 * MAX_STAGES * 8;
-  m.rows = m.flags + 16;                       // Rows
-  m.table = m.rows + 48;                       // the layer records
+  m.rows = m.flags + 16;                       // (flags: a wait ran out; the epoch; stages issued) Rows
+  m.table = m.rows + 64;                       // the layer records
   m.total = m.table + p.n_layers * static_cast<int>(sizeof(lcq_decode_layer));
   return m;
 }
@@ -157,7 +160,64 @@ struct Order {
     } else part = N_PARTS;
   }
 };
-struct Rows { int qkv0, qkv, hid0, hid, int0, inter, voc0, voc, stages[4]; };   // this CTA's shares: first row, rows; stages of PART_O .. PART_DOWN
+// The way of a set of warps through the stream: of gate|up, down and the lm_head each set takes every other stage; o is the first
+// set's alone, q|k|v the second's.
+struct Walk {
+  int set, part, layer;
+  int ahead;            // o is that of layer + ahead: of the first two layers before them, later of the layer after next
+  int done;             // stages of the lm_head that are done: it is taken in pieces
+  __host__ __device__ inline explicit Walk(int set_) : set(set_), part(set_ == 0 ? PART_O : PART_GATE), layer(0), ahead(0), done(0) {}
+  __host__ __device__ inline bool joint() const { return part == PART_GATE || part == PART_DOWN || part == PART_HEAD; }
+  // The set's first of the n stages that are next, and the distance to the one after it.  (The set that has more to do besides takes the smaller half.)
+  __host__ __device__ inline int first() const { return !joint() ? 0 : part == PART_DOWN ? 1 - set : set; }
+  __host__ __device__ inline int step() const { return joint() ? 2 : 1; }
+  __host__ __device__ inline int count(const int* stages) const { return part == PART_HEAD ? min2(stages[PART_HEAD] - done, HEAD_SLABS) : stages[part]; }
+  // The other set's stages before the first of this set's own.
+  static __host__ __device__ inline int skipped_at_first(int set, int n_layers, const int* stages) { return set == 0 ? 0 : min2(n_layers, 2) * stages[PART_O]; }
+  // On to what is next; returns how many stages of the stream in between are the other set's.  (The end: N_PARTS.)
+  __host__ __device__ inline int next(int n_layers, const int* stages) {
+    int skipped = 0;
+    if (part == PART_GATE) {
+      part = set == 0 ? PART_DOWN : PART_QKV;
+      return set == 0 ? stages[PART_QKV] : 0;
+    }
+    if (part == PART_QKV) {
+      part = PART_DOWN;
+      return 0;
+    }
+    if (part == PART_HEAD) {
+      done += HEAD_SLABS;
+      if (done >= stages[PART_HEAD]) part = N_PARTS;
+      return 0;
+    }
+    if (part == PART_DOWN) {
+      if (layer + 2 < n_layers) {
+        if (set == 0) { part = PART_O; return 0; }
+        skipped = stages[PART_O];
+      }
+      ++layer;
+    } else {
+      if (ahead == 0 && n_layers > 1) { ahead = 1; return 0; }
+      if (ahead == 2) ++layer;
+      ahead = 2;
+    }
+    part = layer < n_layers ? PART_GATE : PART_HEAD;
+    return skipped;
+  }
+};
+
+// The shares of a CTA: first row, rows (gate|up: of each), stages.
+struct Rows { int row0[N_PARTS], rows[N_PARTS], stages[N_PARTS]; };
+__host__ __device__ inline Rows rows_of(const Params& p, int b) {
+  const int n[N_PARTS] = {p.sh.hidden, p.sh.inter, p.sh.qkv, p.sh.hidden, p.sh.vocab};
+  Rows r;
+  for (int i = 0; i < N_PARTS; ++i) {
+    r.row0[i] = share(n[i], b, p.ctas);
+    r.rows[i] = share(n[i], b + 1, p.ctas) - r.row0[i];
+    r.stages[i] = stages_of(p.part[i], r.rows[i]);
+  }
+  return r;
+}
 
 // Shared memory by 32-bit addresses: generic pointers would take two registers each and a slower load.
 __device__ __forceinline__ uint32_t ld32(uint32_t a) { uint32_t v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
@@ -175,9 +235,6 @@ __device__ __forceinline__ uint16_t ld16(uint32_t a) {
   uint16_t v;
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
   return v;
-}
-__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
 }
 // The sum of 4 or 8 floats.
 template <int N> __device__ __forceinline__ float sum_words(uint32_t a) {
@@ -217,13 +274,28 @@ __device__ __forceinline__ bool over(unsigned long long& t0, uint32_t flag_abort
   if (t0 == 0) t0 = now;
   return ld32(flag_abort) != 0u || now - t0 > wait_limit_ns();
 }
-// Bounded wait for a stage; gives up when another warp of the CTA has, too.
+// Bounded wait for a phase of a stage's barrier; gives up when another warp of the CTA has, too.  A parity tells only neighbouring phases apart:
+// who waits has to know that the phase before has completed.
 __device__ __forceinline__ bool wait_stage(uint32_t bar, uint32_t parity, uint32_t flag_abort) {
   unsigned long long t0 = 0;
 #pragma unroll 1
   while (!try_wait(bar, parity))
     if (over(t0, flag_abort)) return false;
   return true;
+}
+
+// Bounded wait until more than q stages of the stream have been issued.  A set does not see the other's stages, so this is how it knows which use of a place
+// of the ring it waits for: stage q is issued once stage q - n_stages has been consumed, thus has landed.
+__device__ __forceinline__ void count_issued(uint32_t a, int n) { asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(a), "r"(n) : "memory"); }
+__device__ __forceinline__ bool wait_issued(uint32_t a, int q, uint32_t flag_abort) {
+  unsigned long long t0 = 0;
+#pragma unroll 1
+  for (;;) {
+    int n;
+    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(n) : "r"(a) : "memory");
+    if (n > q) return true;
+    if (over(t0, flag_abort)) return false;
+  }
 }
 
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
@@ -246,7 +318,7 @@ __device__ __forceinline__ void describe(const Part& q, PartInfo& info, int lane
 template <int SET>
 struct Matvec {
   static constexpr int U = Threads<SET>::U;
-  int j, n, step;                              // the set's next stage, number of stages, distance
+  int q, end, step;                            // the set's next stage, counted over the whole stream; the end of its stages, their distance
   int i;                                       // its place in the ring
   uint32_t phase;
   int unit, units;                             // of the stage: this warp's next group, and how many it has
@@ -257,23 +329,23 @@ struct Matvec {
   uint32_t a[U], b[U];                         // words of both rows, their scales
   uint32_t c[U];
 
-  __device__ __forceinline__ void begin(const Params& p, uint32_t info, int n_, int first, int step_, int s, uint32_t phase_) {
+  __device__ __forceinline__ void begin(const Params& p, uint32_t info, int n, int first, int step_, int pos, int turn) {
     const int w = (threadIdx.x >> 5) & (SET - 1), lane = threadIdx.x & 31;
-    const uint2 q = ld64(info), x = ld64(info + 16 + 512 + lane * 8);
+    const uint2 head = ld64(info), x = ld64(info + 16 + 512 + lane * 8);
     at = ld128(info + 16 + lane * 16);
-    units = (static_cast<int>(q.x) - w + SET - 1) / SET;
-    second = q.y != 0;
+    units = (static_cast<int>(head.x) - w + SET - 1) / SET;
+    second = head.y != 0;
     const uint32_t r = SET == 8 ? (w + x.y) & 7 : w;       // (w where the rows do not turn)
     at.x += r * 16; at.y += r * 16; at.z += r * 2; at.w += r * 2;
     xt = x.x + r * 64;
-    j = first; n = n_; step = step_; i = s + first; phase = phase_; unit = 0;
+    q = pos + first; end = pos + n; step = step_; i = turn + first; phase = 0; unit = 0;
 #pragma unroll 1
     while (i >= p.n_stages) { i -= p.n_stages; phase ^= 1u; }
   }
-  // the next groups of stage j
+  // the next groups of stage q
   __device__ __forceinline__ void fetch(const Params& p, uint32_t base, bool& dead, uint32_t flag_abort) {
     if (unit == 0 && !dead) {
-      const bool ok = wait_stage(base + p.map.bars + i * 8, phase, flag_abort);
+      const bool ok = wait_issued(base + p.map.flags + 8, q, flag_abort) && wait_stage(base + p.map.bars + i * 8, phase, flag_abort);
       if (__any_sync(0xffffffffu, !ok)) { dead = true; st32(flag_abort, 1.0f); atomicExch(&g_device_status, 51); }
     }
     const uint32_t st = base + i * p.stage_bytes;
@@ -291,13 +363,13 @@ struct Matvec {
       }
     }
   }
-  // all of it, the first groups fetched before; the sums of a stage go to sums + stage * STAGE_SUMS: [row][warp]
+  // all of it, the first groups fetched before; the sums of stage q go to sums + q * STAGE_SUMS: [row][warp]
   __device__ __forceinline__ void run(const Params& p, uint32_t base, uint32_t x, uint32_t sums, bool& dead, uint32_t flag_abort) {
     const int w = (threadIdx.x >> 5) & (SET - 1), lane = threadIdx.x & 31, g = lane >> 2;
     const bool odd = g & 1;
     float sum0 = 0.0f, sum1 = 0.0f;
 #pragma unroll 1
-    while (j < n) {
+    while (q < end) {
       const uint32_t x0 = x + xt + unit * (SET * 64);
       float d[U][4];
       uint4 xv[U];
@@ -325,16 +397,16 @@ struct Matvec {
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(base + p.map.bars + (MAX_STAGES + i) * 8) : "memory");
         if ((lane & 3) == (g >> 1)) {
-          const uint32_t to = sums + j * STAGE_SUMS + g * ROW_SUMS + w * 4;
+          const uint32_t to = sums + static_cast<uint32_t>(q) * STAGE_SUMS + g * ROW_SUMS + w * 4;
           st32(to, sum0);
           st32(to + 8 * ROW_SUMS, sum1);
         }
         sum0 = 0.0f; sum1 = 0.0f;
-        unit = 0; j += step; i += step;
+        unit = 0; q += step; i += step;
 #pragma unroll 1
         while (i >= p.n_stages) { i -= p.n_stages; phase ^= 1u; }
       }
-      if (j < n) fetch(p, base, dead, flag_abort);
+      if (q < end) fetch(p, base, dead, flag_abort);
     }
   }
 };
@@ -381,15 +453,9 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
 #pragma unroll 1
     for (int i = 0; i < p.n_stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], SET); }
     st32(flag_abort, 0.0f);
+    count_issued(flag_abort + 8, 0);
     *smem_epoch = *reinterpret_cast<volatile uint32_t*>(epoch);
-    Rows r;
-    r.qkv0 = share(sh.qkv, b, p.ctas); r.qkv = share(sh.qkv, b + 1, p.ctas) - r.qkv0;
-    r.hid0 = share(sh.hidden, b, p.ctas); r.hid = share(sh.hidden, b + 1, p.ctas) - r.hid0;
-    r.int0 = share(sh.inter, b, p.ctas); r.inter = share(sh.inter, b + 1, p.ctas) - r.int0;
-    r.voc0 = share(sh.vocab, b, p.ctas); r.voc = share(sh.vocab, b + 1, p.ctas) - r.voc0;
-    r.stages[PART_O] = stages_of(p.part[PART_O], r.hid); r.stages[PART_GATE] = stages_of(p.part[PART_GATE], r.inter);
-    r.stages[PART_QKV] = stages_of(p.part[PART_QKV], r.qkv); r.stages[PART_DOWN] = stages_of(p.part[PART_DOWN], r.hid);
-    *reinterpret_cast<Rows*>(smem + L.rows) = r;
+    *reinterpret_cast<Rows*>(smem + L.rows) = rows_of(p, b);
     fence_barrier_init();
   }
 #pragma unroll 1
@@ -397,13 +463,13 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
     reinterpret_cast<uint64_t*>(smem + L.table)[i] = static_cast<const uint64_t*>(p.d.layers)[i];
   if (warp < N_PARTS) describe(p.part[warp], reinterpret_cast<PartInfo*>(smem + L.info)[warp], lane, SET == 8);
   __syncthreads();
-  const volatile Rows& mine = *reinterpret_cast<const volatile Rows*>(smem + L.rows);      // (volatile: read when needed, registers are scarce)
+  const Rows& mine = *reinterpret_cast<const Rows*>(smem + L.rows);
 
   if (warp >= NCW) {
     // ------------------------------------------------------------ producer: one thread, the whole stream in order.  (A copy takes it 60 clocks
     // to issue, also where several lanes issue one each: with a copy per row that alone was 2000 a stage.)
     if (lane == 0) {
-    int s = 0, in_flight = 0;                  // the next stage; stages before it whose copies may be on their way
+    int s = 0, issued = 0, in_flight = 0;      // the next stage; stages before it, and how many of them may be on their way
     uint32_t phase = 0;
     bool ok = true;
 #pragma unroll 1
@@ -413,8 +479,7 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
       const bool paired = o.part == PART_GATE;
       const uint8_t* w = static_cast<const uint8_t*>(o.part == PART_O ? l->o_w : paired ? l->gate_up_w : o.part == PART_QKV ? l->qkv_w : o.part == PART_DOWN ? l->down_w : p.d.head_w);
       const uint8_t* sc = static_cast<const uint8_t*>(o.part == PART_O ? l->o_s : paired ? l->gate_up_s : o.part == PART_QKV ? l->qkv_s : o.part == PART_DOWN ? l->down_s : p.d.head_s);
-      const int n = paired ? mine.inter : o.part == PART_QKV ? mine.qkv : o.part == PART_HEAD ? mine.voc : mine.hid;
-      const int row0 = paired ? mine.int0 : o.part == PART_QKV ? mine.qkv0 : o.part == PART_HEAD ? mine.voc0 : mine.hid0;
+      const int n = mine.rows[o.part], row0 = mine.row0[o.part];
       const int row_w = q.K / 2, row_s = q.K / 16;
 #pragma unroll 1
       for (int r = 0; r < n; r += q.per) {
@@ -426,6 +491,7 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
           break;
         }
         mbar_expect_tx(&full[s], static_cast<uint32_t>(rows * (row_w + row_s)) << (paired ? 1 : 0));
+        count_issued(flag_abort + 8, ++issued);
         const uint32_t dst = smem_u32(smem) + s * p.stage_bytes, dst_s = dst + q.slots * q.groups * 16;
         bulk_load(dst, w + static_cast<long long>(row0 + r) * row_w, rows * row_w, &full[s]);
         bulk_load(dst_s, sc + static_cast<long long>(row0 + r) * row_s, rows * row_s, &full[s]);
@@ -455,13 +521,13 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
     const uint32_t sums_c = base + L.sums, sums_s = base + L.side;
     const uint32_t tag0 = *smem_epoch * static_cast<uint32_t>(2 * p.n_layers + 1) + 1u;
     const int words = 3 * sh.hidden + sh.inter, copy = (b % COPIES) * words;       // the copy that is read here; warp w writes copy w
-    int s = 0;                                 // the next stage of the stream
-    uint32_t phase = 0;
+    int pos = 0, turn = 0;                     // stages of the stream that are behind, and these modulo two rounds of the ring
     bool dead = false;
     const auto pass = [&](int n) {
-      s += n;
+      pos += n;
+      turn += n;
 #pragma unroll 1
-      while (s >= p.n_stages) { s -= p.n_stages; phase ^= 1u; }
+      while (turn >= 2 * p.n_stages) turn -= 2 * p.n_stages;
     };
     // the sum of row i of a slab (half: of its first or second half) whose sums begin at `sums`: v short rows of a partial sum per warp
     const auto row_sum = [&](uint32_t sums, int i, int v) {
@@ -576,22 +642,21 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
     // One loop body for all of them: it is small enough to stay in the instruction cache next to the schedulers.
     // tags: o of layer l 2 l, its activation 2 l + 1, its down projection 2 l + 2 (o has buffers of its own, the layers' in turn)
     const int layer_out = sh.qkv + 2 * sh.hidden + 2 * sh.inter;
-    int layer = 0, ahead = 0;                  // o is that of layer + ahead
-    int part = set == 0 ? PART_O : PART_GATE, done = 0;  // rows of the lm_head that are done
+    Walk to(set);
     unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem + L.red);     // the best logit of each warp
-    if (set == 1) pass(min2(p.n_layers, 2) * mine.stages[PART_O]);
+    pass(Walk::skipped_at_first(set, p.n_layers, mine.stages));
 #pragma unroll 1
-    for (;;) {
+    while (to.part != N_PARTS) {
+      const int part = to.part, layer = to.layer;
       const uint32_t tag = tag0 + 2u * layer;
       __half* out = static_cast<__half*>(p.d.outputs) + static_cast<long long>(layer) * layer_out;     // the layer's q|k|v, o, gate|up, down
-      const bool joint = part == PART_GATE || part == PART_DOWN || part == PART_HEAD;
-      const int head_rows = min2(mine.voc - done, HEAD_SLABS * p.part[PART_HEAD].per);
-      const int n = part == PART_HEAD ? stages_of(p.part[PART_HEAD], head_rows) : mine.stages[part];
+      const int n = to.count(mine.stages);
       const uint32_t sums = part == PART_QKV ? sums_s : part == PART_O ? sums_s + mine.stages[PART_QKV] * STAGE_SUMS : sums_c;
       const int v = p.part[part].v;
       Matvec<SET> m;
-      m.begin(p, base + L.info + part * PART_INFO_BYTES, n, !joint ? 0 : part == PART_DOWN ? 1 - set : set, joint ? 2 : 1, s, phase);
-      if (m.j < n) m.fetch(p, base, dead, flag_abort);
+      m.begin(p, base + L.info + part * PART_INFO_BYTES, n, to.first(), to.step(), pos, turn);
+      if (m.q < m.end) m.fetch(p, base, dead, flag_abort);
+      const uint32_t sums_q = sums - static_cast<uint32_t>(pos) * STAGE_SUMS;
       pass(n);
       if (set == 0) {
         if (part == PART_DOWN) {               // the activation
@@ -611,22 +676,17 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
           }
           dead = __any_sync(0xffffffffu, dead);
         }
-      } else if (part == PART_GATE || (part == PART_HEAD && done == 0)) {
+      } else if (part == PART_GATE || (part == PART_HEAD && to.done == 0)) {
         norms(layer == 0 ? nullptr : p.d_buf + copy, part == PART_HEAD ? nullptr : p.o_buf + (layer & 1) * sh.hidden + copy, tag & 0xFFFFu);
       }
-      if (joint) named_bar_sync(BAR_ALL, NCT);
+      if (to.joint()) named_bar_sync(BAR_ALL, NCT);
       else if (set == 0) named_bar_sync(BAR_SET0, SET_T);          // (the sums of o before have been read)
-      m.run(p, base, part == PART_DOWN ? xm : part == PART_O ? xq : part == PART_GATE ? xn + 2 * sh.hidden : xn, sums, dead, flag_abort);
+      m.run(p, base, part == PART_DOWN ? xm : part == PART_O ? xq : part == PART_GATE ? xn + 2 * sh.hidden : xn, sums_q, dead, flag_abort);
 
       if (part == PART_GATE || part == PART_DOWN) {
         if (set == 1) {
           bar_arrive(BAR_SUMS, NCT);
-          if (part == PART_GATE) {
-            part = PART_QKV;
-          } else {
-            if (layer + 2 < p.n_layers) pass(mine.stages[PART_O]);
-            part = ++layer < p.n_layers ? PART_GATE : PART_HEAD;
-          }
+          pass(to.next(p.n_layers, mine.stages));
           continue;
         }
         named_bar_sync(BAR_SUMS, NCT);
@@ -634,7 +694,7 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
       if (part == PART_GATE) {
         const int per = p.part[PART_GATE].per;
 #pragma unroll 1
-        for (int i = lane; i < mine.inter; i += 32) {
+        for (int i = lane; i < mine.rows[PART_GATE]; i += 32) {
           const int j = i * v >> 3;            // a slab is 8 / v rows of each (the last may be less)
           const uint32_t slab = sums + j * STAGE_SUMS;
           const int r = i - j * per;
@@ -642,51 +702,39 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
           const float x = __half2float(gate);
           const __half y = __float2half_rn((x * (1.0f / (1.0f + expf(-x)))) * __half2float(up));
 #pragma unroll
-          for (int c = 0; c < COPIES / SET; ++c) publish(p.m_buf + (w + c * SET) * words + mine.int0 + i, y, (tag + 1u) & 0xFFFFu);
+          for (int c = 0; c < COPIES / SET; ++c) publish(p.m_buf + (w + c * SET) * words + mine.row0[PART_GATE] + i, y, (tag + 1u) & 0xFFFFu);
           if (w == 0) {                        // what the caller sees
-            __half* o = out + sh.qkv + sh.hidden + mine.int0 + i;
+            __half* o = out + sh.qkv + sh.hidden + mine.row0[PART_GATE] + i;
             o[0] = gate;
             o[sh.inter] = up;
-            if (layer + 1 == p.n_layers) static_cast<__half*>(p.d.mlp_out)[mine.int0 + i] = y;
+            if (layer + 1 == p.n_layers) static_cast<__half*>(p.d.mlp_out)[mine.row0[PART_GATE] + i] = y;
           }
         }
-        pass(mine.stages[PART_QKV]);
-        part = PART_DOWN;
       } else if (part == PART_DOWN || part == PART_O) {
         const bool down = part == PART_DOWN;
         if (!down) named_bar_sync(BAR_SET0, SET_T);
-        uint32_t* to = (down ? p.d_buf : p.o_buf + ((layer + ahead) & 1) * sh.hidden) + w * words + mine.hid0;
-        __half* o = out + (down ? layer_out - sh.hidden : ahead * layer_out + sh.qkv) + mine.hid0;
-        const uint32_t t = (tag + (down ? 2u : 2u * ahead)) & 0xFFFFu;
+        uint32_t* words_out = (down ? p.d_buf : p.o_buf + ((layer + to.ahead) & 1) * sh.hidden) + w * words + mine.row0[part];
+        __half* o = out + (down ? layer_out - sh.hidden : to.ahead * layer_out + sh.qkv) + mine.row0[part];
+        const uint32_t t = (tag + (down ? 2u : 2u * to.ahead)) & 0xFFFFu;
 #pragma unroll 1
-        for (int i = lane; i < mine.hid; i += 32) {
+        for (int i = lane; i < mine.rows[part]; i += 32) {
           const __half y = __float2half_rn(sum_of(sums, i, v));
 #pragma unroll
-          for (int c = 0; c < COPIES / SET; ++c) publish(to + c * SET * words + i, y, t);
+          for (int c = 0; c < COPIES / SET; ++c) publish(words_out + c * SET * words + i, y, t);
           if (w == 0) o[i] = y;
-        }
-        if (down && layer + 2 < p.n_layers) {
-          part = PART_O;
-        } else if (!down && ahead == 0 && p.n_layers > 1) {
-          ahead = 1;                           // (once: o of the second layer)
-        } else {
-          if (down || ahead == 2) ++layer;
-          ahead = 2;
-          part = layer < p.n_layers ? PART_GATE : PART_HEAD;
         }
       } else if (part == PART_QKV) {
         fetch_norms(layer + 1);
         named_bar_sync(BAR_SET1, SET_T);
 #pragma unroll 1
-        for (int i = st; i < mine.qkv; i += SET_T) out[mine.qkv0 + i] = __float2half_rn(sum_of(sums, i, v));
-        part = PART_DOWN;
+        for (int i = st; i < mine.rows[PART_QKV]; i += SET_T) out[mine.row0[PART_QKV] + i] = __float2half_rn(sum_of(sums, i, v));
       } else {
         // the key of a logit orders as np.argmax does: by value, NaN above all, the lowest index among equals
         named_bar_sync(BAR_ALL, NCT);
-        const int v0 = mine.voc0 + done;
+        const int r0 = to.done * p.part[PART_HEAD].per, v0 = mine.row0[PART_HEAD] + r0, rows = min2(mine.rows[PART_HEAD] - r0, HEAD_SLABS * p.part[PART_HEAD].per);
         unsigned long long key = 0;
 #pragma unroll 1
-        for (int i = tid; i < head_rows; i += NCT) {
+        for (int i = tid; i < rows; i += NCT) {
           const __half y = __float2half_rn(sum_of(sums, i, v));
           static_cast<__half*>(p.d.logits)[v0 + i] = y;
           const float f = __half2float(y) + 0.0f;        // -0 counts as 0
@@ -700,11 +748,10 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
           const unsigned long long k = __shfl_xor_sync(0xffffffffu, key, off);
           if (k > key) key = k;
         }
-        if (lane == 0 && (done == 0 || key > keys[warp])) keys[warp] = key;
-        done += head_rows;
-        if (done >= mine.voc) break;
-        named_bar_sync(BAR_ALL, NCT);          // the sums have been read
+        if (lane == 0 && (to.done == 0 || key > keys[warp])) keys[warp] = key;
+        if (r0 + rows < mine.rows[PART_HEAD]) named_bar_sync(BAR_ALL, NCT);          // the sums have been read
       }
+      pass(to.next(p.n_layers, mine.stages));
     }
     if (b == 0) {
 #pragma unroll 1

@@ -715,6 +715,193 @@ int lcq_decode_step(const lcq_decode_stack* stack, void* stream) {
   return step::launch(*stack, di.sm_count, static_cast<cudaStream_t>(stream));
 }
 
+// The schedule of one CTA of the step, replayed.  Actors: the producer, the copies, and of each set a warp that goes ahead and one
+// that lags (priority decides); a barrier, a stage and a poll let them on as on the device.
+namespace {
+struct StepReplay {
+  enum Op { WAIT, USE, POLL, SYNC, ARRIVE, PUBLISH, READ };
+  enum { ALL, SUMS, SET0, SET1, N_BARS };                  // named barriers
+  enum { CHAIN, QKV, O, N_SUMS };                          // partial sums in shared memory
+  struct Item { Op op; int a, b; };                        // stage; barrier; phase; sums, piece
+  const lcq::step::Params& p;
+  const lcq::step::Rows rows;
+  std::vector<int> stages;                                 // part of each stage of the stream
+  std::vector<Item> program[2];
+  int early = 0;                                           // waits that a parity alone would have let through too early
+  const char* fault = nullptr;
+
+  StepReplay(const lcq::step::Params& p_, int cta) : p(p_), rows(lcq::step::rows_of(p_, cta)) {
+    using namespace lcq::step;
+    for (Order o = {0, PART_O, false}; o.part != N_PARTS; o.next(p.n_layers))
+      for (int i = 0; i < rows.stages[o.part]; ++i) stages.push_back(o.part);
+    for (int set = 0; set < 2; ++set) write(set);
+  }
+  void write(int set) {                                    // what a warp of the set does, in order
+    using namespace lcq::step;
+    std::vector<Item>& v = program[set];
+    int pos = Walk::skipped_at_first(set, p.n_layers, rows.stages);
+    for (Walk to(set); to.part != N_PARTS;) {
+      const int part = to.part, n = to.count(rows.stages), sums = part == PART_QKV ? QKV : part == PART_O ? O : CHAIN;
+      int q = pos + to.first();
+      if (q < pos + n) v.push_back({WAIT, q, part});
+      if (set == 0 && part == PART_DOWN) v.push_back({POLL, 3 * to.layer, 0});
+      if (set == 1 && (part == PART_GATE || (part == PART_HEAD && to.done == 0))) {
+        if (to.layer > 0) v.push_back({POLL, 3 * to.layer - 2, 0});
+        if (part == PART_GATE) v.push_back({POLL, 3 * to.layer + 2, 0});
+        v.push_back({SYNC, SET1, 0});
+      }
+      if (to.joint()) v.push_back({SYNC, ALL, 0});
+      else if (set == 0) v.push_back({SYNC, SET0, 0});
+      for (; q < pos + n; q += to.step()) {
+        if (q != pos + to.first()) v.push_back({WAIT, q, part});
+        v.push_back({USE, q, sums * (1 << 28) + pos});
+      }
+      if (part == PART_GATE || part == PART_DOWN) v.push_back({set == 1 ? ARRIVE : SYNC, SUMS, 0});
+      else v.push_back({SYNC, part == PART_HEAD ? ALL : set == 0 ? SET0 : SET1, 0});
+      if (n > 0 && (set == 0 || !to.joint() || part == PART_HEAD)) v.push_back({READ, sums, pos});
+      if (set == 0 && part != PART_HEAD)
+        v.push_back({PUBLISH, part == PART_GATE ? 3 * to.layer : part == PART_DOWN ? 3 * to.layer + 1 : 3 * (to.layer + to.ahead) + 2, 0});
+      if (part == PART_HEAD && to.done + n < rows.stages[part]) v.push_back({SYNC, ALL, 0});
+      pos += n;
+      pos += to.next(p.n_layers, rows.stages);
+    }
+    if (pos != static_cast<int>(stages.size())) fault = "a set does not end with the stream";
+  }
+
+  // `order`: the actors by priority (0 producer, 1 copies, 2 + 2 * set + which); late: the copy issued last lands first
+  bool run(const int (&order)[6], bool late) {
+    const int ring = p.n_stages, total = static_cast<int>(stages.size());
+    std::vector<int> landed(ring, 0), released(ring, 0), arrivals(ring, 0), holds(ring, -1), used(total, 0), seen(4 * static_cast<size_t>(total), 0);
+    std::vector<int> published(3 * p.n_layers, 0), in_flight;
+    struct Barrier { unsigned here = 0; int round = 0; } bars[N_BARS];
+    const unsigned members[N_BARS] = {15u, 15u, 3u, 12u};
+    struct Warp { size_t at = 0; int round = -1; } warps[4];
+    struct Region { int piece = -1, readers = 0; } sums[N_SUMS];
+    int issued = 0;
+    const auto passes = [](int completed, int parity) { return (completed & 1) != parity; };      // mbarrier try_wait.parity
+    const auto warp_step = [&](int k) {
+      const std::vector<Item>& v = program[k / 2];
+      Warp& w = warps[k];
+      if (w.at == v.size()) return false;
+      const Item& it = v[w.at];
+      switch (it.op) {
+        case WAIT: {
+          const int slot = it.a % ring, use = it.a / ring;
+          const bool lets = passes(landed[slot], use & 1), there = landed[slot] == use + 1 && holds[slot] == it.a;
+          if (stages[it.a] != it.b) { fault = "a set's stage is of another part"; return false; }
+          if (lets && !there && !seen[4 * static_cast<size_t>(it.a) + k]++) ++early;
+          if (issued <= it.a || !lets) return false;
+          if (!there) { fault = "a wait ended before its stage had landed"; return false; }
+          break;
+        }
+        case USE: {
+          const int slot = it.a % ring, region = it.b >> 28, piece = it.b & ((1 << 28) - 1);
+          if (holds[slot] != it.a) { fault = "a stage was overwritten in use"; return false; }
+          if (sums[region].piece != piece) {
+            if (sums[region].readers != 0) { fault = "sums were overwritten before they were read"; return false; }
+            sums[region].piece = piece;
+            sums[region].readers = region == CHAIN && it.a >= total - rows.stages[lcq::step::PART_HEAD] ? 4 : 2;
+          }
+          ++used[it.a];
+          if (++arrivals[slot] == 2) { arrivals[slot] = 0; ++released[slot]; }
+          break;
+        }
+        case POLL: if (published[it.a] != 2) return false; break;
+        case SYNC: case ARRIVE: {
+          Barrier& b = bars[it.a];
+          if (w.round < 0) {                               // arrives
+            if (b.here >> k & 1u) { fault = "a warp is at a barrier twice"; return false; }
+            b.here |= 1u << k;
+            w.round = b.round;
+            if (b.here == members[it.a]) { b.here = 0; ++b.round; }
+          }
+          if (it.op == SYNC && b.round == w.round) return false;
+          w.round = -1;
+          break;
+        }
+        case PUBLISH: ++published[it.a]; break;
+        case READ:
+          if (sums[it.a].piece != it.b || sums[it.a].readers-- == 0) { fault = "sums were read that are not there"; return false; }
+          break;
+      }
+      ++w.at;
+      return true;
+    };
+    for (bool moved = true; moved && !fault;) {
+      moved = false;
+      for (int i = 0; i < 6 && !moved && !fault; ++i) {
+        if (order[i] == 0) {
+          const int slot = issued % ring, use = issued / ring;
+          if (issued == total || !passes(released[slot], (use & 1) ^ 1)) continue;
+          if (released[slot] != use || landed[slot] != use) { fault = "the producer overwrites a stage"; continue; }
+          holds[slot] = issued;
+          in_flight.push_back(issued++);
+          moved = true;
+        } else if (order[i] == 1) {
+          if (in_flight.empty()) continue;
+          const size_t at = late ? in_flight.size() - 1 : 0;
+          ++landed[in_flight[at] % ring];
+          in_flight.erase(in_flight.begin() + static_cast<long>(at));
+          moved = true;
+        } else {
+          moved = warp_step(order[i] - 2);
+        }
+      }
+    }
+    if (fault) return false;
+    for (int k = 0; k < 4; ++k) if (warps[k].at != program[k / 2].size()) { fault = "the CTA waits for itself"; return false; }
+    for (int n : used) if (n != 2) { fault = "a stage is not used once by one set"; return false; }
+    return true;
+  }
+};
+}  // namespace
+
+int lcq_decode_step_plan_check(const lcq_decode_stack* stack, int sm_count, int* fields) {
+  using namespace lcq::step;
+  Plan pl;
+  if (!stack || sm_count < 1 || !make_plan(*stack, sm_count, pl)) { set_error("plan check: shape not covered by the decode step kernel"); return LCQ_ERR_UNSUPPORTED; }
+  const Params& p = pl.p;
+  const Smem& m = p.map;
+  const int n_rows[N_PARTS] = {p.sh.hidden, p.sh.inter, p.sh.qkv, p.sh.hidden, p.sh.vocab};
+  if (m.total > 227 * 1024 || p.n_stages < 2 || p.n_stages > MAX_STAGES || p.stage_bytes % 128 != 0) { set_error("plan check: %d bytes of shared memory, ring of %d", m.total, p.n_stages); return LCQ_ERR_BAD_ARG; }
+  const int orders[][6] = {{2, 4, 0, 1, 3, 5}, {4, 2, 0, 1, 5, 3}, {0, 1, 2, 3, 4, 5}, {2, 3, 4, 5, 0, 1}, {4, 5, 2, 3, 0, 1}, {1, 4, 5, 0, 2, 3}, {0, 2, 4, 3, 5, 1}};
+  int early = 0, covered[N_PARTS] = {0, 0, 0, 0, 0};
+  std::vector<Rows> done;
+  for (int b = 0; b < p.ctas; ++b) {
+    StepReplay replay(p, b);
+    const Rows& r = replay.rows;
+    for (int i = 0; i < N_PARTS; ++i) {
+      const Part& q = p.part[i];
+      const bool paired = i == PART_GATE;
+      if (r.row0[i] != covered[i] || (r.rows[i] < 4 && i != PART_QKV)) { set_error("plan check: CTA %d, part %d: rows %d from %d", b, i, r.rows[i], r.row0[i]); return LCQ_ERR_BAD_ARG; }
+      covered[i] += r.rows[i];
+      // copies: whole multiples of 16 bytes between places on 16 bytes, inside a stage, no more short rows than an MMA has
+      const int half_w = q.h1 * q.groups * 16, scales = q.slots * q.groups * 16, half_s = q.h1 * q.groups * 2;
+      if (q.slots > 16 || q.h1 > 8 || q.per * q.v > (paired ? q.h1 : q.slots) || q.groups * 32 * q.v != q.K || scales + q.slots * q.groups * 2 > p.stage_bytes || (paired && (half_w % 16 || half_s % 16))) { set_error("plan check: part %d does not fit a stage", i); return LCQ_ERR_BAD_ARG; }
+      for (int row = 0; row < r.rows[i]; row += q.per) {
+        const long long from = r.row0[i] + row, n = min2(r.rows[i] - row, q.per), K = q.K, other = paired ? p.sh.inter : 0;
+        if (from * (K / 2) % 16 || from * (K / 16) % 16 || n * (K / 2) % 16 || n * (K / 16) % 16 || other * (K / 16) % 16 || scales % 16) { set_error("plan check: part %d, row %lld: a copy off 16 bytes", i, from); return LCQ_ERR_BAD_ARG; }
+      }
+    }
+    // partial sums of the largest pieces
+    const int head = min2(r.stages[PART_HEAD], HEAD_SLABS);
+    if (m.sums + max2(max2(r.stages[PART_GATE], r.stages[PART_DOWN]), head) * STAGE_SUMS > m.side || m.side + (r.stages[PART_QKV] + r.stages[PART_O]) * STAGE_SUMS > m.red) { set_error("plan check: CTA %d: partial sums out of bounds", b); return LCQ_ERR_BAD_ARG; }
+    bool known = false;                                    // (a CTA whose stages another has, too)
+    for (const Rows& o : done) known = known || memcmp(o.stages, r.stages, sizeof(r.stages)) == 0;
+    if (known) continue;
+    done.push_back(r);
+    for (const int (&order)[6] : orders)
+      for (int late = 0; late < 2; ++late) {
+        if (!replay.fault) replay.run(order, late != 0);
+        if (replay.fault) { set_error("plan check: CTA %d: %s", b, replay.fault); return LCQ_ERR_BAD_ARG; }
+      }
+    early += replay.early;
+  }
+  for (int i = 0; i < N_PARTS; ++i) if (covered[i] != n_rows[i]) { set_error("plan check: part %d has %d rows of %d", i, covered[i], n_rows[i]); return LCQ_ERR_BAD_ARG; }
+  if (fields) { fields[0] = p.ctas; fields[1] = p.n_stages; fields[2] = p.stage_bytes; fields[3] = m.total; fields[4] = narrow(p) ? 8 : 16; fields[5] = early; }
+  return LCQ_OK;
+}
+
 // ---------------------------------------------------------------- quantisers
 static int quantize_entry(int wbits, const void* w, void* q, void* scales, int64_t N, int64_t K, int G, int w_dtype,
                           int style, void* stream) {

@@ -1,11 +1,14 @@
 """The one-kernel decode step against the chain of separate kernels it stands for (same arithmetic, other order
 of the float32 sums): per result a relative 2-norm error of 1e-2 -- fp16 rounding (2^-11) of each stored
 value, compounded over at most four layers."""
+import ctypes
+import random
+
 import pytest
 import torch
 
 import locomp_b200 as L
-from locomp_b200 import _lib
+from locomp_b200 import _lib, linear
 from locomp_b200.linear import _one_kernel_pays
 
 # fewer rows than SMs in some phase, hidden beyond one pass of the threads, rows that fill no tile, many tiles
@@ -45,6 +48,44 @@ def test_edges_of_the_schedule(shape):
     test_matches_the_chain_of_kernels(shape)
 
 
+# Rings that are short against what a set of warps leaves to the other one (o of two layers, q|k|v): the widths of 7B- and 8B-class models
+# and those between, with their own query and key widths.
+WIDE = [dict(layers=3, hidden=4096, inter=11008, q_heads=64, kv_heads=64, vocab=2000), dict(layers=3, hidden=4096, inter=14336, q_heads=64, kv_heads=16, vocab=4100),
+        dict(layers=3, hidden=4096, inter=12288, q_heads=64, kv_heads=16, vocab=2000), dict(layers=3, hidden=3584, inter=18944, q_heads=56, kv_heads=8, vocab=2000),
+        dict(layers=3, hidden=3200, inter=8640, q_heads=50, kv_heads=50, vocab=2000), dict(layers=2, hidden=3072, inter=8192, q_heads=48, kv_heads=16, vocab=128256),
+        dict(layers=2, hidden=2560, inter=9728, q_heads=64, kv_heads=16, vocab=151936), dict(layers=3, hidden=5120, inter=5120, q_heads=40, kv_heads=8, vocab=2000)]
+
+
+def _plan_check(layers, hidden, inter, q_heads, kv_heads, vocab, sms=148):
+    """Replays the schedule on the CPU: the status, and {CTAs, stages in the ring, their bytes, shared memory, warps, early waits}."""
+    desc = _lib.DecodeStackDesc(n_layers=layers, hidden=hidden, inter=inter, q_dim=64 * q_heads, qkv=64 * (q_heads + 2 * kv_heads), vocab=vocab)
+    fields = (ctypes.c_int * 6)()
+    return _lib.lib().lcq_decode_step_plan_check(ctypes.byref(desc), sms, fields), list(fields)
+
+
+@pytest.mark.parametrize("shape", SHAPES + EDGES + WIDE)
+def test_schedule_replayed(shape):
+    """On the device a set waits for its stage by the issue count and by the stage's barrier.  The barrier alone, one parity, would have let it on
+    before the stage had landed wherever the other set's stages fill the ring in between: every one of the wide shapes."""
+    for sms in (148, 132, 16, 3):
+        rc, fields = _plan_check(**shape, sms=sms)
+        assert rc == 0 or rc == _lib.ERR_UNSUPPORTED and sms < 132, (sms, _lib.lib().lcq_last_error())
+    rc, fields = _plan_check(**shape)
+    assert rc == 0 and (shape not in WIDE or fields[5] > 0), fields
+
+
+def test_schedules_of_many_shapes():
+    rng = random.Random(1)
+    covered = 0
+    for _ in range(400):
+        hidden, layers = 64 * round(2 ** rng.uniform(0, 6.6)), rng.choice((1, 2, 3, 5, 32))
+        q = max(1, rng.choice((hidden // 64, hidden // 32, hidden // 128)))
+        rc, fields = _plan_check(layers, hidden, 64 * round(2 ** rng.uniform(0, 8.2)), q, max(1, q // rng.choice((1, 2, 4, 8))), 4 * rng.randint(1, 40000))
+        assert rc in (0, _lib.ERR_UNSUPPORTED), (hidden, layers, q, _lib.lib().lcq_last_error())
+        covered += rc == 0
+    assert covered > 200
+
+
 def _results(st):
     return [t.clone() for t in (st.logits, st.hidden, st.normed, st.mlp, st.outputs)]
 
@@ -72,6 +113,13 @@ def test_matches_the_chain_of_kernels(shape):
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(_results(st), got))
     assert _lib.lib().lcq_check_device_status(None) == 0, _lib.lib().lcq_last_error()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", WIDE)
+def test_short_rings(shape, monkeypatch):
+    monkeypatch.setattr(linear, "_one_kernel_pays", lambda *sizes: True)         # whichever form is faster
+    test_matches_the_chain_of_kernels(shape)
 
 
 @pytest.mark.gpu

@@ -52,11 +52,11 @@ template <int SET> struct Threads {
 constexpr int MAX_STAGES = 32;
 enum { BAR_ALL = 1, BAR_SUMS, BAR_SET0, BAR_SET1 };   // named barriers: all consumers; a phase's sums are there; those of a set
 constexpr int STATE_BYTES = 64;                // epoch, argmax counter, argmax key
-constexpr int HEAD_SLABS = 32;                 // slabs of the lm_head whose sums are kept at a time
+constexpr int HEAD_SLABS = 32;                 // slabs of the lm_head whose sums are kept at a time (of the other parts: all of a CTA's, where they fit)
 constexpr int COPIES = 8;                      // of the published words: a CTA polls copy b % 8.  (30 layers of width 576: 1 copy 420 us, 2 363, 4 337, 8 332, 16 325 in an early build)
 constexpr int ROW_SUMS = 48;                   // bytes of a row's partial sums of a stage, one per warp of a set (eight at most; rows sit in different banks)
 constexpr int STAGE_SUMS = 16 * ROW_SUMS;
-constexpr int PART_INFO_BYTES = 16 + 32 * 16 + 32 * 8;
+constexpr int PART_INFO_BYTES = 16 + 8 * 16 + 8 * 4;
 
 struct Shape { int hidden, inter, qkv, q_dim, vocab; };
 enum { PART_O, PART_GATE, PART_QKV, PART_DOWN, PART_HEAD, N_PARTS };
@@ -64,10 +64,12 @@ enum { PART_O, PART_GATE, PART_QKV, PART_DOWN, PART_HEAD, N_PARTS };
 // those, the rows of an MMA's A operand, as they lie in memory: one copy, and one of their scales.  gate|up: up to 8 rows of gate, then the same
 // ones of up, so that both sums of a row end up in the same lane.
 struct Part {
-  int K, v;
+  int K, v, lg_v;       // lg: logarithms
   int groups;           // of 32 columns of a (short) row; 16 bytes each, so that a row is `groups` times 16 bytes
   int h1, slots;        // short rows of the first half of a slab (at most 8), of both
+  int lg;               // short rows of a slab (gate|up: of a half) of a CTA that has more than one
   int per;              // rows that a slab advances by (gate|up: of each)
+  int piece;            // slabs whose sums are kept at a time
 };
 
 // Offsets in shared memory.
@@ -103,10 +105,9 @@ inline Smem smem_map(const Params& p) {
   m.hid = m.xm + s.inter * 2;
   m.gam = m.hid + 2 * s.hidden * 2;            // before and after o
   m.sums = m.gam + 2 * s.hidden * 2;           // partial sums of the phases on the chain; of q|k|v, then of o
-  const int head = min2(max_share(s.vocab, p.ctas), HEAD_SLABS * p.part[PART_HEAD].per);
-  m.side = m.sums + max2(max2(stages_of(p.part[PART_GATE], max_share(s.inter, p.ctas)), stages_of(p.part[PART_DOWN], max_share(s.hidden, p.ctas))),
-                         stages_of(p.part[PART_HEAD], head)) * STAGE_SUMS;
-  m.red = m.side + (stages_of(p.part[PART_QKV], max_share(s.qkv, p.ctas)) + stages_of(p.part[PART_O], max_share(s.hidden, p.ctas))) * STAGE_SUMS;
+  const auto slabs = [&](int part, int n) { return min2(stages_of(p.part[part], max_share(n, p.ctas)), p.part[part].piece); };
+  m.side = m.sums + max2(max2(slabs(PART_GATE, s.inter), slabs(PART_DOWN, s.hidden)), slabs(PART_HEAD, s.vocab)) * STAGE_SUMS;
+  m.red = m.side + (slabs(PART_QKV, s.qkv) + slabs(PART_O, s.hidden)) * STAGE_SUMS;
   m.info = m.red + 32 * 8;
   m.bars = m.info + N_PARTS * PART_INFO_BYTES;
   m.flags = m.bars + 2 * MAX_STAGES * 8;
@@ -165,18 +166,21 @@ struct Order {
 struct Walk {
   int set, part, layer;
   int ahead;            // o is that of layer + ahead: of the first two layers before them, later of the layer after next
-  int done;             // stages of the lm_head that are done: it is taken in pieces
+  int done;             // stages of the part that are done: it is taken in pieces
   __host__ __device__ inline explicit Walk(int set_) : set(set_), part(set_ == 0 ? PART_O : PART_GATE), layer(0), ahead(0), done(0) {}
   __host__ __device__ inline bool joint() const { return part == PART_GATE || part == PART_DOWN || part == PART_HEAD; }
   // The set's first of the n stages that are next, and the distance to the one after it.  (The set that has more to do besides takes the smaller half.)
   __host__ __device__ inline int first() const { return !joint() ? 0 : part == PART_DOWN ? 1 - set : set; }
   __host__ __device__ inline int step() const { return joint() ? 2 : 1; }
-  __host__ __device__ inline int count(const int* stages) const { return part == PART_HEAD ? min2(stages[PART_HEAD] - done, HEAD_SLABS) : stages[part]; }
+  __host__ __device__ inline int count(const int* stages, const Part* parts) const { return min2(stages[part] - done, parts[part].piece); }
   // The other set's stages before the first of this set's own.
   static __host__ __device__ inline int skipped_at_first(int set, int n_layers, const int* stages) { return set == 0 ? 0 : min2(n_layers, 2) * stages[PART_O]; }
   // On to what is next; returns how many stages of the stream in between are the other set's.  (The end: N_PARTS.)
-  __host__ __device__ inline int next(int n_layers, const int* stages) {
+  __host__ __device__ inline int next(int n_layers, const int* stages, const Part* parts) {
     int skipped = 0;
+    done += parts[part].piece;
+    if (done < stages[part]) return 0;
+    done = 0;
     if (part == PART_GATE) {
       part = set == 0 ? PART_DOWN : PART_QKV;
       return set == 0 ? stages[PART_QKV] : 0;
@@ -186,8 +190,7 @@ struct Walk {
       return 0;
     }
     if (part == PART_HEAD) {
-      done += HEAD_SLABS;
-      if (done >= stages[PART_HEAD]) part = N_PARTS;
+      part = N_PARTS;
       return 0;
     }
     if (part == PART_DOWN) {
@@ -300,13 +303,15 @@ __device__ __forceinline__ bool wait_issued(uint32_t a, int q, uint32_t flag_abo
 
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
-// What a consumer needs to know of a part, in shared memory: one copy for the CTA, addresses inside a stage and of x per lane.
-struct PartInfo { int groups, second, pad[2]; uint4 lane[32]; uint2 x[32]; };
+// What a consumer needs to know of a part, in shared memory: one copy for the CTA, addresses inside a stage and of x per row of the MMA.
+struct PartInfo { int groups, second, pad[2]; uint4 row[8]; uint32_t x[8]; };
 static_assert(sizeof(PartInfo) == PART_INFO_BYTES, "PartInfo layout");
 __device__ __forceinline__ void describe(const Part& q, PartInfo& info, int lane, bool turn) {
-  const int g = lane >> 2, t4 = lane & 3, ra = min2(g, q.h1 - 1), rb = q.h1 + min2(g, max2(q.slots - q.h1, 1) - 1), sc = q.slots * q.groups * 16;
-  info.lane[lane] = make_uint4(ra * q.groups * 16 + t4 * 4, rb * q.groups * 16 + t4 * 4, sc + ra * q.groups * 2, sc + rb * q.groups * 2);
-  info.x[lane] = make_uint2((g % q.v) * (q.K / q.v) * 2 + t4 * 16, turn && q.groups % 8 == 0 ? g : 0);
+  if (lane < 8) {
+    const int g = lane, ra = min2(g, q.h1 - 1), rb = q.h1 + min2(g, max2(q.slots - q.h1, 1) - 1), sc = q.slots * q.groups * 16;
+    info.row[g] = make_uint4(ra * q.groups * 16, rb * q.groups * 16, sc + ra * q.groups * 2, sc + rb * q.groups * 2);
+    info.x[g] = (g & (q.v - 1)) * q.groups * 64 + (turn && q.groups % 8 == 0 ? g : 0);      // (an offset of whole 64 bytes; below, how far its groups are turned)
+  }
   if (lane == 0) { info.groups = q.groups; info.second = q.slots > q.h1; }
 }
 
@@ -331,13 +336,15 @@ struct Matvec {
 
   __device__ __forceinline__ void begin(const Params& p, uint32_t info, int n, int first, int step_, int pos, int turn) {
     const int w = (threadIdx.x >> 5) & (SET - 1), lane = threadIdx.x & 31;
-    const uint2 head = ld64(info), x = ld64(info + 16 + 512 + lane * 8);
-    at = ld128(info + 16 + lane * 16);
+    const int g = lane >> 2, t4 = lane & 3;
+    const uint2 head = ld64(info);
+    const uint32_t x = ld32(info + 16 + 128 + g * 4);
+    at = ld128(info + 16 + g * 16);
     units = (static_cast<int>(head.x) - w + SET - 1) / SET;
     second = head.y != 0;
-    const uint32_t r = SET == 8 ? (w + x.y) & 7 : w;       // (w where the rows do not turn)
-    at.x += r * 16; at.y += r * 16; at.z += r * 2; at.w += r * 2;
-    xt = x.x + r * 64;
+    const uint32_t r = SET == 8 ? (w + x) & 7 : w;         // (w where the rows do not turn)
+    at.x += r * 16 + t4 * 4; at.y += r * 16 + t4 * 4; at.z += r * 2; at.w += r * 2;
+    xt = (x & ~7u) + t4 * 16 + r * 64;
     q = pos + first; end = pos + n; step = step_; i = turn + first; phase = 0; unit = 0;
 #pragma unroll 1
     while (i >= p.n_stages) { i -= p.n_stages; phase ^= 1u; }
@@ -538,8 +545,8 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
       }
       return t;
     };
-    // row i of a part that is not gate|up: 16 / v rows a slab
-    const auto sum_of = [&](uint32_t sums, int i, int v) { return row_sum(sums + (i * v >> 4) * STAGE_SUMS, i & (16 / v - 1), v); };
+    // row i of a piece of a part that is not gate|up
+    const auto sum_of = [&](uint32_t sums, int i, const Part& q) { return row_sum(sums + (i << q.lg_v >> q.lg) * STAGE_SUMS, i & ((1 << (q.lg - q.lg_v)) - 1), q.v); };
     // A thread's share of the hidden state and of the next norms' weights, 8 values of every 8 * SET_T, lies in shared memory.
     const uint32_t hid = base + L.hid;
     const auto fetch_norms = [&](int of) {           // a layer ahead: they may come from HBM.  A thread fetches what it will use.
@@ -650,16 +657,16 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
       const int part = to.part, layer = to.layer;
       const uint32_t tag = tag0 + 2u * layer;
       __half* out = static_cast<__half*>(p.d.outputs) + static_cast<long long>(layer) * layer_out;     // the layer's q|k|v, o, gate|up, down
-      const int n = to.count(mine.stages);
-      const uint32_t sums = part == PART_QKV ? sums_s : part == PART_O ? sums_s + mine.stages[PART_QKV] * STAGE_SUMS : sums_c;
-      const int v = p.part[part].v;
+      const int n = to.count(mine.stages, p.part);
+      const uint32_t sums = part == PART_QKV ? sums_s : part == PART_O ? sums_s + min2(mine.stages[PART_QKV], p.part[PART_QKV].piece) * STAGE_SUMS : sums_c;
+      const int v = p.part[part].v, r0 = to.done * p.part[part].per, rows = min2(mine.rows[part] - r0, n * p.part[part].per);       // rows of this piece
       Matvec<SET> m;
       m.begin(p, base + L.info + part * PART_INFO_BYTES, n, to.first(), to.step(), pos, turn);
       if (m.q < m.end) m.fetch(p, base, dead, flag_abort);
       const uint32_t sums_q = sums - static_cast<uint32_t>(pos) * STAGE_SUMS;
       pass(n);
       if (set == 0) {
-        if (part == PART_DOWN) {               // the activation
+        if (part == PART_DOWN && to.done == 0) {          // the activation
 #pragma unroll 1
           for (int i = 8 * st; i < sh.inter; i += 2 * 8 * SET_T) {
             const int i2 = i + 8 * SET_T;      // two at a time
@@ -676,66 +683,66 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
           }
           dead = __any_sync(0xffffffffu, dead);
         }
-      } else if (part == PART_GATE || (part == PART_HEAD && to.done == 0)) {
+      } else if (to.done == 0 && (part == PART_GATE || part == PART_HEAD)) {
         norms(layer == 0 ? nullptr : p.d_buf + copy, part == PART_HEAD ? nullptr : p.o_buf + (layer & 1) * sh.hidden + copy, tag & 0xFFFFu);
       }
       if (to.joint()) named_bar_sync(BAR_ALL, NCT);
-      else if (set == 0) named_bar_sync(BAR_SET0, SET_T);          // (the sums of o before have been read)
+      else if (set == 0) named_bar_sync(BAR_SET0, SET_T);          // (the sums of the piece before have been read)
+      else if (to.done != 0) named_bar_sync(BAR_SET1, SET_T);
       m.run(p, base, part == PART_DOWN ? xm : part == PART_O ? xq : part == PART_GATE ? xn + 2 * sh.hidden : xn, sums_q, dead, flag_abort);
 
       if (part == PART_GATE || part == PART_DOWN) {
         if (set == 1) {
           bar_arrive(BAR_SUMS, NCT);
-          pass(to.next(p.n_layers, mine.stages));
+          pass(to.next(p.n_layers, mine.stages, p.part));
           continue;
         }
         named_bar_sync(BAR_SUMS, NCT);
       }
       if (part == PART_GATE) {
-        const int per = p.part[PART_GATE].per;
+        const int lg_v = p.part[PART_GATE].lg_v, lg = p.part[PART_GATE].lg, mine0 = mine.row0[PART_GATE] + r0;
 #pragma unroll 1
-        for (int i = lane; i < mine.rows[PART_GATE]; i += 32) {
-          const int j = i * v >> 3;            // a slab is 8 / v rows of each (the last may be less)
-          const uint32_t slab = sums + j * STAGE_SUMS;
-          const int r = i - j * per;
+        for (int i = lane; i < rows; i += 32) {
+          const uint32_t slab = sums + (i << lg_v >> lg) * STAGE_SUMS;
+          const int r = i & ((1 << (lg - lg_v)) - 1);
           const __half gate = __float2half_rn(row_sum(slab, r, v)), up = __float2half_rn(row_sum(slab + 8 * ROW_SUMS, r, v));
           const float x = __half2float(gate);
           const __half y = __float2half_rn((x * (1.0f / (1.0f + expf(-x)))) * __half2float(up));
 #pragma unroll
-          for (int c = 0; c < COPIES / SET; ++c) publish(p.m_buf + (w + c * SET) * words + mine.row0[PART_GATE] + i, y, (tag + 1u) & 0xFFFFu);
+          for (int c = 0; c < COPIES / SET; ++c) publish(p.m_buf + (w + c * SET) * words + mine0 + i, y, (tag + 1u) & 0xFFFFu);
           if (w == 0) {                        // what the caller sees
-            __half* o = out + sh.qkv + sh.hidden + mine.row0[PART_GATE] + i;
+            __half* o = out + sh.qkv + sh.hidden + mine0 + i;
             o[0] = gate;
             o[sh.inter] = up;
-            if (layer + 1 == p.n_layers) static_cast<__half*>(p.d.mlp_out)[mine.row0[PART_GATE] + i] = y;
+            if (layer + 1 == p.n_layers) static_cast<__half*>(p.d.mlp_out)[mine0 + i] = y;
           }
         }
       } else if (part == PART_DOWN || part == PART_O) {
         const bool down = part == PART_DOWN;
         if (!down) named_bar_sync(BAR_SET0, SET_T);
-        uint32_t* words_out = (down ? p.d_buf : p.o_buf + ((layer + to.ahead) & 1) * sh.hidden) + w * words + mine.row0[part];
-        __half* o = out + (down ? layer_out - sh.hidden : to.ahead * layer_out + sh.qkv) + mine.row0[part];
+        uint32_t* words_out = (down ? p.d_buf : p.o_buf + ((layer + to.ahead) & 1) * sh.hidden) + w * words + mine.row0[part] + r0;
+        __half* o = out + (down ? layer_out - sh.hidden : to.ahead * layer_out + sh.qkv) + mine.row0[part] + r0;
         const uint32_t t = (tag + (down ? 2u : 2u * to.ahead)) & 0xFFFFu;
 #pragma unroll 1
-        for (int i = lane; i < mine.rows[part]; i += 32) {
-          const __half y = __float2half_rn(sum_of(sums, i, v));
+        for (int i = lane; i < rows; i += 32) {
+          const __half y = __float2half_rn(sum_of(sums, i, p.part[part]));
 #pragma unroll
           for (int c = 0; c < COPIES / SET; ++c) publish(words_out + c * SET * words + i, y, t);
           if (w == 0) o[i] = y;
         }
       } else if (part == PART_QKV) {
-        fetch_norms(layer + 1);
+        if (to.done == 0) fetch_norms(layer + 1);
         named_bar_sync(BAR_SET1, SET_T);
 #pragma unroll 1
-        for (int i = st; i < mine.rows[PART_QKV]; i += SET_T) out[mine.row0[PART_QKV] + i] = __float2half_rn(sum_of(sums, i, v));
+        for (int i = st; i < rows; i += SET_T) out[mine.row0[PART_QKV] + r0 + i] = __float2half_rn(sum_of(sums, i, p.part[part]));
       } else {
         // the key of a logit orders as np.argmax does: by value, NaN above all, the lowest index among equals
         named_bar_sync(BAR_ALL, NCT);
-        const int r0 = to.done * p.part[PART_HEAD].per, v0 = mine.row0[PART_HEAD] + r0, rows = min2(mine.rows[PART_HEAD] - r0, HEAD_SLABS * p.part[PART_HEAD].per);
+        const int v0 = mine.row0[PART_HEAD] + r0;
         unsigned long long key = 0;
 #pragma unroll 1
         for (int i = tid; i < rows; i += NCT) {
-          const __half y = __float2half_rn(sum_of(sums, i, v));
+          const __half y = __float2half_rn(sum_of(sums, i, p.part[part]));
           static_cast<__half*>(p.d.logits)[v0 + i] = y;
           const float f = __half2float(y) + 0.0f;        // -0 counts as 0
           uint32_t u = __float_as_uint(f);
@@ -749,9 +756,8 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
           if (k > key) key = k;
         }
         if (lane == 0 && (to.done == 0 || key > keys[warp])) keys[warp] = key;
-        if (r0 + rows < mine.rows[PART_HEAD]) named_bar_sync(BAR_ALL, NCT);          // the sums have been read
       }
-      pass(to.next(p.n_layers, mine.stages));
+      pass(to.next(p.n_layers, mine.stages, p.part));
     }
     if (b == 0) {
 #pragma unroll 1
@@ -781,19 +787,26 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
 
 // ---------------------------------------------------------------------------- host side
 struct Plan { Params p; size_t smem, state_bytes; };
+constexpr int LONG_ROW = 2560, MAX_STAGE = 227 * 1024;       // columns; bytes
 
 // A weight of rows of K columns, of which a CTA has at most `rows`: cut into short rows where they would be long, or so few that they
-// left rows of the MMA empty.  (Copies of scales start on 16 bytes: a slab is whole units of 4 rows.)
-inline Part make_part(int K, int rows, bool paired) {
+// left rows of the MMA empty; fewer rows a slab where a stage would still be longer than max_bytes.  (Copies of scales are whole 16 bytes: 256 columns.)
+inline Part make_part(int K, int rows, bool paired, int max_bytes) {
   Part q;
   q.K = K;
-  q.v = 1;
-  const int slab = paired ? 8 : 16;
-  while (q.v < (paired ? 2 : 4) && K % (64 * q.v) == 0 && (K / q.v > 2560 || rows * q.v * 2 <= slab)) q.v *= 2;
+  q.lg_v = 0;
+  q.lg = paired ? 3 : 4;
+  const auto whole = [&](int lg, int lg_v) { return lg >= lg_v && K % (32 << lg_v) == 0 && (K << (lg - lg_v)) % 256 == 0; };
+  const auto bytes = [&]() { return (paired ? 2 : 1) * (min2(1 << q.lg, rows << q.lg_v) * (K >> q.lg_v) / 32) * 18; };
+  while (whole(q.lg, q.lg_v + 1) && ((K >> q.lg_v > LONG_ROW && q.lg_v < (paired ? 1 : 2)) || rows << (q.lg_v + 1) <= 1 << q.lg)) ++q.lg_v;
+  while (bytes() > max_bytes && whole(q.lg - 1, q.lg_v)) --q.lg;
+  q.v = 1 << q.lg_v;
   q.groups = K / q.v / 32;
-  q.h1 = min2(8, rows * q.v);
-  q.slots = paired ? 2 * q.h1 : min2(16, rows * q.v);
-  q.per = (paired ? q.h1 : q.slots) / q.v;
+  const int n = min2(1 << q.lg, rows * q.v);
+  q.h1 = min2(8, n);
+  q.slots = paired ? 2 * n : n;
+  q.per = n / q.v;
+  q.piece = 1 << 30;
   return q;
 }
 
@@ -805,27 +818,39 @@ inline bool narrow(const Params& p) { return p.sh.hidden <= 640; }
 inline bool make_plan(const lcq_decode_stack& d, int sm_count, Plan& pl) {
   const int H = d.hidden, I = d.inter;
   if (d.n_layers < 1 || H < 64 || I < 64 || d.qkv < 4 || d.q_dim < 64 || d.vocab < 4 || d.n_layers > 256) return false;
-  if (H % 64 || I % 64 || d.q_dim % 64 || d.qkv % 4 || d.vocab % 4 || H > 8192 || I > (1 << 20) || d.vocab > (1 << 24)) return false;
+  if (H % 64 || I % 64 || d.q_dim % 64 || d.qkv % 4 || d.vocab % 4 || H > 8192 || I > (1 << 20) || d.q_dim > (1 << 20) || d.qkv > (1 << 24) || d.vocab > (1 << 24)) return false;
   Params& p = pl.p;
   memset(&p, 0, sizeof(p));
   p.d = d;
   p.sh = {H, I, d.qkv, d.q_dim, d.vocab};
   p.n_layers = d.n_layers;
   p.inv_hidden = 1.0f / static_cast<float>(H);
+  // Four rows of the longest kind fit twice beside the vectors.  (Stages may be shorter; longer rows are the chain's.)
+  const int longest = max2(max2(H, I), d.q_dim), vectors = (6 * H + d.q_dim + I) * 2;
+  if (vectors + 2 * max2(24 * 1024, longest / 4 * 9) + d.n_layers * static_cast<int>(sizeof(lcq_decode_layer)) > 227 * 1024) return false;
   int units = H / 4;                           // every CTA needs a unit of 4 rows in every phase
   if (I / 4 < units) units = I / 4;
   if (d.vocab / 4 < units) units = d.vocab / 4;
   p.ctas = sm_count < units ? sm_count : units;
   const int hid = max_share(H, p.ctas), qkv = max_share(d.qkv, p.ctas);
-  p.part[PART_O] = make_part(d.q_dim, hid, false);
-  p.part[PART_GATE] = make_part(H, max_share(I, p.ctas), true);
-  p.part[PART_QKV] = make_part(H, qkv, false);
-  p.part[PART_DOWN] = make_part(I, hid, false);
-  p.part[PART_HEAD] = make_part(H, max_share(d.vocab, p.ctas), false);
-  for (const Part& q : p.part) p.stage_bytes = max2(p.stage_bytes, (q.slots * q.groups * 18 + 127) & ~127);
-  p.n_stages = (227 * 1024 - smem_map(p).total) / p.stage_bytes;
-  if (p.n_stages > MAX_STAGES) p.n_stages = MAX_STAGES;
-  if (p.n_stages < 2) return false;
+  // The longest stages and the largest pieces with which two stages fit.
+  for (int max_bytes = MAX_STAGE; p.n_stages < 2; max_bytes /= 2) {
+    if (max_bytes < 1024) return false;
+    p.part[PART_O] = make_part(d.q_dim, hid, false, max_bytes);
+    p.part[PART_GATE] = make_part(H, max_share(I, p.ctas), true, max_bytes);
+    p.part[PART_QKV] = make_part(H, qkv, false, max_bytes);
+    p.part[PART_DOWN] = make_part(I, hid, false, max_bytes);
+    p.part[PART_HEAD] = make_part(H, max_share(d.vocab, p.ctas), false, max_bytes);
+    p.part[PART_HEAD].piece = HEAD_SLABS;
+    p.stage_bytes = 0;
+    for (const Part& q : p.part) p.stage_bytes = max2(p.stage_bytes, (q.slots * q.groups * 18 + 127) & ~127);
+    for (int piece = HEAD_SLABS; piece >= 2; piece /= 4) {
+      if (piece < HEAD_SLABS) for (Part& q : p.part) q.piece = piece;
+      p.n_stages = 0;
+      p.n_stages = min2(MAX_STAGES, (227 * 1024 - smem_map(p).total) / p.stage_bytes);
+      if (p.n_stages >= 2) break;
+    }
+  }
   p.map = smem_map(p);
   pl.smem = static_cast<size_t>(p.map.total);
   pl.state_bytes = STATE_BYTES + (static_cast<size_t>(3) * H + I) * 4 * COPIES;

@@ -741,17 +741,18 @@ struct StepReplay {
     std::vector<Item>& v = program[set];
     int pos = Walk::skipped_at_first(set, p.n_layers, rows.stages);
     for (Walk to(set); to.part != N_PARTS;) {
-      const int part = to.part, n = to.count(rows.stages), sums = part == PART_QKV ? QKV : part == PART_O ? O : CHAIN;
+      const int part = to.part, n = to.count(rows.stages, p.part), sums = part == PART_QKV ? QKV : part == PART_O ? O : CHAIN;
       int q = pos + to.first();
       if (q < pos + n) v.push_back({WAIT, q, part});
-      if (set == 0 && part == PART_DOWN) v.push_back({POLL, 3 * to.layer, 0});
-      if (set == 1 && (part == PART_GATE || (part == PART_HEAD && to.done == 0))) {
+      if (set == 0 && part == PART_DOWN && to.done == 0) v.push_back({POLL, 3 * to.layer, 0});
+      if (set == 1 && to.done == 0 && (part == PART_GATE || part == PART_HEAD)) {
         if (to.layer > 0) v.push_back({POLL, 3 * to.layer - 2, 0});
         if (part == PART_GATE) v.push_back({POLL, 3 * to.layer + 2, 0});
         v.push_back({SYNC, SET1, 0});
       }
       if (to.joint()) v.push_back({SYNC, ALL, 0});
       else if (set == 0) v.push_back({SYNC, SET0, 0});
+      else if (to.done != 0) v.push_back({SYNC, SET1, 0});
       for (; q < pos + n; q += to.step()) {
         if (q != pos + to.first()) v.push_back({WAIT, q, part});
         v.push_back({USE, q, sums * (1 << 28) + pos});
@@ -759,11 +760,10 @@ struct StepReplay {
       if (part == PART_GATE || part == PART_DOWN) v.push_back({set == 1 ? ARRIVE : SYNC, SUMS, 0});
       else v.push_back({SYNC, part == PART_HEAD ? ALL : set == 0 ? SET0 : SET1, 0});
       if (n > 0 && (set == 0 || !to.joint() || part == PART_HEAD)) v.push_back({READ, sums, pos});
-      if (set == 0 && part != PART_HEAD)
+      if (set == 0 && part != PART_HEAD && to.done + n == rows.stages[part])
         v.push_back({PUBLISH, part == PART_GATE ? 3 * to.layer : part == PART_DOWN ? 3 * to.layer + 1 : 3 * (to.layer + to.ahead) + 2, 0});
-      if (part == PART_HEAD && to.done + n < rows.stages[part]) v.push_back({SYNC, ALL, 0});
       pos += n;
-      pos += to.next(p.n_layers, rows.stages);
+      pos += to.next(p.n_layers, rows.stages, p.part);
     }
     if (pos != static_cast<int>(stages.size())) fault = "a set does not end with the stream";
   }
@@ -877,15 +877,14 @@ int lcq_decode_step_plan_check(const lcq_decode_stack* stack, int sm_count, int*
       covered[i] += r.rows[i];
       // copies: whole multiples of 16 bytes between places on 16 bytes, inside a stage, no more short rows than an MMA has
       const int half_w = q.h1 * q.groups * 16, scales = q.slots * q.groups * 16, half_s = q.h1 * q.groups * 2;
-      if (q.slots > 16 || q.h1 > 8 || q.per * q.v > (paired ? q.h1 : q.slots) || q.groups * 32 * q.v != q.K || scales + q.slots * q.groups * 2 > p.stage_bytes || (paired && (half_w % 16 || half_s % 16))) { set_error("plan check: part %d does not fit a stage", i); return LCQ_ERR_BAD_ARG; }
+      if (q.slots > 16 || q.h1 > 8 || q.v != 1 << q.lg_v || (r.stages[i] > 1 && q.per * q.v != 1 << q.lg) || (q.per * q.v > 1 << q.lg) || q.per * q.v > (paired ? q.h1 : q.slots) || q.groups * 32 * q.v != q.K || scales + q.slots * q.groups * 2 > p.stage_bytes || (paired && (half_w % 16 || half_s % 16))) { set_error("plan check: part %d does not fit a stage", i); return LCQ_ERR_BAD_ARG; }
       for (int row = 0; row < r.rows[i]; row += q.per) {
         const long long from = r.row0[i] + row, n = min2(r.rows[i] - row, q.per), K = q.K, other = paired ? p.sh.inter : 0;
-        if (from * (K / 2) % 16 || from * (K / 16) % 16 || n * (K / 2) % 16 || n * (K / 16) % 16 || other * (K / 16) % 16 || scales % 16) { set_error("plan check: part %d, row %lld: a copy off 16 bytes", i, from); return LCQ_ERR_BAD_ARG; }
+        if (from * (K / 2) % 16 || from * (K / 16) % 16 || n * (K / 2) % 16 || n * (K / 16) % 16 || other * (K / 2) % 16 || other * (K / 16) % 16 || scales % 16) { set_error("plan check: part %d, row %lld: a copy off 16 bytes", i, from); return LCQ_ERR_BAD_ARG; }
       }
     }
-    // partial sums of the largest pieces
-    const int head = min2(r.stages[PART_HEAD], HEAD_SLABS);
-    if (m.sums + max2(max2(r.stages[PART_GATE], r.stages[PART_DOWN]), head) * STAGE_SUMS > m.side || m.side + (r.stages[PART_QKV] + r.stages[PART_O]) * STAGE_SUMS > m.red) { set_error("plan check: CTA %d: partial sums out of bounds", b); return LCQ_ERR_BAD_ARG; }
+    const auto slabs = [&](int part) { return min2(r.stages[part], p.part[part].piece); };      // of the largest pieces
+    if (m.sums + max2(max2(slabs(PART_GATE), slabs(PART_DOWN)), slabs(PART_HEAD)) * STAGE_SUMS > m.side || m.side + (slabs(PART_QKV) + slabs(PART_O)) * STAGE_SUMS > m.red) { set_error("plan check: CTA %d: partial sums out of bounds", b); return LCQ_ERR_BAD_ARG; }
     bool known = false;                                    // (a CTA whose stages another has, too)
     for (const Rows& o : done) known = known || memcmp(o.stages, r.stages, sizeof(r.stages)) == 0;
     if (known) continue;

@@ -56,6 +56,14 @@ WIDE = [dict(layers=3, hidden=4096, inter=11008, q_heads=64, kv_heads=64, vocab=
         dict(layers=2, hidden=2560, inter=9728, q_heads=64, kv_heads=16, vocab=151936), dict(layers=3, hidden=5120, inter=5120, q_heads=40, kv_heads=8, vocab=2000)]
 
 
+# Little shared memory beside the vectors: parts in pieces of eight and of two stages, one CTA for everything, stages of fewer rows (rows that
+# can't be cut in powers of two, long ones), a ring of two, the widest.
+TIGHT = [dict(layers=2, hidden=768, inter=2048, q_heads=24, kv_heads=6, vocab=4), dict(layers=2, hidden=6144, inter=18432, q_heads=192, kv_heads=48, vocab=1000),
+         dict(layers=3, hidden=1792, inter=9408, q_heads=28, kv_heads=28, vocab=4), dict(layers=2, hidden=7680, inter=3840, q_heads=240, kv_heads=60, vocab=2000),
+         dict(layers=2, hidden=4096, inter=21568, q_heads=64, kv_heads=16, vocab=2000), dict(layers=2, hidden=3072, inter=24576, q_heads=24, kv_heads=24, vocab=2000),
+         dict(layers=3, hidden=8192, inter=8192, q_heads=64, kv_heads=8, vocab=1000), dict(layers=2, hidden=5120, inter=13760, q_heads=80, kv_heads=20, vocab=1000)]
+
+
 def _plan_check(layers, hidden, inter, q_heads, kv_heads, vocab, sms=148):
     """Replays the schedule on the CPU: the status, and {CTAs, stages in the ring, their bytes, shared memory, warps, early waits}."""
     desc = _lib.DecodeStackDesc(n_layers=layers, hidden=hidden, inter=inter, q_dim=64 * q_heads, qkv=64 * (q_heads + 2 * kv_heads), vocab=vocab)
@@ -63,7 +71,7 @@ def _plan_check(layers, hidden, inter, q_heads, kv_heads, vocab, sms=148):
     return _lib.lib().lcq_decode_step_plan_check(ctypes.byref(desc), sms, fields), list(fields)
 
 
-@pytest.mark.parametrize("shape", SHAPES + EDGES + WIDE)
+@pytest.mark.parametrize("shape", SHAPES + EDGES + WIDE + TIGHT)
 def test_schedule_replayed(shape):
     """On the device a set waits for its stage by the issue count and by the stage's barrier.  The barrier alone, one parity, would have let it on
     before the stage had landed wherever the other set's stages fill the ring in between: every one of the wide shapes."""
@@ -116,7 +124,7 @@ def test_matches_the_chain_of_kernels(shape):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape", WIDE)
+@pytest.mark.parametrize("shape", WIDE + TIGHT)
 def test_short_rings(shape, monkeypatch):
     monkeypatch.setattr(linear, "_one_kernel_pays", lambda *sizes: True)         # whichever form is faster
     test_matches_the_chain_of_kernels(shape)

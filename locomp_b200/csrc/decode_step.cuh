@@ -787,18 +787,22 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
 
 // ---------------------------------------------------------------------------- host side
 struct Plan { Params p; size_t smem, state_bytes; };
-constexpr int LONG_ROW = 2560, MAX_STAGE = 227 * 1024;       // columns; bytes
+constexpr int CUT_ROW = 3584, LONG_ROW = 4096, MAX_STAGE = 40 * 1024;      // columns; bytes
 
-// A weight of rows of K columns, of which a CTA has at most `rows`: cut into short rows where they would be long, or so few that they
-// left rows of the MMA empty; fewer rows a slab where a stage would still be longer than max_bytes.  (Copies of scales are whole 16 bytes: 256 columns.)
-inline Part make_part(int K, int rows, bool paired, int max_bytes) {
+// A weight of rows of K columns, of which a CTA has at most `rows`: cut into short rows where they would be longer than `whole_row` (then to CUT_ROW at
+// most), or so few that they left rows of the MMA empty; fewer rows a slab where a stage would still be longer than max_bytes.  (Copies of scales are
+// whole 16 bytes: 256 columns.)
+// A stage costs a warp its rounds of U groups and about one more, so long rows are cheaper as long as the ring keeps three stages.  us a step with
+// rows cut to 2560 at most / to 3584: 8 layers of 3072 / 8192 with 128,256 rows 291 / 272, 4 of 3200 / 8640 194 / 181, 6 of 3584 / 18944 603 / 423,
+// 4 of 3072 / 24576 359 / 244; to 1536: 8 of 2048 / 8192 250 instead of 185.
+inline Part make_part(int K, int rows, bool paired, int whole_row, int max_bytes) {
   Part q;
   q.K = K;
   q.lg_v = 0;
   q.lg = paired ? 3 : 4;
   const auto whole = [&](int lg, int lg_v) { return lg >= lg_v && K % (32 << lg_v) == 0 && (K << (lg - lg_v)) % 256 == 0; };
   const auto bytes = [&]() { return (paired ? 2 : 1) * (min2(1 << q.lg, rows << q.lg_v) * (K >> q.lg_v) / 32) * 18; };
-  while (whole(q.lg, q.lg_v + 1) && ((K >> q.lg_v > LONG_ROW && q.lg_v < (paired ? 1 : 2)) || rows << (q.lg_v + 1) <= 1 << q.lg)) ++q.lg_v;
+  while (whole(q.lg, q.lg_v + 1) && ((K > whole_row && K >> q.lg_v > CUT_ROW) || rows << (q.lg_v + 1) <= 1 << q.lg)) ++q.lg_v;
   while (bytes() > max_bytes && whole(q.lg - 1, q.lg_v)) --q.lg;
   q.v = 1 << q.lg_v;
   q.groups = K / q.v / 32;
@@ -833,22 +837,30 @@ inline bool make_plan(const lcq_decode_stack& d, int sm_count, Plan& pl) {
   if (d.vocab / 4 < units) units = d.vocab / 4;
   p.ctas = sm_count < units ? sm_count : units;
   const int hid = max_share(H, p.ctas), qkv = max_share(d.qkv, p.ctas);
-  // The longest stages and the largest pieces with which two stages fit.
-  for (int max_bytes = MAX_STAGE; p.n_stages < 2; max_bytes /= 2) {
-    if (max_bytes < 1024) return false;
-    p.part[PART_O] = make_part(d.q_dim, hid, false, max_bytes);
-    p.part[PART_GATE] = make_part(H, max_share(I, p.ctas), true, max_bytes);
-    p.part[PART_QKV] = make_part(H, qkv, false, max_bytes);
-    p.part[PART_DOWN] = make_part(I, hid, false, max_bytes);
-    p.part[PART_HEAD] = make_part(H, max_share(d.vocab, p.ctas), false, max_bytes);
+  const auto cut = [&](int whole_row, int max_bytes) {
+    p.part[PART_O] = make_part(d.q_dim, hid, false, whole_row, max_bytes);
+    p.part[PART_GATE] = make_part(H, max_share(I, p.ctas), true, whole_row, max_bytes);
+    p.part[PART_QKV] = make_part(H, qkv, false, whole_row, max_bytes);
+    p.part[PART_DOWN] = make_part(I, hid, false, whole_row, max_bytes);
+    p.part[PART_HEAD] = make_part(H, max_share(d.vocab, p.ctas), false, whole_row, max_bytes);
     p.part[PART_HEAD].piece = HEAD_SLABS;
     p.stage_bytes = 0;
     for (const Part& q : p.part) p.stage_bytes = max2(p.stage_bytes, (q.slots * q.groups * 18 + 127) & ~127);
+  };
+  // The longest stages and the largest pieces with which three stages fit, or two.
+  for (int fit = 3, max_bytes = MAX_STAGE; p.n_stages < fit; max_bytes /= 2) {
+    if (max_bytes < MAX_STAGE / 16) {
+      if (--fit < 2) return false;
+      max_bytes = MAX_STAGE;
+    }
+    cut(CUT_ROW, max_bytes);
+    // (rows of up to 4096 whole where that makes the stages half as long again at most; cut / whole: 6 of 4096 / 14336 349 / 331, but 6 of 4096 / 4096 169 / 176)
+    if (p.stage_bytes * 3 / 2 >= 16 * LONG_ROW / 32 * 18) cut(LONG_ROW, max_bytes);
     for (int piece = HEAD_SLABS; piece >= 2; piece /= 4) {
       if (piece < HEAD_SLABS) for (Part& q : p.part) q.piece = piece;
       p.n_stages = 0;
       p.n_stages = min2(MAX_STAGES, (227 * 1024 - smem_map(p).total) / p.stage_bytes);
-      if (p.n_stages >= 2) break;
+      if (p.n_stages >= fit) break;
     }
   }
   p.map = smem_map(p);

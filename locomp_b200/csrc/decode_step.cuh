@@ -289,16 +289,16 @@ __device__ __forceinline__ bool wait_stage(uint32_t bar, uint32_t parity, uint32
 
 // Bounded wait until more than q stages of the stream have been issued.  A set does not see the other's stages, so this is how it knows which use of a place
 // of the ring it waits for: stage q is issued once stage q - n_stages has been consumed, thus has landed.
+// `issued` is what the warp knows already; the producer is mostly far ahead.
 __device__ __forceinline__ void count_issued(uint32_t a, int n) { asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(a), "r"(n) : "memory"); }
-__device__ __forceinline__ bool wait_issued(uint32_t a, int q, uint32_t flag_abort) {
+__device__ __forceinline__ bool wait_issued(uint32_t a, int q, int& issued, uint32_t flag_abort) {
   unsigned long long t0 = 0;
 #pragma unroll 1
-  for (;;) {
-    int n;
-    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(n) : "r"(a) : "memory");
-    if (n > q) return true;
-    if (over(t0, flag_abort)) return false;
+  while (issued <= q) {
+    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(issued) : "r"(a) : "memory");
+    if (issued <= q && over(t0, flag_abort)) return false;
   }
+  return true;
 }
 
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
@@ -350,11 +350,15 @@ struct Matvec {
     while (i >= p.n_stages) { i -= p.n_stages; phase ^= 1u; }
   }
   // the next groups of stage q
-  __device__ __forceinline__ void fetch(const Params& p, uint32_t base, bool& dead, uint32_t flag_abort) {
+  __device__ __forceinline__ void fetch(const Params& p, uint32_t base, int& issued, bool& dead, uint32_t flag_abort) {
     if (unit == 0 && !dead) {
-      const bool ok = wait_issued(base + p.map.flags + 8, q, flag_abort) && wait_stage(base + p.map.bars + i * 8, phase, flag_abort);
-      if (__any_sync(0xffffffffu, !ok)) { dead = true; st32(flag_abort, 1.0f); atomicExch(&g_device_status, 51); }
+      if (!wait_issued(base + p.map.flags + 8, q, issued, flag_abort) || !wait_stage(base + p.map.bars + i * 8, phase, flag_abort)) {
+        dead = true;                           // (of this lane; the warp agrees on it where it polls next)
+        st32(flag_abort, 1.0f);
+        atomicExch(&g_device_status, 51);
+      }
     }
+    __syncwarp();                              // (no vote, here it costs more than what it guards: 30 layers of 576 / 1536 195 -> 185 us, 8 of 4096 / 11008 459 -> 467)
     const uint32_t st = base + i * p.stage_bytes;
     const uint32_t a0 = st + at.x + unit * (SET * 16), b0 = st + at.y + unit * (SET * 16), s0 = st + at.z + unit * (SET * 2), t0 = st + at.w + unit * (SET * 2);
 #pragma unroll
@@ -371,7 +375,7 @@ struct Matvec {
     }
   }
   // all of it, the first groups fetched before; the sums of stage q go to sums + q * STAGE_SUMS: [row][warp]
-  __device__ __forceinline__ void run(const Params& p, uint32_t base, uint32_t x, uint32_t sums, bool& dead, uint32_t flag_abort) {
+  __device__ __forceinline__ void run(const Params& p, uint32_t base, uint32_t x, uint32_t sums, int& issued, bool& dead, uint32_t flag_abort) {
     const int w = (threadIdx.x >> 5) & (SET - 1), lane = threadIdx.x & 31, g = lane >> 2;
     const bool odd = g & 1;
     float sum0 = 0.0f, sum1 = 0.0f;
@@ -413,7 +417,7 @@ struct Matvec {
 #pragma unroll 1
         while (i >= p.n_stages) { i -= p.n_stages; phase ^= 1u; }
       }
-      if (q < end) fetch(p, base, dead, flag_abort);
+      if (q < end) fetch(p, base, issued, dead, flag_abort);
     }
   }
 };
@@ -529,6 +533,7 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
     const uint32_t tag0 = *smem_epoch * static_cast<uint32_t>(2 * p.n_layers + 1) + 1u;
     const int words = 3 * sh.hidden + sh.inter, copy = (b % COPIES) * words;       // the copy that is read here; warp w writes copy w
     int pos = 0, turn = 0;                     // stages of the stream that are behind, and these modulo two rounds of the ring
+    int issued = 0;                            // stages that are known to have been issued
     bool dead = false;
     const auto pass = [&](int n) {
       pos += n;
@@ -662,7 +667,7 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
       const int v = p.part[part].v, r0 = to.done * p.part[part].per, rows = min2(mine.rows[part] - r0, n * p.part[part].per);       // rows of this piece
       Matvec<SET> m;
       m.begin(p, base + L.info + part * PART_INFO_BYTES, n, to.first(), to.step(), pos, turn);
-      if (m.q < m.end) m.fetch(p, base, dead, flag_abort);
+      if (m.q < m.end) m.fetch(p, base, issued, dead, flag_abort);
       const uint32_t sums_q = sums - static_cast<uint32_t>(pos) * STAGE_SUMS;
       pass(n);
       if (set == 0) {
@@ -689,7 +694,7 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
       if (to.joint()) named_bar_sync(BAR_ALL, NCT);
       else if (set == 0) named_bar_sync(BAR_SET0, SET_T);          // (the sums of the piece before have been read)
       else if (to.done != 0) named_bar_sync(BAR_SET1, SET_T);
-      m.run(p, base, part == PART_DOWN ? xm : part == PART_O ? xq : part == PART_GATE ? xn + 2 * sh.hidden : xn, sums_q, dead, flag_abort);
+      m.run(p, base, part == PART_DOWN ? xm : part == PART_O ? xq : part == PART_GATE ? xn + 2 * sh.hidden : xn, sums_q, issued, dead, flag_abort);
 
       if (part == PART_GATE || part == PART_DOWN) {
         if (set == 1) {

@@ -317,7 +317,7 @@ int lcq_set_wait_limit_ns(unsigned long long limit_ns);
  * device with sm_count SMs and replays its device-side schedule on the CPU, checking that
  * every (row block, k tile) is produced exactly once and that scratch slots and contributor
  * counts agree.  fields (may be NULL) receives {grid, row blocks, k ranges, tiles per range,
- * CTAs per range, max split, shared-memory bytes, m tiles}.  No counterpart in the reference.
+ * CTAs per range, max split (1: every CTA takes whole row blocks), shared-memory bytes, m tiles}.  No counterpart in the reference.
  */
 int lcq_gemv_tc_plan_check(int M, int N, int K, int sm_count, int* fields);
 

@@ -103,7 +103,7 @@ struct Params {
   int S;                // tiles (of 256 k) per k-range; the last range may hold fewer
   int nst;              // ceil(K / 256)
   int ctas_per_kr;      // CTAs working on one k-range
-  int max_split;        // scratch slots per (row block, k-range)
+  int max_split;        // scratch slots per (row block, k-range); 1: whole row blocks
   int x_tiles;          // k tiles of x a CTA keeps in shared memory (S, or ceil(S / cluster) in cluster mode)
   int cluster;          // CTAs per row block that reduce through distributed shared memory (1 = none)
   int whole;            // a CTA's share is whole row blocks
@@ -1077,10 +1077,11 @@ inline Plan make_plan(int M, int N, int K, int sm_count) {
     if (want < p.ctas_per_kr) p.ctas_per_kr = static_cast<int>(want);
   }
   // Whole row blocks where they leave no CTA with much more than its equal share: no scratch, no counters, and the tail of a
-  // row block that two CTAs share (a round trip to L2 under full load) costs as much as three to four tiles.  us a call, cut / whole,
-  // tiles of the busiest CTA: M = 1 512 -> 49152 8.1 / 5.9 (2.6, 4), 2048 -> 32000 13.4 / 9.3 (6.8, 8), 4096 -> 28672 17.7 / 16.0 (12.1, 16),
-  // 1536 -> 49152 13.1 / 12.4 (7.8, 12), 2048 -> 49152 14.9 / 15.7 (10.4, 16), 4096 -> 40000 21.4 / 26.0 (16.9, 32); M = 16 512 -> 49152
-  // 12.5 / 9.8 (5.2, 6), 2048 -> 49152 23.5 / 23.1 (20.8, 24), 2048 -> 20000 14.2 / 16.2 (8.5, 16).
+  // row block that two CTAs share (a round trip to L2 under full load) costs as much as three to four tiles.  us a call, cut / whole, 400 calls back to
+  // back in a CUDA graph over weights that together exceed L2 (in parentheses tiles of the busiest CTA): M = 1 512 -> 49152 8.0 / 5.8 (2.6, 4),
+  // 2048 -> 32000 13.0 / 8.9 (6.8, 8), 4096 -> 28672 17.2 / 15.4 (12.1, 16), 1536 -> 49152 12.7 / 12.1 (7.8, 12), 2048 -> 49152 14.5 / 15.1 (10.4, 16),
+  // 4096 -> 40000 20.3 / 25.2 (16.9, 32); M = 3 576 -> 49152 9.8 / 8.6; M = 16 512 -> 49152 12.3 / 9.7 (5.2, 6), 2048 -> 49152 23.1 / 22.6 (20.8, 24),
+  // 2048 -> 20000 13.9 / 16.1 (8.5, 16).
   if (!pl.cluster && p.n_kr == 1) {
     const int ctas = p.ctas_per_kr < p.n_rb ? p.ctas_per_kr : p.n_rb;
     const long long most = static_cast<long long>((p.n_rb + ctas - 1) / ctas) * p.S;
@@ -1096,13 +1097,13 @@ inline Plan make_plan(int M, int N, int K, int sm_count) {
     const int b = static_cast<int>(s.S_kr / (min_tiles > 0 ? min_tiles : 1)) + 2;
     if (b > max_split) max_split = b;
   }
-  p.max_split = max_split;
+  p.max_split = p.whole ? 1 : max_split;       // (whole row blocks write no partials; what callers reserve stays as it is)
   pl.grid = p.n_kr * p.ctas_per_kr;
   pl.fits_32bit = (T + 1) * static_cast<long long>(p.ctas_per_kr) < (1LL << 32);
   pl.smem_bytes = smem_layout(nstages_for(pl.MT, pl.cluster), pl.MPAD, pl.MT, p.x_tiles, p.cluster).total;
   pl.counters_bytes = COUNTER_BYTES;
   pl.workspace_bytes = pl.counters_bytes +
-                       static_cast<size_t>(p.n_rb) * p.n_kr * p.max_split * M * ROWS * sizeof(float);
+                       static_cast<size_t>(p.n_rb) * p.n_kr * max_split * M * ROWS * sizeof(float);
   return pl;
 }
 

@@ -13,6 +13,8 @@ from locomp_b200 import _lib
 
 CASES = [(1, 64, 37889), (1, 512, 49152), (3, 576, 49000), (8, 320, 76001), (1, 1536, 49152), (1, 2048, 49152), (2, 4096, 28672), (4, 2560, 30000),
          (16, 64, 19000), (9, 512, 57000), (16, 832, 18945), (12, 1536, 32000), (16, 2560, 24576)]
+CUT = [(1, 2048, 49152), (16, 2560, 24576), (1, 4096, 40000), (16, 2048, 20000), (3, 2112, 49000), (8, 1856, 40001)]
+CASES += [case for case in CUT if case not in CASES]
 
 
 @pytest.mark.parametrize("m,k,n", CASES)
@@ -21,6 +23,13 @@ def test_plan_covers_every_tile_once(m, k, n):
     for rows in (n, n - 128, n + 128, n // 2):
         for sms in (148, 132, 16, 1):
             assert _lib.lib().lcq_gemv_tc_plan_check(m, rows, k, sms, f) == 0, (rows, sms, _lib.lib().lcq_last_error())
+
+
+@pytest.mark.parametrize("m,k,n", CASES)
+def test_side_of_the_rule(m, k, n):
+    f = (ctypes.c_int * 8)()
+    assert _lib.lib().lcq_gemv_tc_plan_check(m, n, k, 148, f) == 0 and _lib.lib().lcq_gemv_tc_plan_cluster(m, n, k, 148) == 1
+    assert (f[5] > 1) == ((m, k, n) in CUT)   # more than one slot for partials: row blocks are cut
 
 
 @pytest.mark.gpu

@@ -68,11 +68,11 @@ def fuse_rows(parts: Sequence[Tuple[torch.Tensor, torch.Tensor]], group_size: in
 
 def _one_kernel_pays(layers: int, layer_weights: int, head_weights: int) -> bool:
     """Whether a step is faster as one kernel than as a chain of launches.  The kernel saves about 10 us a layer of launches and
-    hand-overs; its matvecs stream weights more slowly than the decode kernel: about 1 us per 30 Mi weights of a
-    layer and per 15 Mi of the lm_head.  Kernel and chain in us: 30 layers of 576 / 1536 217 and 484; 8 of 3072 / 8192
-    with 128,256 rows of lm_head 289 and 344; 8 of 2560 / 9728 with 151,936 315 and 355; wider ones with an earlier kernel: 5 of 4608 / 12288 299
-    and 297; 4 of 6144 / 16384 342 and 296; 6 of 3584 / 18944 with 152,064 rows of lm_head 392 and 370."""
-    return layers * (10.0 - layer_weights / 30e6) > head_weights / 15e6
+    hand-overs; its matvecs stream weights more slowly than the decode kernel: about 1 us per 23.5 million weights of a
+    layer and per 35 million of the lm_head.  Kernel and chain in us (replayed CUDA graphs, six back to back): 30 layers of 576 / 1536 185
+    and 484; 24 of 2048 / 8192 503 and 707; 8 of 3072 / 8192 with 128,256 rows of lm_head 272 and 345; 8 of 4096 / 11008 467 and 479; 5 of 4608 / 12288
+    273 and 298; 6 of 4096 / 14336 337 and 329; 4 of 5120 / 13824 297 and 258; 6 of 3584 / 18944 with 152,064 rows 431 and 372; 4 of 6144 / 16384 361 and 291."""
+    return layers * (10.0 - layer_weights / 23.5e6) > head_weights / 35e6
 
 
 class DecodeStack:
@@ -86,8 +86,8 @@ class DecodeStack:
     input RMS norm, residual add + post-attention norm (one kernel), SiLU * up, residual add, final
     norm, and a greedy argmax of the logits on the device -- a real dependency chain on one hidden
     state.  In fp16 the whole step is one kernel where that covers the shape and is faster, else 8 launches per layer.
-    Since o reads a prepared buffer and not attention output, that kernel computes it beside the down projection of the layer
-    before: two dependent phases a layer, where a model with attention has four."""
+    Since o reads a prepared buffer and not attention output, that kernel computes it two layers
+    ahead: two dependent phases a layer, where a model with attention has four."""
 
     def __init__(self, layers: int = 30, hidden: int = 576, inter: int = 1536, q_heads: int = 9, kv_heads: int = 3,
                  head_dim: int = 64, vocab: int = 49152, fused: bool = False, device="cuda", seed: int = 0,

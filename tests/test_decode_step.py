@@ -18,13 +18,20 @@ SHAPES = [dict(layers=1, hidden=64, inter=64, q_heads=1, kv_heads=1, vocab=4), d
 
 
 # layers, hidden, inter, query and key heads, vocabulary: us of the one kernel, us of the chain
-MEASURED = [((1, 64, 64, 1, 1, 64), 16.6, 16.7), ((12, 256, 768, 4, 4, 32000), 96.8, 140.3), ((30, 576, 1536, 9, 3, 49152), 298.9, 483.7),
-            ((1, 576, 1536, 9, 3, 49152), 26.7, 33.0), ((8, 1024, 3072, 16, 8, 151936), 119.4, 192.6), ((24, 2048, 8192, 32, 32, 49152), 539.2, 726.3),
-            ((1, 2048, 8192, 32, 32, 16384), 37.3, 41.1), ((8, 2560, 9728, 32, 8, 151936), 293.5, 354.6), ((8, 3072, 8192, 24, 8, 128256), 301.3, 344.3),
-            ((4, 3072, 24576, 24, 24, 32000), 238.0, 240.2), ((6, 3584, 18944, 28, 4, 152064), 391.9, 370.0), ((6, 4096, 4096, 32, 8, 32000), 177.0, 210.6),
-            ((8, 4096, 14336, 32, 8, 128256), 466.1, 469.1), ((6, 4096, 14336, 32, 32, 32000), 319.7, 336.4), ((5, 4608, 12288, 36, 36, 32000), 299.0, 296.8),
-            ((5, 5120, 5120, 40, 8, 32000), 201.0, 242.2), ((4, 5120, 13824, 40, 8, 32000), 272.5, 256.9), ((4, 5120, 13824, 40, 40, 32000), 289.5, 281.7),
-            ((4, 6144, 16384, 48, 8, 32000), 342.3, 295.8), ((4, 8192, 8192, 64, 8, 32000), 332.3, 294.4)]
+MEASURED = [((1, 64, 64, 1, 1, 64), 14.7, 16.7), ((12, 256, 768, 4, 4, 32000), 86.0, 141.3), ((30, 576, 1536, 9, 3, 49152), 185.0, 483.6),
+            ((1, 576, 1536, 9, 3, 49152), 25.2, 34.5), ((8, 1024, 3072, 16, 8, 151936), 118.4, 187.7),
+            ((24, 2048, 8192, 32, 32, 49152), 502.8, 706.8), ((1, 2048, 8192, 32, 32, 16384), 37.5, 41.6),
+            ((8, 2560, 9728, 32, 8, 151936), 313.3, 359.1), ((8, 3072, 8192, 24, 8, 128256), 271.7, 344.6),
+            ((4, 3072, 24576, 24, 24, 32000), 245.4, 238.9), ((6, 3584, 18944, 28, 4, 152064), 431.3, 372.0),
+            ((6, 4096, 4096, 32, 8, 32000), 166.2, 213.3), ((8, 4096, 14336, 32, 8, 128256), 486.9, 461.3),
+            ((6, 4096, 14336, 32, 32, 32000), 336.7, 329.0), ((5, 4608, 12288, 36, 36, 32000), 272.7, 297.6),
+            ((5, 5120, 5120, 40, 8, 32000), 217.1, 241.6), ((4, 5120, 13824, 40, 8, 32000), 296.9, 258.0),
+            ((4, 5120, 13824, 40, 40, 32000), 318.6, 279.2), ((4, 6144, 16384, 48, 8, 32000), 361.1, 291.1),
+            ((4, 8192, 8192, 64, 8, 32000), 358.9, 293.5), ((12, 768, 2048, 12, 12, 32000), 96.6, 238.2),
+            ((8, 896, 4864, 14, 2, 32000), 99.0, 176.5), ((6, 1536, 8960, 12, 2, 32000), 108.9, 167.2),
+            ((5, 2048, 8192, 32, 32, 49152), 130.4, 166.5), ((8, 2048, 8192, 32, 32, 32000), 182.6, 243.7),
+            ((8, 2560, 9728, 64, 16, 16000), 267.9, 324.3), ((8, 4096, 11008, 64, 64, 32000), 467.3, 478.7),
+            ((4, 3200, 8640, 50, 50, 32000), 184.3, 206.1)]
 
 
 def test_the_faster_form_is_taken():

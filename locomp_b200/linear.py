@@ -68,11 +68,12 @@ def fuse_rows(parts: Sequence[Tuple[torch.Tensor, torch.Tensor]], group_size: in
 
 def _one_kernel_pays(layers: int, layer_weights: int, head_weights: int) -> bool:
     """Whether a step is faster as one kernel than as a chain of launches.  The kernel saves about 10 us a layer of launches and
-    hand-overs; its matvecs stream weights more slowly than the decode kernel: about 1 us per 23.5 million weights of a
-    layer and per 35 million of the lm_head.  Kernel and chain in us (replayed CUDA graphs, six back to back): 30 layers of 576 / 1536 185
+    hand-overs; its matvecs stream weights more slowly than the decode kernel: about 1 us per 30 million weights of a
+    layer and per 15 million of the lm_head (short stacks pay more for it: 2 layers of 2560 / 9728 with 151,936 rows 148 and 138, 1 of 1024 / 3072
+    with as many 64 and 60).  Kernel and chain in us (replayed CUDA graphs, six back to back): 30 layers of 576 / 1536 185
     and 484; 24 of 2048 / 8192 503 and 707; 8 of 3072 / 8192 with 128,256 rows of lm_head 272 and 345; 8 of 4096 / 11008 467 and 479; 5 of 4608 / 12288
     273 and 298; 6 of 4096 / 14336 337 and 329; 4 of 5120 / 13824 297 and 258; 6 of 3584 / 18944 with 152,064 rows 431 and 372; 4 of 6144 / 16384 361 and 291."""
-    return layers * (10.0 - layer_weights / 23.5e6) > head_weights / 35e6
+    return layers * (10.0 - layer_weights / 30e6) > head_weights / 15e6
 
 
 class DecodeStack:

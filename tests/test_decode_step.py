@@ -31,7 +31,9 @@ MEASURED = [((1, 64, 64, 1, 1, 64), 14.7, 16.7), ((12, 256, 768, 4, 4, 32000), 8
             ((8, 896, 4864, 14, 2, 32000), 99.0, 176.5), ((6, 1536, 8960, 12, 2, 32000), 108.9, 167.2),
             ((5, 2048, 8192, 32, 32, 49152), 130.4, 166.5), ((8, 2048, 8192, 32, 32, 32000), 182.6, 243.7),
             ((8, 2560, 9728, 64, 16, 16000), 267.9, 324.3), ((8, 4096, 11008, 64, 64, 32000), 467.3, 478.7),
-            ((4, 3200, 8640, 50, 50, 32000), 184.3, 206.1)]
+            ((4, 3200, 8640, 50, 50, 32000), 184.3, 206.1), ((1, 1024, 3072, 16, 8, 151936), 64.1, 60.0),
+            ((2, 2560, 9728, 32, 8, 151936), 148.1, 138.2), ((2, 4096, 4096, 32, 8, 128256), 161.8, 135.1),
+            ((2, 4608, 12288, 36, 36, 16000), 121.2, 131.7), ((3, 5120, 5120, 40, 8, 128256), 248.5, 210.2)]
 
 
 def test_the_faster_form_is_taken():

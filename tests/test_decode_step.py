@@ -45,7 +45,7 @@ def test_the_faster_form_is_taken():
 
 # The edges of the schedule: one CTA with several pieces of the lm_head; rows cut in two and in four; groups that are no multiple of the warps, and
 # rows of whole 128 bytes; one to three layers (o runs two layers ahead); both numbers of warps (640 wide and below, above); no key heads' share
-# in some CTAs; stages that go round the ring often.
+# in some CTAs; long rows of down.
 EDGES = [dict(layers=1, hidden=64, inter=64, q_heads=2, kv_heads=1, vocab=1200), dict(layers=2, hidden=256, inter=64, q_heads=4, kv_heads=2, vocab=2052),
          dict(layers=3, hidden=640, inter=1088, q_heads=1, kv_heads=1, vocab=260), dict(layers=3, hidden=704, inter=768, q_heads=11, kv_heads=1, vocab=516),
          dict(layers=2, hidden=2560, inter=2624, q_heads=40, kv_heads=8, vocab=2564), dict(layers=2, hidden=768, inter=20480, q_heads=12, kv_heads=1, vocab=1000)]

@@ -114,25 +114,24 @@ struct Params {
 struct Sched {
   int S_kr;             // tiles per row block in this k-range
   unsigned T;           // n_rb * S_kr
-  int G;                // CTAs on this k-range (<= T / unit)
-  unsigned unit;        // tiles that are not split: 1, or a row block's
+  unsigned unit, units; // tiles that are not split: 1, or a row block's; how many of these the range has
+  int G;                // CTAs on this k-range (<= units)
 };
 
-__host__ __device__ inline Sched make_sched(const Params& p, int kr) {
+// `whole`: p.whole, or a constant false where only cut row blocks come, for kernels that work it out at every row block.
+__host__ __device__ inline Sched make_sched(const Params& p, int kr, bool whole) {
   Sched s;
   const int left = p.nst - kr * p.S;
   s.S_kr = left < p.S ? left : p.S;
   s.T = static_cast<unsigned>(p.n_rb) * static_cast<unsigned>(s.S_kr);
-  s.unit = p.whole ? static_cast<unsigned>(s.S_kr) : 1u;
-  const unsigned units = p.whole ? static_cast<unsigned>(p.n_rb) : s.T;
-  s.G = static_cast<unsigned>(p.ctas_per_kr) < units ? p.ctas_per_kr : static_cast<int>(units);
+  s.unit = whole ? static_cast<unsigned>(s.S_kr) : 1u;
+  s.units = whole ? static_cast<unsigned>(p.n_rb) : s.T;
+  s.G = static_cast<unsigned>(p.ctas_per_kr) < s.units ? p.ctas_per_kr : static_cast<int>(s.units);
   return s;
 }
-__host__ __device__ inline unsigned tile_begin(const Sched& s, int j) {
-  return (static_cast<unsigned>(j) * (s.T / s.unit)) / static_cast<unsigned>(s.G) * s.unit;
-}
+__host__ __device__ inline unsigned tile_begin(const Sched& s, int j) { return (static_cast<unsigned>(j) * s.units) / static_cast<unsigned>(s.G) * s.unit; }
 __host__ __device__ inline int owner_of(const Sched& s, unsigned t) {
-  return static_cast<int>(((t / s.unit + 1u) * static_cast<unsigned>(s.G) - 1u) / (s.T / s.unit));
+  return static_cast<int>(((t / s.unit + 1u) * static_cast<unsigned>(s.G) - 1u) / s.units);
 }
 // CTAs j0..j1 (inclusive) of this k-range contribute to row block rb.
 __host__ __device__ inline void cover(const Sched& s, int rb, int& j0, int& j1) {
@@ -142,7 +141,7 @@ __host__ __device__ inline void cover(const Sched& s, int rb, int& j0, int& j1) 
 __host__ __device__ inline int contributors(const Params& p, int rb) {
   int total = 0;
   for (int kr = 0; kr < p.n_kr; ++kr) {
-    const Sched s = make_sched(p, kr);
+    const Sched s = make_sched(p, kr, p.whole);
     int j0, j1;
     cover(s, rb, j0, j1);
     total += j1 - j0 + 1;
@@ -381,7 +380,7 @@ template <int MT, int NC>
 __device__ __forceinline__ void flush_row_group(const Params& p, const float (&y)[2][MT][4], int rb, int rg, int g, int t4,
                                              int lane, int seen_lane0, const CtaInfo* info) {
   Sched sch;
-  sch.S_kr = info->S_kr; sch.T = info->T; sch.G = info->G; sch.unit = 1;       // (whole row blocks do not come here)
+  sch.S_kr = info->S_kr; sch.T = sch.units = info->T; sch.G = info->G; sch.unit = 1;       // (whole row blocks do not come here)
   const int kr = info->kr, j = info->j;
   // contributors: identical for every full-length k-range, the last range may differ
   int j0, j1, c_full, c_last;
@@ -390,11 +389,11 @@ __device__ __forceinline__ void flush_row_group(const Params& p, const float (&y
   if (p.n_kr > 1) {
     int a0, a1;
     if (kr == p.n_kr - 1) {
-      const Sched sf = make_sched(p, 0);
+      const Sched sf = make_sched(p, 0, false);
       cover(sf, rb, a0, a1);
       c_full = a1 - a0 + 1;
     } else {
-      const Sched sl = make_sched(p, p.n_kr - 1);
+      const Sched sl = make_sched(p, p.n_kr - 1, false);
       cover(sl, rb, a0, a1);
       c_last = a1 - a0 + 1;
     }
@@ -569,7 +568,7 @@ w4a16_gemv_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     ci.abort = 0;
     ci.kr = blockIdx.x % p.n_kr;
     ci.j = blockIdx.x / p.n_kr;
-    const Sched sch = make_sched(p, ci.kr);
+    const Sched sch = make_sched(p, ci.kr, !CL && p.whole);
     ci.leave = ci.j >= sch.G;
     ci.S_kr = sch.S_kr; ci.T = sch.T; ci.G = sch.G;
     ci.t0 = 0; ci.n_tiles = 0; ci.rb0 = 0; ci.ks0 = 0; ci.pad = 0;
@@ -1092,7 +1091,7 @@ inline Plan make_plan(int M, int N, int K, int sm_count) {
   // the last (shorter) range has its own, smaller T -- bound with the worst of the two
   int max_split = 1;
   for (int kr = 0; kr < p.n_kr; ++kr) {
-    const Sched s = make_sched(p, kr);
+    const Sched s = make_sched(p, kr, p.whole);
     const long long min_tiles = s.T / s.G;
     const int b = static_cast<int>(s.S_kr / (min_tiles > 0 ? min_tiles : 1)) + 2;
     if (b > max_split) max_split = b;

@@ -399,7 +399,7 @@ int lcq_gemv_tc_plan_check(int M, int N, int K, int sm_count, int* fields) {
   std::vector<int> slot_used(static_cast<size_t>(p.n_rb) * p.n_kr * p.max_split, 0);
   for (int b = 0; b < pl.grid; ++b) {
     const int kr = b % p.n_kr, j = b / p.n_kr;
-    const gemv_tc::Sched s = gemv_tc::make_sched(p, kr);
+    const gemv_tc::Sched s = gemv_tc::make_sched(p, kr, p.whole);
     if (j >= s.G) continue;
     const long long t0 = gemv_tc::tile_begin(s, j), t1 = gemv_tc::tile_begin(s, j + 1);
     if (!pl.fits_32bit) { set_error("plan check: schedule does not fit 32 bits"); return LCQ_ERR_UNSUPPORTED; }

@@ -1076,15 +1076,18 @@ inline Plan make_plan(int M, int N, int K, int sm_count) {
     if (want < p.ctas_per_kr) p.ctas_per_kr = static_cast<int>(want);
   }
   // Whole row blocks where they leave no CTA with much more than its equal share: no scratch, no counters, and the tail of a
-  // row block that two CTAs share (a round trip to L2 under full load) costs as much as three to four tiles.  us a call, cut / whole, 400 calls back to
-  // back in a CUDA graph over weights that together exceed L2 (in parentheses tiles of the busiest CTA): M = 1 512 -> 49152 8.0 / 5.8 (2.6, 4),
-  // 2048 -> 32000 13.0 / 8.9 (6.8, 8), 4096 -> 28672 17.2 / 15.4 (12.1, 16), 1536 -> 49152 12.7 / 12.1 (7.8, 12), 2048 -> 49152 14.5 / 15.1 (10.4, 16),
-  // 4096 -> 40000 20.3 / 25.2 (16.9, 32); M = 3 576 -> 49152 9.8 / 8.6; M = 16 512 -> 49152 12.3 / 9.7 (5.2, 6), 2048 -> 49152 23.1 / 22.6 (20.8, 24),
-  // 2048 -> 20000 13.9 / 16.1 (8.5, 16).
+  // row block that two CTAs share (a round trip to L2 under full load) costs as much as some tiles.  How many: us a call, cut / whole, 200 to 400 calls
+  // back to back in a CUDA graph over weights that together exceed L2 (in parentheses the tiles of the busiest CTA beyond its equal share).  M <= 8:
+  // 512 -> 49152 8.0 / 5.8 (1.4), 2560 -> 25309 12.9 / 11.1 (3.3), 4096 -> 28672 17.2 / 15.4 (3.9), 1536 -> 49152 12.7 / 12.1 (4.2), 1280 -> 116937
+  // 20.9 / 21.5 (4.6), 2048 -> 49152 14.5 / 15.1 (5.6).  M > 8: 512 -> 49152 12.3 / 9.7 (0.8), 2048 -> 49152 23.1 / 22.6 (3.2), 1536 -> 63430 22.9 / 23.2 (3.9),
+  // 2048 -> 20000 13.9 / 16.1 (7.5).  Less where a tile's scales come in 4-byte pieces: M <= 8 576 -> 49152 9.8 / 8.6 (2.1), 576 -> 122741 15.1 / 15.8 (2.3),
+  // 2624 -> 64986 26.1 / 27.4 (3.1), M > 8 1472 -> 30310 16.2 / 15.8 (2.4), 1984 -> 49268 27.1 / 28.9 (3.2); but not with one row block a CTA, 3200 -> 27130 17.1 / 16.2 (3.7).
+  // More where an equal share is six tiles or less: 1280 -> 42092 13.6 / 12.4 (4.4), 832 -> 45728 11.1 / 10.6 (3.2), M > 8 2112 -> 10550 13.2 / 11.4 (4.0).
   if (!pl.cluster && p.n_kr == 1) {
     const int ctas = p.ctas_per_kr < p.n_rb ? p.ctas_per_kr : p.n_rb;
     const long long most = static_cast<long long>((p.n_rb + ctas - 1) / ctas) * p.S;
-    p.whole = 16 * most * p.ctas_per_kr <= 17 * T + 64LL * p.ctas_per_kr;
+    const int quarters = (pl.ragged && p.n_rb > ctas ? (pl.MT == 1 ? 9 : 10) : (pl.MT == 1 ? 17 : 14)) + (T <= 6LL * p.ctas_per_kr ? 6 : 0);
+    p.whole = 4 * (most * p.ctas_per_kr - T) <= static_cast<long long>(quarters) * p.ctas_per_kr;
     if (p.whole) p.ctas_per_kr = ctas;
   }
   // a row block of S tiles can straddle at most S / min_tiles_per_cta + 2 CTAs of a k-range;

@@ -47,9 +47,9 @@
 namespace lcq {
 namespace step {
 
-// Two sets of SET consumer warps, and the producer; U groups of 32 columns of a warp's share of a stage at a time.
+// Two sets of SET consumer warps, and the producer; of a warp's share of a stage U groups of 32 columns at a time.
 template <int SET> struct Threads {
-  static constexpr int NCW = 2 * SET, NCT = NCW * 32, SET_T = SET * 32, ALL = NCT + 32, U = SET == 4 ? 5 : 3;
+  static constexpr int NCW = 2 * SET, NCT = NCW * 32, SET_T = SET * 32, ALL = NCT + 32;
 };
 constexpr int MAX_STAGES = 32;
 enum { BAR_ALL = 1, BAR_SUMS, BAR_SET0, BAR_SET1 };   // named barriers: all consumers; a phase's sums are there; those of a set
@@ -322,9 +322,8 @@ __device__ __forceinline__ void describe(const Part& q, PartInfo& info, int lane
 // another group of the eight, g further on, so that the eight rows that a quarter of the A operand takes sit in different banks.  Column g of the B
 // operand is x at the group that row g takes (and row g + 8), so the sums of both are in column g of the result.
 // What does not need x -- waiting for the stage, fetching up to U groups of weights -- is done before x is there (fetch).
-template <int SET>
+template <int SET, int U>
 struct Matvec {
-  static constexpr int U = Threads<SET>::U;
   int q, end, step;                            // the set's next stage, counted over the whole stream; the end of its stages, their distance
   int i;                                       // its place in the ring
   uint32_t phase;
@@ -447,7 +446,7 @@ struct Poll {
   }
 };
 
-template <int SET>
+template <int SET, int U>
 __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const __grid_constant__ Params p) {
   constexpr int NCW = Threads<SET>::NCW, NCT = Threads<SET>::NCT, SET_T = Threads<SET>::SET_T;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -667,7 +666,7 @@ __global__ void __launch_bounds__(Threads<SET>::ALL, 1) decode_step_kernel(const
       const int n = to.count(mine.stages, p.part);
       const uint32_t sums = part == PART_QKV ? sums_s : part == PART_O ? sums_s + min2(mine.stages[PART_QKV], p.part[PART_QKV].piece) * STAGE_SUMS : sums_c;
       const int v = p.part[part].v, r0 = to.done * p.part[part].per, rows = min2(mine.rows[part] - r0, n * p.part[part].per);       // rows of this piece
-      Matvec<SET> m;
+      Matvec<SET, U> m;
       m.begin(p, base + L.info + part * PART_INFO_BYTES, n, to.first(), to.step(), pos, turn);
       if (m.q < m.end) m.fetch(p, base, issued, dead, flag_abort);
       const uint32_t sums_q = sums - static_cast<uint32_t>(pos) * STAGE_SUMS;
@@ -826,6 +825,23 @@ inline Part make_part(int K, int rows, bool paired, int whole_row, int max_bytes
 // 8 of 1024 / 3072 with 151,936 rows 129 / 118, 5 of 2048 / 8192 201 / 130.
 inline bool narrow(const Params& p) { return p.sh.hidden <= 640; }
 
+// Groups that a warp of eight takes at a time: two or three, whichever leaves fewer empty places in the stages of the stack.  A round costs
+// as much as its groups and 0.85 of one more.  us a step with two / three: 8 layers of 2560 / 9728 (10 groups a warp and stage) 303 / 314, 5 of
+// 5120 / 5120 (10) 210 / 218, 8 of 1024 / 3072 with 151,936 rows (4) 107 / 119; 5 of 4608 / 12288 (9) 308 / 274, 6 of 1536 / 8960 (6) 117 / 109.
+inline int round_of(const Params& p) {
+  if (narrow(p)) return 5;
+  const int rows[N_PARTS] = {p.sh.hidden, p.sh.inter, p.sh.qkv, p.sh.hidden, p.sh.vocab};
+  long long cost[2] = {0, 0};
+  for (int i = 0; i < N_PARTS; ++i) {
+    const Part& q = p.part[i];
+    const int stages = stages_of(q, max_share(rows[i], p.ctas)), units = (q.groups + 7) / 8;
+    const long long turns = static_cast<long long>(i == PART_O || i == PART_QKV ? stages : (stages + 1) / 2) * (i == PART_HEAD ? 1 : p.n_layers);      // (a set's)
+    cost[0] += turns * ((units + 1) / 2) * (40 + 17);
+    cost[1] += turns * ((units + 2) / 3) * (60 + 17);
+  }
+  return cost[0] < cost[1] ? 2 : 3;
+}
+
 inline bool make_plan(const lcq_decode_stack& d, int sm_count, Plan& pl) {
   const int H = d.hidden, I = d.inter;
   if (d.n_layers < 1 || H < 64 || I < 64 || d.qkv < 4 || d.q_dim < 64 || d.vocab < 4 || d.n_layers > 256) return false;
@@ -891,15 +907,16 @@ inline int launch(const lcq_decode_stack& d, int sm_count, cudaStream_t stream) 
   int dev = 0;
   LCQ_CUDA_TRY(cudaGetDevice(&dev));
   if (configured_device != dev) {
-    LCQ_CUDA_TRY(cudaFuncSetAttribute(decode_step_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    LCQ_CUDA_TRY(cudaFuncSetAttribute(decode_step_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    LCQ_CUDA_TRY(cudaFuncSetAttribute(decode_step_kernel<4, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    LCQ_CUDA_TRY(cudaFuncSetAttribute(decode_step_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    LCQ_CUDA_TRY(cudaFuncSetAttribute(decode_step_kernel<8, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     configured_device = dev;
   }
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(p.ctas);
-  const bool four = narrow(p);
-  cfg.blockDim = dim3(four ? Threads<4>::ALL : Threads<8>::ALL);
+  const int round = round_of(p);
+  cfg.blockDim = dim3(round == 5 ? Threads<4>::ALL : Threads<8>::ALL);
   cfg.dynamicSmemBytes = pl.smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -907,7 +924,7 @@ inline int launch(const lcq_decode_stack& d, int sm_count, cudaStream_t stream) 
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, four ? decode_step_kernel<4> : decode_step_kernel<8>, p));
+  LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, round == 5 ? decode_step_kernel<4, 5> : round == 2 ? decode_step_kernel<8, 2> : decode_step_kernel<8, 3>, p));
   return LCQ_OK;
 }
 

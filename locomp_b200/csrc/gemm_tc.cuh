@@ -73,23 +73,48 @@ template <int CG> __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, u
   if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
   else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem descriptor].  Called by a whole warp, issued by one elected lane: with
-// every operand uniform over the warp the compiler keeps them in uniform registers, where the
-// instruction wants them.  From a branch that one lane takes alone they are moved there one by one,
-// and an MMA takes ~80 clocks to issue whatever its size (M = 64 on 8192 -> 28672: 55.6 us, this way 48.2).
-template <int CG> __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  if (CG == 2) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
-        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-  }
+// D[tmem] (+)= A[tmem] * B[smem descriptor] for 64 k: four MMAs.  Called by a whole warp, issued by one elected
+// lane: with every operand uniform over the warp the compiler keeps them in uniform registers, where the
+// instruction wants them.  `b`: the low word of the descriptor (its start address); `first`: 0 overwrites D.
+#define LCQ_MMA(CG, A, B, P) \
+  "mov.b64 bd, {" B ", %5};\n\ttcgen05.mma.cta_group::" #CG ".kind::f16 [%0], [" A "], bd, %3, " P ";\n\t"
+#define LCQ_MMA_STEP(CG, K, P0) \
+  "add.u32 a1, a" #K ", 8;\n\tadd.u32 a2, a" #K ", 16;\n\tadd.u32 a3, a" #K ", 24;\n\t" \
+  "add.u32 b1, b" #K ", 2;\n\tadd.u32 b2, b" #K ", 4;\n\tadd.u32 b3, b" #K ", 6;\n\t" \
+  LCQ_MMA(CG, "a" #K, "b" #K, P0) LCQ_MMA(CG, "a1", "b1", "q") LCQ_MMA(CG, "a2", "b2", "q") LCQ_MMA(CG, "a3", "b3", "q")
+#define LCQ_MMA_BEGIN \
+  "{\n\t.reg .pred p, q, e;\n\t.reg .b64 bd;\n\t.reg .b32 a0, a1, a2, a3, a4, a8, a12, b0, b1, b2, b3, b4, b8, b12;\n\t" \
+  "elect.sync _|e, 0xffffffff;\n\t@!e bra ISSUED;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 q, 0, 0;\n\t" \
+  "mov.b32 a0, %1;\n\tmov.b32 b0, %2;\n\t"
+#define LCQ_MMA_END "ISSUED:\n\t}"
+// High word of the descriptor: 1024 bytes between 8-row groups, descriptor version (sm_100), 128-byte swizzle.
+constexpr uint32_t B_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+template <int CG> __device__ __forceinline__ void umma_step(uint32_t d_tmem, uint32_t a_tmem, uint32_t b, uint32_t idesc, uint32_t first) {
+  if (CG == 2)
+    asm volatile(LCQ_MMA_BEGIN LCQ_MMA_STEP(2, 0, "p") LCQ_MMA_END ::"r"(d_tmem), "r"(a_tmem), "r"(b), "r"(idesc), "r"(first), "n"(B_DESC_HI) : "memory");
+  else
+    asm volatile(LCQ_MMA_BEGIN LCQ_MMA_STEP(1, 0, "p") LCQ_MMA_END ::"r"(d_tmem), "r"(a_tmem), "r"(b), "r"(idesc), "r"(first), "n"(B_DESC_HI) : "memory");
 }
+// The same for a whole stage of 256 k (`step`: descriptor units between 64-k steps).  One election and one branch for
+// sixteen MMAs: the issuing warp shares its scheduler with four dequant warps, and what it can issue bounds tiles of
+// few rows.  Clocks per MMA beside four busy warps on the scheduler, N <= 64: an election per MMA in a loop over
+// the steps 168, all sixteen unrolled 61, one election for four 63, one for all with predicated MMAs 52, with a branch 45.
+template <int CG> __device__ __forceinline__ void umma_stage(uint32_t d_tmem, uint32_t a_tmem, uint32_t b, uint32_t step, uint32_t idesc, uint32_t first) {
+#define LCQ_MMA_STAGE(G)                                                                                                     \
+  LCQ_MMA_BEGIN                                                                                                              \
+  "add.u32 a4, %1, 32;\n\tadd.u32 a8, %1, 64;\n\tadd.u32 a12, %1, 96;\n\t"                                                   \
+  "add.u32 b4, %2, %6;\n\tadd.u32 b8, b4, %6;\n\tadd.u32 b12, b8, %6;\n\t"                                                   \
+  LCQ_MMA_STEP(G, 0, "p") LCQ_MMA_STEP(G, 4, "q") LCQ_MMA_STEP(G, 8, "q") LCQ_MMA_STEP(G, 12, "q") LCQ_MMA_END
+  if (CG == 2)
+    asm volatile(LCQ_MMA_STAGE(2) ::"r"(d_tmem), "r"(a_tmem), "r"(b), "r"(idesc), "r"(first), "n"(B_DESC_HI), "r"(step) : "memory");
+  else
+    asm volatile(LCQ_MMA_STAGE(1) ::"r"(d_tmem), "r"(a_tmem), "r"(b), "r"(idesc), "r"(first), "n"(B_DESC_HI), "r"(step) : "memory");
+#undef LCQ_MMA_STAGE
+}
+#undef LCQ_MMA
+#undef LCQ_MMA_STEP
+#undef LCQ_MMA_BEGIN
+#undef LCQ_MMA_END
 // Arrives on this barrier (CG = 2: and on its counterpart in the other CTA) once the MMAs issued so far
 // have completed.  Whole warp, like the MMAs: the same lane is elected.
 template <int CG> __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -136,17 +161,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
       : "r"(taddr) : "memory");
 }
 
-// Shared-memory matrix descriptor: K-major tile of 128-byte rows, 128-byte swizzle,
-// 1024 bytes between 8-row groups.
-__device__ __forceinline__ uint64_t make_b_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);   // start address
-  d |= static_cast<uint64_t>(1) << 16;                        // leading byte offset (unused for swizzled K-major)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;                // stride byte offset
-  d |= static_cast<uint64_t>(1) << 46;                        // descriptor version (sm_100)
-  d |= static_cast<uint64_t>(2) << 61;                        // 128-byte swizzle
-  return d;
-}
+// Low word of the shared-memory matrix descriptor of a K-major tile of 128-byte rows, 128-byte swizzle, 1024 bytes
+// between 8-row groups: the start address, and a leading byte offset that is not used for swizzled K-major tiles.
+__device__ __forceinline__ uint32_t make_b_desc(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
 // The N of a kind::f16 MMA is a multiple of this.  For the pair form (M = 256) it is 32 that is specified; 48, 80 and 112 gave the
 // right results, and are not used.
 __host__ __device__ constexpr int mma_n_step(int cg) { return 16 * cg; }
@@ -570,15 +587,15 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   } else if (warp == WARP_MMA) {
     // ------------------------------------------------------------ MMA issuer: one warp for the team
     if (crank == 0) {
-      const uint64_t desc0 = make_b_desc(smem_u32(smem));                                 // descriptors count 16-byte units
-      const uint64_t desc_stage = static_cast<uint64_t>(x_stage_bytes(p.bm, CG) >> 4);
+      const uint32_t desc0 = make_b_desc(smem_u32(smem));                                 // descriptors count 16-byte units
+      const uint32_t desc_stage = static_cast<uint32_t>(x_stage_bytes(p.bm, CG) >> 4);
       Ring rx = {0, 0}, ra = {0, 0}, rd = {0, 0};
       bool ok = true;
       for (Walk w(p, team); ok && w.next(p); rd.step(p.nd)) {
         if (!warp_wait(flag_abort, &empty_d[rd.i], rd.phase ^ 1u)) { if (lane == 0) LCQ_GIVE_UP(12); ok = false; break; }
         tc_fence_after();
         const uint32_t idesc = make_idesc(w.bm, CG);
-        const uint64_t desc_step = static_cast<uint64_t>(x_step_bytes(w.bm, CG) >> 4);
+        const uint32_t desc_step = static_cast<uint32_t>(x_step_bytes(w.bm, CG) >> 4);
         const uint32_t d_t = tmem_base + rd.i * p.bm;
         uint32_t acc = 0;
         for (int i = TERMS * w.st0; i < TERMS * w.st1; ++i, ra.step(p.nas)) {
@@ -590,15 +607,11 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             break;
           }
           tc_fence_after();
-          uint64_t bdesc = desc0 + rx.i * desc_stage;
-          uint32_t a_t = a_base + ra.i * A_SLOT_COLS;
-          for (int k = 0; k < steps; ++k, bdesc += desc_step, a_t += A_STEP_COLS) {
-#pragma unroll
-            for (int j = 0; j < BK / 16; ++j) {
-              umma_ts<CG>(d_t, a_t + j * 8, bdesc + static_cast<uint64_t>(2 * j), idesc, acc);
-              acc = 1;
-            }
-          }
+          const uint32_t bdesc = desc0 + rx.i * desc_stage, a_t = a_base + ra.i * A_SLOT_COLS;
+          if (!RAGGED || steps == WK / BK) umma_stage<CG>(d_t, a_t, bdesc, desc_step, idesc, acc);
+          else
+            for (int k = 0; k < steps; ++k) umma_step<CG>(d_t, a_t + k * A_STEP_COLS, bdesc + k * desc_step, idesc, k == 0 ? acc : 1u);
+          acc = 1;
           if (TERMS == 1 || (i & 1)) {
             umma_commit<CG>(&empty_x[rx.i]);
             rx.step(p.nxs);

@@ -6,9 +6,15 @@
 // Because K % G == 0, the scale of flat element e = r*K + k is scales_flat[e / G], so the
 // fast paths index everything flat and never need the row.
 //
-// HBM-bound (write dominated: 4 B out per 0.5 B in for f32).  The fast int4 path reads one
-// 32-bit word per lane (128 B per warp, coalesced), redistributes nibbles with two warp
-// shuffles so that every store instruction writes 32 x 16 B = 512 contiguous bytes.
+// HBM-bound (write dominated: 4 B out per 0.5 B in for f32).  The fast path gives a thread whole octets of weights: one word
+// (int4) or two (int8) in, one scale, and one store of 32 bytes (f32) or 16 (16-bit outputs).
+//
+// What it measured (4096 x 14336, us a call among others over three weights; floor 41.1 for int4 -> f32 at 6525 GB/s): int4 -> f32 49.0
+// before, 41.4 now, -> f16 32.7 / 27.0; int8 -> f32 56.1 / 46.3, -> f16 41.5 / 28.9.  Before: one wave of blocks that looped, int4
+// words spread over the lanes by shuffles to get 16-byte stores, int8 one word a thread.  What gave it: blocks that end
+// after one round of loads and stores instead of looping (a loop's next loads wait behind its stores; 53 -> 43 in a kernel by
+// itself), fp16 scales converted only after all loads are issued (33.6 -> 27.0 for f16 outputs), and a launch whose blocks are
+// there when the kernel before ends (-2).  Octets a thread: f32 1 / 2 / 4 46.5 / 41.6 / 41.6, f16 1 / 2 / 4 39.2 / 29.4 / 27.0.
 #pragma once
 #include "common.cuh"
 
@@ -40,9 +46,21 @@ __device__ __forceinline__ long long scale_index(long long e, int G, int gshift)
   return gshift >= 0 ? (e >> gshift) : (e / G);
 }
 
-template <typename OT> struct Out8;   // 8 consecutive 16-bit outputs, one 16-byte store
+// 8 consecutive outputs: one 16-byte store of 16-bit values, one of 32 bytes of float32 values (or, where out is on 16 bytes only, two of 16).
+template <typename OT> struct Out8;
+template <> struct Out8<float> {
+  static __device__ __forceinline__ void store(float* p, const float (&f)[8], bool on_32) {
+    if (on_32) {
+      asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                   ::"l"(p), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]), "f"(f[4]), "f"(f[5]), "f"(f[6]), "f"(f[7]) : "memory");
+    } else {
+      Out4<float>::store(p, f[0], f[1], f[2], f[3]);
+      Out4<float>::store(p + 4, f[4], f[5], f[6], f[7]);
+    }
+  }
+};
 template <> struct Out8<__half> {
-  static __device__ __forceinline__ void store(__half* p, const float (&f)[8]) {
+  static __device__ __forceinline__ void store(__half* p, const float (&f)[8], bool) {
     __half2 h[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
@@ -50,7 +68,7 @@ template <> struct Out8<__half> {
   }
 };
 template <> struct Out8<__nv_bfloat16> {
-  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&f)[8]) {
+  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&f)[8], bool) {
     __nv_bfloat162 h[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
@@ -58,73 +76,63 @@ template <> struct Out8<__nv_bfloat16> {
   }
 };
 
-template <> struct Out8<float> {
-  static __device__ __forceinline__ void store(float*, const float (&)[8]) {}   // never taken: float32 goes through Out4
+// float(int8) for the 4 bytes of a word without conversion instructions.
+__device__ __forceinline__ void int8x4_to_f32(uint32_t v, float* f) {
+  v ^= 0x80808080u;  // bias to unsigned: b + 128
+  f[0] = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7540)) - 8388736.0f;
+  f[1] = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7541)) - 8388736.0f;
+  f[2] = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7542)) - 8388736.0f;
+  f[3] = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7543)) - 8388736.0f;
+}
+
+// The 8 weights of an octet as they are stored: one word (int4), two (int8).
+template <int WBITS> struct Octet;
+template <> struct Octet<4> {
+  uint32_t v;
+  __device__ __forceinline__ void load(const void* w, long long i) { v = __ldg(static_cast<const uint32_t*>(w) + i); }
+  __device__ __forceinline__ void scaled(float s, float (&f)[8]) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = (small_uint_to_f32((v >> (4 * i)) & 15u) - 8.0f) * s;
+  }
+};
+template <> struct Octet<8> {
+  uint2 v;
+  __device__ __forceinline__ void load(const void* w, long long i) { v = __ldg(static_cast<const uint2*>(w) + i); }
+  __device__ __forceinline__ void scaled(float s, float (&f)[8]) const {
+    int8x4_to_f32(v.x, f);
+    int8x4_to_f32(v.y, f + 4);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] *= s;
+  }
 };
 
-// Independent 128-byte warp loads in flight per warp, as measured best on a 4096 x 14336 weight:
-// int4 -> f32 4, int4 -> 16-bit 2, int8 1 (more only costs registers, hence resident blocks).
-template <typename OT> __host__ __device__ constexpr int dq4_unroll() { return sizeof(OT) == 4 ? 4 : 2; }
-constexpr int DQ8_UNROLL = 1;
-
-// ---- int4 fast path: K % 8 == 0, G % 8 == 0, w 4-byte aligned, out 16-byte aligned.
-// total_words = N*K/8.  A warp iteration covers dq4_unroll<OT>() blocks of 32 words (256 weights each): all
-// loads of weights and scales are issued before the first store.  float32 output: two shuffles hand
-// every lane 4 consecutive weights per store, so a store instruction writes 512 contiguous bytes.
-// 16-bit output: a lane's own word is 8 outputs = 16 bytes, contiguous across the warp as it is.
-template <typename ST, typename OT>
-__global__ void __launch_bounds__(256) dequant_w4_words_kernel(const uint32_t* __restrict__ w,
-                                                               const ST* __restrict__ scales,
-                                                               OT* __restrict__ out,
-                                                               long long total_words, int G, int gshift) {
-  constexpr bool WIDE = sizeof(OT) == 4;
-  constexpr int DQ_UNROLL = dq4_unroll<OT>();
-  constexpr int NS = WIDE ? 2 : 1;              // stores (and scales) per lane and block
-  const int lane = threadIdx.x & 31;
-  const long long warp_id = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long n_warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
-  const long long n_blocks = (total_words + 31) >> 5;
-  for (long long it = warp_id * DQ_UNROLL; it < n_blocks; it += n_warps * DQ_UNROLL) {
-    uint32_t word[DQ_UNROLL];
-    float sc[DQ_UNROLL][NS];
+// ---- fast path: K % 8 == 0, G % 8 == 0, w on the size of an octet and out on 16 bytes.  A thread has dq_unroll<OT>() octets, a block's
+// width apart, and loads all of them and their scales before its first conversion.  (The loop is for more octets than a grid has
+// threads; ordinary sizes take one round.)
+template <typename OT> __host__ __device__ constexpr int dq_unroll() { return sizeof(OT) == 4 ? 2 : 4; }
+template <int WBITS, typename ST, typename OT>
+__global__ void __launch_bounds__(256) dequant_octets_kernel(const void* __restrict__ w, const ST* __restrict__ scales, OT* __restrict__ out,
+                                                             long long octets, int G, int gshift, bool on_32) {
+  constexpr int U = dq_unroll<OT>();
+  griddep_wait();                              // (and no early start for the next kernel: the outputs may be a linear layer's scales)
+  for (long long i0 = static_cast<long long>(blockIdx.x) * (256 * U) + threadIdx.x; i0 < octets; i0 += static_cast<long long>(gridDim.x) * (256 * U)) {
+    Octet<WBITS> q[U];
+    ST s[U];
 #pragma unroll
-    for (int u = 0; u < DQ_UNROLL; ++u) {
-      const long long wi = ((it + u) << 5) + lane;
-      word[u] = (wi < total_words) ? __ldg(w + wi) : 0u;
-#pragma unroll
-      for (int j = 0; j < NS; ++j) {
-        // WIDE: store j of lane l covers half (l & 1) of word 16j + l/2 of the block; else the lane's own word
-        const long long src_word = WIDE ? (((it + u) << 5) + 16 * j + (lane >> 1)) : wi;
-        const long long e0 = src_word * 8 + (WIDE ? 4 * (lane & 1) : 0);
-        sc[u][j] = (src_word < total_words) ? to_f32<ST>(__ldg(scales + scale_index(e0, G, gshift))) : 0.0f;
+    for (int u = 0; u < U; ++u) {
+      const long long i = i0 + u * 256;
+      if (i < octets) {
+        q[u].load(w, i);
+        s[u] = __ldg(scales + scale_index(i * 8, G, gshift));
       }
     }
 #pragma unroll
-    for (int u = 0; u < DQ_UNROLL; ++u) {
-      if (WIDE) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const uint32_t wj = __shfl_sync(0xffffffffu, word[u], 16 * j + (lane >> 1));
-          const long long src_word = ((it + u) << 5) + 16 * j + (lane >> 1);
-          if (src_word < total_words) {
-            const uint32_t nib = (wj >> (16 * (lane & 1))) & 0xFFFFu;
-            const long long e0 = src_word * 8 + 4 * (lane & 1);
-            const float s = sc[u][j];
-            const float f0 = (small_uint_to_f32(nib & 15u) - 8.0f) * s;
-            const float f1 = (small_uint_to_f32((nib >> 4) & 15u) - 8.0f) * s;
-            const float f2 = (small_uint_to_f32((nib >> 8) & 15u) - 8.0f) * s;
-            const float f3 = (small_uint_to_f32((nib >> 12) & 15u) - 8.0f) * s;
-            Out4<OT>::store(out + e0, f0, f1, f2, f3);
-          }
-        }
-      } else {
-        const long long wi = ((it + u) << 5) + lane;
-        if (wi < total_words) {
-          float f[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) f[i] = (small_uint_to_f32((word[u] >> (4 * i)) & 15u) - 8.0f) * sc[u][0];
-          Out8<OT>::store(out + wi * 8, f);
-        }
+    for (int u = 0; u < U; ++u) {
+      const long long i = i0 + u * 256;
+      if (i < octets) {
+        float f[8];
+        q[u].scaled(to_f32<ST>(s[u]), f);
+        Out8<OT>::store(out + i * 8, f, on_32);
       }
     }
   }
@@ -150,42 +158,18 @@ __global__ void __launch_bounds__(256) dequant_w4_bytes_kernel(const uint8_t* __
   }
 }
 
-// float(int8) for the 4 bytes of a word without conversion instructions.
-__device__ __forceinline__ void int8x4_to_f32(uint32_t v, float (&f)[4]) {
-  v ^= 0x80808080u;  // bias to unsigned: b + 128
-  f[0] = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7540)) - 8388736.0f;
-  f[1] = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7541)) - 8388736.0f;
-  f[2] = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7542)) - 8388736.0f;
-  f[3] = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7543)) - 8388736.0f;
-}
-
-// ---- int8 fast path: K % 4 == 0, G % 4 == 0; one 32-bit word (4 weights) per thread and load,
-// DQ8_UNROLL loads in flight.
+// ---- int8, K % 4 == 0, G % 4 == 0: one 32-bit word (4 weights) per thread and load.
 template <typename ST, typename OT>
 __global__ void __launch_bounds__(256) dequant_w8_words_kernel(const uint32_t* __restrict__ w,
                                                                const ST* __restrict__ scales,
                                                                OT* __restrict__ out,
                                                                long long total_words, int G, int gshift) {
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  for (long long i0 = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < total_words; i0 += stride * DQ8_UNROLL) {
-    uint32_t word[DQ8_UNROLL];
-    float sc[DQ8_UNROLL];
-#pragma unroll
-    for (int u = 0; u < DQ8_UNROLL; ++u) {
-      const long long i = i0 + u * stride;
-      const bool ok = i < total_words;
-      word[u] = ok ? __ldg(w + i) : 0u;
-      sc[u] = ok ? to_f32<ST>(__ldg(scales + scale_index(i * 4, G, gshift))) : 0.0f;
-    }
-#pragma unroll
-    for (int u = 0; u < DQ8_UNROLL; ++u) {
-      const long long i = i0 + u * stride;
-      if (i < total_words) {
-        float f[4];
-        int8x4_to_f32(word[u], f);
-        Out4<OT>::store(out + i * 4, f[0] * sc[u], f[1] * sc[u], f[2] * sc[u], f[3] * sc[u]);
-      }
-    }
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total_words; i += stride) {
+    const float s = to_f32<ST>(__ldg(scales + scale_index(i * 4, G, gshift)));
+    float f[4];
+    int8x4_to_f32(__ldg(w + i), f);
+    Out4<OT>::store(out + i * 4, f[0] * s, f[1] * s, f[2] * s, f[3] * s);
   }
 }
 
@@ -229,26 +213,23 @@ int launch_dequant(int wbits, const void* w, const void* scales, void* out, long
   const size_t out_vec_align = 4 * sizeof(OT);
   int gshift = -1;
   if (G > 0 && (G & (G - 1)) == 0) { gshift = 0; while ((1 << gshift) < G) ++gshift; }
-  if (wbits == 4) {
-    const bool fast = (K % 8 == 0) && (G % 8 == 0) && aligned(w, 4) && aligned(out, 16);
-    if (fast) {
-      const long long words = total / 8;
-      // 8 warps per block, each taking dq4_unroll<OT>() blocks of 32 words per iteration
-      const int grid = one_wave_grid<dequant_w4_words_kernel<ST, OT>>((words + 31) / 32, 8 * dq4_unroll<OT>(), sm_count);
-      dequant_w4_words_kernel<ST, OT><<<grid, 256, 0, stream>>>(
-          static_cast<const uint32_t*>(w), static_cast<const ST*>(scales), static_cast<OT*>(out), words, G, gshift);
-    } else {
-      const long long bytes = total / 2;
-      const int grid = one_wave_grid<dequant_w4_bytes_kernel<ST, OT>>(bytes, 256, sm_count);
-      dequant_w4_bytes_kernel<ST, OT><<<grid, 256, 0, stream>>>(
-          static_cast<const uint8_t*>(w), static_cast<const ST*>(scales), static_cast<OT*>(out), bytes,
-          static_cast<int>(K), G);
-    }
+  if (K % 8 == 0 && G % 8 == 0 && aligned(w, wbits) && aligned(out, 16)) {
+    const long long octets = total / 8, per_block = 256 * dq_unroll<OT>(), need = (octets + per_block - 1) / per_block;
+    const int grid = static_cast<int>(need < (1 << 30) ? need : (1 << 30));
+    auto kern = wbits == 4 ? dequant_octets_kernel<4, ST, OT> : dequant_octets_kernel<8, ST, OT>;
+    const WaitingLaunch launch(grid, 256, stream);
+    LCQ_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, kern, w, static_cast<const ST*>(scales), static_cast<OT*>(out), octets, G, gshift, aligned(out, 32)));
+  } else if (wbits == 4) {
+    const long long bytes = total / 2;
+    const int grid = one_wave_grid<dequant_w4_bytes_kernel<ST, OT>>(bytes, 256, sm_count);
+    dequant_w4_bytes_kernel<ST, OT><<<grid, 256, 0, stream>>>(
+        static_cast<const uint8_t*>(w), static_cast<const ST*>(scales), static_cast<OT*>(out), bytes,
+        static_cast<int>(K), G);
   } else {
     const bool fast = (K % 4 == 0) && (G % 4 == 0) && aligned(w, 4) && aligned(out, out_vec_align);
     if (fast) {
       const long long words = total / 4;
-      const int grid = one_wave_grid<dequant_w8_words_kernel<ST, OT>>(words, 256 * DQ8_UNROLL, sm_count);
+      const int grid = one_wave_grid<dequant_w8_words_kernel<ST, OT>>(words, 256, sm_count);
       dequant_w8_words_kernel<ST, OT><<<grid, 256, 0, stream>>>(
           static_cast<const uint32_t*>(w), static_cast<const ST*>(scales), static_cast<OT*>(out), words, G, gshift);
     } else {

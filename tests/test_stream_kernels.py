@@ -1,0 +1,73 @@
+"""The dequantisers and quantisers at the edges of their fast paths: one octet, a block's octets and one more or less, several blocks, groups that
+are no power of two, and every alignment that the entry points take.  Bit for bit the oracle's results, as the operations are exact or
+rounded once."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import locomp_b200 as L
+from locomp_b200 import _lib
+from oracle import qmm_oracle as O
+
+pytestmark = pytest.mark.gpu
+KINDS = {"f32": (torch.float32, _lib.F32), "f16": (torch.float16, _lib.F16), "bf16": (torch.bfloat16, _lib.BF16)}
+SHAPES = [(1, 8, 8), (1, 32, 32), (3, 24, 24), (2, 4096, 32), (1, 4104, 8), (1, 8184, 24), (5, 8192, 64), (257, 576, 32), (129, 8200, 40), (7, 100, 20), (9, 12, 4), (3, 36, 18)]
+
+
+def _placed(t, offset):
+    """The same values at an address `offset` bytes past a multiple of 512."""
+    raw = torch.zeros(t.numel() * t.element_size() + 512, dtype=torch.uint8, device="cuda")
+    view = raw[offset:offset + t.numel() * t.element_size()].view(t.dtype).view(t.shape)
+    view.copy_(t)
+    return view
+
+
+@pytest.mark.parametrize("n,k,g", SHAPES)
+@pytest.mark.parametrize("scales", ["f32", "f16"])
+@pytest.mark.parametrize("out", ["f32", "f16", "bf16"])
+def test_dequantise_at_every_alignment(n, k, g, scales, out):
+    rng = np.random.default_rng(n * k + g)
+    for bits, make, dequantise, call in ((4, O.make_w4, O.dequant_int4, _lib.lib().lcq_dequant_int4), (8, O.make_w8, O.dequant_int8, _lib.lib().lcq_dequant_int8)):
+        w, s = make(rng, n, k, g, np.float32 if scales == "f32" else np.float16)
+        want = O.round_to(dequantise(w, s, g), out).astype(np.float32)
+        ws, ss = torch.from_numpy(w).cuda(), torch.from_numpy(s).cuda()
+        for w_off, out_off in ((0, 0), (0, 16), (8, 32), (4, 0), (4, 8), (1, 4), (0, 48)):
+            placed = _placed(ws, w_off)
+            dst = _placed(torch.full((n, k), 77.0, device="cuda").to(KINDS[out][0]), out_off)
+            rc = call(ctypes.c_void_p(placed.data_ptr()), ctypes.c_void_p(ss.data_ptr()), ctypes.c_void_p(dst.data_ptr()), n, k, g,
+                      KINDS[scales][1], KINDS[out][1], ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+            assert rc == 0, _lib.lib().lcq_last_error()
+            assert np.array_equal(dst.float().cpu().numpy().view(np.uint32), want.view(np.uint32)), (bits, w_off, out_off)
+
+
+@pytest.mark.parametrize("n,k,g", [(1, 8, 8), (1, 32, 32), (3, 2048, 16), (1, 4104, 8), (2, 4096, 256), (257, 576, 64), (9, 8192, 128), (1025, 8, 8), (3, 24, 24)])
+@pytest.mark.parametrize("kind", ["f32", "f16", "bf16"])
+def test_quantise_at_every_alignment(n, k, g, kind):
+    gen = torch.Generator(device="cuda").manual_seed(n + k)
+    w = (torch.randn(n, k, device="cuda", generator=gen) * 0.1).to(KINDS[kind][0])
+    for bits, quantise in ((4, O.quantize_int4), (8, O.quantize_int8)):
+        q_ref, s_ref = quantise(w.float().cpu().numpy(), g)
+        for offset in (0, 16, 32, 4):
+            q = L.quantize(_placed(w, offset), g, bits=bits)
+            assert np.array_equal(q.w.cpu().numpy(), q_ref), (bits, offset)
+            assert np.array_equal(q.scales.cpu().numpy().view(np.uint32), s_ref.view(np.uint32))
+
+
+def test_a_linear_layer_right_behind_sees_its_weights():
+    """Kernels of linear layers fetch weights and scales before the kernel in front of them has ended: those that write them must not let them start early."""
+    n, k = 4096, 4096
+    layer = L.QuantLinear(torch.zeros(n, k // 2, dtype=torch.uint8, device="cuda"), torch.zeros(n, k // 32, dtype=torch.float16, device="cuda"), 32, 4)
+    x = torch.ones(1, k, dtype=torch.float16, device="cuda")
+    codes = torch.randint(-127, 128, (n, k // 32), dtype=torch.int8, device="cuda")
+    for i in range(20):
+        unit = torch.full((n, 1), float(i + 1) / 8192, device="cuda")
+        w = torch.full((n, k), float(i + 1), device="cuda")
+        q = L.quantize(w, 32)
+        scales = L.dequantize(codes, unit, n, k // 32, k // 32, bits=8, out_dtype="f16")
+        y = L.QuantLinear(q.w, scales, 32, 4)(x)
+        want = (codes.double() * unit.double()).half().double().sum(1) * 7 * 32
+        got = y.double()[0]
+        assert bool(((got - want).abs() <= 2.0 ** -10 * want.abs() + 1e-3 * (codes.double().abs() * unit.double()).sum(1)).all()), i
+    assert float(layer(x).abs().max()) == 0.0

@@ -14,9 +14,9 @@
 // rint is round-half-to-even (np.round); both divisions are IEEE float32 divisions.
 //
 // Streaming kernel, HBM-bound: 4 B read per weight (float32 input), 0.5 B + 4/G B written.
-// One thread owns 8 consecutive weights (one packed 32-bit word) and has the next 8 on their way; the
-// G/8 threads of a group combine their maxima with warp shuffles, so loads are 32 B per thread and stores
-// 4 B per thread, both coalesced.  Group sizes that are not 8, 16, 32, 64, 128 or 256 take a generic
+// One thread owns a few octets of 8 consecutive weights (one packed 32-bit word each) and has all of them on their way before it
+// starts on the first; the G/8 threads of a group combine their maxima with warp shuffles, so loads are 32 B per thread and
+// stores 4 B per thread, both coalesced.  Group sizes that are not 8, 16, 32, 64, 128 or 256 take a generic
 // kernel with one thread per group.
 //
 // The rounded quotient without dividing.  t = w * (1 / denom) differs from the IEEE quotient by less than
@@ -24,9 +24,12 @@
 // to the same integer unless t lies that close to a half-integer.  Adding 1.5 * 2^23 rounds t to an integer
 // (to even) and leaves it in the low bits of the sum; t minus that integer is exact, and when it comes
 // within the bound of 1/2 (or t is no number) the thread divides.  Dividing every weight and converting
-// with rint / min / max / float-to-int instructions bound the kernel: 4096 x 14336, int4, float32 weights 84 us a
-// call, now 48 (the kernel alone, from a cold cache, 44 us for 235 MB read and 37 MB written, most of which are still in
-// L2 when it ends); back to back float16 takes 48 us, bfloat16 60 (its ties: one octet in a few has one).
+// with rint / min / max / float-to-int instructions bound the kernel.
+//
+// What it measured (4096 x 14336, us a call among others over three weights): int4 from float32 48.6 before, 47.3 now (235 MB
+// read, 37 MB written; floor 41.6 at 6525 GB/s), from float16 49.1 / 38.6, from bfloat16 61.4 / 47.9 (its ties: one octet in a few
+// divides); int8 from float32 52.4 / 50.6, from float16 50.9 / 41.4.  Before: one wave of blocks that looped with one octet ahead,
+// converted as it arrived.
 #pragma once
 #include "common.cuh"
 #include "gemv_simt.cuh"
@@ -34,24 +37,44 @@
 namespace lcq {
 namespace quant {
 
-// 8 values read once: past L1, and not kept in it.
-template <typename XT> __device__ __forceinline__ void load8_once(const XT* p, float (&v)[8]);
-template <> __device__ __forceinline__ void load8_once<float>(const float* p, float (&v)[8]) {
-  const float4 a = __ldcs(reinterpret_cast<const float4*>(p)), b = __ldcs(reinterpret_cast<const float4*>(p) + 1);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-template <> __device__ __forceinline__ void load8_once<__half>(const __half* p, float (&v)[8]) {
-  const uint4 r = __ldcs(reinterpret_cast<const uint4*>(p));
+// 8 values read once (past L1, and not kept in it), as they are stored: all loads of a thread are issued before the first conversion.
+// Float32 values in one 32-byte load where they are on 32 bytes.
+template <typename XT> struct Raw8 {           // 16-bit types
+  uint4 r;
+  __device__ __forceinline__ void load(const XT* p, bool) { r = __ldcs(reinterpret_cast<const uint4*>(p)); }
+  __device__ __forceinline__ void zero() { r = make_uint4(0u, 0u, 0u, 0u); }
+  __device__ __forceinline__ void get(float (&v)[8]) const;
+};
+template <> __device__ __forceinline__ void Raw8<__half>::get(float (&v)[8]) const {
   const __half2* h = reinterpret_cast<const __half2*>(&r);
 #pragma unroll
   for (int i = 0; i < 4; ++i) { const float2 f = __half22float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
 }
-template <> __device__ __forceinline__ void load8_once<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[8]) {
-  const uint4 r = __ldcs(reinterpret_cast<const uint4*>(p));
+template <> __device__ __forceinline__ void Raw8<__nv_bfloat16>::get(float (&v)[8]) const {
   const uint32_t* u = reinterpret_cast<const uint32_t*>(&r);
 #pragma unroll
   for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(u[i] << 16); v[2 * i + 1] = __uint_as_float(u[i] & 0xFFFF0000u); }
 }
+template <> struct Raw8<float> {
+  float f[8];
+  __device__ __forceinline__ void load(const float* p, bool on_32) {
+    if (on_32) {
+      asm volatile("ld.global.nc.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "l"(p));
+    } else {
+      const float4 a = __ldcs(reinterpret_cast<const float4*>(p)), b = __ldcs(reinterpret_cast<const float4*>(p) + 1);
+      f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+    }
+  }
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = 0.0f;
+  }
+  __device__ __forceinline__ void get(float (&v)[8]) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = f[i];
+  }
+};
 
 __device__ __forceinline__ float group_scale(float amax, float qmax, int style, int wbits) {
   if (style == 0) return amax > 0.0f ? __fdiv_rn(amax, qmax) : 1.0f;
@@ -130,37 +153,40 @@ __device__ __forceinline__ uint2 quantize_octet(const float (&v)[8], float amax,
 
 // Fast path: G in {8, ..., 256} (a power of two), K % 8 == 0, rows 16-byte aligned.
 // total_oct = N*K/8 octets; octet e belongs to group e / (G/8).
+// Octets a thread: float32 1 / 2 / 4 / 8 48.2 / 48.9 / 47.3 / 57, float16 42.9 / 38.6 / 37.9, bfloat16 52.7 / 47.9 / 48.2 us (4096 x 14336, int4).
+template <typename XT> __host__ __device__ constexpr int q_unroll() { return sizeof(XT) == 4 ? 4 : 2; }
 template <typename XT, int WBITS>
 __global__ void __launch_bounds__(256) quantize_octets_kernel(const XT* __restrict__ w, uint8_t* __restrict__ q,
                                                               float* __restrict__ scales, long long total_oct,
-                                                              int group_shift, int style) {
+                                                              int group_shift, int style, bool on_32) {
+  constexpr int U = q_unroll<XT>();
+  griddep_wait();                              // (and no early start for the next kernel: a linear layer fetches its weights without waiting)
   const int lanes_per_group = 1 << group_shift;
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  // whole warps iterate together so the shuffles below are convergent
-  const long long n_iter = (total_oct + stride - 1) / stride;
-  long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  float next[8];
-  const auto fetch = [&](long long o) {
+  // whole blocks iterate together so the shuffles below are convergent
+  for (long long first = static_cast<long long>(blockIdx.x) * (256 * U); first < total_oct; first += static_cast<long long>(gridDim.x) * (256 * U)) {
+    Raw8<XT> raw[U];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) next[i] = 0.0f;
-    if (o < total_oct) load8_once<XT>(w + o * 8, next);
-  };
-  fetch(e);
-  for (long long it = 0; it < n_iter; ++it, e += stride) {
-    float v[8];
+    for (int u = 0; u < U; ++u) {
+      const long long e = first + u * 256 + threadIdx.x;
+      if (e < total_oct) raw[u].load(w + e * 8, on_32);
+      else raw[u].zero();
+    }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = next[i];
-    fetch(e + stride);
-    float amax = 0.0f;
+    for (int u = 0; u < U; ++u) {
+      const long long e = first + u * 256 + threadIdx.x;
+      float v[8];
+      raw[u].get(v);
+      float amax = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
-    for (int off = 1; off < lanes_per_group; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-    const float scale = group_scale(amax, WBITS == 4 ? 7.0f : 127.0f, style, WBITS);
-    if (e >= total_oct) continue;
-    if ((e & (lanes_per_group - 1)) == 0) scales[e >> group_shift] = scale;
-    const uint2 out = quantize_octet<WBITS>(v, amax, group_denom(scale, style));
-    if (WBITS == 4) reinterpret_cast<uint32_t*>(q)[e] = out.x;
-    else reinterpret_cast<uint2*>(q)[e] = out;
+      for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+      for (int off = 1; off < lanes_per_group; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+      const float scale = group_scale(amax, WBITS == 4 ? 7.0f : 127.0f, style, WBITS);
+      if (e >= total_oct) continue;
+      if ((e & (lanes_per_group - 1)) == 0) scales[e >> group_shift] = scale;
+      const uint2 out = quantize_octet<WBITS>(v, amax, group_denom(scale, style));
+      if (WBITS == 4) reinterpret_cast<uint32_t*>(q)[e] = out.x;
+      else reinterpret_cast<uint2*>(q)[e] = out;
+    }
   }
 }
 
@@ -199,9 +225,11 @@ int launch_quantize(const void* w, void* q, void* scales, long long N, long long
     const long long oct = total / 8;
     int shift = 0;
     while ((8 << shift) < G) ++shift;
-    const int grid = one_wave_grid<quantize_octets_kernel<XT, WBITS>>(oct, 256, sm_count);
-    quantize_octets_kernel<XT, WBITS><<<grid, 256, 0, st>>>(
-        static_cast<const XT*>(w), static_cast<uint8_t*>(q), static_cast<float*>(scales), oct, shift, style);
+    const long long need = (oct + 256 * q_unroll<XT>() - 1) / (256 * q_unroll<XT>());
+    const int grid = static_cast<int>(need < (1 << 30) ? need : (1 << 30));
+    const WaitingLaunch launch(grid, 256, st);
+    auto kern = quantize_octets_kernel<XT, WBITS>;
+    LCQ_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, kern, static_cast<const XT*>(w), static_cast<uint8_t*>(q), static_cast<float*>(scales), oct, shift, style, aligned(w, 32)));
   } else {
     const long long groups = total / G;
     long long blocks = (groups + 255) / 256;

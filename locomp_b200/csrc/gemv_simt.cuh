@@ -37,6 +37,86 @@ template <> __device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bflo
   }
 }
 
+// Two float32 values in one 64-bit register: the FMA pipe takes them as one instruction, each rounded as by itself.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float sum2(f32x2 v) {
+  float a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+  return a + b;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// 8 values of x in pairs
+__device__ __forceinline__ void load8_pairs(const float* p, f32x2 (&v)[4]) {
+  const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2*>(p)), b = __ldg(reinterpret_cast<const ulonglong2*>(p) + 1);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+template <typename XT> __device__ __forceinline__ void load8_pairs(const XT* p, f32x2 (&v)[4]) {
+  float f[8];
+  load8<XT>(p, f);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = pack2(f[2 * i], f[2 * i + 1]);
+}
+// An octet of int4 weights: bits of 2^23 + q, from which 2^23 + 8 is taken exactly.  By a mask per nibble parity and a byte permute
+// a weight; a shift and a mask for each nibble take five more instructions.
+__device__ __forceinline__ void int4_bits(uint32_t w, uint32_t (&v)[8]) {
+  const uint32_t even = w & 0x0F0F0F0Fu, odd = (w >> 4) & 0x0F0F0F0Fu;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __byte_perm(i & 1 ? odd : even, 0x4B000000u, 0x7540 + i / 2);
+}
+__device__ __forceinline__ void int4_pairs(uint32_t w, f32x2 (&v)[4]) {
+  uint32_t bits[8];
+  int4_bits(w, bits);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = add2(pack2(__uint_as_float(bits[2 * i]), __uint_as_float(bits[2 * i + 1])), pack2(-8388616.0f, -8388616.0f));
+}
+// SHIFTS: by a shift and a mask for each nibble, for float32 scales and more than one row of x, where calls of some us are faster with them (M = 3,
+// 2048 -> 6000 8.8 us, permutes 9.7; M = 8, 4096 -> 8192 35.3 / 31.1); 16-bit scales: M = 8, 8192 -> 16000 186 / 111.
+template <bool SHIFTS> __device__ __forceinline__ void int4_floats(uint32_t w, float (&v)[8]) {
+  if (SHIFTS) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(0x4B000000u | ((w >> (4 * i)) & 15u)) - 8388616.0f;
+  } else {
+    uint32_t bits[8];
+    int4_bits(w, bits);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(bits[i]) - 8388616.0f;
+  }
+}
+// The sums of gemv_rows_kernel, in one register or as two halves.
+template <bool PAIRS> struct RowSums { typedef float type; };
+template <> struct RowSums<true> { typedef f32x2 type; };
+__device__ __forceinline__ void scaled_sum(float& acc, float s, float p) { acc = fmaf(s, p, acc); }
+__device__ __forceinline__ void scaled_sum(f32x2& acc, float s, f32x2 p) { acc = fma2(pack2(s, s), p, acc); }
+__device__ __forceinline__ void scaled_sum(f32x2&, float, float) {}            // (never taken)
+__device__ __forceinline__ void scaled_sum(float&, float, f32x2) {}            // (never taken)
+__device__ __forceinline__ f32x2 dot8(const f32x2 (&x)[4], const f32x2 (&w)[4]) {
+  f32x2 p = mul2(x[0], w[0]);
+#pragma unroll
+  for (int i = 1; i < 4; ++i) p = fma2(x[i], w[i], p);
+  return p;
+}
+__device__ __forceinline__ float row_sum(float v) { return v; }
+__device__ __forceinline__ float row_sum(f32x2 v) { return sum2(v); }
+
 template <int WBITS, typename XT, typename ST, typename OT, int MT, bool VEC>
 __global__ void __launch_bounds__(256) gemv_simt_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w,
                                                         const ST* __restrict__ scales, OT* __restrict__ out,
@@ -170,8 +250,9 @@ __global__ void __launch_bounds__(256) gemv_simt_kernel(const XT* __restrict__ x
 // dequantised weight MT rows of x.  `splits` warps of a block share a row group's K when N alone gives too few
 // warps, and add up in shared memory.
 // M = 4, K = 2176, N = 8056, int8, f16: 23.8 us before, now 10.5; M = 8, K = 8192, N = 7000, int4, f32: 129, now 61;
-// M = 1, K = 8192, N = 16000, int8, f32: 56.7, now 36.7.
-template <int WBITS, typename XT, typename ST, typename OT, int MT>
+// M = 1, K = 8192, N = 16000, int8, f32: 56.7, now 35.4, int4 47.2, now 30.1.  Scales stay in their type until they are used: a conversion
+// of fp16 scales between the loads held the next load up (M = 4, 640 -> 12000, int4, f16: 9.0 -> 6.1).
+template <int WBITS, typename XT, typename ST, typename OT, int MT, int C>
 __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w,
                                                         const ST* __restrict__ scales, OT* __restrict__ out,
                                                         int M, int N, int K, int G, int gshift, int split_shift) {
@@ -181,7 +262,7 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
   const int splits = 1 << split_shift, part = warp & (splits - 1);
   const int n0 = (blockIdx.x * (8 >> split_shift) + (warp >> split_shift)) * R;
   const int m0 = blockIdx.y * MT;
-  const int nchunks = K >> 3, ns = K / G, row_bytes = WBITS == 4 ? (K >> 1) : K;
+  const int nchunks = K >> (2 + C), ns = K / G, row_bytes = WBITS == 4 ? (K >> 1) : K;
   const uint8_t* wrow[R];
   const ST* srow[R];
 #pragma unroll
@@ -193,26 +274,37 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
   const XT* xrow[MT];
 #pragma unroll
   for (int m = 0; m < MT; ++m) xrow[m] = x + static_cast<long long>(m0 + m < M ? m0 + m : M - 1) * K;
-  float acc[MT][R];
+  // C = 2 (int4, one row of x): two octets a lane and load, so that as many bytes are on their way as with int8; even and odd k add up
+  // in the halves of 64-bit registers.  M = 1, f32: 4096 -> 8192 16.5 us before, now 9.2, 8192 -> 16000 47.2 / 30.1, 3072 -> 3000 5.1 / 4.0.
+  // (int8 with two octets: 4096 -> 8192 10.7 -> 9.4, but 3072 -> 3000 4.5 -> 5.5; halves with two and four rows of x cost registers: M = 2,
+  // 1024 -> 12000 5.4 -> 6.0, M = 8 33 -> 39.)
+  static_assert(C == 1 || (C == 2 && MT == 1 && WBITS == 4), "two octets a lane: int4, one row of x");
+  constexpr bool PAIRS = C == 2;
+  typedef typename RowSums<PAIRS>::type Sum;
+  Sum acc[MT][R];
 #pragma unroll
   for (int m = 0; m < MT; ++m) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[m][r] = 0.0f;
+    for (int r = 0; r < R; ++r) acc[m][r] = 0;
   }
-  uint32_t lo[R], hi[R];                       // the next chunk, on its way (four chunks ahead cost occupancy: 37 -> 90 us for one case)
-  float sc[R];
+  constexpr int NW = C * (WBITS / 4);          // words of a chunk
+  uint32_t next[R][NW];                        // the next chunk, on its way (four chunks ahead cost occupancy: 37 -> 90 us for one case)
+  ST sc[R];
   const auto fetch = [&](int c) {
     if (c >= nchunks) return;
-    const int g = gshift >= 0 ? (c << 3) >> gshift : (c << 3) / G;
+    const int g = gshift >= 0 ? (c << (2 + C)) >> gshift : (c << (2 + C)) / G;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      if (WBITS == 4) {
-        lo[r] = __ldg(reinterpret_cast<const uint32_t*>(wrow[r]) + c);
+      if (NW == 1) {
+        next[r][0] = __ldg(reinterpret_cast<const uint32_t*>(wrow[r]) + c);
+      } else if (NW == 2) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(wrow[r]) + c);
+        next[r][0] = v.x; next[r][1 % NW] = v.y;
       } else {
-        const uint2 two = __ldg(reinterpret_cast<const uint2*>(wrow[r]) + c);
-        lo[r] = two.x; hi[r] = two.y;
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(wrow[r]) + c);
+        next[r][0] = v.x; next[r][1 % NW] = v.y; next[r][2 % NW] = v.z; next[r][3 % NW] = v.w;
       }
-      sc[r] = to_f32<ST>(__ldg(srow[r] + g));
+      sc[r] = __ldg(srow[r] + g);
     }
   };
   int c = part * 32 + lane;
@@ -220,30 +312,55 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
   griddep_launch_dependents();
   griddep_wait();
   for (; c < nchunks; c += 32 << split_shift) {
-    float wq[R][8], s[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      s[r] = sc[r];
-      if (WBITS == 4) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) wq[r][i] = __uint_as_float(0x4B000000u | ((lo[r] >> (4 * i)) & 15u)) - 8388616.0f;   // 2^23 + q, exact
-      } else {
-        float f[4];
-        int8x4_to_f32(lo[r], f); wq[r][0] = f[0]; wq[r][1] = f[1]; wq[r][2] = f[2]; wq[r][3] = f[3];
-        int8x4_to_f32(hi[r], f); wq[r][4] = f[0]; wq[r][5] = f[1]; wq[r][6] = f[2]; wq[r][7] = f[3];
-      }
-    }
-    fetch(c + (32 << split_shift));
-#pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      float xv[8];
-      load8<XT>(xrow[m] + (c << 3), xv);
+    if (PAIRS) {
+      uint32_t now[R][NW];
+      float s[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        float p = 0.0f;
+        s[r] = to_f32<ST>(sc[r]);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) p = fmaf(xv[i], wq[r][i], p);
-        acc[m][r] = fmaf(s[r], p, acc[m][r]);
+        for (int i = 0; i < NW; ++i) now[r][i] = next[r][i];
+      }
+      fetch(c + (32 << split_shift));
+      f32x2 p[R];
+#pragma unroll
+      for (int h = 0; h < C; ++h) {
+        f32x2 xv[4];
+        load8_pairs(xrow[0] + (c * C + h) * 8, xv);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          f32x2 wq[4];
+          int4_pairs(now[r][h], wq);
+          const f32x2 octet = dot8(xv, wq);
+          p[r] = h == 0 ? octet : add2(p[r], octet);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) scaled_sum(acc[0][r], s[r], p[r]);
+    } else {
+      float wq[R][8], s[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        s[r] = to_f32<ST>(sc[r]);
+        if (WBITS == 4) {
+          int4_floats<(MT == 2 || (MT > 1 && sizeof(ST) == 4))>(next[r][0], wq[r]);
+        } else {
+          int8x4_to_f32(next[r][0], wq[r]);
+          int8x4_to_f32(next[r][NW - 1], wq[r] + 4);
+        }
+      }
+      fetch(c + (32 << split_shift));
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        float xv[8];
+        load8<XT>(xrow[m] + (c << 3), xv);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float p = 0.0f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) p = fmaf(xv[i], wq[r][i], p);
+          scaled_sum(acc[m][r], s[r], p);
+        }
       }
     }
   }
@@ -254,7 +371,7 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
   constexpr int V = R * MT;
   float v[V];
 #pragma unroll
-  for (int i = 0; i < V; ++i) v[i] = acc[i / R][i % R];
+  for (int i = 0; i < V; ++i) v[i] = row_sum(acc[i / R][i % R]);
   int index = 0;
 #pragma unroll
   for (int h = V / 2, off = 16; h > 0; h >>= 1, off >>= 1) {
@@ -309,18 +426,23 @@ int launch_gemv_simt(const void* x, const void* w, const void* s, void* out, int
                                     op, M, N, K, G));                                                \
   } while (0)
   if (vec && (M > 1 || static_cast<long long>(N) * K > (1LL << 21))) {
-    // 8 warps a block; the warps of a block share K while there are fewer than 12 warps an SM and each of them still has a
-    // chunk per lane
+    // 8 warps a block; the warps of a block share K while there are too few warps an SM and each of them still has a chunk per
+    // lane: 12 warps, and with one row of x more where their shares stay long: int8 24 (4096 -> 8192 with 14 warps an SM 19.0 us, with
+    // 28 10.5, but 1152 -> 5000 with 17 and with 34 3.9 / 4.5), int4 32 (8192 -> 16000 with 27 and with 54 37.7 / 30.1).
     int split = 0;
     const long long groups = (N + 3) / 4;
     const int mt = M == 1 ? 1 : M == 2 ? 2 : 4, m_blocks = (M + mt - 1) / mt;
-    while (split < 3 && ((groups * m_blocks) << split) < sm_count * 12LL && (K >> 3) >= (64 << split)) ++split;
+    const bool two = WBITS == 4 && mt == 1 && K % 16 == 0 && G % 16 == 0 && aligned(w, 8);
+    const long long few = sm_count * 12LL, more = sm_count * (mt > 1 ? 12LL : WBITS == 4 ? 32LL : 24LL);
+    const int chunk_k = two ? 1024 : 512, long_k = two ? 1024 : 2048;
+    while (split < 3 && ((((groups * m_blocks) << split) < few && K >= (chunk_k << split)) || (((groups * m_blocks) << split) < more && K >= (long_k << split)))) ++split;
     int gshift = -1;
     if ((G & (G - 1)) == 0) { gshift = 0; while ((1 << gshift) < G) ++gshift; }
     cfg.gridDim = dim3(static_cast<unsigned>((groups + (8 >> split) - 1) / (8 >> split)), m_blocks);
-    if (mt == 1) LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 1>, xp, wp, sp, op, M, N, K, G, gshift, split));
-    else if (mt == 2) LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 2>, xp, wp, sp, op, M, N, K, G, gshift, split));
-    else LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 4>, xp, wp, sp, op, M, N, K, G, gshift, split));
+    if (two) LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<4, XT, ST, OT, 1, 2>, xp, wp, sp, op, M, N, K, G, gshift, split));
+    else if (mt == 1) LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 1, 1>, xp, wp, sp, op, M, N, K, G, gshift, split));
+    else if (mt == 2) LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 2, 1>, xp, wp, sp, op, M, N, K, G, gshift, split));
+    else LCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_rows_kernel<WBITS, XT, ST, OT, 4, 1>, xp, wp, sp, op, M, N, K, G, gshift, split));
   } else if (vec) {
     LCQ_SIMT_LAUNCH(1, true);
   } else {

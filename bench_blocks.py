@@ -198,7 +198,7 @@ def block_dequant(ctx: Ctx) -> dict:
     us = graph_us(ctx, [mk(i) for i in range(nbuf)], min_launches=30)
     moved = n * k // 2 + n * (k // GROUP) * 2 + 4 * n * k
     gbs = moved / us / 1e3
-    return {"workload": "dequant_int4 4096x14336 -> f32", "kernel": "dequant_w4_words_kernel", "us_per_call": us,
+    return {"workload": "dequant_int4 4096x14336 -> f32", "kernel": "dequant_octets_kernel", "us_per_call": us,
             "algorithmic_bytes": moved, "value": gbs, "unit": "GB/s (read + written)",
             "roofline": {"bound": "hbm", "achieved": gbs, "peak": ctx.peaks["hbm_gbs"], "frac": gbs / ctx.peaks["hbm_gbs"]}}
 

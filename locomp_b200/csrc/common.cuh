@@ -40,25 +40,6 @@ inline bool pdl_enabled() {
   return on;
 }
 
-// Launch of a kernel that waits for its predecessor itself (griddep_wait before its first access), so that its blocks are there
-// when that one ends.  It must not let its own successor start early (griddep_launch_dependents) if it writes what a linear
-// layer's kernel takes for constants and fetches without waiting: packed weights or scales.
-struct WaitingLaunch {
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[1];
-  WaitingLaunch(int grid, int block, cudaStream_t stream) {
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.stream = stream;
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
-  }
-  WaitingLaunch(const WaitingLaunch&) = delete;
-};
-
 // ------------------------------------------------------------------ dtype helpers
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }

@@ -20,6 +20,25 @@
 
 namespace lcq {
 
+// Launch of a kernel that waits for its predecessor itself (griddep_wait before its first access), so that its blocks are there
+// when that one ends.  It must not let its own successor start early (griddep_launch_dependents) if it writes what a linear
+// layer's kernel takes for constants and fetches without waiting: packed weights or scales.
+struct WaitingLaunch {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[1];
+  WaitingLaunch(int grid, int block, cudaStream_t stream) {
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  }
+  WaitingLaunch(const WaitingLaunch&) = delete;
+};
+
 template <typename OT> struct Out4;   // 4 consecutive outputs, one vector store
 template <> struct Out4<float> {
   static __device__ __forceinline__ void store(float* p, float a, float b, float c, float d) {

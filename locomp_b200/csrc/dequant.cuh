@@ -104,11 +104,34 @@ __device__ __forceinline__ void int8x4_to_f32(uint32_t v, float* f) {
   f[3] = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7543)) - 8388736.0f;
 }
 
+// Loads of what the kernel before this one may have written while this one was already there (WaitingLaunch): ld.global, since ld.global.nc
+// is for memory that nobody writes during the life of the kernel that reads, and volatile, so that none moves ahead of griddep_wait.
+__device__ __forceinline__ uint32_t load_written(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 load_written(const uint2* p) {
+  uint2 v;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float load_written(const float* p) { return __uint_as_float(load_written(reinterpret_cast<const uint32_t*>(p))); }
+__device__ __forceinline__ unsigned short load_written(const unsigned short* p) {
+  unsigned short v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ __half load_written(const __half* p) { return __ushort_as_half(load_written(reinterpret_cast<const unsigned short*>(p))); }
+__device__ __forceinline__ __nv_bfloat16 load_written(const __nv_bfloat16* p) {
+  return __ushort_as_bfloat16(load_written(reinterpret_cast<const unsigned short*>(p)));
+}
+
 // The 8 weights of an octet as they are stored: one word (int4), two (int8).
 template <int WBITS> struct Octet;
 template <> struct Octet<4> {
   uint32_t v;
-  __device__ __forceinline__ void load(const void* w, long long i) { v = __ldg(static_cast<const uint32_t*>(w) + i); }
+  __device__ __forceinline__ void load(const void* w, long long i) { v = load_written(static_cast<const uint32_t*>(w) + i); }
   __device__ __forceinline__ void scaled(float s, float (&f)[8]) const {
 #pragma unroll
     for (int i = 0; i < 8; ++i) f[i] = (small_uint_to_f32((v >> (4 * i)) & 15u) - 8.0f) * s;
@@ -116,7 +139,7 @@ template <> struct Octet<4> {
 };
 template <> struct Octet<8> {
   uint2 v;
-  __device__ __forceinline__ void load(const void* w, long long i) { v = __ldg(static_cast<const uint2*>(w) + i); }
+  __device__ __forceinline__ void load(const void* w, long long i) { v = load_written(static_cast<const uint2*>(w) + i); }
   __device__ __forceinline__ void scaled(float s, float (&f)[8]) const {
     int8x4_to_f32(v.x, f);
     int8x4_to_f32(v.y, f + 4);
@@ -130,7 +153,7 @@ template <> struct Octet<8> {
 // threads; ordinary sizes take one round.)
 template <typename OT> __host__ __device__ constexpr int dq_unroll() { return sizeof(OT) == 4 ? 2 : 4; }
 template <int WBITS, typename ST, typename OT>
-__global__ void __launch_bounds__(256) dequant_octets_kernel(const void* __restrict__ w, const ST* __restrict__ scales, OT* __restrict__ out,
+__global__ void __launch_bounds__(256) dequant_octets_kernel(const void* w, const ST* scales, OT* out,
                                                              long long octets, int G, int gshift, bool on_32) {
   constexpr int U = dq_unroll<OT>();
   griddep_wait();                              // (and no early start for the next kernel: the outputs may be a linear layer's scales)
@@ -142,7 +165,7 @@ __global__ void __launch_bounds__(256) dequant_octets_kernel(const void* __restr
       const long long i = i0 + u * 256;
       if (i < octets) {
         q[u].load(w, i);
-        s[u] = __ldg(scales + scale_index(i * 8, G, gshift));
+        s[u] = load_written(scales + scale_index(i * 8, G, gshift));
       }
     }
 #pragma unroll

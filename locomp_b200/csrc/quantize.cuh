@@ -38,10 +38,13 @@ namespace lcq {
 namespace quant {
 
 // 8 values read once (past L1, and not kept in it), as they are stored: all loads of a thread are issued before the first conversion.
-// Float32 values in one 32-byte load where they are on 32 bytes.
+// Float32 values in one 32-byte load where they are on 32 bytes.  ld.global and volatile, not .nc: the kernel before this one may write them
+// while this one is already there (load_written, dequant.cuh).
 template <typename XT> struct Raw8 {           // 16-bit types
   uint4 r;
-  __device__ __forceinline__ void load(const XT* p, bool) { r = __ldcs(reinterpret_cast<const uint4*>(p)); }
+  __device__ __forceinline__ void load(const XT* p, bool) {
+    asm volatile("ld.global.cs.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+  }
   __device__ __forceinline__ void zero() { r = make_uint4(0u, 0u, 0u, 0u); }
   __device__ __forceinline__ void get(float (&v)[8]) const;
 };
@@ -59,11 +62,11 @@ template <> struct Raw8<float> {
   float f[8];
   __device__ __forceinline__ void load(const float* p, bool on_32) {
     if (on_32) {
-      asm volatile("ld.global.nc.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                   : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "l"(p));
+      asm volatile("ld.global.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "l"(p) : "memory");
     } else {
-      const float4 a = __ldcs(reinterpret_cast<const float4*>(p)), b = __ldcs(reinterpret_cast<const float4*>(p) + 1);
-      f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+      asm volatile("ld.global.cs.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]) : "l"(p) : "memory");
+      asm volatile("ld.global.cs.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "l"(p + 4) : "memory");
     }
   }
   __device__ __forceinline__ void zero() {
@@ -156,8 +159,7 @@ __device__ __forceinline__ uint2 quantize_octet(const float (&v)[8], float amax,
 // Octets a thread: float32 1 / 2 / 4 / 8 48.2 / 48.9 / 47.3 / 57, float16 42.9 / 38.6 / 37.9, bfloat16 52.7 / 47.9 / 48.2 us (4096 x 14336, int4).
 template <typename XT> __host__ __device__ constexpr int q_unroll() { return sizeof(XT) == 4 ? 4 : 2; }
 template <typename XT, int WBITS>
-__global__ void __launch_bounds__(256) quantize_octets_kernel(const XT* __restrict__ w, uint8_t* __restrict__ q,
-                                                              float* __restrict__ scales, long long total_oct,
+__global__ void __launch_bounds__(256) quantize_octets_kernel(const XT* w, uint8_t* q, float* scales, long long total_oct,
                                                               int group_shift, int style, bool on_32) {
   constexpr int U = q_unroll<XT>();
   griddep_wait();                              // (and no early start for the next kernel: a linear layer fetches its weights without waiting)

@@ -55,6 +55,94 @@ def test_quantise_at_every_alignment(n, k, g, kind):
             assert np.array_equal(q.scales.cpu().numpy().view(np.uint32), s_ref.view(np.uint32))
 
 
+def _call(name, *args):
+    _lib.check(getattr(_lib.lib(), name)(*[ctypes.c_void_p(a.data_ptr()) if isinstance(a, torch.Tensor) else a for a in args],
+                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+
+
+def _unsynchronised_is_synchronised(rounds, step):
+    """step(i) launches a chain of kernels and returns its outputs, in buffers of their own; bit for bit the same with a
+    synchronisation behind every kernel (step calls what it is given between them)."""
+    torch.cuda.synchronize()
+    together = [step(i, lambda: None) for i in range(rounds)]
+    torch.cuda.synchronize()
+    for i in range(rounds):
+        apart = step(i, torch.cuda.synchronize)
+        torch.cuda.synchronize()
+        for a, b in zip(together[i], apart):
+            assert torch.equal(a, b), i
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("kind", ["f32", "f16"])
+@pytest.mark.parametrize("before", ["rms_norm", "silu_mul", "add_inplace", "linear"])
+def test_input_of_a_kernel_that_lets_its_successor_start(before, kind, bits):
+    """The blocks of these kernels are there while such a predecessor still writes what they read, into one buffer whose values change every time."""
+    n, k, rounds, dtype = 1500, 2048, 8, KINDS[kind][0]
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    a = [torch.randn(n, k, device="cuda", generator=gen).to(dtype) for _ in range(rounds)]
+    weight = torch.randn(k, device="cuda", generator=gen).to(dtype)
+    buffer = torch.zeros(n, k, device="cuda", dtype=dtype)
+    layer = L.QuantLinear(torch.randint(0, 256, (k, k // 2), dtype=torch.uint8, device="cuda", generator=gen),
+                          torch.rand(k, k // 32, device="cuda", generator=gen).to(dtype) * 0.01, 32, 4)
+
+    def step(i, between):
+        if before == "rms_norm":
+            L.rms_norm(a[i], weight, out=buffer)
+        elif before == "silu_mul":
+            L.silu_mul(a[i], a[i - 1], out=buffer)
+        elif before == "add_inplace":
+            L.add_inplace(buffer.zero_(), a[i])
+        else:
+            layer(a[i], out=buffer)
+        between()
+        q = torch.empty(n, k * bits // 8, dtype=torch.uint8, device="cuda")
+        s = torch.empty(n, k // 32, device="cuda")
+        _call(f"lcq_quantize_int{bits}", buffer, q, s, n, k, 32, KINDS[kind][1], 0)
+        between()
+        back = torch.empty(n, k, device="cuda")
+        _call(f"lcq_dequant_int{bits}", q, s, back, n, k, 32, _lib.F32, _lib.F32)
+        return q, s, back
+    _unsynchronised_is_synchronised(rounds, step)
+
+
+def test_scales_from_a_linear_layer():
+    """Dequantise behind a kernel that lets it start early and writes its scales."""
+    n, k, rounds = 4096, 4096, 8
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    codes = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen)
+    layer = L.QuantLinear(torch.randint(0, 256, (k // 32, 512), dtype=torch.uint8, device="cuda", generator=gen),
+                          torch.rand(k // 32, 32, device="cuda", generator=gen).half() * 0.01, 32, 4)
+    x = [torch.randn(n, 1024, device="cuda", generator=gen).half() for _ in range(rounds)]
+    scales = torch.zeros(n, k // 32, dtype=torch.float16, device="cuda")
+
+    def step(i, between):
+        layer(x[i], out=scales)
+        between()
+        back = torch.empty(n, k, device="cuda", dtype=torch.float16)
+        _call("lcq_dequant_int4", codes, scales, back, n, k, 32, _lib.F16, _lib.F16)
+        return back,
+    _unsynchronised_is_synchronised(rounds, step)
+
+
+def test_quantise_into_weights_that_a_linear_layer_still_reads():
+    n, k, rounds = 16000, 4096, 6
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    w = [torch.randn(n, k, device="cuda", generator=gen) for _ in range(2)]
+    layer = L.QuantLinear(torch.zeros(n, k // 2, dtype=torch.uint8, device="cuda"), torch.zeros(n, k // 32, device="cuda"), 32, 4)
+    x = torch.randn(4, k, device="cuda", generator=gen)
+
+    def step(i, between):
+        _call("lcq_quantize_int4", w[i % 2], layer.w, layer.scales, n, k, 32, _lib.F32, 0)
+        torch.cuda.synchronize()                               # (the weights of a linear layer are to be complete)
+        y = layer(x)
+        between()
+        _call("lcq_quantize_int4", w[1 - i % 2], layer.w, layer.scales, n, k, 32, _lib.F32, 0)
+        torch.cuda.synchronize()
+        return y,
+    _unsynchronised_is_synchronised(rounds, step)
+
+
 def test_a_linear_layer_right_behind_sees_its_weights():
     """Kernels of linear layers fetch weights and scales before the kernel in front of them has ended: those that write them must not let them start early."""
     n, k = 4096, 4096

@@ -14,8 +14,8 @@
 // rint is round-half-to-even (np.round); both divisions are IEEE float32 divisions.
 //
 // Streaming kernel, HBM-bound: 4 B read per weight (float32 input), 0.5 B + 4/G B written.
-// One thread owns a few octets of 8 consecutive weights (one packed 32-bit word each) and has all of them on their way before it
-// starts on the first; the G/8 threads of a group combine their maxima with warp shuffles, so loads are 32 B per thread and
+// One thread owns one to four octets of 8 consecutive weights (one packed 32-bit word each) and has all of them on their way before
+// it starts on the first; the G/8 threads of a group combine their maxima with warp shuffles, so loads are 32 B per thread and
 // stores 4 B per thread, both coalesced.  Group sizes that are not 8, 16, 32, 64, 128 or 256 take a generic
 // kernel with one thread per group.
 //
@@ -156,12 +156,10 @@ __device__ __forceinline__ uint2 quantize_octet(const float (&v)[8], float amax,
 
 // Fast path: G in {8, ..., 256} (a power of two), K % 8 == 0, rows 16-byte aligned.
 // total_oct = N*K/8 octets; octet e belongs to group e / (G/8).
-// Octets a thread: float32 1 / 2 / 4 / 8 48.2 / 48.9 / 47.3 / 57, float16 42.9 / 38.6 / 37.9, bfloat16 52.7 / 47.9 / 48.2 us (4096 x 14336, int4).
-template <typename XT> __host__ __device__ constexpr int q_unroll() { return sizeof(XT) == 4 ? 4 : 2; }
-template <typename XT, int WBITS>
+// U octets a thread.
+template <typename XT, int WBITS, int U>
 __global__ void __launch_bounds__(256) quantize_octets_kernel(const XT* w, uint8_t* q, float* scales, long long total_oct,
                                                               int group_shift, int style, bool on_32) {
-  constexpr int U = q_unroll<XT>();
   griddep_wait();                              // (and no early start for the next kernel: a linear layer fetches its weights without waiting)
   const int lanes_per_group = 1 << group_shift;
   // whole blocks iterate together so the shuffles below are convergent
@@ -227,10 +225,16 @@ int launch_quantize(const void* w, void* q, void* scales, long long N, long long
     const long long oct = total / 8;
     int shift = 0;
     while ((8 << shift) < G) ++shift;
-    const long long need = (oct + 256 * q_unroll<XT>() - 1) / (256 * q_unroll<XT>());
+    // Octets a thread: two of 16-bit weights (1 / 2 / 4: float16 42.9 / 38.6 / 37.9 us, bfloat16 52.7 / 47.9 / 48.2, 4096 x 14336, int4).  Float32
+    // weights: one up to 32 Mi weights, where four make few and long blocks that leave SMs idle (int4, one / four: 192 x 576 1.33 / 2.40, 1536 x 576
+    // 2.43 / 3.37, 2048 x 2048 4.89 / 6.28, 3000 x 4096 10.7 / 11.8, 7000 x 4096 22.4 / 22.8, 8192 x 4096 26.0 / 26.2), and four beyond (10240 x 4096 32.8 / 32.0,
+    // 4096 x 14336 48.2 / 47.3).
+    constexpr int FEW = sizeof(XT) == 4 ? 1 : 2, MANY = sizeof(XT) == 4 ? 4 : 2;
+    const bool many = total > (1LL << 25);
+    const long long per_block = 256 * (many ? MANY : FEW), need = (oct + per_block - 1) / per_block;
     const int grid = static_cast<int>(need < (1 << 30) ? need : (1 << 30));
     const WaitingLaunch launch(grid, 256, st);
-    auto kern = quantize_octets_kernel<XT, WBITS>;
+    auto kern = many ? quantize_octets_kernel<XT, WBITS, MANY> : quantize_octets_kernel<XT, WBITS, FEW>;
     LCQ_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, kern, static_cast<const XT*>(w), static_cast<uint8_t*>(q), static_cast<float*>(scales), oct, shift, style, aligned(w, 32)));
   } else {
     const long long groups = total / G;

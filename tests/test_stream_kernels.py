@@ -55,6 +55,17 @@ def test_quantise_at_every_alignment(n, k, g, kind):
             assert np.array_equal(q.scales.cpu().numpy().view(np.uint32), s_ref.view(np.uint32))
 
 
+@pytest.mark.parametrize("offset", [0, 16])
+@pytest.mark.parametrize("bits", [4, 8])
+def test_quantise_a_large_weight(bits, offset):
+    """Float32 weights have one octet a thread up to 32 Mi weights and four beyond: a weight just beyond, whole and in two parts."""
+    n, k, g = 4099, 8200, 8
+    assert n * k > 1 << 25 and n * k // 8 % 1024
+    w = _placed(torch.randn(n, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(6)), offset)
+    whole, parts = L.quantize(w, g, bits=bits), [L.quantize(part, g, bits=bits) for part in (w[:1000], w[1000:])]
+    assert torch.equal(whole.w, torch.cat([q.w for q in parts])) and torch.equal(whole.scales, torch.cat([q.scales for q in parts]))
+
+
 def _call(name, *args):
     _lib.check(getattr(_lib.lib(), name)(*[ctypes.c_void_p(a.data_ptr()) if isinstance(a, torch.Tensor) else a for a in args],
                                          ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))

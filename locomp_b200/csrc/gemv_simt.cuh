@@ -428,14 +428,32 @@ int launch_gemv_simt(const void* x, const void* w, const void* s, void* out, int
   if (vec && (M > 1 || static_cast<long long>(N) * K > (1LL << 21))) {
     // 8 warps a block; the warps of a block share K while there are too few warps an SM and each of them still has a chunk per
     // lane: 12 warps, and with one row of x more where their shares stay long: int8 24 (4096 -> 8192 with 14 warps an SM 19.0 us, with
-    // 28 10.5, but 1152 -> 5000 with 17 and with 34 3.9 / 4.5), int4 32 (8192 -> 16000 with 27 and with 54 37.7 / 30.1).
+    // 28 10.5, but 1152 -> 5000 with 17 and with 34 3.9 / 4.5), int4 32.
     int split = 0;
     const long long groups = (N + 3) / 4;
     const int mt = M == 1 ? 1 : M == 2 ? 2 : 4, m_blocks = (M + mt - 1) / mt;
-    const bool two = WBITS == 4 && mt == 1 && K % 16 == 0 && G % 16 == 0 && aligned(w, 8);
-    const long long few = sm_count * 12LL, more = sm_count * (mt > 1 ? 12LL : WBITS == 4 ? 32LL : 24LL);
-    const int chunk_k = two ? 1024 : 512, long_k = two ? 1024 : 2048;
-    while (split < 3 && ((((groups * m_blocks) << split) < few && K >= (chunk_k << split)) || (((groups * m_blocks) << split) < more && K >= (long_k << split)))) ++split;
+    bool two = WBITS == 4 && mt == 1 && K % 16 == 0 && G % 16 == 0 && aligned(w, 8) && K > 256;
+    const long long wave_two = sm_count * 24LL, wave_one = sm_count * 32LL;      // warps that are resident, two octets a lane (80 registers) and one (64)
+    if (two) {
+      // Two octets a lane: as many shares as still make one wave, however short (1536 -> 2800 in 2 / 4 shares 3.2 / 2.4 us, 8 are two waves: 4.0;
+      // 8000 rows of 1152 in 1 / 2 4.9 / 5.7).  Long shares are worth a second wave: 8192 -> 8000 in 1 / 4 20.4 / 17.4.
+      while (split < 3 && (groups << (split + 1)) <= wave_two && K >= (256 << split)) ++split;
+      const int next = groups > wave_two ? 0 : split + 1;
+      const bool one_wave_of_one = next <= 3 && (groups << next) > wave_two && (groups << next) <= wave_one;
+      if (one_wave_of_one && K < (sizeof(XT) == 4 ? 1536 : 1024) && (next == 0 || K > 512)) {
+        // One octet: a wave of it holds 4/3 of the warps.  float32, one octet in one wave / two in two: 16000 rows of 512 3.3 / 4.0, of 1152 6.9 / 7.7, of
+        // 1536 8.4 / 8.3; 2000 rows of 1152 in 8 shares 1.9, two octets in 4 2.4.  float16: 16000 rows of 768 4.6 / 5.4, of 1024 6.0 / 5.4.
+        two = false;
+        split = next;
+      } else if (sizeof(XT) == 4 && K > 512 && K <= 768 && groups > wave_one * 5 / 4) {
+        two = false;                           // three rounds of one octet against two of two, the second half empty: 768 -> 50000 11.5 / 12.0
+      } else {
+        while (split < 3 && (groups << split) < wave_one && K >= (1792 << split)) ++split;
+      }
+    } else {
+      const long long few = sm_count * 12LL, more = mt > 1 ? few : sm_count * (WBITS == 4 ? 32LL : 24LL);
+      while (split < 3 && ((((groups * m_blocks) << split) < few && K >= (512 << split)) || (((groups * m_blocks) << split) < more && K >= (2048 << split)))) ++split;
+    }
     int gshift = -1;
     if ((G & (G - 1)) == 0) { gshift = 0; while ((1 << gshift) < G) ++gshift; }
     cfg.gridDim = dim3(static_cast<unsigned>((groups + (8 >> split) - 1) / (8 >> split)), m_blocks);

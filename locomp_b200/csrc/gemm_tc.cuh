@@ -97,21 +97,27 @@ template <int CG> __device__ __forceinline__ void umma_step(uint32_t d_tmem, uin
   else
     asm volatile(LCQ_MMA_BEGIN LCQ_MMA_STEP(1, 0, "p") LCQ_MMA_END ::"r"(d_tmem), "r"(a_tmem), "r"(b), "r"(idesc), "r"(first), "n"(B_DESC_HI) : "memory");
 }
-// The same for a whole stage of 256 k (`step`: descriptor units between 64-k steps).  One election and one branch for
-// sixteen MMAs: the issuing warp shares its scheduler with four dequant warps, and what it can issue bounds tiles of
+// The same for a whole stage of 256 k (STEPS = 4) or half of one (2); `step`: descriptor units between 64-k steps.  One election and
+// one branch for all: the issuing warp shares its scheduler with four dequant warps, and what it can issue bounds tiles of
 // few rows.  Clocks per MMA beside four busy warps on the scheduler, N <= 64: an election per MMA in a loop over
 // the steps 168, all sixteen unrolled 61, one election for four 63, one for all with predicated MMAs 52, with a branch 45.
-template <int CG> __device__ __forceinline__ void umma_stage(uint32_t d_tmem, uint32_t a_tmem, uint32_t b, uint32_t step, uint32_t idesc, uint32_t first) {
-#define LCQ_MMA_STAGE(G)                                                                                                     \
+template <int CG, int STEPS> __device__ __forceinline__ void umma_steps(uint32_t d_tmem, uint32_t a_tmem, uint32_t b, uint32_t step, uint32_t idesc, uint32_t first) {
+#define LCQ_MMA_TWO_STEPS(G)                                                                                                 \
+  LCQ_MMA_BEGIN "add.u32 a4, %1, 32;\n\tadd.u32 b4, %2, %6;\n\t" LCQ_MMA_STEP(G, 0, "p") LCQ_MMA_STEP(G, 4, "q")
+#define LCQ_MMA_FOUR_STEPS(G)                                                                                                \
   LCQ_MMA_BEGIN                                                                                                              \
   "add.u32 a4, %1, 32;\n\tadd.u32 a8, %1, 64;\n\tadd.u32 a12, %1, 96;\n\t"                                                   \
   "add.u32 b4, %2, %6;\n\tadd.u32 b8, b4, %6;\n\tadd.u32 b12, b8, %6;\n\t"                                                   \
-  LCQ_MMA_STEP(G, 0, "p") LCQ_MMA_STEP(G, 4, "q") LCQ_MMA_STEP(G, 8, "q") LCQ_MMA_STEP(G, 12, "q") LCQ_MMA_END
-  if (CG == 2)
-    asm volatile(LCQ_MMA_STAGE(2) ::"r"(d_tmem), "r"(a_tmem), "r"(b), "r"(idesc), "r"(first), "n"(B_DESC_HI), "r"(step) : "memory");
+  LCQ_MMA_STEP(G, 0, "p") LCQ_MMA_STEP(G, 4, "q") LCQ_MMA_STEP(G, 8, "q") LCQ_MMA_STEP(G, 12, "q")
+  static_assert(STEPS == 4 || (STEPS == 2 && CG == 1), "the forms that are used");
+  if constexpr (CG == 2)
+    asm volatile(LCQ_MMA_FOUR_STEPS(2) LCQ_MMA_END ::"r"(d_tmem), "r"(a_tmem), "r"(b), "r"(idesc), "r"(first), "n"(B_DESC_HI), "r"(step) : "memory");
+  else if constexpr (STEPS == 4)
+    asm volatile(LCQ_MMA_FOUR_STEPS(1) LCQ_MMA_END ::"r"(d_tmem), "r"(a_tmem), "r"(b), "r"(idesc), "r"(first), "n"(B_DESC_HI), "r"(step) : "memory");
   else
-    asm volatile(LCQ_MMA_STAGE(1) ::"r"(d_tmem), "r"(a_tmem), "r"(b), "r"(idesc), "r"(first), "n"(B_DESC_HI), "r"(step) : "memory");
-#undef LCQ_MMA_STAGE
+    asm volatile(LCQ_MMA_TWO_STEPS(1) LCQ_MMA_END ::"r"(d_tmem), "r"(a_tmem), "r"(b), "r"(idesc), "r"(first), "n"(B_DESC_HI), "r"(step) : "memory");
+#undef LCQ_MMA_TWO_STEPS
+#undef LCQ_MMA_FOUR_STEPS
 }
 #undef LCQ_MMA
 #undef LCQ_MMA_STEP
@@ -484,7 +490,13 @@ __device__ __noinline__ void drain(const Params& p, uint8_t* smem, int team, uin
 // before this one took them: a weight is the sum of two fp16 numbers, RN((q - 8) * s) and what that rounds off
 // ((q - 8) * s and its rounding are multiples of 2^-24, so the rest is an fp16 number), in two A slots that meet the
 // same X stage.  The first set of dequant warps writes the one, the second set the other.
-template <int CG, typename OT, bool PERM, bool RAGGED>
+//
+// HALVES: the sixteen MMAs of a stage under two elections, for tiles of more than 64 rows on one SM.  An MMA takes 48 clocks and up there, which hides
+// the second election, while with all in one block the instance spills 60 bytes instead of 24, and calls of few stages pay for that: 116 x 1024 -> 9850
+// 9.2 us with an election per MMA, 9.6 with one, 9.2 with two; 277 x 1280 -> 4077 10.0 / 10.2 / 9.9; 486 x 768 -> 3174 7.8 / 8.05 / 7.7; 128 x 2048 ->
+// 16000 13.0 / 12.9 / 12.7.  Up to 64 rows one is faster on long K: 17 x 12032 -> 26539 60.4 / 45.2 / 46.0, 32 x 8192 -> 28672 46.1 / 35.2 / 35.7 (64 x 1280 ->
+// 16000 9.1 / 8.5 / 8.4).  Pairs and RAGGED calls spill the same either way.
+template <int CG, typename OT, bool PERM, bool RAGGED, bool HALVES>
 __global__ void __launch_bounds__(NTHREADS, 1)
 w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_piece,
                   const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
@@ -610,9 +622,14 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           }
           tc_fence_after();
           const uint32_t bdesc = desc0 + rx.i * desc_stage, a_t = a_base + ra.i * A_SLOT_COLS;
-          if (!RAGGED || steps == WK / BK) umma_stage<CG>(d_t, a_t, bdesc, desc_step, idesc, acc);
-          else
+          if constexpr (HALVES) {
+            umma_steps<1, 2>(d_t, a_t, bdesc, desc_step, idesc, acc);
+            umma_steps<1, 2>(d_t, a_t + 2 * A_STEP_COLS, bdesc + 2 * desc_step, desc_step, idesc, 1u);
+          } else if (!RAGGED || steps == WK / BK) {
+            umma_steps<CG, 4>(d_t, a_t, bdesc, desc_step, idesc, acc);
+          } else {
             for (int k = 0; k < steps; ++k) umma_step<CG>(d_t, a_t + k * A_STEP_COLS, bdesc + k * desc_step, idesc, k == 0 ? acc : 1u);
+          }
           acc = 1;
           if (TERMS == 1 || (i & 1)) {
             umma_commit<CG>(&empty_x[rx.i]);
@@ -956,9 +973,12 @@ inline void pdl_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
 }
 
-template <int CG, typename OT, bool PERM, bool RAGGED>
+template <int CG, typename OT, bool PERM, bool RAGGED, bool HALVES = false>
 int launch_t(const CUtensorMap* tm, const Params& p, cudaStream_t stream) {
-  auto kern = w4a16_gemm_kernel<CG, OT, PERM, RAGGED>;
+  if constexpr (CG == 1 && !RAGGED && !HALVES) {
+    if (p.bm > 64) return launch_t<CG, OT, PERM, RAGGED, true>(tm, p, stream);
+  }
+  auto kern = w4a16_gemm_kernel<CG, OT, PERM, RAGGED, HALVES>;
   static thread_local int configured_device = -1;
   int dev = 0;
   LCQ_CUDA_TRY(cudaGetDevice(&dev));

@@ -38,7 +38,8 @@ def test_pairs_multiply_rows_in_multiples_of_32(m, n, k):
 
 CASES = [(17, 1, 64), (17, 257, 320), (31, 255, 256), (32, 256, 576), (33, 513, 1984), (64, 300, 4096), (96, 1000, 832),
          (128, 129, 4096), (160, 640, 1024), (161, 128, 768), (193, 700, 512), (224, 256, 2048), (250, 384, 448), (257, 2000, 1088),
-         (40, 30000, 512), (300, 20000, 320), (1000, 4000, 512), (520, 9600, 1024)]
+         (40, 30000, 512), (300, 20000, 320), (1000, 4000, 512), (520, 9600, 1024),
+         (64, 300, 256), (65, 300, 256), (96, 200, 512), (128, 400, 768), (116, 9850, 1024)]          # one to four stages, both sides of 64 rows
 
 
 @pytest.mark.gpu

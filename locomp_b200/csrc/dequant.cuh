@@ -13,16 +13,18 @@
 // before, 41.4 now, -> f16 32.7 / 27.0; int8 -> f32 56.1 / 46.3, -> f16 41.5 / 28.9.  Before: one wave of blocks that looped, int4
 // words spread over the lanes by shuffles to get 16-byte stores, int8 one word a thread.  What gave it: blocks that end
 // after one round of loads and stores instead of looping (a loop's next loads wait behind its stores; 53 -> 43 in a kernel by
-// itself), fp16 scales converted only after all loads are issued (33.6 -> 27.0 for f16 outputs), and a launch whose blocks are
-// there when the kernel before ends (-2).  Octets a thread: f32 1 / 2 / 4 46.5 / 41.6 / 41.6, f16 1 / 2 / 4 39.2 / 29.4 / 27.0.
+// itself), fp16 scales converted only after all loads are issued (33.6 -> 27.0 for f16 outputs), and the programmatic attribute, without
+// which a launch starts up to 2 us late whatever is in front of it (-2).  Octets a thread: f32 1 / 2 / 4 46.5 / 41.6 / 41.6, f16 1 / 2 / 4 39.2 / 29.4 / 27.0.
 #pragma once
 #include "common.cuh"
 
 namespace lcq {
 
-// Launch of a kernel that waits for its predecessor itself (griddep_wait before its first access), so that its blocks are there
-// when that one ends.  It must not let its own successor start early (griddep_launch_dependents) if it writes what a linear
-// layer's kernel takes for constants and fetches without waiting: packed weights or scales.
+// Launch of a kernel that waits for its predecessor itself (griddep_wait before its first access).  Behind a kernel that lets its successor start
+// early its blocks are there when that one ends; behind any other the attribute saves the up to 2 us by which a launch without it starts late.
+// A kernel that writes packed weights or scales does not let its own successor start early (griddep_launch_dependents): a linear layer's kernel fetches
+// those without waiting, and would do so while they are being written.  That does not free the caller from synchronising between writing
+// weights and the first call of the layer (locomp_b200.h): that the stores of blocks which have ended are visible to a fetch ahead of the wait is not specified.
 struct WaitingLaunch {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
@@ -156,7 +158,7 @@ template <int WBITS, typename ST, typename OT>
 __global__ void __launch_bounds__(256) dequant_octets_kernel(const void* w, const ST* scales, OT* out,
                                                              long long octets, int G, int gshift, bool on_32) {
   constexpr int U = dq_unroll<OT>();
-  griddep_wait();                              // (and no early start for the next kernel: the outputs may be a linear layer's scales)
+  griddep_wait();                              // (no early start for the next kernel: the outputs may be a linear layer's scales, see WaitingLaunch)
   for (long long i0 = static_cast<long long>(blockIdx.x) * (256 * U) + threadIdx.x; i0 < octets; i0 += static_cast<long long>(gridDim.x) * (256 * U)) {
     Octet<WBITS> q[U];
     ST s[U];

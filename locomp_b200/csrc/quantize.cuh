@@ -160,7 +160,7 @@ __device__ __forceinline__ uint2 quantize_octet(const float (&v)[8], float amax,
 template <typename XT, int WBITS, int U>
 __global__ void __launch_bounds__(256) quantize_octets_kernel(const XT* w, uint8_t* q, float* scales, long long total_oct,
                                                               int group_shift, int style, bool on_32) {
-  griddep_wait();                              // (and no early start for the next kernel: a linear layer fetches its weights without waiting)
+  griddep_wait();                              // (no early start for the next kernel, which may be a linear layer with these weights, see WaitingLaunch)
   const int lanes_per_group = 1 << group_shift;
   // whole blocks iterate together so the shuffles below are convergent
   for (long long first = static_cast<long long>(blockIdx.x) * (256 * U); first < total_oct; first += static_cast<long long>(gridDim.x) * (256 * U)) {

@@ -154,19 +154,29 @@ def test_quantise_into_weights_that_a_linear_layer_still_reads():
     _unsynchronised_is_synchronised(rounds, step)
 
 
-def test_a_linear_layer_right_behind_sees_its_weights():
-    """Kernels of linear layers fetch weights and scales before the kernel in front of them has ended: those that write them must not let them start early."""
-    n, k = 4096, 4096
-    layer = L.QuantLinear(torch.zeros(n, k // 2, dtype=torch.uint8, device="cuda"), torch.zeros(n, k // 32, dtype=torch.float16, device="cuda"), 32, 4)
-    x = torch.ones(1, k, dtype=torch.float16, device="cuda")
-    codes = torch.randint(-127, 128, (n, k // 32), dtype=torch.int8, device="cuda")
-    for i in range(20):
-        unit = torch.full((n, 1), float(i + 1) / 8192, device="cuda")
-        w = torch.full((n, k), float(i + 1), device="cuda")
-        q = L.quantize(w, 32)
-        scales = L.dequantize(codes, unit, n, k // 32, k // 32, bits=8, out_dtype="f16")
-        y = L.QuantLinear(q.w, scales, 32, 4)(x)
-        want = (codes.double() * unit.double()).half().double().sum(1) * 7 * 32
-        got = y.double()[0]
-        assert bool(((got - want).abs() <= 2.0 ** -10 * want.abs() + 1e-3 * (codes.double().abs() * unit.double()).sum(1)).all()), i
-    assert float(layer(x).abs().max()) == 0.0
+@pytest.mark.parametrize("written", ["weights", "scales"])
+def test_a_linear_layer_does_not_start_while_its_weights_are_written(written):
+    """Kernels of linear layers fetch weights and scales before they wait for the kernel in front of them, which is why a caller has to synchronise between
+    writing weights and the first call.  The quantisers and dequantisers do their part: they do not let a linear layer directly behind them
+    start early, so that it does not fetch what was there before.  Other weights every time, in the same buffers."""
+    n, k, rounds = 8192, 4096, 12
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    if written == "weights":
+        source = [torch.randn(n, k, device="cuda", generator=gen) for _ in range(4)]
+        layer = L.QuantLinear(torch.zeros(n, k // 2, dtype=torch.uint8, device="cuda"), torch.zeros(n, k // 32, device="cuda"), 32, 4)
+        x = torch.randn(1, k, device="cuda", generator=gen)
+    else:
+        source = [torch.randint(0, 256, (n, k // 32), dtype=torch.uint8, device="cuda", generator=gen) for _ in range(4)]
+        unit = torch.rand(n, 1, device="cuda", generator=gen) * 0.01
+        layer = L.QuantLinear(torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen),
+                              torch.zeros(n, k // 32, dtype=torch.float16, device="cuda"), 32, 4)
+        x = torch.randn(1, k, device="cuda", generator=gen).half()
+
+    def step(i, between):
+        if written == "weights":
+            _call("lcq_quantize_int4", source[i % 4], layer.w, layer.scales, n, k, 32, _lib.F32, 0)
+        else:
+            _call("lcq_dequant_int8", source[i % 4], unit, layer.scales, n, k // 32, k // 32, _lib.F32, _lib.F16)
+        between()
+        return layer(x),
+    _unsynchronised_is_synchronised(rounds, step)

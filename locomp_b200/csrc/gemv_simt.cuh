@@ -88,8 +88,11 @@ __device__ __forceinline__ void int4_pairs(uint32_t w, f32x2 (&v)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) v[i] = add2(pack2(__uint_as_float(bits[2 * i]), __uint_as_float(bits[2 * i + 1])), pack2(-8388616.0f, -8388616.0f));
 }
-// SHIFTS: by a shift and a mask for each nibble, for float32 scales and more than one row of x, where calls of some us are faster with them (M = 3,
-// 2048 -> 6000 8.8 us, permutes 9.7; M = 8, 4096 -> 8192 35.3 / 31.1); 16-bit scales: M = 8, 8192 -> 16000 186 / 111.
+// SHIFTS: by a shift and a mask for each nibble; else by permutes, which take fewer instructions and more registers.  Shifts for two rows of x, and for
+// float32 scales with more: the forms in which permutes lost somewhere.  us, shifts / permutes.  Two rows, float32: 4096 -> 8192 13.5 / 17.3, 2048 -> 2000
+// 2.8 / 3.2, 8192 -> 16000 51.0 / 54.1, but 1024 -> 12000 7.5 / 5.3; float16: 8192 -> 16000 52.7 / 53.9, but 4096 -> 8192 21.6 / 18.2, 1024 -> 12000 6.0 / 5.2.  Three and
+// more, float32: M = 8, 3072 -> 3000 12.6 / 13.1, M = 3, 2048 -> 6000 9.7 / 9.9, but M = 8, 4096 -> 8192 35.5 / 31.2, 8192 -> 16000 123 / 111, M = 5, 1536 -> 3690 7.8 / 6.9;
+// float16: M = 8, 4096 -> 8192 40.4 / 32.1, 8192 -> 16000 184 / 111.
 template <bool SHIFTS> __device__ __forceinline__ void int4_floats(uint32_t w, float (&v)[8]) {
   if (SHIFTS) {
 #pragma unroll
@@ -106,8 +109,6 @@ template <bool PAIRS> struct RowSums { typedef float type; };
 template <> struct RowSums<true> { typedef f32x2 type; };
 __device__ __forceinline__ void scaled_sum(float& acc, float s, float p) { acc = fmaf(s, p, acc); }
 __device__ __forceinline__ void scaled_sum(f32x2& acc, float s, f32x2 p) { acc = fma2(pack2(s, s), p, acc); }
-__device__ __forceinline__ void scaled_sum(f32x2&, float, float) {}            // (never taken)
-__device__ __forceinline__ void scaled_sum(float&, float, f32x2) {}            // (never taken)
 __device__ __forceinline__ f32x2 dot8(const f32x2 (&x)[4], const f32x2 (&w)[4]) {
   f32x2 p = mul2(x[0], w[0]);
 #pragma unroll
@@ -249,9 +250,9 @@ __global__ void __launch_bounds__(256) gemv_simt_kernel(const XT* __restrict__ x
 // it from L1 per half byte of weight -- and that bound the kernel; here a chunk of x serves four rows and a
 // dequantised weight MT rows of x.  `splits` warps of a block share a row group's K when N alone gives too few
 // warps, and add up in shared memory.
-// M = 4, K = 2176, N = 8056, int8, f16: 23.8 us before, now 10.5; M = 8, K = 8192, N = 7000, int4, f32: 129, now 61;
-// M = 1, K = 8192, N = 16000, int8, f32: 56.7, now 35.4, int4 47.2, now 30.1.  Scales stay in their type until they are used: a conversion
-// of fp16 scales between the loads held the next load up (M = 4, 640 -> 12000, int4, f16: 9.0 -> 6.1).
+// M = 4, K = 2176, N = 8056, int8, f16: 23.8 us before, now 10.1; M = 8, K = 8192, N = 7000, int4, f32: 129, now 57;
+// M = 1, K = 8192, N = 16000, int8, f32: 56.7, now 35.1, int4 47, now 29.7.  Scales stay in their type until they are used: a conversion
+// of fp16 scales between the loads held the next load up (M = 4, 640 -> 12000, int4, f16: 9.1 -> 6.6).
 template <int WBITS, typename XT, typename ST, typename OT, int MT, int C>
 __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w,
                                                         const ST* __restrict__ scales, OT* __restrict__ out,
@@ -274,8 +275,9 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
   const XT* xrow[MT];
 #pragma unroll
   for (int m = 0; m < MT; ++m) xrow[m] = x + static_cast<long long>(m0 + m < M ? m0 + m : M - 1) * K;
-  // C = 2 (int4, one row of x): two octets a lane and load, so that as many bytes are on their way as with int8; even and odd k add up
-  // in the halves of 64-bit registers.  M = 1, f32: 4096 -> 8192 16.5 us before, now 9.2, 8192 -> 16000 47.2 / 30.1, 3072 -> 3000 5.1 / 4.0.
+  // C = 2 (int4, one row of x; where, launch_gemv_simt says): two octets a lane and load, so that as many bytes are on their way as with int8; even and
+  // odd k add up in the halves of 64-bit registers.  M = 1, f32, groups of 32, us in a CUDA graph, one octet as it was / now: 4096 -> 8192 23.1 / 10.8, 8192 ->
+  // 16000 46.6 / 29.7, 3072 -> 3000 5.1 / 3.5.
   // (int8 with two octets: 4096 -> 8192 10.7 -> 9.4, but 3072 -> 3000 4.5 -> 5.5; halves with two and four rows of x cost registers: M = 2,
   // 1024 -> 12000 5.4 -> 6.0, M = 8 33 -> 39.)
   static_assert(C == 1 || (C == 2 && MT == 1 && WBITS == 4), "two octets a lane: int4, one row of x");
@@ -295,14 +297,11 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
     const int g = gshift >= 0 ? (c << (2 + C)) >> gshift : (c << (2 + C)) / G;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      if (NW == 1) {
+      if constexpr (NW == 1) {
         next[r][0] = __ldg(reinterpret_cast<const uint32_t*>(wrow[r]) + c);
-      } else if (NW == 2) {
-        const uint2 v = __ldg(reinterpret_cast<const uint2*>(wrow[r]) + c);
-        next[r][0] = v.x; next[r][1 % NW] = v.y;
       } else {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(wrow[r]) + c);
-        next[r][0] = v.x; next[r][1 % NW] = v.y; next[r][2 % NW] = v.z; next[r][3 % NW] = v.w;
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(wrow[r]) + c);
+        next[r][0] = v.x; next[r][1] = v.y;
       }
       sc[r] = __ldg(srow[r] + g);
     }
@@ -312,7 +311,7 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const XT* __restrict__ x
   griddep_launch_dependents();
   griddep_wait();
   for (; c < nchunks; c += 32 << split_shift) {
-    if (PAIRS) {
+    if constexpr (PAIRS) {
       uint32_t now[R][NW];
       float s[R];
 #pragma unroll

@@ -19,7 +19,7 @@
 //
 // What bounds it.  In one call by itself at bm >= 192 the tensor cores (an MMA with its A operand in TMEM takes N / 2 clocks from
 // N = 32 on); below, the dequant warps' instructions and HBM, and what is left of the issue of the MMAs beside them (see
-// umma_stage).  The hand-over between the dequant warps, the MMA warp and back is a chain of barrier round trips -- hence whole 256-k
+// umma_steps).  The hand-over between the dequant warps, the MMA warp and back is a chain of barrier round trips -- hence whole 256-k
 // stages per barrier (with 64-k steps every step took ~750 clocks whatever bm), two sets of dequant warps that take the
 // stages in turn, and MMAs issued by an elected lane of a uniform warp.  Call after call, everything from M = 32 on large
 // weights upwards runs at the GPU's 1000 W: then a call takes as long as its energy lasts.
@@ -868,8 +868,11 @@ __global__ void __launch_bounds__(256) bf16_to_f16_perm_kernel(const uint4* __re
 // ---------------------------------------------------------------------------- host side
 struct Tiling { int cg, bm, n_tiles_n, n_tiles, teams, sk_tiles, full, tail, split, nd, nas, nxs, nws; };
 
-// Microseconds of a 64-k step of a tile, measured at K = 8192: with few teams at work the hand-over of the
-// weights through TMEM and the MMAs bound it; with all SMs busy (`used` = 1) L2 and power add to that.
+// Microseconds of a 64-k step of a tile, measured at K = 8192 when every MMA had an election of its own: with few teams at work the hand-over
+// of the weights through TMEM and the MMAs bound it; with all SMs busy (`used` = 1) L2 and power add to that.  Since the MMAs of a stage are
+// issued in one block, steps of up to 64 rows take less than this says (64 x 8192 -> 28672: 0.22 us by the formula, 0.19 by the call's 42 us; 32 rows 46 ->
+// 36 us a call), so low tiles, pieces and shares of K are priced too high against high tiles.  The constants have not been fitted again: forms are chosen as they
+// were, and calls have become faster in them.  Two terms per weight are taken to cost twice as much, which has not been measured by itself.
 inline double step_us(int cg, int bm, double used) {
   const double alone = 0.145 + 0.0005 * bm;
   const double busy = cg == 1 ? 0.145 + 0.00117 * bm : bm <= 128 ? 0.152 + 0.00088 * bm : 0.150 + 0.00100 * bm;
